@@ -130,6 +130,175 @@ TabLayout make_layout(const int* R, int d, int max_rows) {
   return T;
 }
 
+// Folded last-axis range of a run: columns c = |n| from fold_lo to fold_hi.
+int fold_lo(const GridRun& g) {
+  return (g.a <= 0 && g.b >= 0) ? 0 : std::min(std::abs(g.a), std::abs(g.b));
+}
+int fold_hi(const GridRun& g) { return std::max(std::abs(g.a), std::abs(g.b)); }
+
+void sort_by_fold(std::vector<GridRun>& runs) {
+  std::stable_sort(runs.begin(), runs.end(), [](const GridRun& x, const GridRun& y) {
+    return fold_hi(x) - fold_lo(x) > fold_hi(y) - fold_lo(y);
+  });
+}
+
+// What cco_problem_pass1_form reports: the (24-run x 16 cq-column) blocks of a
+// k-set of d >= 2 whose blocks hold at least half (d = 3: all) as many rows as
+// cells, cells counted per 6 runs; 0 for sparser ones and in 1-D.
+int folded_blocks(std::vector<GridRun> runs, int d, int m) {
+  if (d < 2 || runs.empty()) return 0;
+  sort_by_fold(runs);
+  double best = 0.0;
+  int blocks = 0;
+  for (int cols = 16; cols <= 48; cols += 16) {
+    double cells = 0.0;
+    int nb = 0;
+    for (size_t r0 = 0; r0 < runs.size(); r0 += 24) {
+      const int nrun = (int)std::min<size_t>(24, runs.size() - r0);
+      int lo = 1 << 30, hi = 0;
+      for (int r = 0; r < nrun; ++r) {
+        lo = std::min(lo, fold_lo(runs[r0 + r]));
+        hi = std::max(hi, fold_hi(runs[r0 + r]));
+      }
+      const int win = (hi - lo) / cols + 1;
+      cells += (double)((nrun + 5) / 6 * 6) * cols * win;
+      nb += win;
+    }
+    if (cols == 16 || cells <= best) {
+      best = cells;
+      blocks = nb;
+    }
+  }
+  return (double)m >= (d == 3 ? 1.0 : 0.5) * best ? blocks : 0;
+}
+
+// The grid of a k-set (cco_grid.cuh): runs, strips of 8, blocks, quads.
+struct GridPlan {
+  std::vector<GridRun> runs;
+  std::vector<GridStrip> strips;
+  std::vector<GridBlock> blocks;
+  std::vector<GridQuad> quads;
+  int entries = 0;   // widest block's table entries
+  int cols = 0;      // widest block's columns
+};
+
+void grid_layout(std::vector<GridRun> runs, int d, GridPlan* out) {
+  *out = GridPlan{};
+  sort_by_fold(runs);
+  out->runs = runs;
+  const int nr = (int)runs.size(), ns = (nr + 7) / 8;
+  const int nbr = (ns + kGridStrips - 1) / kGridStrips;   // block rows, of even height
+  for (int br = 0; br < nbr; ++br) {
+    const int s0 = (int)((long long)ns * br / nbr), s1 = (int)((long long)ns * (br + 1) / nbr);
+    int lo = 1 << 30, hi = 0;
+    for (int r = 8 * s0; r < std::min(nr, 8 * s1); ++r) {
+      lo = std::min(lo, fold_lo(runs[r]));
+      hi = std::max(hi, fold_hi(runs[r]));
+    }
+    const int range = hi - lo + 1, nw = (range + kGridCols - 1) / kGridCols;
+    const int width = ((range + nw - 1) / nw + 7) / 8 * 8;
+    for (int w = lo; w <= hi; w += width) {
+      GridBlock b{};
+      b.strip0 = (int)out->strips.size();
+      b.lo = w;
+      b.m0 = b.m1 = 1 << 30;
+      int M0 = -(1 << 30), M1 = -(1 << 30);
+      for (int s = s0; s < s1; ++s) {
+        GridStrip g{};
+        g.run0 = 8 * s;
+        g.nrun = std::min(8, nr - 8 * s);
+        int top = -1;
+        for (int r = g.run0; r < g.run0 + g.nrun; ++r)
+          if (fold_hi(runs[r]) >= w && fold_lo(runs[r]) < w + width)
+            top = std::max(top, std::min(fold_hi(runs[r]) - w, width - 1));
+        if (top < 0) continue;
+        g.nq = top / 4 + 1;
+        g.slot0 = 32 * (int)out->quads.size();
+        for (int q = 0; q < g.nq; ++q) out->quads.push_back(GridQuad{g.run0, g.nrun, w + 4 * q, 0});
+        out->strips.push_back(g);
+        b.nstrip += 1;
+        b.ncol = std::max(b.ncol, (g.nq + 1) / 2 * 8);
+        for (int r = g.run0; r < g.run0 + g.nrun; ++r) {
+          b.m0 = std::min(b.m0, runs[r].n0);
+          M0 = std::max(M0, runs[r].n0);
+          b.m1 = std::min(b.m1, runs[r].n1);
+          M1 = std::max(M1, runs[r].n1);
+        }
+      }
+      if (b.nstrip == 0) continue;
+      b.c0 = M0 - b.m0 + 1;
+      b.c1 = d == 3 ? M1 - b.m1 + 1 : 0;
+      if (d != 3) b.m1 = 0;
+      out->entries = std::max(out->entries, b.ncol + b.c0 + b.c1);
+      out->cols = std::max(out->cols, b.ncol);
+      out->blocks.push_back(b);
+    }
+  }
+}
+
+// Runs of a 1-D k-set on columns |c| <= C: n = q (2 C + 1) + c.
+std::vector<GridRun> split_runs_1d(const std::vector<GridRun>& runs, int C) {
+  const int S = 2 * C + 1;
+  auto fdiv = [](int x, int y) { return x >= 0 ? x / y : -((-x + y - 1) / y); };
+  std::vector<GridRun> out;
+  for (const GridRun& g : runs)
+    for (int q = fdiv(g.a + C, S); q <= fdiv(g.b + C, S); ++q) {
+      const int a = std::max(g.a, q * S - C), b = std::min(g.b, q * S + C);
+      out.push_back(GridRun{q, 0, a - q * S, b - q * S, g.kstart + a - g.a, 0});
+    }
+  return out;
+}
+
+// Whether and how FP64 lanes of a problem run the grid form. The form costs 12
+// FMAs per grid cell and particle (4 density, 8 gradient) plus the tables,
+// where the recurrences need 14 or more instructions per k-set row: it is taken
+// when the slots (cells with their padding) are at most twice the rows.
+void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
+  if (runs.empty()) return;
+  int step = 1;
+  if (P->d == 1) {
+    // the column count that costs least: cells and table entries per particle
+    double best = 0.0;
+    int best_c = -1;
+    for (int nc = 4; nc <= kGridCols; nc += 4) {
+      GridPlan g;
+      grid_layout(split_runs_1d(runs, nc - 1), 1, &g);
+      double cost = 0.0;
+      for (const GridBlock& b : g.blocks) cost += 16.0 * (b.ncol + b.c0);
+      cost += 8.0 * 32.0 * (double)g.quads.size();
+      if (g.entries <= kGridMaxEntries && (best_c < 0 || cost < best)) {
+        best = cost;
+        best_c = nc;
+      }
+    }
+    if (best_c < 0) return;
+    grid_layout(split_runs_1d(runs, best_c - 1), 1, gp);
+    step = 2 * (best_c - 1) + 1;
+  } else {
+    grid_layout(runs, P->d, gp);
+  }
+  const long long slots = 32ll * (long long)gp->quads.size();
+  if (gp->entries > kGridMaxEntries || slots > 2ll * P->M) return;
+  P->grid = 1;
+  P->ngblk = (int)gp->blocks.size();
+  P->gcls = gp->cols <= 24 ? 0 : 1;
+  P->gts = gp->entries | 1;
+  P->gstep = step;
+  P->gslots = (int)slots;
+  // larger pass-1 tiles for larger N keep the partials (32 bytes per slot and
+  // tile) and the reduction small once there are enough tiles to fill the GPU
+  P->gtile = P->N <= 2048 ? 64 : P->N <= 8192 ? 128 : 256;
+  P->gntile = (P->N + P->gtile - 1) / P->gtile;
+  P->grhow = (int)slots * (P->d == 1 ? 2 : 4) + (reduce_chunks((int)slots) + 1) / 2;
+}
+
+template <class T>
+cudaError_t to_device(T** dst, const std::vector<T>& src) {
+  const cudaError_t e = cudaMalloc(dst, std::max<size_t>(src.size(), 1) * sizeof(T));
+  if (e != cudaSuccess || src.empty()) return e;
+  return cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice);
+}
+
 // Absolute table rows of the digits of v on axis a (+ sign bit 24).
 int pack_rows(int v, const TabLayout& T, int a) {
   const int neg = v < 0;
@@ -243,7 +412,7 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
 
   // runs -> segments (headers carry each pass's absolute table rows)
   std::vector<SegHdr> s1, s2;
-  std::vector<GemmRun> runs;
+  std::vector<GridRun> runs;
   auto emit = [&](std::vector<SegHdr>& dst, const TabLayout& T, int kstart, int len, int maxlen) {
     for (int off = 0; off < len; off += maxlen) {
       SegHdr h{};
@@ -270,7 +439,7 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
       emit(s1, P.t1, start, k - start, kSeg1Len);
       emit(s2, P.t2, start, k - start, kSeg2Len);
       const int* nv = n_vectors + (size_t)order[start] * d;
-      GemmRun g{};
+      GridRun g{};
       g.n0 = d >= 2 ? nv[0] : 0;
       g.n1 = d >= 3 ? nv[1] : 0;
       g.a = nv[d - 1];
@@ -280,114 +449,11 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
       start = k;
     }
   }
-  // GEMM pass 1: runs grouped kGemmRows at a time by length, each group's
-  // last-axis range cut into column windows. Used when the blocks cost at
-  // most 8 FMAs per k-set row and particle (4 for d = 3): m >= cells / 2
-  // (m >= cells), cells counted with the warps' 6-row granularity (a folded
-  // cell serves two rows)
-  // (CCO_PASS1_GEMM=0 turns it off).
-  std::vector<GemmRun> grun;
-  std::vector<GemmBlock> gblk;
-  {
-    const char* env = getenv("CCO_PASS1_GEMM");
-    const bool allow = d >= 2 && !(env && atoi(env) == 0);
-    // The last axis is folded: columns are c = |n|, a run [a, b] covers
-    // [ca, cb] (its folded range), and one cell (run, c) yields C(c) and C(-c).
-    // Its window width is 16 cq columns (cq = 1..3), the width that computes
-    // the fewest cells for this k-set (the widest on ties: fewer blocks).
-    auto fa = [](const GemmRun& g) {
-      return (g.a <= 0 && g.b >= 0) ? 0 : std::min(std::abs(g.a), std::abs(g.b));
-    };
-    auto fb = [](const GemmRun& g) { return std::max(std::abs(g.a), std::abs(g.b)); };
-    std::vector<GemmRun> sorted = runs;
-    std::stable_sort(sorted.begin(), sorted.end(), [&](const GemmRun& x, const GemmRun& y) {
-      return (fb(x) - fa(x)) > (fb(y) - fa(y));
-    });
-    int c0 = 0, c1 = 0;      // widest group prefix windows
-    double computed = 0.0;   // grid cells the blocks multiply (4 FMAs per particle each)
-    auto group = [&](int cols) {
-      grun.clear();
-      gblk.clear();
-      c0 = c1 = 0;
-      computed = 0.0;
-      for (size_t r0 = 0; r0 < sorted.size(); r0 += kGemmRows) {
-        const int nrun = (int)std::min<size_t>(kGemmRows, sorted.size() - r0);
-        int lo = 1 << 30, hi = -(1 << 30);
-        int gm0 = 1 << 30, gM0 = -(1 << 30), gm1 = 1 << 30, gM1 = -(1 << 30);
-        for (int r = 0; r < nrun; ++r) {
-          const GemmRun& g = sorted[r0 + r];
-          lo = std::min(lo, fa(g));
-          hi = std::max(hi, fb(g));
-          gm0 = std::min(gm0, g.n0);
-          gM0 = std::max(gM0, g.n0);
-          gm1 = std::min(gm1, g.n1);
-          gM1 = std::max(gM1, g.n1);
-        }
-        // each group's prefix tables cover only its own prefixes
-        const int gc0 = gM0 - gm0 + 1, gc1 = d >= 3 ? gM1 - gm1 + 1 : 0;
-        c0 = std::max(c0, gc0);
-        c1 = std::max(c1, gc1);
-        const int run0 = (int)grun.size();
-        for (int r = 0; r < nrun; ++r) grun.push_back(sorted[r0 + r]);
-        // warps whose 6 rows lie past the group's runs skip their products
-        computed += (double)((nrun + 5) / 6 * 6) * cols * ((hi - lo) / cols + 1);
-        for (int w = lo; w <= hi; w += cols) {
-          GemmBlock b{};
-          b.run0 = run0;
-          b.nrun = nrun;
-          b.lo = w;
-          b.nb = std::min(cols, hi - w + 1);
-          b.m0 = gm0;
-          b.c0 = gc0;
-          b.m1 = d >= 3 ? gm1 : 0;
-          b.c1 = gc1;
-          gblk.push_back(b);
-        }
-      }
-    };
-    int best = 1;
-    double best_cells = 0.0;
-    for (int cq = 1; cq <= kGemmFoldMaxCq; ++cq) {
-      group(16 * cq);
-      if (cq == 1 || computed <= best_cells) {
-        best = cq;
-        best_cells = computed;
-      }
-    }
-    const int cols = 16 * best;
-    P.gcq = best;
-    group(cols);
-    const double cells = computed;
-    // d = 3 builds an A phase per chunk and only broke even with the
-    // per-segment kernel at about 3.5 FMAs per row (d=3 N=4000 chi=0.45: 1.480
-    // vs 1.481 ms per 32-lane evaluation; at 6.2 FMAs, N=2000 chi=0.20, it lost
-    // 4%), so 3-D k-sets take the GEMM form only at <= 4 FMAs per row
-    const double need = d == 3 ? 1.0 : 0.5;
-    P.gemm = allow && !runs.empty() && c0 <= kGemmMaxPrefix && c1 <= kGemmMaxPrefix &&
-             (double)m >= need * cells;
-    P.ngblk = (int)gblk.size();
-    P.gm0 = 0;
-    P.gc0 = c0;
-    P.gm1 = 0;
-    P.gc1 = c1;
-    P.gs0 = (c0 + 1) | 1;   // odd, with a spare column c0 (zeros in the d = 2 kernel)
-    P.gs1 = c1 > 0 ? (c1 | 1) : 0;
-    // fill units: the fewest rounds of one unit per thread, then the
-    // shortest chains (each unit seeds with sincospi, then multiplies)
-    const int per_round = kGemmThreads / kGemmChunk;
-    bool found = false;
-    for (int rounds = 1; !found; ++rounds)
-      for (int L = 8; L <= kGemmMaxRun && !found; ++L) {
-        const int u0 = (c0 + L - 1) / L, u1 = (c1 + L - 1) / L, uz = (cols + L - 1) / L;
-        if (u0 + u1 + uz <= per_round * rounds) {
-          P.gL = L;
-          P.gu0 = u0;
-          P.gu1 = u1;
-          P.guz = uz;
-          found = true;
-        }
-      }
-  }
+  GridPlan gp;
+  const char* env = getenv("CCO_PASS1_GEMM");   // 0: the per-segment form everywhere
+  const bool allow = !(env && atoi(env) == 0);
+  const int dense_blocks = allow ? folded_blocks(runs, d, m) : 0;
+  if (allow) plan_grid(runs, &P, &gp);
   // longest segments first: pass-1 warps share trip counts, pass 2 pairs
   // segments of similar length
   auto by_len = [](const SegHdr& x, const SegHdr& y) { return x.len > y.len; };
@@ -443,14 +509,16 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
   if (e == cudaSuccess) e = cudaMemcpy(pr->run2ref, r2r.data(), m * sizeof(int), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&pr->krow, m * sizeof(double4));
   if (e == cudaSuccess) e = cudaMemcpy(pr->krow, krow.data(), m * sizeof(double4), cudaMemcpyHostToDevice);
-  if (P.gemm) {
-    if (e == cudaSuccess) e = cudaMalloc(&pr->grun, grun.size() * sizeof(GemmRun));
-    if (e == cudaSuccess) e = cudaMalloc(&pr->gblk, gblk.size() * sizeof(GemmBlock));
-    if (e == cudaSuccess) e = cudaMemcpy(pr->grun, grun.data(), grun.size() * sizeof(GemmRun), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(pr->gblk, gblk.data(), gblk.size() * sizeof(GemmBlock), cudaMemcpyHostToDevice);
+  if (P.grid) {
+    if (e == cudaSuccess) e = to_device(&pr->grun, gp.runs);
+    if (e == cudaSuccess) e = to_device(&pr->gblk, gp.blocks);
+    if (e == cudaSuccess) e = to_device(&pr->gstrip, gp.strips);
+    if (e == cudaSuccess) e = to_device(&pr->gquad, gp.quads);
   }
   P.grun = pr->grun;
   P.gblk = pr->gblk;
+  P.gstrip = pr->gstrip;
+  P.gquad = pr->gquad;
   P.seg1 = pr->seg1;
   P.seg2 = pr->seg2;
   P.w_run = pr->w_run;
@@ -460,6 +528,8 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
   pr->smem1 = smem1;
   pr->smem2 = smem2;
   pr->smemG = eval_smemG(P);
+  pr->smemH = eval_smemH(P);
+  pr->dense_blocks = dense_blocks;
   if (e != cudaSuccess) {
     cco_problem_destroy(pr);
     return cuda_fail(e, "cco_problem_create upload");
@@ -477,6 +547,8 @@ int cco_problem_destroy(cco_problem* p) {
   cudaFree(p->run2ref);
   if (p->grun) cudaFree(p->grun);
   if (p->gblk) cudaFree(p->gblk);
+  if (p->gstrip) cudaFree(p->gstrip);
+  if (p->gquad) cudaFree(p->gquad);
   if (p->krow) cudaFree(p->krow);
   cudaFree(p->dev);
   delete p;
@@ -497,7 +569,7 @@ int cco_problem_info(const cco_problem* p, int* d, int* n_particles, int* m, int
 
 int cco_problem_pass1_form(const cco_problem* p, int* gemm_blocks) {
   if (!p || !gemm_blocks) return fail(CCO_ERR_ARG, "null argument");
-  *gemm_blocks = p->host.gemm ? p->host.ngblk : 0;
+  *gemm_blocks = p->dense_blocks;
   return CCO_OK;
 }
 
@@ -506,12 +578,11 @@ int cco_problem_pass1_form(const cco_problem* p, int* gemm_blocks) {
 // ------------------------------------------------------------ eval workspace
 namespace {
 
-__global__ void k_make_lanes(EvalLane* lanes, EvalItem* it1, EvalItem* it2, EvalItem* itG,
-                             int B, int nt1, int nt2, int ntG, int total, const double* s,
-                             size_t s_stride, double* f,
+__global__ void k_make_lanes(EvalLane* lanes, EvalItem* it1, EvalItem* it2, int B, int nt1,
+                             int nt2, int total, const double* s, size_t s_stride, double* f,
                              size_t f_stride, double* g, size_t g_stride, double2* rho,
-                             double2* rhow, double2* part, int M, const int64_t* status,
-                             size_t status_stride, int prec) {
+                             double2* rhow, double2* part, int M, size_t rhow_stride,
+                             size_t part_stride, int prec) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     if (i < B) {
       EvalLane L;
@@ -519,9 +590,9 @@ __global__ void k_make_lanes(EvalLane* lanes, EvalItem* it1, EvalItem* it2, Eval
       L.f = f + (size_t)i * f_stride;
       L.g = g ? g + (size_t)i * g_stride : nullptr;
       L.rho = rho + (size_t)i * M;
-      L.rhow = rhow + (size_t)i * M;
-      L.part = part + (size_t)i * nt1 * M;
-      L.status = status ? status + (size_t)i * status_stride : nullptr;
+      L.rhow = rhow + (size_t)i * rhow_stride;
+      L.part = part + (size_t)i * part_stride;
+      L.status = nullptr;
       L.prec = nullptr;
       L.fixed_prec = prec;
       L.prob = 0;
@@ -531,83 +602,85 @@ __global__ void k_make_lanes(EvalLane* lanes, EvalItem* it1, EvalItem* it2, Eval
     if (j >= 0) {
       if (j < B * nt1) it1[j] = EvalItem{j / nt1, j % nt1};
       if (j < B * nt2) it2[j] = EvalItem{j / nt2, j % nt2};
-      if (itG && j < B * ntG) itG[j] = EvalItem{j / ntG, j % ntG};
     }
   }
 }
 
 // Device buffers of one batched evaluation: densities, partials and the plan.
+// One problem and one arithmetic, so every lane takes the same form: it1 and
+// it2 hold the items of that form's two passes.
 struct EvalWS {
   EvalLane* lanes = nullptr;
   EvalItem* it1 = nullptr;
   EvalItem* it2 = nullptr;
-  EvalItem* itG = nullptr;   // GEMM pass-1 items (problems with p->host.gemm)
   double2* rho = nullptr;
   double2* rhow = nullptr;
   double2* part = nullptr;
   EvalPlan plan{};
   int prec = PREC_FP64;   // arithmetic of every lane of this workspace
 
-  static int gemm_tiles(const cco_problem* p) {
-    return p->host.gemm ? p->host.ntile1 * p->host.ngblk : 0;
-  }
-
-  // pass-2 threads per particle and tiles per configuration for a batch of B
-  static int split_for(const cco_problem* p, int B) {
-    return pass2_split((long long)B * p->host.ntile2);
+  // Element counts of a batch of B (b_*: of the whole batch).
+  struct Sizes {
+    bool grid;
+    int split, nt1, nt2;
+    size_t rhow, part;   // double2 words per lane
+  };
+  static Sizes sizes(const cco_problem* p, int B, int prec) {
+    Sizes z;
+    const ProbDev& h = p->host;
+    z.grid = h.grid && prec == PREC_FP64;
+    z.split = pass2_split((long long)B * h.ntile2);
+    z.nt1 = z.grid ? h.gntile * h.ngblk : h.ntile1;
+    z.nt2 = z.grid ? (h.N + kGridTile2 - 1) / kGridTile2 : pass2_tiles(h, z.split);
+    z.rhow = z.grid ? (size_t)h.grhow : (size_t)h.M;
+    z.part = z.grid ? 2 * (size_t)h.gntile * h.gslots : (size_t)h.ntile1 * h.M;
+    return z;
   }
   cudaError_t alloc(const cco_problem* p, int B, cudaStream_t st) {
-    const int M = p->M, nt1 = p->host.ntile1, nt2 = pass2_tiles(p->host, split_for(p, B));
+    const Sizes z = sizes(p, B, prec);
     cudaError_t e = pool_alloc(&lanes, sizeof(EvalLane) * B, st);
-    if (e == cudaSuccess) e = pool_alloc(&it1, sizeof(EvalItem) * (size_t)B * nt1, st);
-    if (e == cudaSuccess) e = pool_alloc(&it2, sizeof(EvalItem) * (size_t)B * nt2, st);
-    if (e == cudaSuccess && gemm_tiles(p) > 0)
-      e = pool_alloc(&itG, sizeof(EvalItem) * (size_t)B * gemm_tiles(p), st);
-    if (e == cudaSuccess) e = pool_alloc(&rho, sizeof(double2) * (size_t)B * M, st);
-    if (e == cudaSuccess) e = pool_alloc(&rhow, sizeof(double2) * (size_t)B * M, st);
-    if (e == cudaSuccess) e = pool_alloc(&part, sizeof(double2) * (size_t)B * nt1 * M, st);
+    if (e == cudaSuccess) e = pool_alloc(&it1, sizeof(EvalItem) * (size_t)B * z.nt1, st);
+    if (e == cudaSuccess) e = pool_alloc(&it2, sizeof(EvalItem) * (size_t)B * z.nt2, st);
+    if (e == cudaSuccess) e = pool_alloc(&rho, sizeof(double2) * (size_t)B * p->M, st);
+    if (e == cudaSuccess) e = pool_alloc(&rhow, sizeof(double2) * (size_t)B * z.rhow, st);
+    if (e == cudaSuccess) e = pool_alloc(&part, sizeof(double2) * (size_t)B * z.part, st);
     return e;
   }
   cudaError_t build(const cco_problem* p, int B, const double* s, size_t s_stride, double* f,
-                    size_t f_stride, double* g, size_t g_stride, const int64_t* status,
-                    size_t status_stride, cudaStream_t st) {
-    const int split = split_for(p, B);
-    const int nt1 = p->host.ntile1, nt2 = pass2_tiles(p->host, split);
-    const int ntG = itG ? gemm_tiles(p) : 0;
-    const int total = B * std::max(std::max(nt1, nt2), ntG) + B;
+                    size_t f_stride, double* g, size_t g_stride, cudaStream_t st) {
+    const Sizes z = sizes(p, B, prec);
+    const int total = B * std::max(z.nt1, z.nt2) + B;
     const int blocks = std::min(1024, (total + 255) / 256);
-    k_make_lanes<<<blocks, 256, 0, st>>>(lanes, it1, it2, itG, B, nt1, nt2, ntG, total, s,
-                                         s_stride, f, f_stride, g, g_stride, rho, rhow, part,
-                                         p->M, status, status_stride, prec);
+    k_make_lanes<<<blocks, 256, 0, st>>>(lanes, it1, it2, B, z.nt1, z.nt2, total, s, s_stride, f,
+                                         f_stride, g, g_stride, rho, rhow, part, p->M, z.rhow,
+                                         z.part, prec);
     plan.probs = p->dev;
     plan.lanes = lanes;
-    plan.items1 = it1;
-    plan.items2 = it2;
-    plan.itemsG = itG;
+    plan.items1 = plan.itemsG = it1;
+    plan.items2 = plan.itemsH = it2;
     plan.n_lanes = B;
-    // the per-segment pass 1 covers FP32 lanes, and FP64 lanes of problems
-    // without the GEMM form
-    plan.n_items1 = (ntG > 0 && prec == PREC_FP64) ? 0 : B * nt1;
-    plan.n_items2 = B * nt2;
-    plan.n_itemsG = (prec == PREC_FP64) ? B * ntG : 0;
+    plan.n_items1 = z.grid ? 0 : B * z.nt1;
+    plan.n_items2 = z.grid ? 0 : B * z.nt2;
+    const int nG = z.grid ? B * z.nt1 : 0, nH = z.grid ? B * z.nt2 : 0;
     for (int D = 0; D <= 3; ++D) {
       plan.d_off1[D] = D >= p->d ? plan.n_items1 : 0;
       plan.d_off2[D] = D >= p->d ? plan.n_items2 : 0;
-      plan.d_offG[D] = D >= p->d ? plan.n_itemsG : 0;
+      plan.d_offH[D] = D >= p->d ? nH : 0;
     }
-    // one problem: its GEMM items are all of its window width
-    for (int D = 2; D <= 3; ++D)
-      for (int c = 0; c <= kGemmFoldMaxCq; ++c)
-        plan.q_offG[D - 2][c] = (D == p->d && c >= p->host.gcq) ? plan.n_itemsG : 0;
+    // one problem: its items are all of its column class
+    for (int D = 1; D <= 3; ++D)
+      for (int c = 0; c <= kGridClasses; ++c)
+        plan.q_offG[D - 1][c] = (D == p->d && c > p->host.gcls) ? nG : 0;
     plan.smemG = p->smemG;
+    plan.smemH = p->smemH;
     plan.dyn_prec = prec == PREC_FP32 ? 1 : 0;
     plan.max_d = p->d;
     plan.smem1 = p->smem1;
-    plan.smem2 = eval_smem2(p->host, split);
-    plan.smem2_f32 = eval_smem2(p->host, split, true);
-    plan.split2 = split;
+    plan.smem2 = eval_smem2(p->host, z.split);
+    plan.smem2_f32 = eval_smem2(p->host, z.split, true);
+    plan.split2 = z.split;
     plan.chunks1 = 1;
-    plan.red_chunks = reduce_chunks(p->M);
+    plan.red_chunks = reduce_chunks(z.grid ? p->host.gslots : p->M);
     plan.want_grad = g != nullptr;
     return cudaGetLastError();
   }
@@ -615,12 +688,10 @@ struct EvalWS {
     cudaFreeAsync(lanes, st);
     cudaFreeAsync(it1, st);
     cudaFreeAsync(it2, st);
-    if (itG) cudaFreeAsync(itG, st);
     cudaFreeAsync(rho, st);
     cudaFreeAsync(rhow, st);
     cudaFreeAsync(part, st);
     lanes = nullptr;
-    itG = nullptr;
   }
 };
 
@@ -637,7 +708,7 @@ extern "C" int cco_energy_grad(cco_problem* p, void* stream, int batch, const do
   EvalWS ws;
   CCO_CUDA(ws.alloc(p, batch, st));
   const size_t nd = (size_t)p->N * p->d;
-  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, grad, nd, nullptr, 0, st));
+  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, grad, nd, st));
   CCO_CUDA(eval_launch(ws.plan, st));
   if (rho_re || rho_im)
     CCO_CUDA(rho_scatter(ws.rho, p->run2ref, p->M, batch, p->M, rho_re, rho_im, st));
@@ -658,7 +729,7 @@ extern "C" int cco_energy_grad_fp32(cco_problem* p, void* stream, int batch, con
   ws.prec = PREC_FP32;
   CCO_CUDA(ws.alloc(p, batch, st));
   const size_t nd = (size_t)p->N * p->d;
-  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, grad, nd, nullptr, 0, st));
+  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, grad, nd, st));
   CCO_CUDA(eval_launch(ws.plan, st));
   ws.release(st);
   CCO_CUDA(cudaGetLastError());
@@ -679,7 +750,7 @@ extern "C" int cco_hessian(cco_problem* p, void* stream, int batch, const double
   CCO_CUDA(ws.alloc(p, batch, st));
   CCO_CUDA(pool_alloc(&phi, sizeof(double) * batch, st));
   const size_t nd = (size_t)p->N * p->d;
-  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, nullptr, 0, nullptr, 0, st));
+  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, nullptr, 0, st));
   CCO_CUDA(eval_launch(ws.plan, st));   // the density the diagonal blocks need
   CCO_CUDA(hessian_launch(p, st, batch, s, ws.rho, hess));
   ws.release(st);
@@ -727,37 +798,63 @@ extern "C" int cco_energy_grad_noalloc(cco_problem* p, void* stream, int batch, 
   if (batch < 0) return fail(CCO_ERR_ARG, "batch must be >= 0");
   if (batch == 0) return CCO_OK;
   if (!s || !phi) return fail(CCO_ERR_ARG, "null s or phi");
-  const size_t B = (size_t)batch, M = (size_t)p->M;
-  const size_t nt1 = (size_t)p->host.ntile1;
-  const size_t nt2 = (size_t)pass2_tiles(p->host, EvalWS::split_for(p, batch));
-  const size_t b_lanes = round256(sizeof(EvalLane) * B);
-  const size_t b_it1 = round256(sizeof(EvalItem) * B * nt1);
-  const size_t b_it2 = round256(sizeof(EvalItem) * B * nt2);
-  const size_t b_itG = round256(sizeof(EvalItem) * B * (size_t)EvalWS::gemm_tiles(p));
-  const size_t b_rho = round256(sizeof(double2) * B * M);
-  const size_t b_part = round256(sizeof(double2) * B * nt1 * M);
-  const size_t need = b_lanes + b_it1 + b_it2 + 2 * b_rho + b_part + b_itG;
-  if (need > CCO_NOALLOC_SCRATCH_BYTES)
-    return fail(CCO_ERR_ARG,
-                "batch %d needs %zu bytes of fixed scratch, the limit is %zu: split the batch",
-                batch, need, (size_t)CCO_NOALLOC_SCRATCH_BYTES);
+  // The scratch a call may ask for: rho, w rho and the per-segment partials of
+  // the batch plus its items. The grid form's layout of the same data can be
+  // larger (padded cells), so such a batch runs in parts that fit; its lanes
+  // do not depend on one another.
+  const size_t M = (size_t)p->M;
+  {
+    const size_t B = (size_t)batch, nt1 = (size_t)p->host.ntile1;
+    const size_t nt2 = (size_t)pass2_tiles(p->host, pass2_split((long long)batch * p->host.ntile2));
+    const size_t gemm = (size_t)p->dense_blocks * nt1;
+    const size_t need = round256(sizeof(EvalLane) * B) + round256(sizeof(EvalItem) * B * nt1) +
+                        round256(sizeof(EvalItem) * B * nt2) + 2 * round256(sizeof(double2) * B * M) +
+                        round256(sizeof(double2) * B * nt1 * M) + round256(sizeof(EvalItem) * B * gemm);
+    if (need > CCO_NOALLOC_SCRATCH_BYTES)
+      return fail(CCO_ERR_ARG,
+                  "batch %d needs %zu bytes of fixed scratch, the limit is %zu: split the batch",
+                  batch, need, (size_t)CCO_NOALLOC_SCRATCH_BYTES);
+  }
   DeviceGuard guard(p->device);
   unsigned char* base = nullptr;
   const int rc = noalloc_scratch(p->device, &base);
   if (rc != CCO_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  EvalWS ws;  // carved from the fixed scratch; never released
-  ws.lanes = reinterpret_cast<EvalLane*>(base);
-  ws.it1 = reinterpret_cast<EvalItem*>(base + b_lanes);
-  ws.it2 = reinterpret_cast<EvalItem*>(base + b_lanes + b_it1);
-  ws.rho = reinterpret_cast<double2*>(base + b_lanes + b_it1 + b_it2);
-  ws.rhow = reinterpret_cast<double2*>(base + b_lanes + b_it1 + b_it2 + b_rho);
-  ws.part = reinterpret_cast<double2*>(base + b_lanes + b_it1 + b_it2 + 2 * b_rho);
-  ws.itG = b_itG > 0 ? reinterpret_cast<EvalItem*>(base + b_lanes + b_it1 + b_it2 + 2 * b_rho + b_part)
-                     : nullptr;
   const size_t nd = (size_t)p->N * p->d;
-  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, grad, nd, nullptr, 0, st));
-  CCO_CUDA(eval_launch(ws.plan, st));
+  struct Carve {
+    size_t lanes, it1, it2, rho, rhow, total;
+  };
+  auto carve = [&](int b, int prec_form) {
+    const EvalWS::Sizes z = EvalWS::sizes(p, b, prec_form);
+    Carve c;
+    c.lanes = 0;
+    c.it1 = round256(sizeof(EvalLane) * b);
+    c.it2 = c.it1 + round256(sizeof(EvalItem) * (size_t)b * z.nt1);
+    c.rho = c.it2 + round256(sizeof(EvalItem) * (size_t)b * z.nt2);
+    c.rhow = c.rho + round256(sizeof(double2) * (size_t)b * M);
+    const size_t part = c.rhow + round256(sizeof(double2) * (size_t)b * z.rhow);
+    c.total = part + round256(sizeof(double2) * (size_t)b * z.part);
+    return std::make_pair(c, part);
+  };
+  int part_b = batch;
+  while (part_b > 1 && carve(part_b, PREC_FP64).first.total > CCO_NOALLOC_SCRATCH_BYTES)
+    part_b = (part_b + 1) / 2;
+  const auto [c, part] = carve(part_b, PREC_FP64);
+  if (c.total > CCO_NOALLOC_SCRATCH_BYTES)
+    return fail(CCO_ERR_ARG, "one configuration needs %zu bytes of fixed scratch, the limit is %zu",
+                c.total, (size_t)CCO_NOALLOC_SCRATCH_BYTES);
+  for (int lo = 0; lo < batch; lo += part_b) {
+    const int b = std::min(part_b, batch - lo);
+    EvalWS ws;  // carved from the fixed scratch; never released
+    ws.lanes = reinterpret_cast<EvalLane*>(base + c.lanes);
+    ws.it1 = reinterpret_cast<EvalItem*>(base + c.it1);
+    ws.it2 = reinterpret_cast<EvalItem*>(base + c.it2);
+    ws.rho = reinterpret_cast<double2*>(base + c.rho);
+    ws.rhow = reinterpret_cast<double2*>(base + c.rhow);
+    ws.part = reinterpret_cast<double2*>(base + part);
+    CCO_CUDA(ws.build(p, b, s + (size_t)lo * nd, nd, phi + lo, 1,
+                      grad ? grad + (size_t)lo * nd : nullptr, nd, st));
+    CCO_CUDA(eval_launch(ws.plan, st));
+  }
   return CCO_OK;
 }
-

@@ -17,6 +17,10 @@
 // trig error. No theta matrix ever reaches HBM: traffic per evaluation is s
 // in, g out and the M-row density, so both passes are FP64-pipe bound.
 //
+// Dense k-sets run both FP64 passes on the matrix pipe instead (k_grid1 and
+// k_grid2, cco_grid.cuh); the recurrences below serve sparse k-sets (more than
+// two grid slots per row) and FP32 lanes.
+//
 //   pass 1 (k_pass1): CTA = (configuration, 64-particle tile), 128 threads.
 //     A thread owns a segment of <= 8 rows and streams the tile's particles
 //     four at a time (four independent phase chains), accumulating 8 complex
@@ -35,49 +39,33 @@
 #include <cstdlib>
 
 #include "cco_eval_bodies.cuh"
+#include "cco_grid.cuh"
 #include "cco_internal.cuh"
 
 namespace cco {
 
 namespace {
 
-// One kernel per (dimension, window width): each holds one body, so the
-// instruction cache serves one folded product loop.
-template <int D, int CQ>
-__global__ void __launch_bounds__(kGemmThreads, 4) k_pass1_gemm(EvalPlan plan) {
+// Grid form (cco_grid.cuh), pass 1: one kernel per (dimension, column class),
+// each holding the accumulators of NT = 3 or 6 column tiles.
+template <int D, int NT>
+__global__ void __launch_bounds__(kGridThreads, NT == 3 ? 4 : 3) k_grid1(EvalPlan plan) {
   extern __shared__ double2 smem[];
   __shared__ ProbDev sp;
-  const EvalItem it = plan.itemsG[plan.q_offG[D - 2][CQ - 1] + blockIdx.x];
+  const EvalItem it = plan.itemsG[plan.q_offG[D - 1][NT == 3 ? 0 : 1] + blockIdx.x];
   const EvalLane ln = plan.lanes[it.lane];
   if (!lane_active(ln.status)) return;
   if (plan.dyn_prec && lane_prec(ln) == PREC_FP32) return;   // the FP32 body handles it
   if (threadIdx.x == 0) sp = plan.probs[ln.prob];
   __syncthreads();
-  if constexpr (D == 2)
-    pass1_gemm_body_d2<CQ>(sp, ln, it.tile / sp.ngblk, it.tile % sp.ngblk, smem);
-  else
-    pass1_gemm_body<D, CQ>(sp, ln, it.tile / sp.ngblk, it.tile % sp.ngblk, smem);
+  grid_pass1_body<D, NT>(sp, ln, it.tile / sp.ngblk, it.tile % sp.ngblk, blockIdx.x, smem);
 }
 
 template <int D>
-void launch_gemm(const EvalPlan& plan, cudaStream_t s) {
-  const int* q = plan.q_offG[D - 2];
-  if (q[1] > q[0]) k_pass1_gemm<D, 1><<<q[1] - q[0], kGemmThreads, plan.smemG, s>>>(plan);
-  if (q[2] > q[1]) k_pass1_gemm<D, 2><<<q[2] - q[1], kGemmThreads, plan.smemG, s>>>(plan);
-  if (q[3] > q[2]) k_pass1_gemm<D, 3><<<q[3] - q[2], kGemmThreads, plan.smemG, s>>>(plan);
-}
-
-template <int D>
-cudaError_t configure_gemm() {
-  cudaError_t e = cudaFuncSetAttribute(k_pass1_gemm<D, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       227 * 1024 - 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_pass1_gemm<D, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             227 * 1024 - 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_pass1_gemm<D, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             227 * 1024 - 1024);
-  return e;
+void launch_grid1(const EvalPlan& plan, cudaStream_t s) {
+  const int* q = plan.q_offG[D - 1];
+  if (q[1] > q[0]) k_grid1<D, 3><<<q[1] - q[0], kGridThreads, plan.smemG, s>>>(plan);
+  if (q[2] > q[1]) k_grid1<D, 6><<<q[2] - q[1], kGridThreads, plan.smemG, s>>>(plan);
 }
 
 // One kernel per dimension D and arithmetic keeps each kernel's code small:
@@ -97,13 +85,18 @@ __global__ void __launch_bounds__(kPass1Threads, 4) k_pass1(EvalPlan plan) {
   __syncthreads();
   if (F32) {
     pass1_body_f32<D>(sp, ln, it.tile, smem);
-  } else if (!sp.gemm) {   // GEMM problems: k_pass1_gemm
+  } else if (!sp.grid) {   // grid problems: k_grid1
     const int C = pass1_chunks(sp, plan.chunks1);
     pass1_body<D>(sp, ln, it.tile / C, smem, it.tile % C, C);
   }
 }
 
-// Reduction (grid: k-chunks x lanes): rho_k = sum over tiles of the pass-1
+// Chunk energies of a grid-form lane: after the pass-2 weights.
+__device__ __forceinline__ double* grid_energies(const ProbDev& P, const EvalLane& ln) {
+  return reinterpret_cast<double*>(ln.rhow + (size_t)P.gslots * (P.d == 1 ? 2 : 4));
+}
+
+// Reduction (grid: chunks x lanes): rho_k = sum over tiles of the pass-1
 // partials in tile order, the weighted density for pass 2, and this chunk's
 // part of sum w |rho|^2, stored over the chunk's first partial (which only
 // this block reads).
@@ -112,6 +105,18 @@ __global__ void __launch_bounds__(kReduceChunk) k_reduce(EvalPlan plan) {
   const EvalLane ln = plan.lanes[blockIdx.y];
   if (!lane_active(ln.status)) return;
   const ProbDev& P = plan.probs[ln.prob];
+  if (P.grid && lane_prec(ln) == PREC_FP64) {
+    if ((int)(blockIdx.x * kReduceChunk) >= P.gslots) return;
+    const int slot = blockIdx.x * kReduceChunk + threadIdx.x;
+    double e = 0.0;
+    if (slot < P.gslots) {
+      if (P.d == 1) e = grid_reduce_slot<true>(P, ln, slot);
+      else e = grid_reduce_slot<false>(P, ln, slot);
+    }
+    e = block_sum(e, red);
+    if (threadIdx.x == 0) grid_energies(P, ln)[blockIdx.x] = e;
+    return;
+  }
   const int M = P.M, nt = P.ntile1;
   const int k0 = blockIdx.x * kReduceChunk;
   if (k0 >= M) return;
@@ -153,9 +158,15 @@ __global__ void __launch_bounds__(kReduceChunk) k_reduce(EvalPlan plan) {
 // Energy of one lane (one warp): the chunk energies summed in a fixed order.
 __device__ __forceinline__ void lane_energy(const EvalPlan& plan, const EvalLane& ln) {
   const ProbDev& P = plan.probs[ln.prob];
-  const int nc = reduce_chunks(P.M);
   double e = 0.0;
-  for (int c = threadIdx.x; c < nc; c += 32) e += ln.part[(size_t)c * kReduceChunk].x;
+  if (P.grid && lane_prec(ln) == PREC_FP64) {
+    const double* ec = grid_energies(P, ln);
+    const int nc = reduce_chunks(P.gslots);
+    for (int c = threadIdx.x; c < nc; c += 32) e += ec[c];
+  } else {
+    const int nc = reduce_chunks(P.M);
+    for (int c = threadIdx.x; c < nc; c += 32) e += ln.part[(size_t)c * kReduceChunk].x;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
   if (threadIdx.x == 0) *ln.f = e / P.vol;
@@ -170,6 +181,22 @@ __global__ void k_energy(EvalPlan plan) {
   lane_energy(plan, ln);
 }
 
+// Grid form, pass 2.
+template <int D>
+__global__ void __launch_bounds__(kGridThreads, 4) k_grid2(EvalPlan plan) {
+  extern __shared__ double2 smem[];
+  __shared__ ProbDev sp;
+  const EvalItem it = plan.itemsH[plan.d_offH[D - 1] + blockIdx.x];
+  const EvalLane ln = plan.lanes[it.lane];
+  if (!lane_active(ln.status)) return;
+  if (plan.dyn_prec && lane_prec(ln) == PREC_FP32) return;   // the FP32 body handles it
+  if (it.tile == 0 && threadIdx.x < 32) lane_energy(plan, ln);
+  if (ln.g == nullptr) return;
+  if (threadIdx.x == 0) sp = plan.probs[ln.prob];
+  __syncthreads();
+  grid_pass2_body<D>(sp, ln, it.tile, smem);
+}
+
 template <int D, bool F32>
 __global__ void __launch_bounds__(kPass2Threads, 4) k_pass2(EvalPlan plan) {
   extern __shared__ double2 smem[];
@@ -178,6 +205,7 @@ __global__ void __launch_bounds__(kPass2Threads, 4) k_pass2(EvalPlan plan) {
   const EvalLane ln = plan.lanes[it.lane];
   if (!lane_active(ln.status)) return;
   if ((lane_prec(ln) == PREC_FP32) != F32) return;   // the other kernel's lane
+  if (!F32 && plan.probs[ln.prob].grid) return;      // grid problems: k_grid2
   if (it.tile == 0 && threadIdx.x < 32) lane_energy(plan, ln);
   if (ln.g == nullptr) return;
   if (threadIdx.x == 0) sp = plan.probs[ln.prob];
@@ -231,13 +259,11 @@ size_t eval_smem1(const ProbDev& p) {
 }
 
 size_t eval_smemG(const ProbDev& p) {
-  if (!p.gemm) return 0;
-  if (p.d == 2)   // two table sets (prefix, last axis) and two root sets
-    return (size_t)kGemmChunk * (2 * (p.gs0 + gemm_fold_zstride(p.gcq)) + 2 * p.d) *
-           sizeof(double2);
-  const int s1 = p.d == 3 ? p.gs1 : 0;
-  return (size_t)kGemmChunk * (p.gs0 + s1 + gemm_fold_zstride(p.gcq) + kGemmRows + 2 * p.d) *
-         sizeof(double2);
+  return p.grid ? (size_t)kGridChunk * p.gts * sizeof(double2) : 0;
+}
+
+size_t eval_smemH(const ProbDev& p) {
+  return p.grid ? (size_t)kGridTile2 * p.gts * sizeof(double2) : 0;
 }
 
 size_t eval_smem2(const ProbDev& p, int split, bool f32) {
@@ -278,6 +304,24 @@ cudaError_t configure_d() {
                               227 * 1024 - 1024);
 }
 
+template <int D>
+cudaError_t configure_grid() {
+  constexpr int most = 227 * 1024 - 1024;
+  cudaError_t e =
+      cudaFuncSetAttribute(k_grid1<D, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_grid1<D, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_grid2<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  return e;
+}
+
+template <int D>
+void launch_grid2(const EvalPlan& plan, cudaStream_t s) {
+  const int n = plan.d_offH[D] - plan.d_offH[D - 1];
+  if (n > 0) k_grid2<D><<<n, kGridThreads, plan.smemH, s>>>(plan);
+}
+
 template <int D, bool F32>
 void launch_d(const EvalPlan& plan, bool pass2, cudaStream_t stream) {
   if (!pass2) {
@@ -292,8 +336,9 @@ void launch_d(const EvalPlan& plan, bool pass2, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t eval_configure() {
-  cudaError_t e = configure_gemm<2>();
-  if (e == cudaSuccess) e = configure_gemm<3>();
+  cudaError_t e = configure_grid<1>();
+  if (e == cudaSuccess) e = configure_grid<2>();
+  if (e == cudaSuccess) e = configure_grid<3>();
   if (e == cudaSuccess) e = configure_d<1, false>();
   if (e == cudaSuccess) e = configure_d<2, false>();
   if (e == cudaSuccess) e = configure_d<3, false>();
@@ -305,22 +350,20 @@ cudaError_t eval_configure() {
 
 namespace {
 
-// The pass kernels of dimension D on stream s (pass 1: per-segment and GEMM forms).
+// The pass kernels of dimension D on stream s (per-segment and grid forms).
 // FP64 lanes run the F32 = false kernels whatever the plan; a plan that may
 // hold FP32 lanes (dyn_prec) launches the F32 = true kernels as well.
+template <int D>
+void launch_dim_d(const EvalPlan& plan, bool pass2, cudaStream_t s) {
+  launch_d<D, false>(plan, pass2, s);
+  if (plan.dyn_prec) launch_d<D, true>(plan, pass2, s);
+  if (pass2) launch_grid2<D>(plan, s);
+  else launch_grid1<D>(plan, s);
+}
 void launch_dim(const EvalPlan& plan, bool pass2, int D, cudaStream_t s) {
-  if (D == 1) {
-    launch_d<1, false>(plan, pass2, s);
-    if (plan.dyn_prec) launch_d<1, true>(plan, pass2, s);
-  } else if (D == 2) {
-    launch_d<2, false>(plan, pass2, s);
-    if (plan.dyn_prec) launch_d<2, true>(plan, pass2, s);
-    if (!pass2) launch_gemm<2>(plan, s);
-  } else {
-    launch_d<3, false>(plan, pass2, s);
-    if (plan.dyn_prec) launch_d<3, true>(plan, pass2, s);
-    if (!pass2) launch_gemm<3>(plan, s);
-  }
+  if (D == 1) launch_dim_d<1>(plan, pass2, s);
+  else if (D == 2) launch_dim_d<2>(plan, pass2, s);
+  else launch_dim_d<3>(plan, pass2, s);
 }
 
 // One pass over every dimension present: in order on `stream`, or, with side
@@ -331,8 +374,7 @@ cudaError_t launch_pass_all(const EvalPlan& plan, bool pass2, cudaStream_t strea
   bool has[4] = {false, false, false, false};
   int nd = 0;
   for (int D = 1; D <= 3; ++D) {
-    has[D] = pass2 ? plan.d_off2[D] > plan.d_off2[D - 1]
-                   : (plan.d_off1[D] > plan.d_off1[D - 1] || plan.d_offG[D] > plan.d_offG[D - 1]);
+    has[D] = eval_has_dim(plan, D);
     nd += has[D];
   }
   if (!side || nd < 2) {

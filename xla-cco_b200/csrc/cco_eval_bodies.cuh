@@ -1,5 +1,6 @@
-// Device bodies of the evaluation: phase tables, the pass-1 density (per
-// segment and GEMM forms, FP64 and FP32) and the pass-2 gradient. Included
+// Device bodies of the evaluation by phase recurrences: phase tables, the
+// pass-1 density per segment and the pass-2 gradient, in FP64 and FP32 (the
+// tensor-core form of dense k-sets is in cco_grid.cuh). Included
 // by cco_eval.cu (the launched kernels) and cco_persist.cu (the persistent
 // small-lane kernel); each file compiles its own copy.
 #pragma once
@@ -684,256 +685,6 @@ __device__ void pass2_body_f32(const ProbDev& P, const EvalLane& ln, int tile, i
       for (int a = 0; a < D; ++a) gj[a] = P.gpref * G[a];
     }
   }
-}
-
-// ------------------------------------------------------------ GEMM pass 1
-// Powers dst[e] = exp(2 pi i (base + e) s) for e in [e0, e0 + cnt): FP64
-// sincospi of the exact exponent at e0, products with z = exp(2 pi i s) after it.
-__device__ __forceinline__ void fill_powers(double2* dst, int e0, int cnt, int base, double s,
-                                            double2 z) {
-  double sn, cs;
-  sincos_2pi_ms((double)(base + e0), s, &sn, &cs);
-  double2 p = make_double2(cs, sn);
-  for (int e = 0; e < cnt; ++e) {
-    dst[e0 + e] = p;
-    p = cmul(p, z);
-  }
-}
-
-// z = exp(2 pi i s) per (particle, axis) of the chunk starting at particle jb.
-template <int D>
-__device__ __forceinline__ void chunk_roots(double2* zs, const double* s, int jb, int kc) {
-  for (int u = threadIdx.x; u < kGemmChunk * D; u += blockDim.x) {
-    const int j = u / D;
-    double sn = 0.0, cs = 1.0;
-    if (j < kc) sincospi(2.0 * s[(size_t)jb * D + u], &sn, &cs);
-    zs[u] = make_double2(cs, sn);
-  }
-}
-
-// The outputs of a folded block: cell (run 3 tr + i, column lo + tn + 16 q)
-// holds C(c) = (P1 - P2) + i (P3 + P4) and C(-c) = (P1 + P2) + i (P4 - P3);
-// each lands in its run's row if the run contains that n.
-template <int CQ>
-__device__ __forceinline__ void gemm_fold_store(const ProbDev& P, const EvalLane& ln, int tile,
-                                                const GemmBlock& B, int tr, int tn,
-                                                const double (&p1)[3][CQ],
-                                                const double (&p2)[3][CQ],
-                                                const double (&p3)[3][CQ],
-                                                const double (&p4)[3][CQ]) {
-  double2* out = ln.part + (size_t)tile * P.M;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const int r = 3 * tr + i;
-    if (r < B.nrun) {
-      const GemmRun g = P.grun[B.run0 + r];
-#pragma unroll
-      for (int q = 0; q < CQ; ++q) {
-        const int col = tn + 16 * q;
-        const int cv = B.lo + col;
-        if (col < B.nb) {
-          if (cv >= g.a && cv <= g.b)
-            out[g.kstart + (cv - g.a)] = make_double2(p1[i][q] - p2[i][q], p3[i][q] + p4[i][q]);
-          if (cv > 0 && -cv >= g.a && -cv <= g.b)
-            out[g.kstart + (-cv - g.a)] = make_double2(p1[i][q] + p2[i][q], p4[i][q] - p3[i][q]);
-        }
-      }
-    }
-  }
-}
-
-// Pass 1 of one (lane, tile, block) of a 3-D k-set as a complex GEMM over
-// the tile's particles, kGemmChunk at a time: the tables of the chunk (prefix
-// powers per axis, last-axis powers for the block's window) and the A rows
-// (A = T0 T1, the runs' prefix phases) are built in shared memory. The last
-// axis is folded as in the d = 2 body: columns are c = |n2| and the four sums
-// P1..P4 of a cell give C(c) and C(-c). Each thread accumulates 3 runs x CQ
-// columns (tn, tn + 16, ...). Each k-set row is written once. The roots z of
-// the next chunk are formed while the A rows are built.
-template <int D, int CQ>
-__device__ void pass1_gemm_body(const ProbDev& P, const EvalLane& ln, int tile, int blk,
-                                double2* smem) {
-  constexpr int KC = kGemmChunk, ZS = gemm_fold_zstride(CQ), W = 16 * CQ;
-  const GemmBlock B = P.gblk[blk];
-  const int j0 = tile * kPass1Tile;
-  const int nj = min(kPass1Tile, P.N - j0);
-  const int c0 = B.c0, c1 = D == 3 ? B.c1 : 0;   // this group's prefix windows
-  const int s0 = P.gs0, s1 = D == 3 ? P.gs1 : 0;
-  double2* T0 = smem;                       // [KC][s0]
-  double2* T1 = T0 + KC * s0;               // [KC][s1]
-  double2* Z = T1 + KC * s1;                // [KC][ZS]
-  double2* A = Z + KC * ZS;                 // [KC][kGemmRows]
-  double2* R = A + KC * kGemmRows;          // [2][KC * D] roots, double-buffered
-  const int tr = threadIdx.x >> 4, tn = threadIdx.x & 15;
-  double p1[3][CQ], p2[3][CQ], p3[3][CQ], p4[3][CQ];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int q = 0; q < CQ; ++q) p1[i][q] = p2[i][q] = p3[i][q] = p4[i][q] = 0.0;
-  const int L = P.gL, u0 = P.gu0, u1 = D == 3 ? P.gu1 : 0, uz = P.guz;
-  chunk_roots<D>(R, ln.s, j0, min(KC, nj));
-  int buf = 0;
-  for (int jc = 0; jc < nj; jc += KC) {
-    const int kc = min(KC, nj - jc);
-    const double2* zs = R + buf * KC * D;
-    __syncthreads();   // the previous chunk's products and this chunk's roots are done
-    for (int u = threadIdx.x; u < KC * (u0 + u1 + uz); u += blockDim.x) {
-      const int j = u % KC, q = u / KC;
-      const double* sj = ln.s + (size_t)(j0 + jc + j) * D;
-      const bool live = j < kc;
-      if (q < u0) {
-        if (L * q < c0)
-          fill_powers(T0 + j * s0, L * q, min(L, c0 - L * q), B.m0, live ? sj[0] : 0.0,
-                      zs[j * D]);
-      } else if (q < u0 + u1) {
-        const int qq = q - u0;
-        if (L * qq < c1)
-          fill_powers(T1 + j * s1, L * qq, min(L, c1 - L * qq), B.m1, live ? sj[1] : 0.0,
-                      zs[j * D + 1]);
-      } else {
-        const int qq = q - u0 - u1;
-        fill_powers(Z + j * ZS, L * qq, min(L, W - L * qq), B.lo, live ? sj[D - 1] : 0.0,
-                    zs[j * D + D - 1]);
-      }
-    }
-    __syncthreads();
-    for (int u = threadIdx.x; u < KC * kGemmRows; u += blockDim.x) {
-      const int j = u / kGemmRows, r = u - j * kGemmRows;
-      double2 v = make_double2(0.0, 0.0);
-      if (j < kc && r < B.nrun) {
-        const GemmRun g = P.grun[B.run0 + r];
-        v = T0[j * s0 + (g.n0 - B.m0)];
-        if (D == 3) v = cmul(v, T1[j * s1 + (g.n1 - B.m1)]);
-      }
-      A[j * kGemmRows + r] = v;
-    }
-    if (jc + KC < nj) chunk_roots<D>(R + (buf ^ 1) * KC * D, ln.s, j0 + jc + KC, min(KC, nj - jc - KC));
-    buf ^= 1;
-    __syncthreads();
-    const int kr = 6 * (threadIdx.x >> 5) < B.nrun ? kc : 0;   // warps past the runs skip
-    for (int j = 0; j < kr; ++j) {
-      double2 a[3], z[CQ];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) a[i] = A[j * kGemmRows + 3 * tr + i];
-#pragma unroll
-      for (int q = 0; q < CQ; ++q) z[q] = Z[j * ZS + tn + 16 * q];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int q = 0; q < CQ; ++q) {
-          p1[i][q] = fma(a[i].x, z[q].x, p1[i][q]);
-          p2[i][q] = fma(a[i].y, z[q].y, p2[i][q]);
-          p3[i][q] = fma(a[i].x, z[q].y, p3[i][q]);
-          p4[i][q] = fma(a[i].y, z[q].x, p4[i][q]);
-        }
-    }
-  }
-  gemm_fold_store<CQ>(P, ln, tile, B, tr, tn, p1, p2, p3, p4);
-}
-
-// d = 2: the A rows are a gather from the prefix table (A[r][j] = T0[j][n0(r)]),
-// so there is no A phase. The last axis is folded: the block's columns are
-// c = |n|, and with A = a + ib and z^c = u + iv the four sums P1 = sum a u,
-// P2 = sum b v, P3 = sum a v, P4 = sum b u give C(c) = (P1 - P2) + i (P3 + P4)
-// and C(-c) = A conj(z^c) summed = (P1 + P2) + i (P4 - P3): four FMAs per
-// cell and particle for two k-set rows. Each thread accumulates 3 runs x CQ
-// columns (tn, tn + 16, ...). The tables are double-buffered: while the CTA
-// multiplies chunk c it fills chunk c + 1 (and the roots of chunk c + 2), one
-// barrier per chunk. Rows past the group's runs read the zero column c0.
-// CQ: columns per thread (tn, tn + 16, ...), the problem's window is 16 CQ.
-template <int CQ>
-__device__ void pass1_gemm_body_d2(const ProbDev& P, const EvalLane& ln, int tile, int blk,
-                                   double2* smem) {
-  constexpr int KC = kGemmChunk, D = 2, ZS = gemm_fold_zstride(CQ), W = 16 * CQ;
-  const GemmBlock B = P.gblk[blk];
-  const int j0 = tile * kPass1Tile;
-  const int nj = min(kPass1Tile, P.N - j0);
-  const int c0 = B.c0, s0 = P.gs0;           // s0 > P.gc0 >= c0: column P.gc0 holds zeros
-  const int zc = P.gc0;
-  const int buf = KC * (s0 + ZS);            // one table set
-  double2* R = smem + 2 * buf;               // [2][KC * D] roots
-  const int tr = threadIdx.x >> 4, tn = threadIdx.x & 15;
-  const bool rows_live = 6 * (threadIdx.x >> 5) < B.nrun;   // this warp's rows 6w .. 6w + 5
-  int off[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const int r = 3 * tr + i;
-    off[i] = r < B.nrun ? P.grun[B.run0 + r].n0 - B.m0 : zc;
-  }
-  double p1[3][CQ], p2[3][CQ], p3[3][CQ], p4[3][CQ];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int q = 0; q < CQ; ++q) p1[i][q] = p2[i][q] = p3[i][q] = p4[i][q] = 0.0;
-  const int L = P.gL, u0 = P.gu0, uz = P.guz;
-  const int nch = (nj + KC - 1) / KC;
-  auto fill = [&](int c) {   // tables of chunk c into buffer c & 1 (roots in R[c & 1])
-    double2* T0 = smem + (c & 1) * buf;
-    double2* Z = T0 + KC * s0;
-    const double2* zs = R + (c & 1) * KC * D;
-    const int jc = c * KC, kc = min(KC, nj - jc);
-    for (int u = threadIdx.x; u < KC * (u0 + uz); u += blockDim.x) {
-      const int j = u % KC, q = u / KC;
-      const double* sj = ln.s + (size_t)(j0 + jc + j) * D;
-      const bool live = j < kc;
-      if (q < u0) {
-        if (L * q < c0)   // the problem's widest window sets the units; this one may be narrower
-          fill_powers(T0 + j * s0, L * q, min(L, c0 - L * q), B.m0, live ? sj[0] : 0.0, zs[j * D]);
-      } else {
-        const int qq = q - u0;
-        fill_powers(Z + j * ZS, L * qq, min(L, W - L * qq), B.lo, live ? sj[1] : 0.0,
-                    zs[j * D + 1]);
-      }
-    }
-    if (threadIdx.x < KC) T0[threadIdx.x * s0 + zc] = make_double2(0.0, 0.0);
-  };
-  chunk_roots<D>(R, ln.s, j0, min(KC, nj));
-  if (nch > 1) chunk_roots<D>(R + KC * D, ln.s, j0 + KC, min(KC, nj - KC));
-  __syncthreads();
-  fill(0);
-  __syncthreads();
-  for (int c = 0; c < nch; ++c) {
-    if (c + 1 < nch) fill(c + 1);
-    if (c + 2 < nch)   // roots of chunk c + 2 replace those of chunk c (used by fill(c), done)
-      chunk_roots<D>(R + (c & 1) * KC * D, ln.s, j0 + (c + 2) * KC, min(KC, nj - (c + 2) * KC));
-    const double2* T0 = smem + (c & 1) * buf;
-    const double2* Z = T0 + KC * s0;
-    const int kc = rows_live ? min(KC, nj - c * KC) : 0;
-    for (int j = 0; j < kc; ++j) {
-      double2 a[3], z[CQ];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) a[i] = T0[j * s0 + off[i]];
-#pragma unroll
-      for (int q = 0; q < CQ; ++q) z[q] = Z[j * ZS + tn + 16 * q];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int q = 0; q < CQ; ++q) {
-          p1[i][q] = fma(a[i].x, z[q].x, p1[i][q]);
-          p2[i][q] = fma(a[i].y, z[q].y, p2[i][q]);
-          p3[i][q] = fma(a[i].x, z[q].y, p3[i][q]);
-          p4[i][q] = fma(a[i].y, z[q].x, p4[i][q]);
-        }
-    }
-    __syncthreads();
-  }
-  gemm_fold_store<CQ>(P, ln, tile, B, tr, tn, p1, p2, p3, p4);
-}
-
-// The folded 3-D body at the problem's window width.
-__device__ __forceinline__ void pass1_gemm_d3(const ProbDev& P, const EvalLane& ln, int tile,
-                                              int blk, double2* smem) {
-  if (P.gcq == 1) pass1_gemm_body<3, 1>(P, ln, tile, blk, smem);
-  else if (P.gcq == 2) pass1_gemm_body<3, 2>(P, ln, tile, blk, smem);
-  else pass1_gemm_body<3, 3>(P, ln, tile, blk, smem);
-}
-
-// The folded d = 2 body at the problem's window width.
-__device__ __forceinline__ void pass1_gemm_d2(const ProbDev& P, const EvalLane& ln, int tile,
-                                              int blk, double2* smem) {
-  if (P.gcq == 1) pass1_gemm_body_d2<1>(P, ln, tile, blk, smem);
-  else if (P.gcq == 2) pass1_gemm_body_d2<2>(P, ln, tile, blk, smem);
-  else pass1_gemm_body_d2<3>(P, ln, tile, blk, smem);
 }
 
 }  // namespace

@@ -41,8 +41,8 @@ __host__ __device__ __forceinline__ FlView fl_view(double* rec, int ld) {
   return v;
 }
 
-__host__ __device__ __forceinline__ size_t fl_record_doubles(int ld, int M, int nt1) {
-  return kFlHead + 12 * (size_t)ld + 2 * (size_t)M * (2 + nt1);
+__host__ __device__ __forceinline__ size_t fl_record_doubles(int ld, size_t scratch) {
+  return kFlHead + 12 * (size_t)ld + 2 * scratch;
 }
 
 struct FlArgs {

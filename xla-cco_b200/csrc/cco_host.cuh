@@ -25,10 +25,13 @@ struct cco_problem {
   cco::SegHdr* seg2 = nullptr;
   double* w_run = nullptr;
   int* run2ref = nullptr;
-  cco::GemmRun* grun = nullptr;
-  cco::GemmBlock* gblk = nullptr;
+  cco::GridRun* grun = nullptr;
+  cco::GridBlock* gblk = nullptr;
+  cco::GridStrip* gstrip = nullptr;
+  cco::GridQuad* gquad = nullptr;
   double4* krow = nullptr;     // run-order rows (n_0, n_1, n_2, w) for the Hessian kernels
-  size_t smem1 = 0, smem2 = 0, smemG = 0;
+  size_t smem1 = 0, smem2 = 0, smemG = 0, smemH = 0;
+  int dense_blocks = 0;        // cco_problem_pass1_form
 };
 
 namespace cco {
@@ -97,10 +100,11 @@ struct RecordShape {
 inline size_t record_doubles(const RecordShape& R, const cco_problem* p) {
   const int ld = pad4(p->N * p->d);
   size_t n = 0;
-  if (R.method == Method::Descent) n = ds_record_doubles(ld, p->M, p->host.ntile1);
-  else if (R.method == Method::Flow) n = fl_record_doubles(ld, p->M, p->host.ntile1);
-  else if (R.method == Method::Md) n = md_record_doubles(ld, p->M, p->host.ntile1, R.waves);
-  else n = lb_record_doubles(R.m, R.tri_len, ld, p->M, p->host.ntile1, R.keep_s0);
+  const size_t sw = eval_scratch_words(p->host);
+  if (R.method == Method::Descent) n = ds_record_doubles(ld, sw);
+  else if (R.method == Method::Flow) n = fl_record_doubles(ld, sw);
+  else if (R.method == Method::Md) n = md_record_doubles(ld, sw, R.waves);
+  else n = lb_record_doubles(R.m, R.tri_len, ld, sw, R.keep_s0);
   return (n + 31) & ~(size_t)31;   // records start on 256-byte boundaries
 }
 
@@ -144,7 +148,7 @@ inline EvalLane eval_lane(const RecordShape& R, const LaneRef& L, const cco_prob
   }
   e.rho = dens;
   e.rhow = dens + p->M;
-  e.part = dens + 2 * (size_t)p->M;
+  e.part = e.rhow + eval_rhow_words(p->host);
   e.status = rec_status(L.rec);
   e.prob = prob_index;
   return e;
@@ -157,15 +161,17 @@ struct EvalSet {
   EvalItem* it1 = nullptr;
   EvalItem* it2 = nullptr;
   EvalItem* itG = nullptr;
+  EvalItem* itH = nullptr;
   EvalPlan plan{};
 
   cudaError_t build(const RecordShape& R, const std::vector<LaneRef>& refs,
                     const std::vector<const cco_problem*>& probs_of, int lo, int hi,
                     cudaStream_t st, bool may_fp32 = false) {
+    // the recurrence kernels run lanes without the grid form, and FP32 lanes
     long long tiles1 = 0, seg_tiles = 0;
     for (int i = lo; i < hi; ++i) {
       tiles1 += probs_of[i]->host.ntile2;
-      if (!probs_of[i]->host.gemm) seg_tiles += probs_of[i]->host.ntile1;
+      if (!probs_of[i]->host.grid) seg_tiles += probs_of[i]->host.ntile1;
     }
     const int split = pass2_split(tiles1);
     // pass-1 segment chunks: enough CTAs for the per-segment FP64 tiles
@@ -174,51 +180,55 @@ struct EvalSet {
     std::vector<const cco_problem*> uniq;
     std::vector<ProbDev> pv;
     std::vector<EvalLane> lv;
-    std::vector<EvalItem> g1[3], g2[3];   // items grouped by d
-    std::vector<EvalItem> gG[3][kGemmFoldMaxCq];   // GEMM items by d and window width
-    size_t smem1 = 0, smem2 = 0, smem2f = 0, smemG = 0;
-    int max_d = 1, max_m = 1;
+    std::vector<EvalItem> g1[3], g2[3], gH[3];   // items grouped by d
+    std::vector<EvalItem> gG[3][kGridClasses];   // grid pass-1 items by d and column class
+    size_t smem1 = 0, smem2 = 0, smem2f = 0, smemG = 0, smemH = 0;
+    int max_d = 1, chunks_red = 1;
     for (int i = lo; i < hi; ++i) {
       const cco_problem* p = probs_of[i];
+      const ProbDev& h = p->host;
       int u = 0;
       while (u < (int)uniq.size() && uniq[u] != p) ++u;
       if (u == (int)uniq.size()) {
         uniq.push_back(p);
-        pv.push_back(p->host);
+        pv.push_back(h);
         smem1 = std::max(smem1, p->smem1);
-        smem2 = std::max(smem2, eval_smem2(p->host, split));
-        smem2f = std::max(smem2f, eval_smem2(p->host, split, true));
+        smem2 = std::max(smem2, eval_smem2(h, split));
+        smem2f = std::max(smem2f, eval_smem2(h, split, true));
         smemG = std::max(smemG, p->smemG);
+        smemH = std::max(smemH, p->smemH);
         max_d = std::max(max_d, p->d);
-        max_m = std::max(max_m, p->M);
+        if (h.grid) chunks_red = std::max(chunks_red, reduce_chunks(h.gslots));
+        if (!h.grid || may_fp32) chunks_red = std::max(chunks_red, reduce_chunks(p->M));
       }
       const int j = i - lo;
       lv.push_back(eval_lane(R, refs[i], p, u));
-      if (p->host.gemm) {
-        const int ntG = p->host.ntile1 * p->host.ngblk;
-        for (int t = 0; t < ntG; ++t) gG[p->d - 1][p->host.gcq - 1].push_back(EvalItem{j, t});
+      if (h.grid) {
+        const int ntG = h.gntile * h.ngblk, ntH = (h.N + kGridTile2 - 1) / kGridTile2;
+        for (int t = 0; t < ntG; ++t) gG[p->d - 1][h.gcls].push_back(EvalItem{j, t});
+        for (int t = 0; t < ntH; ++t) gH[p->d - 1].push_back(EvalItem{j, t});
       }
-      // the per-segment pass 1: FP32 lanes, and problems without the GEMM form
-      if (!p->host.gemm || may_fp32) {
-        const int C = pass1_chunks(p->host, chunks);
-        for (int t = 0; t < p->host.ntile1 * C; ++t) g1[p->d - 1].push_back(EvalItem{j, t});
+      if (!h.grid || may_fp32) {
+        const int C = pass1_chunks(h, chunks);
+        for (int t = 0; t < h.ntile1 * C; ++t) g1[p->d - 1].push_back(EvalItem{j, t});
+        const int nt2 = pass2_tiles(h, split);
+        for (int t = 0; t < nt2; ++t) g2[p->d - 1].push_back(EvalItem{j, t});
       }
-      const int nt2 = pass2_tiles(p->host, split);
-      for (int t = 0; t < nt2; ++t) g2[p->d - 1].push_back(EvalItem{j, t});
     }
-    std::vector<EvalItem> i1, i2, iG;
-    plan.d_off1[0] = plan.d_off2[0] = plan.d_offG[0] = 0;
+    std::vector<EvalItem> i1, i2, iG, iH;
+    plan.d_off1[0] = plan.d_off2[0] = plan.d_offH[0] = 0;
     for (int D = 0; D < 3; ++D) {
       i1.insert(i1.end(), g1[D].begin(), g1[D].end());
       i2.insert(i2.end(), g2[D].begin(), g2[D].end());
-      for (int c = 0; c < kGemmFoldMaxCq; ++c) {
-        if (D >= 1) plan.q_offG[D - 1][c] = (int)iG.size();
+      iH.insert(iH.end(), gH[D].begin(), gH[D].end());
+      for (int c = 0; c < kGridClasses; ++c) {
+        plan.q_offG[D][c] = (int)iG.size();
         iG.insert(iG.end(), gG[D][c].begin(), gG[D][c].end());
       }
-      if (D >= 1) plan.q_offG[D - 1][kGemmFoldMaxCq] = (int)iG.size();
+      plan.q_offG[D][kGridClasses] = (int)iG.size();
       plan.d_off1[D + 1] = (int)i1.size();
       plan.d_off2[D + 1] = (int)i2.size();
-      plan.d_offG[D + 1] = (int)iG.size();
+      plan.d_offH[D + 1] = (int)iH.size();
     }
     plan.dyn_prec = may_fp32 ? 1 : 0;
     cudaError_t e = upload(&probs, pv, st);
@@ -226,13 +236,15 @@ struct EvalSet {
     if (e == cudaSuccess) e = upload(&it1, i1, st);
     if (e == cudaSuccess) e = upload(&it2, i2, st);
     if (e == cudaSuccess) e = upload(&itG, iG, st);
+    if (e == cudaSuccess) e = upload(&itH, iH, st);
     plan.probs = probs;
     plan.lanes = lanes;
     plan.items1 = it1;
     plan.items2 = it2;
     plan.itemsG = itG;
-    plan.n_itemsG = (int)iG.size();
+    plan.itemsH = itH;
     plan.smemG = smemG;
+    plan.smemH = smemH;
     plan.n_lanes = hi - lo;
     plan.n_items1 = (int)i1.size();
     plan.n_items2 = (int)i2.size();
@@ -240,7 +252,7 @@ struct EvalSet {
     plan.smem1 = smem1;
     plan.smem2 = smem2;
     plan.smem2_f32 = smem2f;
-    plan.red_chunks = reduce_chunks(max_m);
+    plan.red_chunks = chunks_red;
     plan.split2 = split;
     plan.chunks1 = chunks;
     plan.want_grad = true;
@@ -252,10 +264,10 @@ struct EvalSet {
     if (it1) cudaFreeAsync(it1, st);
     if (it2) cudaFreeAsync(it2, st);
     if (itG) cudaFreeAsync(itG, st);
-    itG = nullptr;
+    if (itH) cudaFreeAsync(itH, st);
     probs = nullptr;
     lanes = nullptr;
-    it1 = it2 = nullptr;
+    it1 = it2 = itG = itH = nullptr;
   }
 };
 

@@ -43,27 +43,31 @@ struct SegHdr {
 };
 static_assert(sizeof(SegHdr) == 32, "segment header is two 16-byte loads");
 
-// Pass 1 as a complex GEMM (problems where it is efficient, FP64 lanes): the
-// density of a particle tile on the grid (run r, last-axis n) is
-// C[r][n] = sum_j A[r][j] Z[n][j] with A the run's prefix phase and Z the
-// last-axis power z_j^n. The last axis is folded: a block's columns are
-// c = |n|, and the four real products of A z^c give both C(c) and C(-c).
-// Runs are grouped kGemmRows at a time (sorted by folded length) and each
-// group's folded range is cut into windows of 16 cq columns (cq per problem,
-// 1..kGemmFoldMaxCq); a (group, window) is a block, one CTA per (lane, tile,
-// block).
-constexpr int kGemmRows = 24, kGemmChunk = 32, kGemmThreads = 128;
-constexpr int kGemmFoldMaxCq = 3;
-// odd row stride of the last-axis table: table writes spread over banks
-__host__ __device__ constexpr int gemm_fold_zstride(int cq) { return 16 * cq + 1; }
-constexpr int kGemmMaxPrefix = 128;   // table entries per prefix axis
-constexpr int kGemmMaxRun = 16;       // longest power chain between FP64 sincospi seeds
-struct GemmRun {
-  int n0, n1, a, b, kstart, pad_;   // prefix (n0[, n1]), last-axis range [a, b]
+// Tensor-core form of both FP64 passes over the folded grid of the k-set
+// (cco_grid.cuh). A run is a prefix and the last-axis range [a, b] of its rows
+// (k-set rows kstart ..); a strip is 8 runs of similar folded length with nq
+// quads of 4 columns from its block's lo on; a block is up to 4 strips and
+// kGridCols columns whose phase tables a CTA builds together. A slot is one
+// (quad, lane) cell; slots are numbered strip by strip, quad by quad.
+constexpr int kGridCols = 48;      // columns of a block
+constexpr int kGridStrips = 4;     // strips of a block (one per warp in pass 1)
+constexpr int kGridChunk = 32;     // particles whose tables pass 1 holds at a time
+constexpr int kGridTile2 = 64;     // particles of a pass-2 CTA
+constexpr int kGridThreads = 128;
+constexpr int kGridMaxEntries = 200;   // table entries per particle (64 particles: 200 KB)
+constexpr int kGridClasses = 2;    // pass-1 kernels: blocks of <= 24 and <= 48 columns
+struct GridRun {
+  int n0, n1, a, b, kstart, pad_;   // prefix (1-D: n0 = q), last-axis range [a, b]
 };
-struct GemmBlock {
-  int run0, nrun, lo, nb;            // runs [run0, run0 + nrun), columns lo .. lo + nb - 1
-  int m0, c0, m1, c1;                // the group's prefix windows [m, m + c) per axis
+struct GridStrip {
+  int run0, nrun, nq, slot0;
+};
+struct GridBlock {
+  int strip0, nstrip, lo, ncol;      // columns lo .. lo + ncol - 1 (ncol a multiple of 8)
+  int m0, c0, m1, c1;                // prefix windows [m, m + c) of its runs, per axis
+};
+struct GridQuad {
+  int run0, nrun, c0, pad_;          // the strip's runs, the quad's first column
 };
 
 // Per-particle phase tables of one pass: row r holds z_a^(e * base^l) for one
@@ -83,13 +87,17 @@ struct ProbDev {
   TabLayout t1, t2;          // pass-1 / pass-2 table layouts
   int ntile1, ntile2;        // particle tiles of pass 1 / pass 2 (pass 2 at split 1)
   int sl2;                   // logical slices of the pass-2 segment pairs (power of 2, <= 8)
-  int gemm;                  // 1: FP64 pass 1 runs as the GEMM below
-  int ngblk, gm0, gc0, gm1, gc1;   // GEMM blocks; gc0, gc1: the widest group prefix windows
-  int gs0, gs1;              // their shared-memory row strides (odd)
-  int gL, gu0, gu1, guz;     // table fill: gL entries per unit; units per particle per table
-  int gcq, gpad_;            // d = 2: folded window of 16 gcq columns
-  const GemmBlock* gblk;
-  const GemmRun* grun;
+  int grid;                  // 1: FP64 lanes run the tensor-core form below
+  int ngblk, gcls;           // its blocks; pass-1 kernel class (0: <= 24 columns)
+  int gts;                   // table entries per particle (odd)
+  int gstep;                 // 1-D: prefix exponents are gstep n0 (1 otherwise)
+  int gslots;                // slots (a multiple of 32)
+  int gtile, gntile;         // particles per pass-1 tile, tiles
+  int grhow;                 // double2 words of the rhow area (chunk energies after the weights)
+  const GridBlock* gblk;
+  const GridStrip* gstrip;
+  const GridRun* grun;
+  const GridQuad* gquad;
   double vol;                // V
   double gpref;              // 2 (2 pi) / V
   const SegHdr* seg1;
@@ -104,8 +112,8 @@ struct EvalLane {
   double* f;              // [1]
   double* g;              // [N][d] or null
   double2* rho;           // [M] run order
-  double2* rhow;          // [M] weighted density (pass-2 input)
-  double2* part;          // [ntile1][M]
+  double2* rhow;          // pass-2 input: [M] weighted density, or the grid form's weights
+  double2* part;          // [ntile1][M], or [gntile][gslots][2] (grid form)
   const int64_t* status;  // evaluate iff null or *status == RUNNING
   const int32_t* prec;    // arithmetic of this evaluation: *prec, or `fixed_prec` when null
   int prob;
@@ -195,16 +203,17 @@ struct EvalPlan {
   const EvalItem* items2;   // device, grouped the same way (d_off2)
   int n_lanes, n_items1, n_items2;
   int d_off1[4], d_off2[4];
-  const EvalItem* itemsG;   // GEMM pass-1 items (lane, tile * ngblk + block), grouped by d
-  int n_itemsG;
-  int d_offG[4];
-  // within dimension D's GEMM items (D = 2, 3): those of window width 16 cq at
-  // [q_offG[D - 2][cq - 1], q_offG[D - 2][cq]) (one kernel per (D, cq))
-  int q_offG[2][kGemmFoldMaxCq + 1];
-  size_t smemG;
+  // grid form: pass-1 items (lane, tile * ngblk + block) and pass-2 items (lane,
+  // tile), grouped by d; within dimension D the pass-1 items of kernel class c
+  // are [q_offG[D - 1][c], q_offG[D - 1][c + 1])
+  const EvalItem* itemsG;
+  const EvalItem* itemsH;
+  int q_offG[3][kGridClasses + 1];
+  int d_offH[4];
+  size_t smemG, smemH;
   int dyn_prec;             // 1: lanes may be FP32 (the FP32 pass kernels launch too), 0: FP64 only
   int max_d;                // largest d in the plan (template dispatch)
-  int red_chunks;           // k-chunks of the reduction: ceil(max M / kReduceChunk)
+  int red_chunks;           // chunks of the reduction (reduce_chunks, largest in the plan)
   int split2;               // pass-2 threads per particle (1, 2, 4 or 8)
   int chunks1;              // pass-1 segment chunks per tile (FP64 per-segment form; 1 = none)
   size_t smem1, smem2;      // dynamic shared memory of pass 1 / pass 2 (FP64 kernels)
@@ -233,6 +242,20 @@ constexpr int kReduceChunk = 256;
 __host__ __device__ __forceinline__ int reduce_chunks(int M) {
   return (M + kReduceChunk - 1) / kReduceChunk;
 }
+// Scratch of one evaluated configuration, in double2 words: rho [M], the rhow
+// area, the pass-1 partials (the larger of the forms the problem may run).
+__host__ __device__ __forceinline__ size_t eval_rhow_words(const ProbDev& p) {
+  const size_t m = (size_t)p.M, g = p.grid ? (size_t)p.grhow : 0;
+  return m > g ? m : g;
+}
+__host__ __device__ __forceinline__ size_t eval_part_words(const ProbDev& p) {
+  const size_t seg = (size_t)p.ntile1 * p.M;
+  const size_t g = p.grid ? 2 * (size_t)p.gntile * p.gslots : 0;
+  return seg > g ? seg : g;
+}
+__host__ __device__ __forceinline__ size_t eval_scratch_words(const ProbDev& p) {
+  return (size_t)p.M + eval_rhow_words(p) + eval_part_words(p);
+}
 
 // Side streams of one launching stream: when a plan holds lanes of several
 // dimensions, each dimension's pass kernels run on their own stream (forked
@@ -246,30 +269,34 @@ struct EvalSide {
 cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream,
                         const EvalSide* side = nullptr);
 // Kernels one eval_launch of a plan issues: per dimension the per-segment and
-// GEMM pass-1 kernels and the pass-2 kernel that have items, plus the reduction (and
-// the energy kernel when there is no pass 2).
+// grid pass kernels that have items, plus the reduction (and the energy kernel
+// when there is no pass 2).
 inline int eval_kernels(const EvalPlan& p) {
   int n = p.n_lanes > 0 ? (p.want_grad ? 1 : 2) : 0;   // reduce (+ energy without pass 2)
   const int per = p.dyn_prec ? 2 : 1;   // FP64 and FP32 pass kernels
   for (int D = 1; D <= 3; ++D) {
     n += per * (p.d_off1[D] > p.d_off1[D - 1]);
-    if (D >= 2)
-      for (int c = 0; c < kGemmFoldMaxCq; ++c) n += p.q_offG[D - 2][c + 1] > p.q_offG[D - 2][c];
-    if (p.want_grad) n += per * (p.d_off2[D] > p.d_off2[D - 1]);
+    for (int c = 0; c < kGridClasses; ++c) n += p.q_offG[D - 1][c + 1] > p.q_offG[D - 1][c];
+    if (p.want_grad)
+      n += per * (p.d_off2[D] > p.d_off2[D - 1]) + (p.d_offH[D] > p.d_offH[D - 1]);
   }
   return n;
 }
 
+// Whether a plan launches pass kernels of dimension D.
+inline bool eval_has_dim(const EvalPlan& p, int D) {
+  return p.d_off1[D] > p.d_off1[D - 1] || p.q_offG[D - 1][kGridClasses] > p.q_offG[D - 1][0] ||
+         p.d_off2[D] > p.d_off2[D - 1] || p.d_offH[D] > p.d_offH[D - 1];
+}
 // Dimensions whose pass kernels a plan launches (side streams pay off from 2).
 inline int eval_dims(const EvalPlan& p) {
   int n = 0;
-  for (int D = 1; D <= 3; ++D)
-    n += p.d_off1[D] > p.d_off1[D - 1] || p.d_offG[D] > p.d_offG[D - 1] ||
-         p.d_off2[D] > p.d_off2[D - 1];
+  for (int D = 1; D <= 3; ++D) n += eval_has_dim(p, D);
   return n;
 }
 size_t eval_smem1(const ProbDev& p);
-size_t eval_smemG(const ProbDev& p);   // GEMM pass 1 (0 when the problem has none)
+size_t eval_smemG(const ProbDev& p);   // grid pass 1 (0 when the problem has no grid)
+size_t eval_smemH(const ProbDev& p);   // grid pass 2
 // Pass-2 dynamic shared memory at `split` for the FP64 kernels, or with
 // f32 for the FP32 ones (which keep phase tables for 1-D problems too).
 size_t eval_smem2(const ProbDev& p, int split, bool f32 = false);

@@ -61,8 +61,8 @@ __host__ __device__ __forceinline__ MdView md_view(double* rec, int ld, int w = 
 
 __host__ __device__ __forceinline__ size_t md_wave_doubles(int w) { return 8 * (size_t)w; }
 
-__host__ __device__ __forceinline__ size_t md_record_doubles(int ld, int M, int nt1, int w = 0) {
-  return kMdHead + 5 * (size_t)ld + md_wave_doubles(w) + 2 * (size_t)M * (2 + nt1);
+__host__ __device__ __forceinline__ size_t md_record_doubles(int ld, size_t scratch, int w = 0) {
+  return kMdHead + 5 * (size_t)ld + md_wave_doubles(w) + 2 * scratch;
 }
 
 enum : int { MD_VERLET = 0, MD_BAOAB = 1 };

@@ -48,7 +48,8 @@ __host__ __device__ __forceinline__ int64_t* rec_status(double* rec) {
 
 // ------------------------------------------------------------ descent
 // Record: [0, 16) DsState and the probe energy pf at [15]; then s, g, ps, pg
-// (ld each); then the evaluation scratch (double2: rho M, rhow M, part nt1 M).
+// (ld each); then the evaluation scratch (`scratch` double2 words:
+// rho, rhow and the pass-1 partials, eval_scratch_words).
 struct DsState {
   int64_t status, it, n_evals, t0, t1;   // t0/t1: %globaltimer at start / completion
   double f, step, norm;
@@ -74,8 +75,8 @@ __host__ __device__ __forceinline__ DsView ds_view(double* rec, int ld) {
   return v;
 }
 
-__host__ __device__ __forceinline__ size_t ds_record_doubles(int ld, int M, int nt1) {
-  return kDsHead + 4 * (size_t)ld + 2 * (size_t)M * (2 + nt1);
+__host__ __device__ __forceinline__ size_t ds_record_doubles(int ld, size_t scratch) {
+  return kDsHead + 4 * (size_t)ld + 2 * scratch;
 }
 
 struct DescentArgs {
@@ -179,10 +180,10 @@ __host__ __device__ __forceinline__ LbView lb_view(double* rec, int m, int tri_l
   return v;
 }
 
-__host__ __device__ __forceinline__ size_t lb_record_doubles(int m, int tri_len, int ld, int M,
-                                                             int nt1, int keep_s0 = 0) {
+__host__ __device__ __forceinline__ size_t lb_record_doubles(int m, int tri_len, int ld,
+                                                             size_t scratch, int keep_s0 = 0) {
   return kLbHead + 2 * (size_t)m * m + tri_len + lb_scal_len(m, ld) +
-         (7 + 2 * (size_t)m + (keep_s0 ? 1 : 0)) * ld + 2 * (size_t)M * (2 + nt1);
+         (7 + 2 * (size_t)m + (keep_s0 ? 1 : 0)) * ld + 2 * scratch;
 }
 
 struct LbArgs {

@@ -6,7 +6,7 @@
 // reference README's d=3 N=100 chi=0.05 relax has 1300 - their launch
 // latency is the whole cost of an iteration. Here a CTA of 128 threads (the
 // evaluation bodies' size) owns one lane and loops: pass 1 over the lane's
-// particle tiles (per-segment or GEMM form), the tile-order reduction to rho,
+// particle tiles (per-segment form), the tile-order reduction to rho,
 // w rho and Phi, pass 2 over its tiles, and the descent update, with block
 // barriers between the stages and no host round trip. Lanes never wait on
 // one another, so there is no inter-CTA synchronization; the loop ends when
@@ -27,7 +27,7 @@ namespace cco {
 
 namespace {
 
-constexpr int kPersistThreads = 128;   // kPass1Threads = kPass2Threads = kGemmThreads
+constexpr int kPersistThreads = 128;   // kPass1Threads = kPass2Threads
 
 // rho_k = sum over tiles of the pass-1 rows in tile order, w rho and Phi
 // (one lane, the whole CTA; fixed-order block sum).
@@ -53,21 +53,9 @@ __device__ void persist_reduce(const ProbDev& P, const EvalLane& ln, double* red
 // Energy, gradient and density of the lane's probe positions (FP64).
 template <int D>
 __device__ void persist_eval(const ProbDev& P, const EvalLane& ln, double2* smem, double* red) {
-  if constexpr (D >= 2) {
-    if (P.gemm) {
-      const int items = P.ntile1 * P.ngblk;
-      for (int it = 0; it < items; ++it) {
-        if constexpr (D == 2) pass1_gemm_d2(P, ln, it / P.ngblk, it % P.ngblk, smem);
-        else pass1_gemm_d3(P, ln, it / P.ngblk, it % P.ngblk, smem);
-        __syncthreads();
-      }
-    }
-  }
-  if (!P.gemm) {
-    for (int t = 0; t < P.ntile1; ++t) {
-      pass1_body<D>(P, ln, t, smem);
-      __syncthreads();
-    }
+  for (int t = 0; t < P.ntile1; ++t) {
+    pass1_body<D>(P, ln, t, smem);
+    __syncthreads();
   }
   persist_reduce(P, ln, red);
   __syncthreads();
@@ -119,9 +107,7 @@ bool persist_eligible(const cco_problem* p) {
 }
 
 size_t persist_smem(const cco_problem* p) {
-  size_t s = std::max(p->smem1, eval_smem2(p->host, 1));
-  if (p->host.gemm) s = std::max(s, p->smemG);
-  return s;
+  return std::max(p->smem1, eval_smem2(p->host, 1));
 }
 
 cudaError_t persist_descent(const DescentArgs& a, const EvalPlan& plan, size_t smem, int dims,

@@ -111,7 +111,7 @@ int cco_stepper_create(int device, void* stream, int method, const void* setting
     a.max_iters = cfg->max_evals / 2;
     a.rec_every = 1;
     a.rec_cap = 0;
-    h->rec_doubles = (ds_record_doubles(h->ld, 0, 0) + 31) & ~(size_t)31;
+    h->rec_doubles = (ds_record_doubles(h->ld, 0) + 31) & ~(size_t)31;
   } else {
     const auto* cfg = static_cast<const cco_lbfgs_settings*>(settings);
     if (cfg->n_rescales < 1 || cfg->n_rescales > CCO_MAX_RESCALES || cfg->memory < 1 ||
@@ -134,7 +134,7 @@ int cco_stepper_create(int device, void* stream, int method, const void* setting
       delete h;
       return rc;
     }
-    h->rec_doubles = (lb_record_doubles(shape.m, shape.tri_len, h->ld, 0, 0) + 31) & ~(size_t)31;
+    h->rec_doubles = (lb_record_doubles(shape.m, shape.tri_len, h->ld, 0) + 31) & ~(size_t)31;
     h->lb.nblkB = lb_nblk(h->ld);
     h->lb.nchA = lb_achunks(h->ld);
   }
