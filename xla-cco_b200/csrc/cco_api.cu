@@ -178,16 +178,28 @@ struct GridPlan {
   std::vector<GridStrip> strips;
   std::vector<GridBlock> blocks;
   std::vector<GridQuad> quads;
+  std::vector<GridRow> rows;
   int entries = 0;   // widest block's table entries
-  int cols = 0;      // widest block's columns
+  int tiles = 0;     // most 8 x 8-cell tiles of a block
 };
 
-void grid_layout(std::vector<GridRun> runs, int d, GridPlan* out) {
+// by_length: strips of runs of the same number of quads (fewest padded cells);
+// otherwise in prefix order (narrowest prefix windows: large or skewed sets).
+// Either way the inner axis runs back and forth, so that a strip that crosses
+// into the next outer value stays at the same end of the inner one.
+void grid_layout(std::vector<GridRun> runs, int d, int max_cols, int max_strips, bool by_length,
+                 GridPlan* out) {
   *out = GridPlan{};
-  sort_by_fold(runs);
+  std::stable_sort(runs.begin(), runs.end(), [by_length](const GridRun& x, const GridRun& y) {
+    const int u = by_length ? fold_hi(x) / 4 : 0, v = by_length ? fold_hi(y) / 4 : 0;
+    if (u != v) return u > v;
+    if (by_length)
+      return x.n1 != y.n1 ? x.n1 < y.n1 : (x.n1 & 1) ? x.n0 > y.n0 : x.n0 < y.n0;
+    return x.n0 != y.n0 ? x.n0 < y.n0 : (x.n0 & 1) ? x.n1 > y.n1 : x.n1 < y.n1;
+  });
   out->runs = runs;
   const int nr = (int)runs.size(), ns = (nr + 7) / 8;
-  const int nbr = (ns + kGridStrips - 1) / kGridStrips;   // block rows, of even height
+  const int nbr = (ns + max_strips - 1) / max_strips;   // block rows, of even height
   for (int br = 0; br < nbr; ++br) {
     const int s0 = (int)((long long)ns * br / nbr), s1 = (int)((long long)ns * (br + 1) / nbr);
     int lo = 1 << 30, hi = 0;
@@ -195,7 +207,7 @@ void grid_layout(std::vector<GridRun> runs, int d, GridPlan* out) {
       lo = std::min(lo, fold_lo(runs[r]));
       hi = std::max(hi, fold_hi(runs[r]));
     }
-    const int range = hi - lo + 1, nw = (range + kGridCols - 1) / kGridCols;
+    const int range = hi - lo + 1, nw = (range + max_cols - 1) / max_cols;
     const int width = ((range + nw - 1) / nw + 7) / 8 * 8;
     for (int w = lo; w <= hi; w += width) {
       GridBlock b{};
@@ -217,6 +229,7 @@ void grid_layout(std::vector<GridRun> runs, int d, GridPlan* out) {
         for (int q = 0; q < g.nq; ++q) out->quads.push_back(GridQuad{g.run0, g.nrun, w + 4 * q, 0});
         out->strips.push_back(g);
         b.nstrip += 1;
+        b.ntile += (g.nq + 1) / 2;
         b.ncol = std::max(b.ncol, (g.nq + 1) / 2 * 8);
         for (int r = g.run0; r < g.run0 + g.nrun; ++r) {
           b.m0 = std::min(b.m0, runs[r].n0);
@@ -230,7 +243,13 @@ void grid_layout(std::vector<GridRun> runs, int d, GridPlan* out) {
       b.c1 = d == 3 ? M1 - b.m1 + 1 : 0;
       if (d != 3) b.m1 = 0;
       out->entries = std::max(out->entries, b.ncol + b.c0 + b.c1);
-      out->cols = std::max(out->cols, b.ncol);
+      out->tiles = std::max(out->tiles, b.ntile);
+      for (int s = b.strip0; s < b.strip0 + b.nstrip; ++s)
+        for (int r = 0; r < 8; ++r) {   // rows past the strip's runs repeat its last (weights 0)
+          const GridRun& g = runs[out->strips[s].run0 + std::min(r, out->strips[s].nrun - 1)];
+          out->rows.push_back(GridRow{b.ncol + g.n0 - b.m0,
+                                      d == 3 ? b.ncol + b.c0 + g.n1 - b.m1 : 0, g.n0, g.n1});
+        }
       out->blocks.push_back(b);
     }
   }
@@ -255,41 +274,61 @@ std::vector<GridRun> split_runs_1d(const std::vector<GridRun>& runs, int C) {
 // when the slots (cells with their padding) are at most twice the rows.
 void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
   if (runs.empty()) return;
+  // the layout that costs least per particle: products and table entries (both
+  // passes), among block shapes whose tables fit
   int step = 1;
+  double best = -1.0;
+  auto consider = [&](const std::vector<GridRun>& r, int cols, int strips, bool by_length, int st) {
+    GridPlan g;
+    grid_layout(r, P->d, cols, strips, by_length, &g);
+    double cost = (P->d == 1 ? 8.0 : 12.0) * 32.0 * (double)g.quads.size();
+    for (const GridBlock& b : g.blocks) cost += 16.0 * (b.ncol + b.c0 + b.c1);
+    if (g.entries > kGridMaxEntries || g.tiles > kGridMaxTiles || (best >= 0.0 && cost >= best)) return;
+    best = cost;
+    step = st;
+    *gp = g;
+  };
   if (P->d == 1) {
-    // the column count that costs least: cells and table entries per particle
-    double best = 0.0;
-    int best_c = -1;
-    for (int nc = 4; nc <= kGridCols; nc += 4) {
-      GridPlan g;
-      grid_layout(split_runs_1d(runs, nc - 1), 1, &g);
-      double cost = 0.0;
-      for (const GridBlock& b : g.blocks) cost += 16.0 * (b.ncol + b.c0);
-      cost += 8.0 * 32.0 * (double)g.quads.size();
-      if (g.entries <= kGridMaxEntries && (best_c < 0 || cost < best)) {
-        best = cost;
-        best_c = nc;
-      }
-    }
-    if (best_c < 0) return;
-    grid_layout(split_runs_1d(runs, best_c - 1), 1, gp);
-    step = 2 * (best_c - 1) + 1;
+    for (const int nc : {4, 8, 12, 16, 24, 32})
+      consider(split_runs_1d(runs, nc - 1), nc, std::min(kGridStrips, (kGridMaxEntries - nc) / 8),
+               true, 2 * nc - 1);
   } else {
-    grid_layout(runs, P->d, gp);
+    static const int shapes[][2] = {{32, 2}, {24, 3}, {24, 4}, {16, 4}, {24, 2}, {16, 2}, {16, 1}, {8, 1}};
+    for (int i = 0; i < 4; ++i) consider(runs, shapes[i][0], shapes[i][1], true, 1);
+    for (int i = 1; i < 8; ++i) consider(runs, shapes[i][0], shapes[i][1], false, 1);
   }
+  if (best < 0.0) return;
   const long long slots = 32ll * (long long)gp->quads.size();
-  if (gp->entries > kGridMaxEntries || slots > 2ll * P->M) return;
+  if (slots > 2ll * P->M) return;
   P->grid = 1;
   P->ngblk = (int)gp->blocks.size();
-  P->gcls = gp->cols <= 24 ? 0 : 1;
+  P->gcls = gp->tiles > 8 ? 2 : P->ngblk >= kGridRootsMin ? 1 : 0;
   P->gts = gp->entries | 1;
   P->gstep = step;
   P->gslots = (int)slots;
   // larger pass-1 tiles for larger N keep the partials (32 bytes per slot and
   // tile) and the reduction small once there are enough tiles to fill the GPU
-  P->gtile = P->N <= 2048 ? 64 : P->N <= 8192 ? 128 : 256;
+  P->gtile = P->N <= 512 ? 64 : P->N <= 8192 ? 128 : 256;
   P->gntile = (P->N + P->gtile - 1) / P->gtile;
   P->grhow = (int)slots * (P->d == 1 ? 2 : 4) + (reduce_chunks((int)slots) + 1) / 2;
+  // seeds per virtual axis: multiples of 16 up to the largest |exponent| used
+  // (the columns of a block's last tile included)
+  int top[3] = {0, 0, 0};
+  for (const GridBlock& b : gp->blocks) {
+    top[0] = std::max({top[0], -b.m0 + 15, b.m0 + b.c0 - 1});
+    if (P->d == 3) top[1] = std::max({top[1], -b.m1 + 15, b.m1 + b.c1 - 1});
+    top[2] = std::max(top[2], b.lo + b.ncol - 1);
+  }
+  P->groff[0] = 0;
+  P->groff[1] = 1 + top[0] / 16;
+  P->groff[2] = P->groff[1] + (P->d == 3 ? 1 + top[1] / 16 : 0);
+  P->groots = P->gcls > 0 ? P->groff[2] + 1 + top[2] / 16 : 0;
+  // cco_energy_grad_noalloc must go on taking what it took
+  const size_t seg = 2 * (size_t)P->M + (size_t)P->ntile1 * P->M;
+  const size_t own = (size_t)P->M + P->grhow + 2 * (size_t)P->gntile * P->gslots + eval_roots_words(*P);
+  if (sizeof(double2) * own > CCO_NOALLOC_SCRATCH_BYTES - 65536 &&
+      sizeof(double2) * seg <= CCO_NOALLOC_SCRATCH_BYTES)
+    P->grid = 0;
 }
 
 template <class T>
@@ -514,11 +553,13 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
     if (e == cudaSuccess) e = to_device(&pr->gblk, gp.blocks);
     if (e == cudaSuccess) e = to_device(&pr->gstrip, gp.strips);
     if (e == cudaSuccess) e = to_device(&pr->gquad, gp.quads);
+    if (e == cudaSuccess) e = to_device(&pr->grow, gp.rows);
   }
   P.grun = pr->grun;
   P.gblk = pr->gblk;
   P.gstrip = pr->gstrip;
   P.gquad = pr->gquad;
+  P.grow = pr->grow;
   P.seg1 = pr->seg1;
   P.seg2 = pr->seg2;
   P.w_run = pr->w_run;
@@ -549,6 +590,7 @@ int cco_problem_destroy(cco_problem* p) {
   if (p->gblk) cudaFree(p->gblk);
   if (p->gstrip) cudaFree(p->gstrip);
   if (p->gquad) cudaFree(p->gquad);
+  if (p->grow) cudaFree(p->grow);
   if (p->krow) cudaFree(p->krow);
   cudaFree(p->dev);
   delete p;
@@ -581,8 +623,9 @@ namespace {
 __global__ void k_make_lanes(EvalLane* lanes, EvalItem* it1, EvalItem* it2, int B, int nt1,
                              int nt2, int total, const double* s, size_t s_stride, double* f,
                              size_t f_stride, double* g, size_t g_stride, double2* rho,
-                             double2* rhow, double2* part, int M, size_t rhow_stride,
-                             size_t part_stride, int prec) {
+                             double2* rhow, double2* part, double2* roots, int M,
+                             size_t rhow_stride, size_t part_stride, size_t roots_stride,
+                             int prec) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     if (i < B) {
       EvalLane L;
@@ -592,6 +635,7 @@ __global__ void k_make_lanes(EvalLane* lanes, EvalItem* it1, EvalItem* it2, int 
       L.rho = rho + (size_t)i * M;
       L.rhow = rhow + (size_t)i * rhow_stride;
       L.part = part + (size_t)i * part_stride;
+      L.roots = roots + (size_t)i * roots_stride;
       L.status = nullptr;
       L.prec = nullptr;
       L.fixed_prec = prec;
@@ -616,6 +660,7 @@ struct EvalWS {
   double2* rho = nullptr;
   double2* rhow = nullptr;
   double2* part = nullptr;
+  double2* roots = nullptr;   // after the partials
   EvalPlan plan{};
   int prec = PREC_FP64;   // arithmetic of every lane of this workspace
 
@@ -623,7 +668,7 @@ struct EvalWS {
   struct Sizes {
     bool grid;
     int split, nt1, nt2;
-    size_t rhow, part;   // double2 words per lane
+    size_t rhow, part, roots;   // double2 words per lane
   };
   static Sizes sizes(const cco_problem* p, int B, int prec) {
     Sizes z;
@@ -634,6 +679,7 @@ struct EvalWS {
     z.nt2 = z.grid ? (h.N + kGridTile2 - 1) / kGridTile2 : pass2_tiles(h, z.split);
     z.rhow = z.grid ? (size_t)h.grhow : (size_t)h.M;
     z.part = z.grid ? 2 * (size_t)h.gntile * h.gslots : (size_t)h.ntile1 * h.M;
+    z.roots = z.grid ? eval_roots_words(h) : 0;
     return z;
   }
   cudaError_t alloc(const cco_problem* p, int B, cudaStream_t st) {
@@ -643,7 +689,8 @@ struct EvalWS {
     if (e == cudaSuccess) e = pool_alloc(&it2, sizeof(EvalItem) * (size_t)B * z.nt2, st);
     if (e == cudaSuccess) e = pool_alloc(&rho, sizeof(double2) * (size_t)B * p->M, st);
     if (e == cudaSuccess) e = pool_alloc(&rhow, sizeof(double2) * (size_t)B * z.rhow, st);
-    if (e == cudaSuccess) e = pool_alloc(&part, sizeof(double2) * (size_t)B * z.part, st);
+    if (e == cudaSuccess) e = pool_alloc(&part, sizeof(double2) * (size_t)B * (z.part + z.roots), st);
+    if (e == cudaSuccess) roots = part + (size_t)B * z.part;
     return e;
   }
   cudaError_t build(const cco_problem* p, int B, const double* s, size_t s_stride, double* f,
@@ -652,8 +699,8 @@ struct EvalWS {
     const int total = B * std::max(z.nt1, z.nt2) + B;
     const int blocks = std::min(1024, (total + 255) / 256);
     k_make_lanes<<<blocks, 256, 0, st>>>(lanes, it1, it2, B, z.nt1, z.nt2, total, s, s_stride, f,
-                                         f_stride, g, g_stride, rho, rhow, part, p->M, z.rhow,
-                                         z.part, prec);
+                                         f_stride, g, g_stride, rho, rhow, part, roots, p->M,
+                                         z.rhow, z.part, z.roots, prec);
     plan.probs = p->dev;
     plan.lanes = lanes;
     plan.items1 = plan.itemsG = it1;
@@ -665,14 +712,18 @@ struct EvalWS {
     for (int D = 0; D <= 3; ++D) {
       plan.d_off1[D] = D >= p->d ? plan.n_items1 : 0;
       plan.d_off2[D] = D >= p->d ? plan.n_items2 : 0;
-      plan.d_offH[D] = D >= p->d ? nH : 0;
     }
     // one problem: its items are all of its column class
     for (int D = 1; D <= 3; ++D)
       for (int c = 0; c <= kGridClasses; ++c)
         plan.q_offG[D - 1][c] = (D == p->d && c > p->host.gcls) ? nG : 0;
+    for (int D = 1; D <= 3; ++D)
+      for (int c = 0; c <= 2; ++c)
+        plan.h_off[D - 1][c] = (D == p->d && c > (p->host.gcls > 0)) ? nH : 0;
     plan.smemG = p->smemG;
     plan.smemH = p->smemH;
+    plan.n_grid = z.roots > 0 ? B : 0;
+    plan.root_chunks = (int)((z.roots + kRootChunk - 1) / kRootChunk);
     plan.dyn_prec = prec == PREC_FP32 ? 1 : 0;
     plan.max_d = p->d;
     plan.smem1 = p->smem1;
@@ -822,24 +873,25 @@ extern "C" int cco_energy_grad_noalloc(cco_problem* p, void* stream, int batch, 
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nd = (size_t)p->N * p->d;
   struct Carve {
-    size_t lanes, it1, it2, rho, rhow, total;
+    size_t lanes, it1, it2, rho, rhow, part, roots, total;
   };
-  auto carve = [&](int b, int prec_form) {
-    const EvalWS::Sizes z = EvalWS::sizes(p, b, prec_form);
+  auto carve = [&](int b) {
+    const EvalWS::Sizes z = EvalWS::sizes(p, b, PREC_FP64);
     Carve c;
     c.lanes = 0;
     c.it1 = round256(sizeof(EvalLane) * b);
     c.it2 = c.it1 + round256(sizeof(EvalItem) * (size_t)b * z.nt1);
     c.rho = c.it2 + round256(sizeof(EvalItem) * (size_t)b * z.nt2);
     c.rhow = c.rho + round256(sizeof(double2) * (size_t)b * M);
-    const size_t part = c.rhow + round256(sizeof(double2) * (size_t)b * z.rhow);
-    c.total = part + round256(sizeof(double2) * (size_t)b * z.part);
-    return std::make_pair(c, part);
+    c.part = c.rhow + round256(sizeof(double2) * (size_t)b * z.rhow);
+    c.roots = c.part + sizeof(double2) * (size_t)b * z.part;
+    c.total = c.roots + round256(sizeof(double2) * (size_t)b * z.roots);
+    return c;
   };
   int part_b = batch;
-  while (part_b > 1 && carve(part_b, PREC_FP64).first.total > CCO_NOALLOC_SCRATCH_BYTES)
+  while (part_b > 1 && carve(part_b).total > CCO_NOALLOC_SCRATCH_BYTES)
     part_b = (part_b + 1) / 2;
-  const auto [c, part] = carve(part_b, PREC_FP64);
+  const Carve c = carve(part_b);
   if (c.total > CCO_NOALLOC_SCRATCH_BYTES)
     return fail(CCO_ERR_ARG, "one configuration needs %zu bytes of fixed scratch, the limit is %zu",
                 c.total, (size_t)CCO_NOALLOC_SCRATCH_BYTES);
@@ -851,7 +903,8 @@ extern "C" int cco_energy_grad_noalloc(cco_problem* p, void* stream, int batch, 
     ws.it2 = reinterpret_cast<EvalItem*>(base + c.it2);
     ws.rho = reinterpret_cast<double2*>(base + c.rho);
     ws.rhow = reinterpret_cast<double2*>(base + c.rhow);
-    ws.part = reinterpret_cast<double2*>(base + part);
+    ws.part = reinterpret_cast<double2*>(base + c.part);
+    ws.roots = reinterpret_cast<double2*>(base + c.roots);
     CCO_CUDA(ws.build(p, b, s + (size_t)lo * nd, nd, phi + lo, 1,
                       grad ? grad + (size_t)lo * nd : nullptr, nd, st));
     CCO_CUDA(eval_launch(ws.plan, st));

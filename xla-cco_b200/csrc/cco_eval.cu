@@ -35,6 +35,7 @@
 //     two rows ahead). Per row: one complex multiply, the coefficient
 //     w(Im rho cos - Re rho sin) and two accumulations; prefix axes are
 //     weighted once per segment.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 
@@ -46,26 +47,58 @@ namespace cco {
 
 namespace {
 
-// Grid form (cco_grid.cuh), pass 1: one kernel per (dimension, column class),
-// each holding the accumulators of NT = 3 or 6 column tiles.
-template <int D, int NT>
-__global__ void __launch_bounds__(kGridThreads, NT == 3 ? 4 : 3) k_grid1(EvalPlan plan) {
-  extern __shared__ double2 smem[];
-  __shared__ ProbDev sp;
-  const EvalItem it = plan.itemsG[plan.q_offG[D - 1][NT == 3 ? 0 : 1] + blockIdx.x];
-  const EvalLane ln = plan.lanes[it.lane];
-  if (!lane_active(ln.status)) return;
-  if (plan.dyn_prec && lane_prec(ln) == PREC_FP32) return;   // the FP32 body handles it
-  if (threadIdx.x == 0) sp = plan.probs[ln.prob];
-  __syncthreads();
-  grid_pass1_body<D, NT>(sp, ln, it.tile / sp.ngblk, it.tile % sp.ngblk, blockIdx.x, smem);
+constexpr int kGridSms = 148;                      // SMs of a B200
+
+
+// An FP64 lane that is still to be evaluated.
+__device__ __forceinline__ bool grid_lane_runs(const EvalPlan& plan, const EvalLane& ln) {
+  return lane_active(ln.status) && !(plan.dyn_prec && lane_prec(ln) == PREC_FP32);
 }
 
+// Grid form: the phases the tables start from.
+__global__ void __launch_bounds__(kRootChunk) k_grid_roots(EvalPlan plan) {
+  const EvalLane& ln = plan.lanes[blockIdx.y];
+  if (!grid_lane_runs(plan, ln)) return;
+  const ProbDev& P = plan.probs[ln.prob];
+  const int w = blockIdx.x * kRootChunk + threadIdx.x;
+  if (!P.grid || w >= P.groots * P.N) return;
+  if (P.d == 1) grid_roots<1>(P, ln, w);
+  else if (P.d == 2) grid_roots<2>(P, ln, w);
+  else grid_roots<3>(P, ln, w);
+}
+
+// Grid form (cco_grid.cuh), pass 1: one kernel per (dimension, class), each
+// holding the accumulators of 2 or 3 tiles per warp. Persistent: four CTAs of
+// four warps per SM walk the items.
+template <int D, int CLS>
+__global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid1(EvalPlan plan) {
+  extern __shared__ double2 smem[];
+  __shared__ GridStage stage;
+  constexpr bool ROOTS = CLS > 0;
+  constexpr int NT = CLS == 2 ? 3 : 2;
+  const EvalItem* items = plan.itemsG + plan.q_offG[D - 1][CLS];
+  const int n = plan.q_offG[D - 1][CLS + 1] - plan.q_offG[D - 1][CLS];
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const EvalItem it = items[i];
+    const EvalLane ln = plan.lanes[it.lane];
+    if (!grid_lane_runs(plan, ln)) continue;   // FP32 lanes: k_pass1
+    const ProbDev& P = plan.probs[ln.prob];
+    grid_pass1<D, ROOTS, NT>(P, ln, it.tile / P.ngblk, it.tile % P.ngblk, stage, smem);
+  }
+}
+
+int grid_ctas(int items) { return std::min(items, kGridCtas * kGridSms); }
+
+template <int D, int CLS>
+void launch_grid1_class(const EvalPlan& plan, cudaStream_t s) {
+  const int n = plan.q_offG[D - 1][CLS + 1] - plan.q_offG[D - 1][CLS];
+  if (n > 0) k_grid1<D, CLS><<<grid_ctas(n), kGridThreads, plan.smemG, s>>>(plan);
+}
 template <int D>
 void launch_grid1(const EvalPlan& plan, cudaStream_t s) {
-  const int* q = plan.q_offG[D - 1];
-  if (q[1] > q[0]) k_grid1<D, 3><<<q[1] - q[0], kGridThreads, plan.smemG, s>>>(plan);
-  if (q[2] > q[1]) k_grid1<D, 6><<<q[2] - q[1], kGridThreads, plan.smemG, s>>>(plan);
+  launch_grid1_class<D, 0>(plan, s);
+  launch_grid1_class<D, 1>(plan, s);
+  launch_grid1_class<D, 2>(plan, s);
 }
 
 // One kernel per dimension D and arithmetic keeps each kernel's code small:
@@ -158,18 +191,19 @@ __global__ void __launch_bounds__(kReduceChunk) k_reduce(EvalPlan plan) {
 // Energy of one lane (one warp): the chunk energies summed in a fixed order.
 __device__ __forceinline__ void lane_energy(const EvalPlan& plan, const EvalLane& ln) {
   const ProbDev& P = plan.probs[ln.prob];
+  const int wl = threadIdx.x & 31;
   double e = 0.0;
   if (P.grid && lane_prec(ln) == PREC_FP64) {
     const double* ec = grid_energies(P, ln);
     const int nc = reduce_chunks(P.gslots);
-    for (int c = threadIdx.x; c < nc; c += 32) e += ec[c];
+    for (int c = wl; c < nc; c += 32) e += ec[c];
   } else {
     const int nc = reduce_chunks(P.M);
-    for (int c = threadIdx.x; c < nc; c += 32) e += ln.part[(size_t)c * kReduceChunk].x;
+    for (int c = wl; c < nc; c += 32) e += ln.part[(size_t)c * kReduceChunk].x;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-  if (threadIdx.x == 0) *ln.f = e / P.vol;
+  if (wl == 0) *ln.f = e / P.vol;
 }
 
 // Energy-only evaluations (no pass 2): one warp per lane. With the gradient,
@@ -182,19 +216,19 @@ __global__ void k_energy(EvalPlan plan) {
 }
 
 // Grid form, pass 2.
-template <int D>
-__global__ void __launch_bounds__(kGridThreads, 4) k_grid2(EvalPlan plan) {
+template <int D, bool ROOTS>
+__global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid2(EvalPlan plan) {
   extern __shared__ double2 smem[];
-  __shared__ ProbDev sp;
-  const EvalItem it = plan.itemsH[plan.d_offH[D - 1] + blockIdx.x];
-  const EvalLane ln = plan.lanes[it.lane];
-  if (!lane_active(ln.status)) return;
-  if (plan.dyn_prec && lane_prec(ln) == PREC_FP32) return;   // the FP32 body handles it
-  if (it.tile == 0 && threadIdx.x < 32) lane_energy(plan, ln);
-  if (ln.g == nullptr) return;
-  if (threadIdx.x == 0) sp = plan.probs[ln.prob];
-  __syncthreads();
-  grid_pass2_body<D>(sp, ln, it.tile, smem);
+  __shared__ GridStage stage;
+  const EvalItem* items = plan.itemsH + plan.h_off[D - 1][ROOTS];
+  const int n = plan.h_off[D - 1][ROOTS + 1] - plan.h_off[D - 1][ROOTS];
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const EvalItem it = items[i];
+    const EvalLane ln = plan.lanes[it.lane];
+    if (!grid_lane_runs(plan, ln)) continue;   // FP32 lanes: k_pass2
+    if (it.tile == 0 && threadIdx.x < 32) lane_energy(plan, ln);
+    if (ln.g) grid_pass2<D, ROOTS>(plan.probs[ln.prob], ln, it.tile, stage, smem);
+  }
 }
 
 template <int D, bool F32>
@@ -306,20 +340,24 @@ cudaError_t configure_d() {
 
 template <int D>
 cudaError_t configure_grid() {
-  constexpr int most = 227 * 1024 - 1024;
-  cudaError_t e =
-      cudaFuncSetAttribute(k_grid1<D, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_grid1<D, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_grid2<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  constexpr int most = kGridTile2 * kGridMaxEntries * sizeof(double2);
+  cudaError_t e = cudaSuccess;
+  auto opt_in = [&](const void* k) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  };
+  opt_in((const void*)k_grid1<D, 0>);
+  opt_in((const void*)k_grid1<D, 1>);
+  opt_in((const void*)k_grid1<D, 2>);
+  opt_in((const void*)k_grid2<D, false>);
+  opt_in((const void*)k_grid2<D, true>);
   return e;
 }
 
-template <int D>
+template <int D, bool ROOTS>
 void launch_grid2(const EvalPlan& plan, cudaStream_t s) {
-  const int n = plan.d_offH[D] - plan.d_offH[D - 1];
-  if (n > 0) k_grid2<D><<<n, kGridThreads, plan.smemH, s>>>(plan);
+  const int n = plan.h_off[D - 1][ROOTS + 1] - plan.h_off[D - 1][ROOTS];
+  if (n > 0) k_grid2<D, ROOTS><<<grid_ctas(n), kGridThreads, plan.smemH, s>>>(plan);
 }
 
 template <int D, bool F32>
@@ -357,8 +395,12 @@ template <int D>
 void launch_dim_d(const EvalPlan& plan, bool pass2, cudaStream_t s) {
   launch_d<D, false>(plan, pass2, s);
   if (plan.dyn_prec) launch_d<D, true>(plan, pass2, s);
-  if (pass2) launch_grid2<D>(plan, s);
-  else launch_grid1<D>(plan, s);
+  if (pass2) {
+    launch_grid2<D, false>(plan, s);
+    launch_grid2<D, true>(plan, s);
+  } else {
+    launch_grid1<D>(plan, s);
+  }
 }
 void launch_dim(const EvalPlan& plan, bool pass2, int D, cudaStream_t s) {
   if (D == 1) launch_dim_d<1>(plan, pass2, s);
@@ -408,6 +450,8 @@ cudaError_t launch_pass_all(const EvalPlan& plan, bool pass2, cudaStream_t strea
 }  // namespace
 
 cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream, const EvalSide* side) {
+  if (plan.n_grid > 0)
+    k_grid_roots<<<dim3(plan.root_chunks, plan.n_lanes), kRootChunk, 0, stream>>>(plan);
   cudaError_t e = launch_pass_all(plan, false, stream, side);
   if (e != cudaSuccess) return e;
   if (plan.n_lanes > 0) {

@@ -21,17 +21,24 @@
 // issue slots and shared-memory reads stop being the limit.
 //
 // Measured against the recurrence kernels it replaced (evaluations with
-// gradient): 256 lanes of d=2 N=1000 M=802 285 -> 186 us, 64 lanes of d=3
-// N=4000 M=5413 2765 -> 1432 us, one lane of d=2 N=20000 M=18000 600 -> 309 us,
-// one of d=1 N=7777 M=3732 109 -> 64 us; forces up to 1.6 times closer to
-// the exact sums. Bound: the FP64 pipe, which the tables share.
+// gradient): 256 lanes of d=2 N=1000 M=802 285 -> 165 us, 64 lanes of d=3
+// N=4000 M=5413 2765 -> 1187 us, one lane of d=2 N=20000 M=18000 600 -> 288 us,
+// one of d=1 N=7777 M=3732 108 -> 56 us; forces up to 2.8 times closer to the
+// exact sums. Bound: the FP64 pipe (DMMA 62% active on the 256 lanes; the two
+// passes' DMMAs alone take 87 us there, a fifth of them on padded cells, and
+// what the table fills, the weight loads (33.2 against 36.8 TFLOP/s in a loop
+// of their own) and a kernel's start and end add comes on top: neither a
+// producer / consumer split of the warps, nor loading items and weights further
+// ahead, nor offsetting the CTAs of an SM made them overlap better).
 //
 // Tiling. Runs are sorted by folded length in strips of 8; a strip's columns
 // are 4-column quads. A slot (quad, lane) is one cell: lane = 4 row + t holds
 // run grid_perm(row) of the strip and column 4 quad + t. Partials and the
 // pass-2 weights are stored slot by slot, which makes both coalesced and is
-// the order the matrix fragments want. Up to 4 strips and 48 columns form a
-// block, whose phase tables a CTA builds together in shared memory.
+// the order the matrix fragments want. Up to 4 strips and 32 columns form a
+// block, whose phase tables a CTA builds together in shared memory: at most 55
+// entries per particle, so that four CTAs with 64 particles' tables share an SM
+// (wider blocks, one or two CTAs per SM, ran N=20000 in 416 instead of 296 us).
 //
 // Bank conflicts. A particle's table entries are contiguous and particles are
 // an odd number of entries apart. Fragment reads then touch 8 distinct 16-byte
@@ -56,66 +63,134 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
-// dst[e] = exp(2 pi i step (m + e) s), e < cnt: FP64 sincospi of the exactly
-// reduced argument at the first entry, products with exp(2 pi i step s) after
-// it. A dead particle (past the tile's end) gets `fillv` instead.
-__device__ __forceinline__ void grid_powers(double2* dst, int m, int cnt, int step, double s,
-                                            bool live, double fillv) {
-  if (!live) {
-    for (int e = 0; e < cnt; ++e) dst[e] = make_double2(fillv, 0.0);
-    return;
-  }
+// Phases that the tables of an evaluation start from. Problems of kGridRootsMin
+// blocks or more, or of more than 8 tiles a block, have a kernel form them once
+// per particle (k_grid_roots): per virtual axis v (prefix 0, prefix 1, columns) the
+// root exp(2 pi i step s) and the seeds exp(2 pi i 16 q step s), q = 1 .., by
+// FP64 sincospi of the exactly reduced argument; word (P.groff[v] + q) N + j of
+// the lane's roots area. Forming them in the passes, once per block, took 350 of
+// 550 FP64 instructions per particle and pass on an 802-row set; with 10 blocks
+// (64 lanes of d=3 N=4000) taking them out cut the passes from 1260 to 1130 us
+// for a 9 us kernel. With few blocks the kernel costs what it saves (one block,
+// 256 lanes of N=1000: passes -8 us, kernel +9 us) and a lone small evaluation
+// one launch more, so there the passes form them.
+template <int D>
+__device__ __forceinline__ void grid_roots(const ProbDev& P, const EvalLane& ln, int w) {
+  const int N = P.N, e = w / N, j = w - e * N;
+  const int v = e >= P.groff[2] ? 2 : e >= P.groff[1] ? 1 : 0;
+  const int q = e - P.groff[v];
+  const double s = ln.s[(size_t)j * D + (v == 2 ? D - 1 : v)];
+  const int step = v == 0 ? P.gstep : 1;
   double sn, cs;
-  sincos_2pi_ms((double)step, s, &sn, &cs);
-  const double2 z = make_double2(cs, sn);
-  double2 p = make_double2(1.0, 0.0);
-  if (m == 1) {
-    p = z;
-  } else if (m != 0) {
-    sincos_2pi_ms((double)((long long)step * m), s, &sn, &cs);
-    p = make_double2(cs, sn);
+  sincos_2pi_ms((double)(q == 0 ? step : 16 * q * step), s, &sn, &cs);
+  ln.roots[w] = make_double2(cs, sn);
+}
+
+// A unit of a block's phase tables: the entries of one virtual axis whose
+// exponents share their multiple of 16. Entry i of the unit is exponent 16 q + i;
+// [i0, i1) are inside the block's window and go to row words off + i.
+struct GridUnit {
+  int v, q, i0, i1, off;
+};
+__device__ __forceinline__ int grid_floor16(int m) { return m >> 4; }
+__device__ __forceinline__ GridUnit grid_unit(const GridBlock& B, int u, int uz, int u0) {
+  int v, m, cnt, first;
+  if (u < uz) {
+    v = 2; m = B.lo; cnt = B.ncol; first = 0;
+  } else if (u < uz + u0) {
+    u -= uz;
+    v = 0; m = B.m0; cnt = B.c0; first = B.ncol;
+  } else {
+    u -= uz + u0;
+    v = 1; m = B.m1; cnt = B.c1; first = B.ncol + B.c0;
   }
-  for (int e = 0; e < cnt; ++e) {
-    dst[e] = p;
-    p = cmul(p, z);
+  GridUnit U;
+  U.v = v;
+  U.q = grid_floor16(m) + u;
+  U.i0 = max(0, m - 16 * U.q);
+  U.i1 = min(16, m + cnt - 16 * U.q);
+  U.off = first + 16 * U.q - m;
+  return U;
+}
+__device__ __forceinline__ int grid_units(int m, int cnt) {
+  return cnt > 0 ? grid_floor16(m + cnt - 1) - grid_floor16(m) + 1 : 0;
+}
+
+// Two units' first phases (exponents 16 q) and roots for particle j.
+template <int D, bool ROOTS>
+__device__ __forceinline__ void grid_seeds(const ProbDev& P, const EvalLane& ln, const GridUnit& A,
+                                           const GridUnit& C, int j, double2& za, double2& a0,
+                                           double2& zc, double2& c0) {
+  a0 = c0 = make_double2(1.0, 0.0);
+  if constexpr (ROOTS) {
+    const double2* ra = ln.roots + (size_t)P.groff[A.v] * P.N + j;
+    const double2* rc = ln.roots + (size_t)P.groff[C.v] * P.N + j;
+    za = ra[0];
+    zc = rc[0];
+    if (A.q != 0) a0 = ra[(size_t)abs(A.q) * P.N];
+    if (C.q != 0) c0 = rc[(size_t)abs(C.q) * P.N];
+    if (A.q < 0) a0.y = -a0.y;
+    if (C.q < 0) c0.y = -c0.y;
+  } else {
+    const double* sj = ln.s + (size_t)j * D;
+    const double sa = sj[A.v == 2 ? D - 1 : A.v], sc = sj[C.v == 2 ? D - 1 : C.v];
+    const int ka = A.v == 0 ? P.gstep : 1, kc = C.v == 0 ? P.gstep : 1;
+    sincos_2pi_ms((double)ka, sa, &za.y, &za.x);
+    sincos_2pi_ms((double)kc, sc, &zc.y, &zc.x);
+    if (A.q != 0 || C.q != 0) {   // warp-uniform
+      sincos_2pi_ms((double)(16 * A.q * ka), sa, &a0.y, &a0.x);
+      sincos_2pi_ms((double)(16 * C.q * kc), sc, &c0.y, &c0.x);
+    }
   }
 }
 
 // Phase tables of a block for TP particles from j0 on: per particle (row of
 // P.gts entries) the columns lo .. lo + ncol - 1, then the prefix windows of
-// axis 0 and (d = 3) axis 1. A unit is up to 16 entries of one table of one
-// particle; a warp's threads share the unit and differ in the particle.
-template <int D, int TP>
+// axis 0 and (d = 3) axis 1. Each unit goes on from its seed by products with
+// the root, even and odd entries apart (at most 8 products of the root's
+// square). A thread forms two units of one particle at a time: four independent
+// chains, since a chain's latency (its operations queue behind other warps'
+// DMMAs) is what a stage waits for. A warp's threads share the units and differ
+// in the particle. Dead particles (past the tile's end) get a zero axis-0
+// prefix and drop out of every product.
+template <int D, bool ROOTS, int TP>
 __device__ __forceinline__ void grid_tables(const ProbDev& P, const GridBlock& B,
-                                            const double* __restrict__ s, int j0, int nj,
-                                            double2* tab) {
-  const int uz = (B.ncol + 15) >> 4, u0 = (B.c0 + 15) >> 4, u1 = D == 3 ? (B.c1 + 15) >> 4 : 0;
-  const int total = (uz + u0 + u1) * TP;
-  for (int w = threadIdx.x; w < total; w += blockDim.x) {
+                                            const EvalLane& ln, int j0, int nj,
+                                            int thread, double2* tab) {
+  const int uz = grid_units(B.lo, B.ncol), u0 = grid_units(B.m0, B.c0);
+  const int units = uz + u0 + (D == 3 ? grid_units(B.m1, B.c1) : 0);
+  const int pairs = (units + 1) >> 1, gts = P.gts;
+  for (int w = thread; w < pairs * TP; w += kGridThreads) {
     const int j = w & (TP - 1), u = w / TP;
     const bool live = j < nj;
-    const double* sj = s + (size_t)(j0 + (live ? j : 0)) * D;
-    double2* row = tab + (size_t)j * P.gts;
-    if (u < uz) {
-      const int L = (B.ncol + uz - 1) / uz, e0 = u * L;
-      grid_powers(row + e0, B.lo + e0, min(L, B.ncol - e0), 1, sj[D - 1], live, 1.0);
-    } else if (u < uz + u0) {
-      const int q = u - uz, L = (B.c0 + u0 - 1) / u0, e0 = q * L;
-      // dead particles drop out of every product through a zero prefix
-      grid_powers(row + B.ncol + e0, B.m0 + e0, min(L, B.c0 - e0), P.gstep, sj[0], live, 0.0);
-    } else if constexpr (D == 3) {
-      const int q = u - uz - u0, L = (B.c1 + u1 - 1) / u1, e0 = q * L;
-      grid_powers(row + B.ncol + B.c0 + e0, B.m1 + e0, min(L, B.c1 - e0), 1, sj[1], live, 1.0);
+    const int jj = j0 + (live ? j : 0);
+    const GridUnit A = grid_unit(B, u, uz, u0);
+    GridUnit C = A;
+    if (u + pairs < units) C = grid_unit(B, u + pairs, uz, u0);
+    else C.i1 = 0;
+    double2 za, zc, a0, c0;
+    grid_seeds<D, ROOTS>(P, ln, A, C, jj, za, a0, zc, c0);
+    if (!live && A.v == 0) a0 = make_double2(0.0, 0.0);
+    if (!live && C.v == 0) c0 = make_double2(0.0, 0.0);
+    double2 a1 = cmul(a0, za), c1 = cmul(c0, zc);
+    za = cmul(za, za);
+    zc = cmul(zc, zc);
+    double2 *da = tab + j * gts + A.off, *dc = tab + j * gts + C.off;
+    const int most = max(A.i1, C.i1);
+    for (int i = 0; i < most; i += 2) {
+      if (i >= A.i0 && i < A.i1) da[i] = a0;
+      if (i + 1 >= A.i0 && i + 1 < A.i1) da[i + 1] = a1;
+      if (i >= C.i0 && i < C.i1) dc[i] = c0;
+      if (i + 1 >= C.i0 && i + 1 < C.i1) dc[i + 1] = c1;
+      a0 = cmul(a0, za);
+      a1 = cmul(a1, za);
+      c0 = cmul(c0, zc);
+      c1 = cmul(c1, zc);
     }
   }
 }
 
-// Table offsets of run `r` of a block (its prefix phase is the product).
-template <int D>
-__device__ __forceinline__ void run_offsets(const GridBlock& B, const GridRun& g, int& o0, int& o1) {
-  o0 = B.ncol + g.n0 - B.m0;
-  o1 = D == 3 ? B.ncol + B.c0 + g.n1 - B.m1 : 0;
-}
+// Prefix phase of a run from its table offsets (one particle's row).
 template <int D>
 __device__ __forceinline__ double2 run_phase(const double2* row, int o0, int o1) {
   const double2 a = row[o0];
@@ -123,67 +198,137 @@ __device__ __forceinline__ double2 run_phase(const double2* row, int o0, int o1)
   return a;
 }
 
-// Pass 1 of one (lane, particle tile, block): a warp owns a strip, 4 DMMAs per
-// 8 columns and 4 particles. NT: column tiles of 8 a warp may hold.
-template <int D, int NT>
-__device__ __forceinline__ void grid_pass1_body(const ProbDev& P, const EvalLane& ln, int tile,
-                                                int blk, int rot, double2* tab) {
-  constexpr int KC = kGridChunk;
-  const GridBlock B = P.gblk[blk];
-  const int jt0 = tile * P.gtile, jt1 = min(P.N, jt0 + P.gtile);
-  const int lane = threadIdx.x & 31, t = lane & 3, pr = grid_perm(lane >> 2);
-  // warps take strips in rotation over the CTAs, so that a block of fewer than
-  // four strips does not leave the same quarter of every SM idle
-  const int sidx = ((threadIdx.x >> 5) + rot) & 3;
-  GridStrip S{};
-  int o0 = 0, o1 = 0;
-  if (sidx < B.nstrip) {
-    S = P.gstrip[B.strip0 + sidx];
-    run_offsets<D>(B, P.grun[S.run0 + min(pr, S.nrun - 1)], o0, o1);
+// CTA barrier that warps may meet in different branches (bar.sync counts
+// arrivals, wherever they come from).
+__device__ __forceinline__ void bar_cta() { asm volatile("bar.sync 0;" ::: "memory"); }
+
+// What a stage's block and item are (loaded once per CTA).
+struct GridStage {
+  double2* buf;   // pass 1: the partials, pass 2: the weights
+  double* g;
+  double gpref;
+  int tile, N, gtile, gts, gslots, ngblk, nstrip, ntile;
+  GridStrip strip[kGridStrips];
+  GridRow row[8 * kGridStrips];
+};
+__device__ __forceinline__ void grid_describe(GridStage& S, const ProbDev& P, const GridBlock& B,
+                                              double2* buf, double* g, int tile) {
+  const int t = threadIdx.x;
+  if (t < 8 * B.nstrip) S.row[t] = P.grow[8 * B.strip0 + t];
+  if (t >= 32 && t < 32 + B.nstrip) S.strip[t - 32] = P.gstrip[B.strip0 + t - 32];
+  if (t == 64) {
+    S.buf = buf;
+    S.g = g;
+    S.gpref = P.gpref;
+    S.tile = tile;
+    S.N = P.N;
+    S.gtile = P.gtile;
+    S.gts = P.gts;
+    S.gslots = P.gslots;
+    S.ngblk = P.ngblk;
+    S.nstrip = B.nstrip;
+    S.ntile = B.ntile;
   }
-  const int nt = (S.nq + 1) >> 1;
-  double p1[NT][2], p2[NT][2], p3[NT][2], p4[NT][2];
+}
+
+// Pass 1 products of one item by a warp that owns the CNT tiles lo .. lo + CNT
+// - 1 of the block: 4 DMMAs per tile and 4 particles. SAME: the tiles are of
+// one strip and share the prefix phase. CNT = 0: the warp only fills.
+template <int D, bool ROOTS, int CNT, bool SAME>
+__device__ __forceinline__ void grid_pass1_item(const ProbDev& P, const GridBlock& B,
+                                                const EvalLane& ln, const GridStage& S, int lo,
+                                                double2* tab) {
+  constexpr int NA = SAME ? 1 : CNT, NC = CNT > 0 ? CNT : 1;
+  const int lane = threadIdx.x & 31, t = lane & 3, pr = grid_perm(lane >> 2);
+  const int jt0 = S.tile * S.gtile, jt1 = min(S.N, jt0 + S.gtile), gts = S.gts;
+  // tile i: run offsets of the lane's row, column, slot (doubled, plus one if
+  // the tile's second quad exists)
+  int o0[NC], o1[NC], col[NC], slot[NC];
+  double p1[NC][2], p2[NC][2], p3[NC][2], p4[NC][2];
+  int at = 0, si = 0, nq = S.strip[0].nq;
 #pragma unroll
-  for (int i = 0; i < NT; ++i)
+  for (int i = 0; i < CNT; ++i) {
+    while (lo + i - at >= ((nq + 1) >> 1)) {
+      at += (nq + 1) >> 1;
+      nq = S.strip[++si].nq;
+    }
+    const int c = lo + i - at;
+    o0[i] = S.row[8 * si + pr].o0;
+    o1[i] = S.row[8 * si + pr].o1;
+    col[i] = 8 * c + pr;
+    slot[i] = 2 * (S.strip[si].slot0 + 64 * c) + (2 * c + 1 < nq ? 1 : 0);
 #pragma unroll
-    for (int c = 0; c < 2; ++c) p1[i][c] = p2[i][c] = p3[i][c] = p4[i][c] = 0.0;
-  for (int j0 = jt0; j0 < jt1; j0 += KC) {
-    __syncthreads();   // the previous chunk's products are done
-    grid_tables<D, KC>(P, B, ln.s, j0, jt1 - j0, tab);
-    __syncthreads();
-    if (nt > 0) {
-      const double2* row = tab + (size_t)t * P.gts;
-      const int dead = min(KC, (jt1 - j0 + 3) & ~3);
-      for (int j = 0; j < dead; j += 4, row += 4 * P.gts) {
-        const double2 a = run_phase<D>(row, o0, o1);
+    for (int h = 0; h < 2; ++h) p1[i][h] = p2[i][h] = p3[i][h] = p4[i][h] = 0.0;
+  }
+  for (int j0 = jt0;;) {
+    if (CNT > 0) {
+      const double2* row = tab + t * gts;
+      const int nj = min(kGridChunk, (jt1 - j0 + 3) & ~3);
+#pragma unroll 2
+      for (int j = 0; j < nj; j += 4, row += 4 * gts) {
+        double2 a[NC], z[NC];
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          if (i < nt) {
-            const double2 z = row[8 * i + pr];
-            dmma(p1[i], a.x, z.x);
-            dmma(p2[i], a.y, z.y);
-            dmma(p3[i], a.x, z.y);
-            dmma(p4[i], a.y, z.x);
-          }
+        for (int i = 0; i < CNT; ++i) z[i] = row[col[i]];
+#pragma unroll
+        for (int i = 0; i < NA; ++i) a[i] = run_phase<D>(row, o0[i], o1[i]);
+#pragma unroll
+        for (int i = 0; i < CNT; ++i) {
+          const double2 ai = a[SAME ? 0 : i];
+          dmma(p1[i], ai.x, z[i].x);
+          dmma(p2[i], ai.y, z[i].y);
+          dmma(p3[i], ai.x, z[i].y);
+          dmma(p4[i], ai.y, z[i].x);
         }
       }
     }
+    j0 += kGridChunk;
+    if (j0 >= jt1) break;
+    bar_cta();
+    grid_tables<D, ROOTS, kGridChunk>(P, B, ln, j0, jt1 - j0, threadIdx.x, tab);
+    bar_cta();
   }
-  if (nt == 0) return;
-  // lane holds the cells (run pr, columns 8 i + t and 8 i + t + 4): one slot of
-  // each of the tile's two quads
-  double2* out = ln.part + 2 * ((size_t)tile * P.gslots + S.slot0 + lane);
+  // lane holds the cells (run pr, columns t and t + 4 of a tile): a slot of each
+  // of the tile's two quads
+  double2* const out = S.buf + 2 * ((size_t)S.tile * S.gslots + lane);
 #pragma unroll
-  for (int i = 0; i < NT; ++i) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int q = 2 * i + c;
-      if (q < S.nq) {
-        out[64 * q] = make_double2(p1[i][c] - p2[i][c], p3[i][c] + p4[i][c]);
-        out[64 * q + 1] = make_double2(p1[i][c] + p2[i][c], p4[i][c] - p3[i][c]);
-      }
+  for (int i = 0; i < CNT; ++i) {
+    double2* o = out + (slot[i] & ~1);
+    o[0] = make_double2(p1[i][0] - p2[i][0], p3[i][0] + p4[i][0]);
+    o[1] = make_double2(p1[i][0] + p2[i][0], p4[i][0] - p3[i][0]);
+    if (slot[i] & 1) {
+      o[64] = make_double2(p1[i][1] - p2[i][1], p3[i][1] + p4[i][1]);
+      o[65] = make_double2(p1[i][1] + p2[i][1], p4[i][1] - p3[i][1]);
     }
   }
+}
+
+// Pass 1 of one item (lane, tile, block): the block's 8 x 8-cell tiles in strip
+// order are cut into four equal ranges, one per warp (at most NT tiles), so
+// that uneven strips do not leave warps idle.
+template <int D, bool ROOTS, int NT>
+__device__ __forceinline__ void grid_pass1(const ProbDev& P, const EvalLane& ln, int tile, int blk,
+                                           GridStage& S, double2* tab) {
+  const GridBlock B = P.gblk[blk];
+  const int jt0 = tile * P.gtile;
+  grid_describe(S, P, B, ln.part, nullptr, tile);
+  grid_tables<D, ROOTS, kGridChunk>(P, B, ln, jt0, min(P.N - jt0, P.gtile), threadIdx.x, tab);
+  bar_cta();
+  const int warp = threadIdx.x >> 5;
+  const int lo = B.ntile * warp >> 2, hi = B.ntile * (warp + 1) >> 2;
+  int at = 0, si = 0;   // the strip of tile lo: whether tile hi - 1 is of it
+  while (lo >= at + ((S.strip[si].nq + 1) >> 1)) at += (S.strip[si++].nq + 1) >> 1;
+  const bool same = hi <= at + ((S.strip[si].nq + 1) >> 1);
+#define CCO_GRID_CASE(CNT)                                                                     \
+  if (CNT <= NT && hi - lo == CNT) {                                                           \
+    if (same) grid_pass1_item<D, ROOTS, CNT <= NT ? CNT : 0, true>(P, B, ln, S, lo, tab);      \
+    else grid_pass1_item<D, ROOTS, CNT <= NT ? CNT : 0, false>(P, B, ln, S, lo, tab);          \
+  }
+  CCO_GRID_CASE(0)
+  CCO_GRID_CASE(1)
+  CCO_GRID_CASE(2)
+  CCO_GRID_CASE(3)
+#undef CCO_GRID_CASE
+  bar_cta();   // the tables and the description are free again
 }
 
 // Reduction of one slot: rho of its two k-set rows summed over the tiles in
@@ -268,100 +413,115 @@ __device__ __forceinline__ double grid_reduce_slot(const ProbDev& P, const EvalL
   return e;
 }
 
-// Pass 2 of one (lane, 64-particle tile): a warp owns 16 particles (two
-// fragment columns of 8) and walks every strip of every block: per quad and
-// 8 particles 8 DMMAs (4 in 1-D) from 4 (2) coalesced 16-byte weight loads and
-// one table read, then the strip's rows are weighted by their prefix phases.
-template <int D>
-__device__ __forceinline__ void grid_pass2_body(const ProbDev& P, const EvalLane& ln, int tile,
-                                                double2* tab) {
-  constexpr int TP = kGridTile2, NW = D == 1 ? 2 : 4, NP = 2;
-  const int j0 = tile * TP, nj = min(TP, P.N - j0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
-  const int pr = grid_perm(lane >> 2);
-  double G[NP][2][D];
+// Sum over a strip's rows (lanes 4 apart) of 8 values: halves are exchanged and
+// added three times, so row r ends with the total of value r (7 shuffles where
+// summing every value everywhere takes 24).
+__device__ __forceinline__ double grid_row_sum(const double (&v)[8], int row) {
+  double a[4], b[2];
 #pragma unroll
-  for (int p = 0; p < NP; ++p)
+  for (int i = 0; i < 4; ++i) {
+    const bool up = row & 4;
+    const double mine = up ? v[i + 4] : v[i], other = up ? v[i] : v[i + 4];
+    a[i] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
+  }
 #pragma unroll
-    for (int c = 0; c < 2; ++c)
+  for (int i = 0; i < 2; ++i) {
+    const bool up = row & 2;
+    const double mine = up ? a[i + 2] : a[i], other = up ? a[i] : a[i + 2];
+    b[i] = mine + __shfl_xor_sync(0xffffffffu, other, 8);
+  }
+  const bool up = row & 1;
+  const double mine = up ? b[1] : b[0], other = up ? b[0] : b[1];
+  return mine + __shfl_xor_sync(0xffffffffu, other, 4);
+}
+
+// Pass 2 of one item (lane, 64-particle tile): a warp owns 16 particles (two
+// fragment columns of 8) and walks every strip of every block: per quad and 8
+// particles 8 DMMAs (4 in 1-D) from 4 (2) coalesced 16-byte weight loads, one
+// quad ahead, and one table read; then the strip's rows are weighted by their
+// prefix phases. The weights of all quads are one stream.
+template <int D, bool ROOTS>
+__device__ __forceinline__ void grid_pass2(const ProbDev& P, const EvalLane& ln, int tile,
+                                           GridStage& S, double2* tab) {
+  constexpr int NW = D == 1 ? 2 : 4, NP = 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3, r8 = lane >> 2;
+  const int pr = grid_perm(r8);
+  const int j0 = tile * kGridTile2, nj = min(kGridTile2, P.N - j0), gts = P.gts, nb = P.ngblk;
+  const double2* __restrict__ wq = ln.rhow + lane;
+  const double2* const wlast = wq + (size_t)((P.gslots >> 5) - 1) * (32 * NW);
+  double2 w[NW];
 #pragma unroll
-      for (int x = 0; x < D; ++x) G[p][c][x] = 0.0;
-  const double2* wtab = tab + (size_t)(warp * 16) * P.gts;
-  for (int b = 0; b < P.ngblk; ++b) {
+  for (int x = 0; x < NW; ++x) w[x] = wq[32 * x];
+  if (wq < wlast) wq += 32 * NW;
+  double G[D][NP][2];
+#pragma unroll
+  for (int x = 0; x < D; ++x)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) G[x][p][0] = G[x][p][1] = 0.0;
+  const double2* wtab = tab + warp * 16 * gts;
+  for (int b = 0; b < nb; ++b) {
     const GridBlock B = P.gblk[b];
-    __syncthreads();
-    grid_tables<D, TP>(P, B, ln.s, j0, nj, tab);
+    grid_describe(S, P, B, nullptr, nullptr, tile);
+    grid_tables<D, ROOTS, kGridTile2>(P, B, ln, j0, nj, threadIdx.x, tab);
     __syncthreads();
     for (int si = 0; si < B.nstrip; ++si) {
-      const GridStrip S = P.gstrip[B.strip0 + si];
+      const int nq = S.strip[si].nq;
+      const GridRow R = S.row[8 * si + pr];
       double acc[NW][NP][2];
 #pragma unroll
-      for (int w = 0; w < NW; ++w)
+      for (int x = 0; x < NW; ++x)
 #pragma unroll
-        for (int p = 0; p < NP; ++p) acc[w][p][0] = acc[w][p][1] = 0.0;
-      const double2* __restrict__ wq = ln.rhow + (size_t)(S.slot0 >> 5) * (32 * NW) + lane;
-      const double2* zr = wtab + (size_t)pr * P.gts + t;
-      double2 w[NW];
+        for (int p = 0; p < NP; ++p) acc[x][p][0] = acc[x][p][1] = 0.0;
+      const double2* zr = wtab + pr * gts + t;
+      for (int q = 0; q < nq; ++q, zr += 4) {
+        double2 wn[NW], z[NP];
 #pragma unroll
-      for (int x = 0; x < NW; ++x) w[x] = wq[32 * x];
-      for (int q = 0; q < S.nq; ++q) {
-        double2 wn[NW];
-        wq += 32 * NW;
-        if (q + 1 < S.nq) {
+        for (int p = 0; p < NP; ++p) z[p] = zr[8 * p * gts];
 #pragma unroll
-          for (int x = 0; x < NW; ++x) wn[x] = wq[32 * x];
-        }
+        for (int x = 0; x < NW; ++x) wn[x] = wq[32 * x];   // past the end: the last quad again
+        if (wq < wlast) wq += 32 * NW;
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const double2 z = zr[(size_t)(8 * p) * P.gts + 4 * q];
+        for (int p = 0; p < NP; ++p)
 #pragma unroll
-          for (int x = 0; x < NW; ++x) dmma(acc[x][p], w[x].x, z.x);
+          for (int x = 0; x < NW; ++x) dmma(acc[x][p], w[x].x, z[p].x);
 #pragma unroll
-          for (int x = 0; x < NW; ++x) dmma(acc[x][p], w[x].y, z.y);
-        }
+        for (int p = 0; p < NP; ++p)
+#pragma unroll
+          for (int x = 0; x < NW; ++x) dmma(acc[x][p], w[x].y, z[p].y);
 #pragma unroll
         for (int x = 0; x < NW; ++x) w[x] = wn[x];
       }
       // lane holds T, T' of run pr for particles t and t + 4 of each eight
-      const GridRun g = P.grun[S.run0 + min(pr, S.nrun - 1)];
-      int o0, o1;
-      run_offsets<D>(B, g, o0, o1);
 #pragma unroll
       for (int p = 0; p < NP; ++p)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          const double2 a = run_phase<D>(wtab + (size_t)(8 * p + 4 * c + t) * P.gts, o0, o1);
+          const double2 a = run_phase<D>(wtab + (8 * p + 4 * c + t) * gts, R.o0, R.o1);
           const double h = a.x * acc[1][p][c] + a.y * acc[0][p][c];
           if (D == 1) {
-            G[p][c][0] += h;
+            G[0][p][c] += h;
           } else {
-            G[p][c][0] += (double)g.n0 * h;
-            if (D == 3) G[p][c][1] += (double)g.n1 * h;
-            G[p][c][D - 1] += a.x * acc[3][p][c] + a.y * acc[2][p][c];
+            G[0][p][c] += (double)R.n0 * h;
+            if (D == 3) G[1][p][c] += (double)R.n1 * h;
+            G[D - 1][p][c] += a.x * acc[3][p][c] + a.y * acc[2][p][c];
           }
         }
     }
+    __syncthreads();   // the tables and the description are free again
   }
-  // sum over the strip rows (lanes 4 apart); lanes 0..3 hold the particles
+  // value 4 x + 2 p + c of the row sums is axis x of particle 8 p + 4 c + t
 #pragma unroll
-  for (int p = 0; p < NP; ++p)
+  for (int h = 0; h < D; h += 2) {
+    double v[8];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-#pragma unroll
-      for (int x = 0; x < D; ++x) {
-        double v = G[p][c][x];
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        G[p][c][x] = v;
-      }
-      const int j = warp * 16 + 8 * p + 4 * c + t;
-      if (lane < 4 && j < nj) {
-        double* gj = ln.g + (size_t)(j0 + j) * D;
-#pragma unroll
-        for (int x = 0; x < D; ++x) gj[x] = P.gpref * G[p][c][x];
-      }
+    for (int i = 0; i < 8; ++i) {
+      const int x = h + (i >> 2);
+      v[i] = x < D ? G[x < D ? x : 0][(i >> 1) & 1][i & 1] : 0.0;
     }
+    const double tot = grid_row_sum(v, r8);
+    const int x = h + (r8 >> 2), j = warp * 16 + 8 * ((r8 >> 1) & 1) + 4 * (r8 & 1) + t;
+    if (x < D && j < nj) ln.g[(size_t)(j0 + j) * D + x] = P.gpref * tot;
+  }
 }
 
 }  // namespace

@@ -29,6 +29,7 @@ struct cco_problem {
   cco::GridBlock* gblk = nullptr;
   cco::GridStrip* gstrip = nullptr;
   cco::GridQuad* gquad = nullptr;
+  cco::GridRow* grow = nullptr;
   double4* krow = nullptr;     // run-order rows (n_0, n_1, n_2, w) for the Hessian kernels
   size_t smem1 = 0, smem2 = 0, smemG = 0, smemH = 0;
   int dense_blocks = 0;        // cco_problem_pass1_form
@@ -149,6 +150,7 @@ inline EvalLane eval_lane(const RecordShape& R, const LaneRef& L, const cco_prob
   e.rho = dens;
   e.rhow = dens + p->M;
   e.part = e.rhow + eval_rhow_words(p->host);
+  e.roots = e.part + eval_part_words(p->host);
   e.status = rec_status(L.rec);
   e.prob = prob_index;
   return e;
@@ -180,10 +182,10 @@ struct EvalSet {
     std::vector<const cco_problem*> uniq;
     std::vector<ProbDev> pv;
     std::vector<EvalLane> lv;
-    std::vector<EvalItem> g1[3], g2[3], gH[3];   // items grouped by d
-    std::vector<EvalItem> gG[3][kGridClasses];   // grid pass-1 items by d and column class
+    std::vector<EvalItem> g1[3], g2[3];   // items grouped by d
+    std::vector<EvalItem> gG[3][kGridClasses], gH[3][2];   // grid items by d and class
     size_t smem1 = 0, smem2 = 0, smem2f = 0, smemG = 0, smemH = 0;
-    int max_d = 1, chunks_red = 1;
+    int max_d = 1, chunks_red = 1, chunks_root = 0, n_grid = 0;
     for (int i = lo; i < hi; ++i) {
       const cco_problem* p = probs_of[i];
       const ProbDev& h = p->host;
@@ -204,9 +206,11 @@ struct EvalSet {
       const int j = i - lo;
       lv.push_back(eval_lane(R, refs[i], p, u));
       if (h.grid) {
+        n_grid += h.groots > 0;
+        chunks_root = std::max(chunks_root, (h.groots * h.N + kRootChunk - 1) / kRootChunk);
         const int ntG = h.gntile * h.ngblk, ntH = (h.N + kGridTile2 - 1) / kGridTile2;
         for (int t = 0; t < ntG; ++t) gG[p->d - 1][h.gcls].push_back(EvalItem{j, t});
-        for (int t = 0; t < ntH; ++t) gH[p->d - 1].push_back(EvalItem{j, t});
+        for (int t = 0; t < ntH; ++t) gH[p->d - 1][h.gcls > 0].push_back(EvalItem{j, t});
       }
       if (!h.grid || may_fp32) {
         const int C = pass1_chunks(h, chunks);
@@ -216,19 +220,22 @@ struct EvalSet {
       }
     }
     std::vector<EvalItem> i1, i2, iG, iH;
-    plan.d_off1[0] = plan.d_off2[0] = plan.d_offH[0] = 0;
+    plan.d_off1[0] = plan.d_off2[0] = 0;
     for (int D = 0; D < 3; ++D) {
       i1.insert(i1.end(), g1[D].begin(), g1[D].end());
       i2.insert(i2.end(), g2[D].begin(), g2[D].end());
-      iH.insert(iH.end(), gH[D].begin(), gH[D].end());
       for (int c = 0; c < kGridClasses; ++c) {
         plan.q_offG[D][c] = (int)iG.size();
         iG.insert(iG.end(), gG[D][c].begin(), gG[D][c].end());
       }
       plan.q_offG[D][kGridClasses] = (int)iG.size();
+      for (int c = 0; c < 2; ++c) {
+        plan.h_off[D][c] = (int)iH.size();
+        iH.insert(iH.end(), gH[D][c].begin(), gH[D][c].end());
+      }
+      plan.h_off[D][2] = (int)iH.size();
       plan.d_off1[D + 1] = (int)i1.size();
       plan.d_off2[D + 1] = (int)i2.size();
-      plan.d_offH[D + 1] = (int)iH.size();
     }
     plan.dyn_prec = may_fp32 ? 1 : 0;
     cudaError_t e = upload(&probs, pv, st);
@@ -245,6 +252,8 @@ struct EvalSet {
     plan.itemsH = itH;
     plan.smemG = smemG;
     plan.smemH = smemH;
+    plan.n_grid = n_grid;
+    plan.root_chunks = chunks_root;
     plan.n_lanes = hi - lo;
     plan.n_items1 = (int)i1.size();
     plan.n_items2 = (int)i2.size();

@@ -49,13 +49,17 @@ static_assert(sizeof(SegHdr) == 32, "segment header is two 16-byte loads");
 // quads of 4 columns from its block's lo on; a block is up to 4 strips and
 // kGridCols columns whose phase tables a CTA builds together. A slot is one
 // (quad, lane) cell; slots are numbered strip by strip, quad by quad.
-constexpr int kGridCols = 48;      // columns of a block
-constexpr int kGridStrips = 4;     // strips of a block (one per warp in pass 1)
-constexpr int kGridChunk = 32;     // particles whose tables pass 1 holds at a time
+constexpr int kGridStrips = 4;     // strips of a block
+constexpr int kGridChunk = 64;     // particles of a pass-1 stage
 constexpr int kGridTile2 = 64;     // particles of a pass-2 CTA
 constexpr int kGridThreads = 128;
-constexpr int kGridMaxEntries = 200;   // table entries per particle (64 particles: 200 KB)
-constexpr int kGridClasses = 2;    // pass-1 kernels: blocks of <= 24 and <= 48 columns
+constexpr int kGridCtas = 4;       // CTAs per SM (registers and shared memory)
+constexpr int kGridMaxEntries = 55;   // table entries per particle: 64 particles, four CTAs per SM
+constexpr int kGridRootsMin = 4;  // blocks from which a kernel forms the phase roots
+// pass-1 kernels by tiles of 8 x 8 cells per warp and where the roots come from:
+// <= 2 (formed in the passes), <= 2, <= 3 (from the roots kernel)
+constexpr int kGridClasses = 3;
+constexpr int kGridMaxTiles = 12;  // tiles of a block
 struct GridRun {
   int n0, n1, a, b, kstart, pad_;   // prefix (1-D: n0 = q), last-axis range [a, b]
 };
@@ -65,6 +69,10 @@ struct GridStrip {
 struct GridBlock {
   int strip0, nstrip, lo, ncol;      // columns lo .. lo + ncol - 1 (ncol a multiple of 8)
   int m0, c0, m1, c1;                // prefix windows [m, m + c) of its runs, per axis
+  int ntile, pad_[3];                // its 8 x 8-cell tiles
+};
+struct GridRow {                     // run r of strip i at 8 i + r: table offsets, prefix
+  int o0, o1, n0, n1;
 };
 struct GridQuad {
   int run0, nrun, c0, pad_;          // the strip's runs, the quad's first column
@@ -88,9 +96,10 @@ struct ProbDev {
   int ntile1, ntile2;        // particle tiles of pass 1 / pass 2 (pass 2 at split 1)
   int sl2;                   // logical slices of the pass-2 segment pairs (power of 2, <= 8)
   int grid;                  // 1: FP64 lanes run the tensor-core form below
-  int ngblk, gcls;           // its blocks; pass-1 kernel class (0: <= 24 columns)
+  int ngblk, gcls;           // its blocks; pass-1 kernel class
   int gts;                   // table entries per particle (odd)
   int gstep;                 // 1-D: prefix exponents are gstep n0 (1 otherwise)
+  int groff[3], groots;      // roots area: first word / N of each virtual axis, words / N (0: none)
   int gslots;                // slots (a multiple of 32)
   int gtile, gntile;         // particles per pass-1 tile, tiles
   int grhow;                 // double2 words of the rhow area (chunk energies after the weights)
@@ -98,6 +107,7 @@ struct ProbDev {
   const GridStrip* gstrip;
   const GridRun* grun;
   const GridQuad* gquad;
+  const GridRow* grow;
   double vol;                // V
   double gpref;              // 2 (2 pi) / V
   const SegHdr* seg1;
@@ -114,6 +124,7 @@ struct EvalLane {
   double2* rho;           // [M] run order
   double2* rhow;          // pass-2 input: [M] weighted density, or the grid form's weights
   double2* part;          // [ntile1][M], or [gntile][gslots][2] (grid form)
+  double2* roots;         // [groots][N] phase roots and seeds (grid form)
   const int64_t* status;  // evaluate iff null or *status == RUNNING
   const int32_t* prec;    // arithmetic of this evaluation: *prec, or `fixed_prec` when null
   int prob;
@@ -209,8 +220,9 @@ struct EvalPlan {
   const EvalItem* itemsG;
   const EvalItem* itemsH;
   int q_offG[3][kGridClasses + 1];
-  int d_offH[4];
-  size_t smemG, smemH;
+  int h_off[3][3];          // pass-2 items likewise: roots formed in the pass, from the kernel
+  int n_grid, root_chunks; // lanes with roots; chunks of their roots (largest)
+  size_t smemG, smemH;     // dynamic shared memory
   int dyn_prec;             // 1: lanes may be FP32 (the FP32 pass kernels launch too), 0: FP64 only
   int max_d;                // largest d in the plan (template dispatch)
   int red_chunks;           // chunks of the reduction (reduce_chunks, largest in the plan)
@@ -238,12 +250,14 @@ __host__ __device__ __forceinline__ int pass1_chunks(const ProbDev& p, int plan_
 // The reduction of the pass-1 partials runs one block per kReduceChunk
 // k-vectors of a lane; a second kernel sums the chunks' energies in a fixed
 // order, so the energy's rounding depends on M alone.
+constexpr int kRootChunk = 256;   // roots per block of the roots kernel
 constexpr int kReduceChunk = 256;
 __host__ __device__ __forceinline__ int reduce_chunks(int M) {
   return (M + kReduceChunk - 1) / kReduceChunk;
 }
 // Scratch of one evaluated configuration, in double2 words: rho [M], the rhow
-// area, the pass-1 partials (the larger of the forms the problem may run).
+// area, the pass-1 partials (the larger of the forms the problem may run) and
+// the grid form's roots.
 __host__ __device__ __forceinline__ size_t eval_rhow_words(const ProbDev& p) {
   const size_t m = (size_t)p.M, g = p.grid ? (size_t)p.grhow : 0;
   return m > g ? m : g;
@@ -253,8 +267,11 @@ __host__ __device__ __forceinline__ size_t eval_part_words(const ProbDev& p) {
   const size_t g = p.grid ? 2 * (size_t)p.gntile * p.gslots : 0;
   return seg > g ? seg : g;
 }
+__host__ __device__ __forceinline__ size_t eval_roots_words(const ProbDev& p) {
+  return p.grid ? (size_t)p.groots * p.N : 0;
+}
 __host__ __device__ __forceinline__ size_t eval_scratch_words(const ProbDev& p) {
-  return (size_t)p.M + eval_rhow_words(p) + eval_part_words(p);
+  return (size_t)p.M + eval_rhow_words(p) + eval_part_words(p) + eval_roots_words(p);
 }
 
 // Side streams of one launching stream: when a plan holds lanes of several
@@ -273,12 +290,14 @@ cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream,
 // when there is no pass 2).
 inline int eval_kernels(const EvalPlan& p) {
   int n = p.n_lanes > 0 ? (p.want_grad ? 1 : 2) : 0;   // reduce (+ energy without pass 2)
+  n += p.n_grid > 0;                                   // roots
   const int per = p.dyn_prec ? 2 : 1;   // FP64 and FP32 pass kernels
   for (int D = 1; D <= 3; ++D) {
     n += per * (p.d_off1[D] > p.d_off1[D - 1]);
     for (int c = 0; c < kGridClasses; ++c) n += p.q_offG[D - 1][c + 1] > p.q_offG[D - 1][c];
     if (p.want_grad)
-      n += per * (p.d_off2[D] > p.d_off2[D - 1]) + (p.d_offH[D] > p.d_offH[D - 1]);
+      n += per * (p.d_off2[D] > p.d_off2[D - 1]) + (p.h_off[D - 1][1] > p.h_off[D - 1][0]) +
+           (p.h_off[D - 1][2] > p.h_off[D - 1][1]);
   }
   return n;
 }
@@ -286,7 +305,7 @@ inline int eval_kernels(const EvalPlan& p) {
 // Whether a plan launches pass kernels of dimension D.
 inline bool eval_has_dim(const EvalPlan& p, int D) {
   return p.d_off1[D] > p.d_off1[D - 1] || p.q_offG[D - 1][kGridClasses] > p.q_offG[D - 1][0] ||
-         p.d_off2[D] > p.d_off2[D - 1] || p.d_offH[D] > p.d_offH[D - 1];
+         p.d_off2[D] > p.d_off2[D - 1] || p.h_off[D - 1][2] > p.h_off[D - 1][0];
 }
 // Dimensions whose pass kernels a plan launches (side streams pay off from 2).
 inline int eval_dims(const EvalPlan& p) {
