@@ -99,3 +99,40 @@ def test_noalloc_batch_larger_than_the_scratch_in_grid_layout():
     assert code == _native.CCO_OK, _native.load().cco_last_error()
     p_ref, g_ref, _, _ = en.evaluate(s)
     assert torch.equal(phi, p_ref) and torch.equal(g, g_ref)
+
+
+@pytest.mark.parametrize("d,n,b,dirs,top", [(2, 65, 2, 5.3, 130), (2, 300, 1, 9.1, 700), (3, 129, 2, 3.2, 90),
+                                            (2, 1, 1, 5.3, 60)])  # fmt: skip
+def test_line_grid_density_vs_direct_sums(monkeypatch, d, n, b, dirs, top):
+    """K-sets of multiples of primitive vectors (the structure factor's): rows with
+    gaps, lines through both half spaces, uneven weights; density, energy and the
+    gradient (whose pass keeps the recurrences) in both forms."""
+    r = int(dirs) + 1
+    g = np.stack(np.meshgrid(*([np.arange(-r, r + 1)] * d), indexing="ij"), axis=-1).reshape(-1, d)
+    g = g[(np.gcd.reduce(np.abs(g), axis=1) == 1) & ((g * g).sum(1) < dirs**2)]
+    first = np.array([x[np.flatnonzero(x)[0]] for x in g])
+    g = g[first > 0]
+    rows = [i * v for v in g for i in range(1, int(top / np.sqrt(v @ v)) + 1) if i % 13 != 5]
+    rows += [-3 * v for v in g[::2]]
+    nv = np.array(rows, dtype=np.int64)
+    rng = np.random.default_rng(n)
+    w = rng.uniform(0.1, 1.0, size=len(nv))
+    s = rng.uniform(size=(b, n, d))
+    out = {}
+    for form in ("lines", "recurrence"):
+        if form == "recurrence":
+            monkeypatch.setenv("CCO_PASS1_GEMM", "0")
+        en = StealthyEnergy(nv.astype(np.float64), w, np.float64(2.0 * n))
+        out[form] = en.evaluate(s, want_rho=True)
+        out[form + " density"] = en.evaluate(s, want_grad=False, want_rho=True)
+    e_ref, g_ref = oracle.energy_grad_accurate(s, nv, w, 2.0 * n)
+    hi = np.round(s * 2.0**26) / 2.0**26   # n hi exact: its whole part leaves before rounding
+    for i in range(b):
+        t = nv @ hi[i].T
+        theta = 2.0 * np.pi * ((t - np.round(t)) + nv @ (s[i] - hi[i]).T)
+        for form, (phi, grad, re, im) in out.items():
+            np.testing.assert_allclose(phi[i], e_ref[i], rtol=RTOL_KERNEL_E, atol=0, err_msg=form)
+            np.testing.assert_allclose(re[i], np.cos(theta).sum(1), rtol=0, atol=1e-13 * n, err_msg=form)
+            np.testing.assert_allclose(im[i], np.sin(theta).sum(1), rtol=0, atol=1e-13 * n, err_msg=form)
+            if grad is not None and n > 1:
+                np.testing.assert_allclose(grad[i], g_ref[i], rtol=0, atol=RTOL_KERNEL_F * np.abs(g_ref[i]).max())

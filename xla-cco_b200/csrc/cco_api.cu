@@ -1,11 +1,14 @@
 // C ABI of libcco: problems, evaluation and the batched relax drivers.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -179,6 +182,8 @@ struct GridPlan {
   std::vector<GridBlock> blocks;
   std::vector<GridQuad> quads;
   std::vector<GridRow> rows;
+  std::vector<GridLine> lines;   // line grids
+  std::vector<int2> slotk;
   int entries = 0;   // widest block's table entries
   int tiles = 0;     // most 8 x 8-cell tiles of a block
 };
@@ -272,6 +277,119 @@ std::vector<GridRun> split_runs_1d(const std::vector<GridRun>& runs, int C) {
 // FMAs per grid cell and particle (4 density, 8 gradient) plus the tables,
 // where the recurrences need 14 or more instructions per k-set row: it is taken
 // when the slots (cells with their padding) are at most twice the rows.
+void grid_sizes(ProbDev* P, const GridPlan& gp);
+// A line grid: `rows` holds the k-set in run order (M x d). Rows are multiples
+// i v of primitive vectors v; a line's multiples are cut into strips of 8 rows
+// i = q step + c, |c| < 4 nq, step = 8 nq - 1, with the nq (at most 4) that
+// costs least; as many strips share a block as its table holds. Only pass 1
+// takes this form (the structure factor's k-set: every multiple up to a large
+// cut-off along each of ~600 directions, runs of one row for the recurrences:
+// 16 densities of N = 1000 on 96 660 rows 11.3 ms, on lines 0.63 ms; two thirds
+// of that is forming tables, three sincospi and 24 products per strip and
+// particle against 512 FMAs of a full strip).
+void plan_lines(const std::vector<int>& rows, ProbDev* P, GridPlan* gp) {
+  const int d = P->d, m = P->M;
+  if (d < 2) return;
+  std::map<std::array<int, 3>, std::vector<std::pair<int, int>>> lines;   // v -> (i, row)
+  for (int k = 0; k < m; ++k) {
+    std::array<int, 3> v{0, 0, 0};
+    int g = 0, sign = 0;
+    for (int a = 0; a < d; ++a) {
+      v[a] = rows[(size_t)k * d + a];
+      g = std::gcd(g, std::abs(v[a]));
+      if (sign == 0) sign = (v[a] > 0) - (v[a] < 0);
+    }
+    for (int a = 0; a < d; ++a) v[a] /= g * sign;
+    lines[v].push_back({g * sign, k});
+  }
+  if ((long long)lines.size() * 16 > m) return;   // short lines: mostly padding
+  struct Strip {
+    GridLine line;
+    int nq;
+    std::vector<int2> k;   // per slot
+  };
+  std::vector<Strip> strips;
+  auto fdiv = [](int x, int y) { return x >= 0 ? x / y : -((-x + y - 1) / y); };
+  for (auto& [v, ms] : lines) {
+    int lo = ms[0].first, hi = lo;
+    for (const auto& e : ms) {
+      lo = std::min(lo, e.first);
+      hi = std::max(hi, e.first);
+    }
+    int nq = 1, best = 0;
+    for (int t = 1; t <= 4; ++t) {
+      const int S = 8 * t - 1, C = 4 * t - 1;
+      const int ns = (fdiv(hi + C, S) - fdiv(lo + C, S)) / 8 + 1;
+      const int cost = ns * (128 * t + 250);   // DMMA work and tables per particle
+      if (t == 1 || cost < best) {
+        best = cost;
+        nq = t;
+      }
+    }
+    const int S = 8 * nq - 1, C = 4 * nq - 1, q_lo = fdiv(lo + C, S);
+    const int ns = (fdiv(hi + C, S) - q_lo) / 8 + 1;
+    const size_t first = strips.size();
+    for (int s = 0; s < ns; ++s)
+      strips.push_back(Strip{GridLine{{v[0], v[1], v[2]}, S, q_lo + 8 * s, (nq + 1) / 2 * 8}, nq,
+                             std::vector<int2>(32 * nq, make_int2(-1, -1))});
+    for (const auto& [i, k] : ms) {
+      const int q = fdiv(i + C, S), c = i - q * S, ac = std::abs(c);
+      Strip& T = strips[first + (q - q_lo) / 8];
+      const int r = (q - q_lo) % 8, row = r < 4 ? 2 * r : 2 * (r - 4) + 1;   // grid_perm(row) = r
+      int2& e = T.k[32 * (ac / 4) + 4 * row + ac % 4];
+      (c >= 0 ? e.x : e.y) = k;
+    }
+  }
+  std::stable_sort(strips.begin(), strips.end(),
+                   [](const Strip& x, const Strip& y) { return x.nq > y.nq; });
+  GridPlan out;
+  for (const Strip& T : strips) {
+    const int entries = T.line.ncol + 8;
+    GridBlock* b = out.blocks.empty() ? nullptr : &out.blocks.back();
+    const int used = b ? b->ncol : 0;   // table entries so far
+    if (!b || used + entries > kGridMaxEntries || b->nstrip == kGridStrips || b->ntile + (T.nq + 1) / 2 > 4) {
+      out.blocks.push_back(GridBlock{});
+      b = &out.blocks.back();
+      b->strip0 = (int)out.strips.size();
+    }
+    GridStrip g{};
+    g.nrun = 8;
+    g.nq = T.nq;
+    g.slot0 = (int)out.slotk.size();
+    g.col0 = b->ncol;
+    for (int r = 0; r < 8; ++r) out.rows.push_back(GridRow{g.col0 + T.line.ncol + r, 0, 0, 0});
+    out.strips.push_back(g);
+    out.lines.push_back(T.line);
+    out.slotk.insert(out.slotk.end(), T.k.begin(), T.k.end());
+    b->nstrip += 1;
+    b->ntile += (T.nq + 1) / 2;
+    b->ncol += entries;
+    out.entries = std::max(out.entries, b->ncol);
+  }
+  if ((long long)out.slotk.size() > 2ll * m) return;
+  *gp = out;
+  P->grid = 2;
+  P->gcls = kGridLines;
+  P->gstep = 1;
+  P->gslots = (int)out.slotk.size();
+  P->grhow = m + (reduce_chunks(P->gslots) + 1) / 2;
+  P->gtile = P->N <= 64 ? 64 : P->N <= 128 ? 128 : 256;   // many blocks: few, large tiles
+  grid_sizes(P, out);
+}
+
+// Tile counts and table stride, and the check that the form fits the fixed
+// scratch of cco_energy_grad_noalloc wherever the recurrence form does.
+void grid_sizes(ProbDev* P, const GridPlan& gp) {
+  P->ngblk = (int)gp.blocks.size();
+  P->gts = gp.entries | 1;
+  P->gntile = (P->N + P->gtile - 1) / P->gtile;
+  const size_t seg = 2 * (size_t)P->M + (size_t)P->ntile1 * P->M;
+  const size_t own = (size_t)P->M + P->grhow + 2 * (size_t)P->gntile * P->gslots + eval_roots_words(*P);
+  if (sizeof(double2) * own > CCO_NOALLOC_SCRATCH_BYTES - 65536 &&
+      sizeof(double2) * seg <= CCO_NOALLOC_SCRATCH_BYTES)
+    P->grid = 0;
+}
+
 void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
   if (runs.empty()) return;
   // the layout that costs least per particle: products and table entries (both
@@ -303,13 +421,11 @@ void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
   P->grid = 1;
   P->ngblk = (int)gp->blocks.size();
   P->gcls = gp->tiles > 8 ? 2 : P->ngblk >= kGridRootsMin ? 1 : 0;
-  P->gts = gp->entries | 1;
   P->gstep = step;
   P->gslots = (int)slots;
   // larger pass-1 tiles for larger N keep the partials (32 bytes per slot and
   // tile) and the reduction small once there are enough tiles to fill the GPU
   P->gtile = P->N <= 512 ? 64 : P->N <= 8192 ? 128 : 256;
-  P->gntile = (P->N + P->gtile - 1) / P->gtile;
   P->grhow = (int)slots * (P->d == 1 ? 2 : 4) + (reduce_chunks((int)slots) + 1) / 2;
   // seeds per virtual axis: multiples of 16 up to the largest |exponent| used
   // (the columns of a block's last tile included)
@@ -323,12 +439,7 @@ void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
   P->groff[1] = 1 + top[0] / 16;
   P->groff[2] = P->groff[1] + (P->d == 3 ? 1 + top[1] / 16 : 0);
   P->groots = P->gcls > 0 ? P->groff[2] + 1 + top[2] / 16 : 0;
-  // cco_energy_grad_noalloc must go on taking what it took
-  const size_t seg = 2 * (size_t)P->M + (size_t)P->ntile1 * P->M;
-  const size_t own = (size_t)P->M + P->grhow + 2 * (size_t)P->gntile * P->gslots + eval_roots_words(*P);
-  if (sizeof(double2) * own > CCO_NOALLOC_SCRATCH_BYTES - 65536 &&
-      sizeof(double2) * seg <= CCO_NOALLOC_SCRATCH_BYTES)
-    P->grid = 0;
+  grid_sizes(P, *gp);
 }
 
 template <class T>
@@ -493,6 +604,12 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
   const bool allow = !(env && atoi(env) == 0);
   const int dense_blocks = allow ? folded_blocks(runs, d, m) : 0;
   if (allow) plan_grid(runs, &P, &gp);
+  if (allow && !P.grid) {
+    std::vector<int> rows((size_t)m * d);
+    for (int k = 0; k < m; ++k)
+      for (int a = 0; a < d; ++a) rows[(size_t)k * d + a] = n_vectors[(size_t)order[k] * d + a];
+    plan_lines(rows, &P, &gp);
+  }
   // longest segments first: pass-1 warps share trip counts, pass 2 pairs
   // segments of similar length
   auto by_len = [](const SegHdr& x, const SegHdr& y) { return x.len > y.len; };
@@ -554,12 +671,16 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
     if (e == cudaSuccess) e = to_device(&pr->gstrip, gp.strips);
     if (e == cudaSuccess) e = to_device(&pr->gquad, gp.quads);
     if (e == cudaSuccess) e = to_device(&pr->grow, gp.rows);
+    if (e == cudaSuccess) e = to_device(&pr->gline, gp.lines);
+    if (e == cudaSuccess) e = to_device(&pr->gslotk, gp.slotk);
   }
   P.grun = pr->grun;
   P.gblk = pr->gblk;
   P.gstrip = pr->gstrip;
   P.gquad = pr->gquad;
   P.grow = pr->grow;
+  P.gline = pr->gline;
+  P.gslotk = pr->gslotk;
   P.seg1 = pr->seg1;
   P.seg2 = pr->seg2;
   P.w_run = pr->w_run;
@@ -591,6 +712,8 @@ int cco_problem_destroy(cco_problem* p) {
   if (p->gstrip) cudaFree(p->gstrip);
   if (p->gquad) cudaFree(p->gquad);
   if (p->grow) cudaFree(p->grow);
+  if (p->gline) cudaFree(p->gline);
+  if (p->gslotk) cudaFree(p->gslotk);
   if (p->krow) cudaFree(p->krow);
   cudaFree(p->dev);
   delete p;
@@ -666,7 +789,7 @@ struct EvalWS {
 
   // Element counts of a batch of B (b_*: of the whole batch).
   struct Sizes {
-    bool grid;
+    bool grid, grid2;   // the grid form in pass 1, in pass 2
     int split, nt1, nt2;
     size_t rhow, part, roots;   // double2 words per lane
   };
@@ -676,7 +799,8 @@ struct EvalWS {
     z.grid = h.grid && prec == PREC_FP64;
     z.split = pass2_split((long long)B * h.ntile2);
     z.nt1 = z.grid ? h.gntile * h.ngblk : h.ntile1;
-    z.nt2 = z.grid ? (h.N + kGridTile2 - 1) / kGridTile2 : pass2_tiles(h, z.split);
+    z.grid2 = z.grid && h.grid == 1;
+    z.nt2 = z.grid2 ? (h.N + kGridTile2 - 1) / kGridTile2 : pass2_tiles(h, z.split);
     z.rhow = z.grid ? (size_t)h.grhow : (size_t)h.M;
     z.part = z.grid ? 2 * (size_t)h.gntile * h.gslots : (size_t)h.ntile1 * h.M;
     z.roots = z.grid ? eval_roots_words(h) : 0;
@@ -707,8 +831,8 @@ struct EvalWS {
     plan.items2 = plan.itemsH = it2;
     plan.n_lanes = B;
     plan.n_items1 = z.grid ? 0 : B * z.nt1;
-    plan.n_items2 = z.grid ? 0 : B * z.nt2;
-    const int nG = z.grid ? B * z.nt1 : 0, nH = z.grid ? B * z.nt2 : 0;
+    plan.n_items2 = z.grid2 ? 0 : B * z.nt2;
+    const int nG = z.grid ? B * z.nt1 : 0, nH = z.grid2 ? B * z.nt2 : 0;
     for (int D = 0; D <= 3; ++D) {
       plan.d_off1[D] = D >= p->d ? plan.n_items1 : 0;
       plan.d_off2[D] = D >= p->d ? plan.n_items2 : 0;

@@ -74,8 +74,8 @@ template <int D, int CLS>
 __global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid1(EvalPlan plan) {
   extern __shared__ double2 smem[];
   __shared__ GridStage stage;
-  constexpr bool ROOTS = CLS > 0;
-  constexpr int NT = CLS == 2 ? 3 : 2;
+  constexpr bool LINES = CLS == kGridLines, ROOTS = CLS > 0 && !LINES;
+  constexpr int NT = CLS == 2 ? 3 : LINES ? 1 : 2;
   const EvalItem* items = plan.itemsG + plan.q_offG[D - 1][CLS];
   const int n = plan.q_offG[D - 1][CLS + 1] - plan.q_offG[D - 1][CLS];
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid1(EvalPlan plan
     const EvalLane ln = plan.lanes[it.lane];
     if (!grid_lane_runs(plan, ln)) continue;   // FP32 lanes: k_pass1
     const ProbDev& P = plan.probs[ln.prob];
-    grid_pass1<D, ROOTS, NT>(P, ln, it.tile / P.ngblk, it.tile % P.ngblk, stage, smem);
+    grid_pass1<D, ROOTS, NT, LINES>(P, ln, it.tile / P.ngblk, it.tile % P.ngblk, stage, smem);
   }
 }
 
@@ -99,6 +99,7 @@ void launch_grid1(const EvalPlan& plan, cudaStream_t s) {
   launch_grid1_class<D, 0>(plan, s);
   launch_grid1_class<D, 1>(plan, s);
   launch_grid1_class<D, 2>(plan, s);
+  if constexpr (D > 1) launch_grid1_class<D, kGridLines>(plan, s);
 }
 
 // One kernel per dimension D and arithmetic keeps each kernel's code small:
@@ -126,7 +127,8 @@ __global__ void __launch_bounds__(kPass1Threads, 4) k_pass1(EvalPlan plan) {
 
 // Chunk energies of a grid-form lane: after the pass-2 weights.
 __device__ __forceinline__ double* grid_energies(const ProbDev& P, const EvalLane& ln) {
-  return reinterpret_cast<double*>(ln.rhow + (size_t)P.gslots * (P.d == 1 ? 2 : 4));
+  return reinterpret_cast<double*>(
+      ln.rhow + (P.grid == 2 ? (size_t)P.M : (size_t)P.gslots * (P.d == 1 ? 2 : 4)));
 }
 
 // Reduction (grid: chunks x lanes): rho_k = sum over tiles of the pass-1
@@ -239,7 +241,7 @@ __global__ void __launch_bounds__(kPass2Threads, 4) k_pass2(EvalPlan plan) {
   const EvalLane ln = plan.lanes[it.lane];
   if (!lane_active(ln.status)) return;
   if ((lane_prec(ln) == PREC_FP32) != F32) return;   // the other kernel's lane
-  if (!F32 && plan.probs[ln.prob].grid) return;      // grid problems: k_grid2
+  if (!F32 && plan.probs[ln.prob].grid == 1) return;      // grid problems: k_grid2
   if (it.tile == 0 && threadIdx.x < 32) lane_energy(plan, ln);
   if (ln.g == nullptr) return;
   if (threadIdx.x == 0) sp = plan.probs[ln.prob];
@@ -349,6 +351,7 @@ cudaError_t configure_grid() {
   opt_in((const void*)k_grid1<D, 0>);
   opt_in((const void*)k_grid1<D, 1>);
   opt_in((const void*)k_grid1<D, 2>);
+  if constexpr (D > 1) opt_in((const void*)k_grid1<D, kGridLines>);
   opt_in((const void*)k_grid2<D, false>);
   opt_in((const void*)k_grid2<D, true>);
   return e;

@@ -190,6 +190,51 @@ __device__ __forceinline__ void grid_tables(const ProbDev& P, const GridBlock& B
   }
 }
 
+// Tables of a block of a line grid: strip by strip the powers of the line's
+// phase z = exp(2 pi i v . s) for its columns and of z^step from row q0 on, a
+// thread per (strip, particle), both chains even and odd apart.
+template <int D, int TP>
+__device__ __forceinline__ void grid_line_tables(const ProbDev& P, const GridBlock& B,
+                                                 const EvalLane& ln, int j0, int nj, int thread,
+                                                 double2* tab) {
+  const int gts = P.gts;
+  for (int w = thread; w < B.nstrip * TP; w += kGridThreads) {
+    const int j = w & (TP - 1), st = B.strip0 + w / TP;
+    const GridLine L = P.gline[st];
+    const bool live = j < nj;
+    const double* sj = ln.s + (size_t)(j0 + (live ? j : 0)) * D;
+    double n1[D], nS[D], nQ[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      n1[a] = (double)L.n[a];
+      nS[a] = (double)(L.n[a] * L.step);
+      nQ[a] = (double)(L.n[a] * L.step * L.q0);
+    }
+    double2 z, y, c0 = make_double2(1.0, 0.0), r0 = c0;
+    sincos_2pi_dot<D>(n1, sj, &z.y, &z.x);
+    sincos_2pi_dot<D>(nS, sj, &y.y, &y.x);
+    if (L.q0 != 0) sincos_2pi_dot<D>(nQ, sj, &r0.y, &r0.x);
+    if (!live) r0 = make_double2(0.0, 0.0);
+    double2 c1 = z, r1 = cmul(r0, y);
+    z = cmul(z, z);
+    y = cmul(y, y);
+    double2* dc = tab + j * gts + P.gstrip[st].col0;
+    double2* dr = dc + L.ncol;
+    for (int e = 0; e < L.ncol; e += 2) {   // ncol is a multiple of 8
+      dc[e] = c0;
+      dc[e + 1] = c1;
+      c0 = cmul(c0, z);
+      c1 = cmul(c1, z);
+      if (e < 8) {
+        dr[e] = r0;
+        dr[e + 1] = r1;
+        r0 = cmul(r0, y);
+        r1 = cmul(r1, y);
+      }
+    }
+  }
+}
+
 // Prefix phase of a run from its table offsets (one particle's row).
 template <int D>
 __device__ __forceinline__ double2 run_phase(const double2* row, int o0, int o1) {
@@ -234,7 +279,7 @@ __device__ __forceinline__ void grid_describe(GridStage& S, const ProbDev& P, co
 // Pass 1 products of one item by a warp that owns the CNT tiles lo .. lo + CNT
 // - 1 of the block: 4 DMMAs per tile and 4 particles. SAME: the tiles are of
 // one strip and share the prefix phase. CNT = 0: the warp only fills.
-template <int D, bool ROOTS, int CNT, bool SAME>
+template <int D, bool ROOTS, int CNT, bool SAME, bool LINES>
 __device__ __forceinline__ void grid_pass1_item(const ProbDev& P, const GridBlock& B,
                                                 const EvalLane& ln, const GridStage& S, int lo,
                                                 double2* tab) {
@@ -255,7 +300,7 @@ __device__ __forceinline__ void grid_pass1_item(const ProbDev& P, const GridBloc
     const int c = lo + i - at;
     o0[i] = S.row[8 * si + pr].o0;
     o1[i] = S.row[8 * si + pr].o1;
-    col[i] = 8 * c + pr;
+    col[i] = S.strip[si].col0 + 8 * c + pr;
     slot[i] = 2 * (S.strip[si].slot0 + 64 * c) + (2 * c + 1 < nq ? 1 : 0);
 #pragma unroll
     for (int h = 0; h < 2; ++h) p1[i][h] = p2[i][h] = p3[i][h] = p4[i][h] = 0.0;
@@ -284,7 +329,8 @@ __device__ __forceinline__ void grid_pass1_item(const ProbDev& P, const GridBloc
     j0 += kGridChunk;
     if (j0 >= jt1) break;
     bar_cta();
-    grid_tables<D, ROOTS, kGridChunk>(P, B, ln, j0, jt1 - j0, threadIdx.x, tab);
+    if constexpr (LINES) grid_line_tables<D, kGridChunk>(P, B, ln, j0, jt1 - j0, threadIdx.x, tab);
+    else grid_tables<D, ROOTS, kGridChunk>(P, B, ln, j0, jt1 - j0, threadIdx.x, tab);
     bar_cta();
   }
   // lane holds the cells (run pr, columns t and t + 4 of a tile): a slot of each
@@ -305,13 +351,16 @@ __device__ __forceinline__ void grid_pass1_item(const ProbDev& P, const GridBloc
 // Pass 1 of one item (lane, tile, block): the block's 8 x 8-cell tiles in strip
 // order are cut into four equal ranges, one per warp (at most NT tiles), so
 // that uneven strips do not leave warps idle.
-template <int D, bool ROOTS, int NT>
+template <int D, bool ROOTS, int NT, bool LINES>
 __device__ __forceinline__ void grid_pass1(const ProbDev& P, const EvalLane& ln, int tile, int blk,
                                            GridStage& S, double2* tab) {
   const GridBlock B = P.gblk[blk];
   const int jt0 = tile * P.gtile;
   grid_describe(S, P, B, ln.part, nullptr, tile);
-  grid_tables<D, ROOTS, kGridChunk>(P, B, ln, jt0, min(P.N - jt0, P.gtile), threadIdx.x, tab);
+  if constexpr (LINES)
+    grid_line_tables<D, kGridChunk>(P, B, ln, jt0, min(P.N - jt0, P.gtile), threadIdx.x, tab);
+  else
+    grid_tables<D, ROOTS, kGridChunk>(P, B, ln, jt0, min(P.N - jt0, P.gtile), threadIdx.x, tab);
   bar_cta();
   const int warp = threadIdx.x >> 5;
   const int lo = B.ntile * warp >> 2, hi = B.ntile * (warp + 1) >> 2;
@@ -320,8 +369,8 @@ __device__ __forceinline__ void grid_pass1(const ProbDev& P, const EvalLane& ln,
   const bool same = hi <= at + ((S.strip[si].nq + 1) >> 1);
 #define CCO_GRID_CASE(CNT)                                                                     \
   if (CNT <= NT && hi - lo == CNT) {                                                           \
-    if (same) grid_pass1_item<D, ROOTS, CNT <= NT ? CNT : 0, true>(P, B, ln, S, lo, tab);      \
-    else grid_pass1_item<D, ROOTS, CNT <= NT ? CNT : 0, false>(P, B, ln, S, lo, tab);          \
+    if (same) grid_pass1_item<D, ROOTS, CNT <= NT ? CNT : 0, true, LINES>(P, B, ln, S, lo, tab);   \
+    else grid_pass1_item<D, ROOTS, CNT <= NT ? CNT : 0, false, LINES>(P, B, ln, S, lo, tab);       \
   }
   CCO_GRID_CASE(0)
   CCO_GRID_CASE(1)
@@ -336,10 +385,16 @@ __device__ __forceinline__ void grid_pass1(const ProbDev& P, const EvalLane& ln,
 // where the grid has no k-set row).
 template <bool ONE_D>
 __device__ __forceinline__ double grid_reduce_slot(const ProbDev& P, const EvalLane& ln, int slot) {
-  const GridQuad Q = P.gquad[slot >> 5];
+  const bool lines = P.grid == 2;
+  GridQuad Q{};
+  if (!lines) Q = P.gquad[slot >> 5];
   const int lane = slot & 31, r = grid_perm(lane >> 2), c = Q.c0 + (lane & 3);
   int kp = -1, km = -1, n0 = 0;
-  if (r < Q.nrun) {
+  if (lines) {
+    const int2 k = P.gslotk[slot];
+    kp = k.x;
+    km = k.y;
+  } else if (r < Q.nrun) {
     const GridRun g = P.grun[Q.run0 + r];
     n0 = g.n0;
     if (c >= g.a && c <= g.b) kp = g.kstart + c - g.a;
@@ -390,6 +445,11 @@ __device__ __forceinline__ double grid_reduce_slot(const ProbDev& P, const EvalL
     } else {
       tm = make_double2(0.0, 0.0);
     }
+  }
+  if (lines) {   // the weighted density of the recurrence pass 2
+    if (kp >= 0) ln.rhow[kp] = tp;
+    if (km >= 0) ln.rhow[km] = tm;
+    return e;
   }
   // -conj(w rho): T = sum_c -(conj(p+) z^c + conj(p-) conj(z^c)), u and v parts
   const double2 re_t = make_double2(-(tp.x + tm.x), tm.y - tp.y);

@@ -30,6 +30,8 @@ struct cco_problem {
   cco::GridStrip* gstrip = nullptr;
   cco::GridQuad* gquad = nullptr;
   cco::GridRow* grow = nullptr;
+  cco::GridLine* gline = nullptr;
+  int2* gslotk = nullptr;
   double4* krow = nullptr;     // run-order rows (n_0, n_1, n_2, w) for the Hessian kernels
   size_t smem1 = 0, smem2 = 0, smemG = 0, smemH = 0;
   int dense_blocks = 0;        // cco_problem_pass1_form
@@ -208,13 +210,16 @@ struct EvalSet {
       if (h.grid) {
         n_grid += h.groots > 0;
         chunks_root = std::max(chunks_root, (h.groots * h.N + kRootChunk - 1) / kRootChunk);
-        const int ntG = h.gntile * h.ngblk, ntH = (h.N + kGridTile2 - 1) / kGridTile2;
+        const int ntG = h.gntile * h.ngblk;
+        const int ntH = h.grid == 1 ? (h.N + kGridTile2 - 1) / kGridTile2 : 0;
         for (int t = 0; t < ntG; ++t) gG[p->d - 1][h.gcls].push_back(EvalItem{j, t});
         for (int t = 0; t < ntH; ++t) gH[p->d - 1][h.gcls > 0].push_back(EvalItem{j, t});
       }
       if (!h.grid || may_fp32) {
         const int C = pass1_chunks(h, chunks);
         for (int t = 0; t < h.ntile1 * C; ++t) g1[p->d - 1].push_back(EvalItem{j, t});
+      }
+      if (h.grid != 1 || may_fp32) {
         const int nt2 = pass2_tiles(h, split);
         for (int t = 0; t < nt2; ++t) g2[p->d - 1].push_back(EvalItem{j, t});
       }

@@ -57,14 +57,21 @@ constexpr int kGridCtas = 4;       // CTAs per SM (registers and shared memory)
 constexpr int kGridMaxEntries = 55;   // table entries per particle: 64 particles, four CTAs per SM
 constexpr int kGridRootsMin = 4;  // blocks from which a kernel forms the phase roots
 // pass-1 kernels by tiles of 8 x 8 cells per warp and where the roots come from:
-// <= 2 (formed in the passes), <= 2, <= 3 (from the roots kernel)
-constexpr int kGridClasses = 3;
+// <= 2 (formed in the passes), <= 2, <= 3 (from the roots kernel); line grids
+constexpr int kGridClasses = 4;
+constexpr int kGridLines = 3;      // their class
 constexpr int kGridMaxTiles = 12;  // tiles of a block
 struct GridRun {
   int n0, n1, a, b, kstart, pad_;   // prefix (1-D: n0 = q), last-axis range [a, b]
 };
 struct GridStrip {
   int run0, nrun, nq, slot0;
+  int col0, pad_;                    // table offset of its first column
+};
+// Line grids (sparse k-sets made of multiples i v of primitive vectors v): each
+// strip has columns and prefixes of its own, i = q step + c along its line v.
+struct GridLine {
+  int n[3], step, q0, ncol;          // rows q0 .. q0 + 7, columns 0 .. ncol - 1
 };
 struct GridBlock {
   int strip0, nstrip, lo, ncol;      // columns lo .. lo + ncol - 1 (ncol a multiple of 8)
@@ -95,7 +102,7 @@ struct ProbDev {
   TabLayout t1, t2;          // pass-1 / pass-2 table layouts
   int ntile1, ntile2;        // particle tiles of pass 1 / pass 2 (pass 2 at split 1)
   int sl2;                   // logical slices of the pass-2 segment pairs (power of 2, <= 8)
-  int grid;                  // 1: FP64 lanes run the tensor-core form below
+  int grid;                  // 1: FP64 lanes run the tensor-core form below, 2: pass 1 only, on lines
   int ngblk, gcls;           // its blocks; pass-1 kernel class
   int gts;                   // table entries per particle (odd)
   int gstep;                 // 1-D: prefix exponents are gstep n0 (1 otherwise)
@@ -108,6 +115,8 @@ struct ProbDev {
   const GridRun* grun;
   const GridQuad* gquad;
   const GridRow* grow;
+  const GridLine* gline;     // line grids: per strip; and per slot its rows n = +c, -c (-1: none)
+  const int2* gslotk;
   double vol;                // V
   double gpref;              // 2 (2 pi) / V
   const SegHdr* seg1;
