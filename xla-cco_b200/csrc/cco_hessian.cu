@@ -4,21 +4,29 @@
 //                           - delta_jl (Re rho_k cos th_kj + Im rho_k sin th_kj)]
 //   th_kj = 2 pi n_k . s_j,  pref = 2 (2 pi)^2 / V        (src/xla_cco/energy.py:272-299)
 //
-// The reference forms the (N, M) cos / sin matrices and two (N, M) x (M, N)
-// products per (a, b). Here no (N, M) array exists: a CTA owns one tile pair
-// (particles J x particles L, L >= J; the Hessian is symmetric, the lower
-// tiles are written as mirrors), walks the k-set in chunks, forms the chunk's
-// phases of both particle tiles in shared memory and accumulates
-//   acc_ab[j][l] += q_kab (cos th_kj cos th_kl + sin th_kj sin th_kl),
-//   q_kab = w_k n_ka n_kb   (a <= b; the (a, b) and (b, a) blocks are equal)
-// in registers, 4 x 4 particle pairs per thread. The delta_jl term needs rho,
-// which the evaluation kernels compute first; a second kernel subtracts it
-// from the diagonal blocks.
+// Three kernels per k-chunk (one chunk unless the phases pass kPhaseBytes):
+//   k_hess_phase  the phases exp(i th_kj) of the chunk, once per (k, particle),
+//                 from the argument n . s reduced exactly (fma products,
+//                 compensated sum, nearest integer removed) before sincospi;
+//   k_hess_diag   the delta_jl sums of the chunk (a warp per particle; rho comes
+//                 from the evaluation kernels);
+//   k_hess_tiles  cos(th_j - th_l) = c_j c_l + s_j s_l makes block (a, b) a real
+//                 matrix product of depth 2 M with weights q_kab = w_k n_ka n_kb
+//                 (a <= b), run on the FP64 matrix pipe (DMMA m8n8k4). A CTA owns
+//                 32 particles x 32 particles at or above the diagonal and all
+//                 component pairs; a warp 16 x 16 of them.
+// The product costs N^2 M (d (d + 1) / 2) FMAs (half of the matrix), against
+// which everything else is small; the tile goes through shared memory so that it
+// and its mirror are written row by row, and an element and its mirror come from
+// the same sum (the matrix is exactly symmetric).
 //
-// Phases use the argument n . s reduced exactly (fma products, compensated
-// sum, nearest integer removed) before sincospi, so |n . s| in the thousands
-// costs no accuracy.
+// d=2 N=700 M=560: before, one sincospi per (k, particle, tile pair) and FP64
+// FMAs took 240 us and a thread per particle walking all k 238 us; now 4 us for
+// the phases, 8 for the diagonal and 88 for the tiles, whose DMMAs alone need
+// 57 us on the SMs that hold two of the 253 CTAs.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "cco_host.cuh"
 #include "cco_internal.cuh"
@@ -26,44 +34,24 @@
 namespace cco {
 namespace {
 
-constexpr int kHessTile = 64;      // particles per tile side
-constexpr int kHessK = 16;         // k rows per shared-memory chunk
-constexpr int kHessThreads = 256;  // 16 x 16 threads, 4 x 4 particle pairs each
+constexpr int kHessTile = 32;      // particles per tile side
+constexpr int kHessK = 16;         // k rows per shared-memory chunk (two chunks held)
+constexpr int kHessThreads = 128;
+constexpr int kHessStride = kHessTile + 2;   // 16-byte words: fragment reads hit 8 banks
+constexpr size_t kPhaseBytes = (size_t)256 << 20;   // phases held at a time
 
-// (a, b) component pairs (a <= b) a CTA accumulates: group g of dimension D.
-// D = 1: (0,0); D = 2: (0,0) (0,1) (1,1); D = 3: two groups of three.
+// Component pair c (a <= b) of dimension D, in row order of the upper triangle.
 template <int D>
-struct Combos;
-template <>
-struct Combos<1> {
-  static constexpr int kGroups = 1, kPer = 1;
-  __device__ static void ab(int, int, int& a, int& b) { a = 0; b = 0; }
-};
-template <>
-struct Combos<2> {
-  static constexpr int kGroups = 1, kPer = 3;
-  __device__ static void ab(int, int c, int& a, int& b) {
+__device__ __forceinline__ void hess_ab(int c, int& a, int& b) {
+  if (D == 1) {
+    a = b = 0;
+  } else if (D == 2) {
     a = c == 2 ? 1 : 0;
     b = c == 0 ? 0 : 1;
+  } else {
+    a = c < 3 ? 0 : c < 5 ? 1 : 2;
+    b = c < 3 ? c : c < 5 ? c - 2 : 2;
   }
-};
-template <>
-struct Combos<3> {
-  static constexpr int kGroups = 2, kPer = 3;
-  __device__ static void ab(int g, int c, int& a, int& b) {
-    // group 0: (0,0) (0,1) (0,2); group 1: (1,1) (1,2) (2,2)
-    if (g == 0) { a = 0; b = c; }
-    else { a = c == 2 ? 2 : 1; b = c == 0 ? 1 : 2; }
-  }
-};
-
-// exp(2 pi i n . s) with n . s reduced exactly before the transcendental.
-template <int D>
-__device__ __forceinline__ double2 exact_phase(const double4& nk, const double* sj) {
-  const double nv[3] = {nk.x, nk.y, nk.z};
-  double sn, cs;
-  sincos_2pi_dot<D>(nv, sj, &sn, &cs);
-  return make_double2(cs, sn);
 }
 
 // Linear index over the upper triangle of T x T tile pairs -> (J, L), L >= J.
@@ -76,156 +64,244 @@ __device__ __forceinline__ void tile_pair(int t, int T, int& J, int& L) {
   L = J + t;
 }
 
+// ph[lane][k - k0][j] = exp(i th_kj)
 template <int D>
-__global__ void __launch_bounds__(kHessThreads, 1)
-k_hess_tiles(const double* __restrict__ s, size_t s_stride, const double4* __restrict__ krow,
-             int N, int M, double pref, double* __restrict__ H, size_t h_stride) {
-  using C = Combos<D>;
-  constexpr int NC = C::kPer;
-  __shared__ double2 zj[kHessK][kHessTile];
-  __shared__ double2 zl[kHessK][kHessTile];
-  __shared__ double q[kHessK][NC];
-  const int T = (N + kHessTile - 1) / kHessTile;
-  int J, L;
-  tile_pair(blockIdx.x, T, J, L);
-  const int g = blockIdx.y, lane = blockIdx.z;
-  const double* sl = s + (size_t)lane * s_stride;
-  double* Hl = H + (size_t)lane * h_stride;
-  const bool diag_tile = J == L;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  int ca[NC], cb[NC];
+__global__ void k_hess_phase(const double* __restrict__ s, const double4* __restrict__ krow, int N,
+                             int k0, int kn, double2* __restrict__ ph) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, lane = blockIdx.z;
+  if (j >= N) return;
+  double sj[D];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) C::ab(g, c, ca[c], cb[c]);
-
-  double acc[4][4][NC];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) acc[u][v][c] = 0.0;
-
-  const int fill = (diag_tile ? 1 : 2) * kHessK * kHessTile;
-  for (int k0 = 0; k0 < M; k0 += kHessK) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < fill; idx += kHessThreads) {
-      const int which = idx / (kHessK * kHessTile);
-      const int r = idx - which * (kHessK * kHessTile);
-      const int kk = r / kHessTile, p = r - kk * kHessTile;
-      const int k = k0 + kk, part = (which ? L : J) * kHessTile + p;
-      double2 z = make_double2(0.0, 0.0);
-      if (k < M && part < N) z = exact_phase<D>(krow[k], sl + (size_t)part * D);
-      if (which) zl[kk][p] = z;
-      else zj[kk][p] = z;
-    }
-    for (int idx = threadIdx.x; idx < kHessK * NC; idx += kHessThreads) {
-      const int kk = idx / NC, c = idx - kk * NC;
-      const int k = k0 + kk;
-      double v = 0.0;
-      if (k < M) {
-        const double4 r = krow[k];
-        const double nv[3] = {r.x, r.y, r.z};
-        v = r.w * nv[ca[c]] * nv[cb[c]];
-      }
-      q[kk][c] = v;
-    }
-    __syncthreads();
-    const double2(*zr)[kHessTile] = diag_tile ? zj : zl;
-#pragma unroll 2
-    for (int kk = 0; kk < kHessK; ++kk) {
-      double2 a[4], b[4];
-      double qc[NC];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a[u] = zj[kk][ty + 16 * u];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) b[v] = zr[kk][tx + 16 * v];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) qc[c] = q[kk][c];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const double t = fma(a[u].x, b[v].x, a[u].y * b[v].y);
-#pragma unroll
-          for (int c = 0; c < NC; ++c) acc[u][v][c] = fma(qc[c], t, acc[u][v][c]);
-        }
-    }
-  }
-  const size_t nd = (size_t)N * D;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int j = J * kHessTile + ty + 16 * u;
-    if (j >= N) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int l = L * kHessTile + tx + 16 * v;
-      if (l >= N) continue;
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const double val = pref * acc[u][v][c];
-        const int a = ca[c], b = cb[c];
-        Hl[(size_t)(j * D + a) * nd + l * D + b] = val;
-        if (a != b) Hl[(size_t)(j * D + b) * nd + l * D + a] = val;
-        if (!diag_tile) {
-          Hl[(size_t)(l * D + b) * nd + j * D + a] = val;
-          if (a != b) Hl[(size_t)(l * D + a) * nd + j * D + b] = val;
-        }
-      }
-    }
+  for (int a = 0; a < D; ++a) sj[a] = s[((size_t)lane * N + j) * D + a];
+  for (int k = blockIdx.y; k < kn; k += gridDim.y) {
+    const double4 r = krow[k0 + k];
+    const double nv[3] = {r.x, r.y, r.z};
+    double sn, cs;
+    sincos_2pi_dot<D>(nv, sj, &sn, &cs);
+    ph[((size_t)lane * kn + k) * N + j] = make_double2(cs, sn);
   }
 }
 
-// Diagonal blocks: H[(j,a),(j,b)] -= pref sum_k q_kab (Re rho_k cos th_kj + Im rho_k sin th_kj).
-// One thread per particle; rho is the evaluation's run-order density.
+// dg[lane][j][c] = sum over the chunk of q_kab (Re rho_k cos th_kj + Im rho_k sin th_kj)
 template <int D>
-__global__ void k_hess_diag(const double* __restrict__ s, size_t s_stride,
-                            const double4* __restrict__ krow, const double2* __restrict__ rho,
-                            int N, int M, double pref, double* __restrict__ H, size_t h_stride) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, lane = blockIdx.y;
+__global__ void k_hess_diag(const double2* __restrict__ ph, const double4* __restrict__ krow,
+                            const double2* __restrict__ rho, int N, int M, int k0, int kn,
+                            double* __restrict__ dg) {
+  constexpr int NC = D * (D + 1) / 2;
+  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = blockIdx.y;
   if (j >= N) return;
-  const double* sj = s + (size_t)lane * s_stride + (size_t)j * D;
-  const double2* rl = rho + (size_t)lane * M;
-  double acc[D][D];
+  double acc[NC];
 #pragma unroll
-  for (int a = 0; a < D; ++a)
-#pragma unroll
-    for (int b = 0; b < D; ++b) acc[a][b] = 0.0;
-  for (int k = 0; k < M; ++k) {
-    const double4 r = krow[k];
-    const double2 z = exact_phase<D>(r, sj);
-    const double2 rh = rl[k];
+  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+  for (int k = threadIdx.x & 31; k < kn; k += 32) {
+    const double4 r = krow[k0 + k];
+    const double2 z = ph[((size_t)lane * kn + k) * N + j];
+    const double2 rh = rho[(size_t)lane * M + k0 + k];
     const double core = r.w * fma(rh.x, z.x, rh.y * z.y);
     const double nv[3] = {r.x, r.y, r.z};
 #pragma unroll
-    for (int a = 0; a < D; ++a)
-#pragma unroll
-      for (int b = a; b < D; ++b) acc[a][b] = fma(core * nv[a], nv[b], acc[a][b]);
-  }
-  const size_t nd = (size_t)N * D;
-  double* Hl = H + (size_t)lane * h_stride;
-#pragma unroll
-  for (int a = 0; a < D; ++a)
-#pragma unroll
-    for (int b = a; b < D; ++b) {
-      Hl[(size_t)(j * D + a) * nd + j * D + b] -= pref * acc[a][b];
-      if (a != b) Hl[(size_t)(j * D + b) * nd + j * D + a] -= pref * acc[a][b];
+    for (int c = 0; c < NC; ++c) {
+      int a, b;
+      hess_ab<D>(c, a, b);
+      acc[c] = fma(core * nv[a], nv[b], acc[c]);
     }
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if ((threadIdx.x & 31) == 0) dg[((size_t)lane * N + j) * NC + c] = acc[c];
+  }
+}
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile(
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+template <int D>
+constexpr size_t hess_smem() {
+  const size_t nc = D * (D + 1) / 2;
+  const size_t chunk =
+      2 * (2 * (size_t)kHessK * kHessStride * sizeof(double2) + kHessK * nc * sizeof(double));
+  const size_t side = (size_t)kHessTile * D, tile = side * (side + 1) * sizeof(double);
+  return chunk > tile ? chunk : tile;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kHessThreads)
+k_hess_tiles(const double2* __restrict__ ph, const double4* __restrict__ krow,
+             const double* __restrict__ dg, int N, int k0, int kn, double pref, bool first,
+             double* __restrict__ H) {
+  constexpr int NC = D * (D + 1) / 2, TS = kHessTile, SIDE = TS * D;
+  extern __shared__ double2 sm[];
+  double2* z2 = sm;   // [2][j, l][kHessK][kHessStride]
+  constexpr int ZW = kHessK * kHessStride;
+  double* q2 = reinterpret_cast<double*>(sm + 4 * ZW);   // [2][kHessK][NC]
+  const int T = (N + TS - 1) / TS;
+  int J, L;
+  tile_pair(blockIdx.x, T, J, L);
+  const int lane = blockIdx.y;
+  const double2* pl = ph + (size_t)lane * kn * N;
+  const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31, t = wl & 3, r = wl >> 2;
+  const int jw = 16 * (warp >> 1), lw = 16 * (warp & 1);
+  double acc[NC][2][2][2];
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) acc[c][u][v][0] = acc[c][u][v][1] = 0.0;
+  // a chunk's phases travel through registers: the next chunk's are loaded while
+  // this one's products run (95 -> 88 us on d=2 N=700), one barrier per chunk
+  constexpr int NL = kHessK * TS / kHessThreads;
+  double2 nj[NL], nl[NL];
+  auto load = [&](int kc) {
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+      const int e = threadIdx.x + i * kHessThreads, k = e / TS, p = e - k * TS;
+      const bool in = kc + k < kn;   // rows past the chunk are zero
+      const size_t row = (size_t)(kc + k) * N;
+      const int j = J * TS + p, l = L * TS + p;
+      nj[i] = in && j < N ? pl[row + j] : make_double2(0.0, 0.0);
+      nl[i] = in && l < N ? pl[row + l] : make_double2(0.0, 0.0);
+    }
+  };
+  auto store = [&](int buf, int kc) {
+    double2 *zj = z2 + 2 * buf * ZW, *zl = zj + ZW;
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+      const int e = threadIdx.x + i * kHessThreads, k = e / TS, p = e - k * TS;
+      zj[k * kHessStride + p] = nj[i];
+      zl[k * kHessStride + p] = nl[i];
+    }
+    for (int e = threadIdx.x; e < kHessK * NC; e += kHessThreads) {
+      const int k = e / NC, c = e - k * NC;
+      double v = 0.0;
+      if (kc + k < kn) {
+        const double4 w = krow[k0 + kc + k];
+        const double nv[3] = {w.x, w.y, w.z};
+        int a, b;
+        hess_ab<D>(c, a, b);
+        v = w.w * nv[a] * nv[b];
+      }
+      q2[buf * kHessK * NC + e] = v;
+    }
+  };
+  load(0);
+  store(0, 0);
+  __syncthreads();
+  for (int kc = 0, buf = 0; kc < kn; kc += kHessK, buf ^= 1) {
+    const bool more = kc + kHessK < kn;
+    if (more) load(kc + kHessK);
+    const double2 *zj = z2 + 2 * buf * ZW, *zl = zj + ZW;
+    const double* q = q2 + buf * kHessK * NC;
+#pragma unroll 2
+    for (int k = 0; k < kHessK; k += 4) {
+      double2 a[2], b[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) a[u] = zj[(k + t) * kHessStride + jw + 8 * u + r];
+#pragma unroll
+      for (int v = 0; v < 2; ++v) b[v] = zl[(k + t) * kHessStride + lw + 8 * v + r];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double qc = q[(k + t) * NC + c];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const double ax = qc * a[u].x, ay = qc * a[u].y;
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            dmma(acc[c][u][v], ax, b[v].x);
+            dmma(acc[c][u][v], ay, b[v].y);
+          }
+        }
+      }
+    }
+    if (more) store(buf ^ 1, kc + kHessK);
+    __syncthreads();
+  }
+  // the tile, scaled and with its share of the diagonal term, into shared memory
+  double* tile = reinterpret_cast<double*>(sm);   // [SIDE][SIDE + 1]
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    int a, b;
+    hess_ab<D>(c, a, b);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int pj = jw + 8 * u + r, p2 = lw + 8 * v + 2 * t + h;
+          double x = pref * acc[c][u][v][h];
+          if (J == L && pj == p2 && J * TS + pj < N)
+            x -= pref * dg[((size_t)lane * N + J * TS + pj) * NC + c];
+          tile[(pj * D + a) * (SIDE + 1) + p2 * D + b] = x;
+          if (a != b) tile[(pj * D + b) * (SIDE + 1) + p2 * D + a] = x;
+        }
+  }
+  __syncthreads();
+  const size_t nd = (size_t)N * D;
+  double* Hl = H + (size_t)lane * nd * nd;
+  const int rows = min(SIDE, (N - J * TS) * D), cols = min(SIDE, (N - L * TS) * D);
+  // a diagonal tile's lower half is the mirror of its upper half (blocks of equal
+  // particles are symmetric as written)
+  for (int e = threadIdx.x; e < SIDE * SIDE; e += kHessThreads) {
+    const int y = e / SIDE, x = e - y * SIDE;
+    if (y >= rows || x >= cols) continue;
+    const bool up = J != L || x / D >= y / D;
+    const double v = up ? tile[y * (SIDE + 1) + x] : tile[x * (SIDE + 1) + y];
+    double* o = Hl + (size_t)(J * SIDE + y) * nd + L * SIDE + x;
+    *o = first ? v : *o + v;
+  }
+  if (J == L) return;
+  for (int e = threadIdx.x; e < SIDE * SIDE; e += kHessThreads) {
+    const int x = e / SIDE, y = e - x * SIDE;   // row x of the mirror tile
+    if (y >= rows || x >= cols) continue;
+    const double v = tile[y * (SIDE + 1) + x];
+    double* o = Hl + (size_t)(L * SIDE + x) * nd + J * SIDE + y;
+    *o = first ? v : *o + v;
+  }
 }
 
 template <int D>
 cudaError_t launch_hessian(const cco_problem* p, cudaStream_t st, int batch, const double* s,
                            const double2* rho, double* H) {
+  constexpr int NC = D * (D + 1) / 2;
   const int N = p->N, M = p->M;
   const int T = (N + kHessTile - 1) / kHessTile;
   const size_t nd = (size_t)N * D;
   const double pref = 2.0 * (2.0 * M_PI) * (2.0 * M_PI) / p->host.vol;
-  dim3 grid((unsigned)(T * (T + 1) / 2), Combos<D>::kGroups, (unsigned)batch);
-  k_hess_tiles<D><<<grid, kHessThreads, 0, st>>>(s, nd, p->krow, N, M, pref, H, nd * nd);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  dim3 g2((unsigned)((N + 127) / 128), (unsigned)batch);
-  k_hess_diag<D><<<g2, 128, 0, st>>>(s, nd, p->krow, rho, N, M, pref, H, nd * nd);
-  return cudaGetLastError();
+  static const cudaError_t opt = cudaFuncSetAttribute(
+      k_hess_tiles<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hess_smem<D>());
+  if (opt != cudaSuccess) return opt;
+  // lanes, then k rows, at a time: phases within kPhaseBytes
+  const size_t per_k = (size_t)N * sizeof(double2);
+  const int kn_max = (int)std::max<size_t>(1, std::min<size_t>(M, kPhaseBytes / per_k));
+  const int lanes = (int)std::max<size_t>(1, std::min<size_t>(batch, kPhaseBytes / (per_k * kn_max)));
+  double2* ph = nullptr;
+  double* dg = nullptr;
+  cudaError_t e = pool_alloc(&ph, per_k * kn_max * lanes, st);
+  if (e == cudaSuccess) e = pool_alloc(&dg, sizeof(double) * NC * N * lanes, st);
+  for (int lo = 0; lo < batch && e == cudaSuccess; lo += lanes) {
+    const int b = std::min(lanes, batch - lo);
+    for (int k0 = 0; k0 < M && e == cudaSuccess; k0 += kn_max) {
+      const int kn = std::min(kn_max, M - k0);
+      const double* sl = s + (size_t)lo * nd;
+      k_hess_phase<D><<<dim3((N + 127) / 128, std::min(kn, 256), b), 128, 0, st>>>(sl, p->krow, N, k0,
+                                                                               kn, ph);
+      k_hess_diag<D><<<dim3((N + 3) / 4, b), 128, 0, st>>>(ph, p->krow, rho + (size_t)lo * M, N, M, k0,
+                                                           kn, dg);
+      k_hess_tiles<D><<<dim3((unsigned)(T * (T + 1) / 2), b), kHessThreads, hess_smem<D>(), st>>>(
+          ph, p->krow, dg, N, k0, kn, pref, k0 == 0, H + (size_t)lo * nd * nd);
+      e = cudaGetLastError();
+    }
+  }
+  if (ph) cudaFreeAsync(ph, st);
+  if (dg) cudaFreeAsync(dg, st);
+  return e;
 }
 
 }  // namespace
