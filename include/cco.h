@@ -75,6 +75,15 @@ int cco_device_count(int* n_devices);
 int cco_problem_create(int device, int d, int n_particles, int m,
                        const int32_t* n_vectors, const double* weights,
                        double volume, cco_problem** out);
+/*
+ * The same with a padded row layout for cco_energy_grad_rows: its densities have
+ * `total` columns, column rows[k] for row k (distinct), and every other column
+ * is a zero (padding) row. cco_problem_create: total = m, rows[k] = k.
+ */
+int cco_problem_create_rows(int device, int d, int n_particles, int m,
+                            const int32_t* n_vectors, const double* weights,
+                            double volume, int total, const int32_t* rows,
+                            cco_problem** out);
 int cco_problem_destroy(cco_problem* p);
 /* Sizes of the device k-set layout (runs split into pass-1/pass-2 segments). */
 int cco_problem_info(const cco_problem* p, int* d, int* n_particles, int* m,
@@ -98,6 +107,22 @@ int cco_problem_pass1_form(const cco_problem* p, int* gemm_blocks);
  */
 int cco_energy_grad(cco_problem* p, void* stream, int batch, const double* s,
                     double* phi, double* grad, double* rho_re, double* rho_im);
+
+/*
+ * cco_energy_grad with the density in the layout of cco_problem_create_rows:
+ * rho_re, rho_im are [batch][total], zero rows N and 0
+ * (StealthyEnergy.value_grad_density, src/xla_cco/energy.py:206-225).
+ */
+int cco_energy_grad_rows(cco_problem* p, void* stream, int batch, const double* s,
+                         double* phi, double* grad, double* rho_re, double* rho_im);
+
+/*
+ * Structure-factor sums of a batch: tot[k] += S, tot2[k] += S^2 over the batch
+ * in order, S = |rho_k|^2 / N, rows as given to cco_problem_create (device
+ * [M], accumulated into; src/xla_cco/analysis/structure.py:150-180).
+ */
+int cco_structure_sums(cco_problem* p, void* stream, int batch, const double* s,
+                       double* tot, double* tot2);
 
 /*
  * Closed-form Hessian d2 Phi / ds_ja ds_lb of `batch` configurations

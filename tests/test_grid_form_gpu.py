@@ -136,3 +136,24 @@ def test_line_grid_density_vs_direct_sums(monkeypatch, d, n, b, dirs, top):
             np.testing.assert_allclose(im[i], np.sin(theta).sum(1), rtol=0, atol=1e-13 * n, err_msg=form)
             if grad is not None and n > 1:
                 np.testing.assert_allclose(grad[i], g_ref[i], rtol=0, atol=RTOL_KERNEL_F * np.abs(g_ref[i]).max())
+
+
+def test_density_layout_with_zero_rows_inside():
+    """Zero (padding) rows anywhere: N and 0 there, every other row in place; the
+    same from NumPy and CUDA inputs, and structure-factor sums in the same order."""
+    import torch
+
+    from xla_cco.analysis.structure import structure_factor
+
+    nv = np.array([[0, 0], [1, 0], [0, 2], [0, 0], [3, -1], [-2, 5], [0, 0]], dtype=np.float64)
+    en = StealthyEnergy(nv, np.where(nv.any(1), 1.0, 0.0), np.float64(5.0))
+    s = np.random.default_rng(9).uniform(size=(3, 41, 2))
+    _, _, re, im = en.evaluate(s, want_rho=True)
+    theta = 2.0 * np.pi * np.einsum("ka,bja->bkj", nv, s)
+    np.testing.assert_allclose(re, np.cos(theta).sum(-1), rtol=0, atol=1e-12 * 41)
+    np.testing.assert_allclose(im, np.sin(theta).sum(-1), rtol=0, atol=1e-12 * 41)
+    assert (re[:, [0, 3, 6]] == 41.0).all() and (im[:, [0, 3, 6]] == 0.0).all()
+    _, _, rt, it = en.evaluate(torch.from_numpy(s).cuda(), want_rho=True)
+    assert np.array_equal(rt.cpu().numpy(), re) and np.array_equal(it.cpu().numpy(), im)
+    sk = structure_factor(s[1], nv)
+    np.testing.assert_allclose(sk, (re[1] ** 2 + im[1] ** 2) / 41, rtol=1e-13)

@@ -442,12 +442,17 @@ void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
   grid_sizes(P, *gp);
 }
 
-template <class T>
-cudaError_t to_device(T** dst, const std::vector<T>& src) {
-  const cudaError_t e = cudaMalloc(dst, std::max<size_t>(src.size(), 1) * sizeof(T));
-  if (e != cudaSuccess || src.empty()) return e;
-  return cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice);
-}
+// Arrays gathered into one upload, each at a 256-byte offset.
+struct Blob {
+  std::vector<unsigned char> bytes;
+  template <class T>
+  size_t add(const std::vector<T>& v) {
+    const size_t o = (bytes.size() + 255) & ~(size_t)255, n = v.size() * sizeof(T);
+    bytes.resize(o + std::max<size_t>(n, 1));
+    if (n) memcpy(bytes.data() + o, v.data(), n);
+    return o;
+  }
+};
 
 // Absolute table rows of the digits of v on axis a (+ sign bit 24).
 int pack_rows(int v, const TabLayout& T, int a) {
@@ -504,6 +509,13 @@ int cco_device_count(int* n_devices) {
 
 int cco_problem_create(int device, int d, int n_particles, int m, const int32_t* n_vectors,
                        const double* weights, double volume, cco_problem** out) {
+  return cco_problem_create_rows(device, d, n_particles, m, n_vectors, weights, volume, m, nullptr,
+                                 out);
+}
+
+int cco_problem_create_rows(int device, int d, int n_particles, int m, const int32_t* n_vectors,
+                            const double* weights, double volume, int total, const int32_t* rows,
+                            cco_problem** out) {
   if (!out) return fail(CCO_ERR_ARG, "out is null");
   *out = nullptr;
   if (d < 1 || d > 3) return fail(CCO_ERR_ARG, "d must be 1, 2 or 3, got %d", d);
@@ -511,6 +523,14 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
   if (m < 1) return fail(CCO_ERR_ARG, "empty k-set: no k-vectors in the shell");
   if (!n_vectors || !weights) return fail(CCO_ERR_ARG, "null k-set arrays");
   if (!(volume > 0.0) || !std::isfinite(volume)) return fail(CCO_ERR_ARG, "volume must be finite and > 0");
+  if (total < m) return fail(CCO_ERR_ARG, "total %d below the %d rows", total, m);
+  std::vector<int> row_of(total, -1);   // padded column -> row, then run-order row
+  for (int k = 0; k < m; ++k) {
+    const int c = rows ? rows[k] : k;
+    if (c < 0 || c >= total || row_of[c] >= 0)
+      return fail(CCO_ERR_ARG, "row %d: column %d is out of range or taken", k, c);
+    row_of[c] = k;
+  }
   int ndev = 0;
   if (cco_device_count(&ndev) != CCO_OK) return CCO_ERR_NODEVICE;
   if (device < 0 || device >= ndev) return fail(CCO_ERR_ARG, "device %d out of range", device);
@@ -653,39 +673,41 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
     const int32_t* nv = n_vectors + (size_t)order[k] * d;
     krow[k] = make_double4(nv[0], d > 1 ? nv[1] : 0, d > 2 ? nv[2] : 0, w_run[k]);
   }
-  cudaError_t e = cudaSuccess;
-  e = cudaMalloc(&pr->seg1, s1.size() * sizeof(SegHdr));
-  if (e == cudaSuccess) e = cudaMalloc(&pr->seg2, s2.size() * sizeof(SegHdr));
-  if (e == cudaSuccess) e = cudaMalloc(&pr->w_run, m * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&pr->run2ref, m * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&pr->dev, sizeof(ProbDev));
-  if (e == cudaSuccess) e = cudaMemcpy(pr->seg1, s1.data(), s1.size() * sizeof(SegHdr), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(pr->seg2, s2.data(), s2.size() * sizeof(SegHdr), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(pr->w_run, w_run.data(), m * sizeof(double), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(pr->run2ref, r2r.data(), m * sizeof(int), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&pr->krow, m * sizeof(double4));
-  if (e == cudaSuccess) e = cudaMemcpy(pr->krow, krow.data(), m * sizeof(double4), cudaMemcpyHostToDevice);
-  if (P.grid) {
-    if (e == cudaSuccess) e = to_device(&pr->grun, gp.runs);
-    if (e == cudaSuccess) e = to_device(&pr->gblk, gp.blocks);
-    if (e == cudaSuccess) e = to_device(&pr->gstrip, gp.strips);
-    if (e == cudaSuccess) e = to_device(&pr->gquad, gp.quads);
-    if (e == cudaSuccess) e = to_device(&pr->grow, gp.rows);
-    if (e == cudaSuccess) e = to_device(&pr->gline, gp.lines);
-    if (e == cudaSuccess) e = to_device(&pr->gslotk, gp.slotk);
+  std::vector<int> run_of(m);
+  for (int k = 0; k < m; ++k) run_of[order[k]] = k;
+  for (int& c : row_of)
+    if (c >= 0) c = run_of[c];
+  pr->run2ref = r2r;
+  pr->total = total;
+  // one device block for everything the problem uploads
+  Blob blob;
+  const size_t o_seg1 = blob.add(s1), o_seg2 = blob.add(s2), o_w = blob.add(w_run),
+               o_r2r = blob.add(r2r), o_krow = blob.add(krow), o_row = blob.add(row_of),
+               o_grun = blob.add(gp.runs), o_gblk = blob.add(gp.blocks),
+               o_gstrip = blob.add(gp.strips), o_gquad = blob.add(gp.quads),
+               o_grow = blob.add(gp.rows), o_gline = blob.add(gp.lines),
+               o_gslotk = blob.add(gp.slotk);
+  const size_t o_dev = blob.add(std::vector<ProbDev>(1));
+  cudaError_t e = cudaMalloc(&pr->block, blob.bytes.size());
+  auto at = [&](size_t o) { return static_cast<void*>(pr->block + o); };
+  if (e == cudaSuccess) {
+    P.seg1 = static_cast<SegHdr*>(at(o_seg1));
+    P.seg2 = static_cast<SegHdr*>(at(o_seg2));
+    P.w_run = static_cast<double*>(at(o_w));
+    P.run2ref = static_cast<int*>(at(o_r2r));
+    P.grun = static_cast<GridRun*>(at(o_grun));
+    P.gblk = static_cast<GridBlock*>(at(o_gblk));
+    P.gstrip = static_cast<GridStrip*>(at(o_gstrip));
+    P.gquad = static_cast<GridQuad*>(at(o_gquad));
+    P.grow = static_cast<GridRow*>(at(o_grow));
+    P.gline = static_cast<GridLine*>(at(o_gline));
+    P.gslotk = static_cast<int2*>(at(o_gslotk));
+    pr->krow = static_cast<double4*>(at(o_krow));
+    pr->row_of = static_cast<int*>(at(o_row));
+    pr->dev = static_cast<ProbDev*>(at(o_dev));
+    memcpy(blob.bytes.data() + o_dev, &P, sizeof(ProbDev));
+    e = cudaMemcpy(pr->block, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice);
   }
-  P.grun = pr->grun;
-  P.gblk = pr->gblk;
-  P.gstrip = pr->gstrip;
-  P.gquad = pr->gquad;
-  P.grow = pr->grow;
-  P.gline = pr->gline;
-  P.gslotk = pr->gslotk;
-  P.seg1 = pr->seg1;
-  P.seg2 = pr->seg2;
-  P.w_run = pr->w_run;
-  P.run2ref = pr->run2ref;
-  if (e == cudaSuccess) e = cudaMemcpy(pr->dev, &P, sizeof(ProbDev), cudaMemcpyHostToDevice);
   pr->host = P;
   pr->smem1 = smem1;
   pr->smem2 = smem2;
@@ -703,19 +725,7 @@ int cco_problem_create(int device, int d, int n_particles, int m, const int32_t*
 int cco_problem_destroy(cco_problem* p) {
   if (!p) return CCO_OK;
   DeviceGuard guard(p->device);
-  cudaFree(p->seg1);
-  cudaFree(p->seg2);
-  cudaFree(p->w_run);
-  cudaFree(p->run2ref);
-  if (p->grun) cudaFree(p->grun);
-  if (p->gblk) cudaFree(p->gblk);
-  if (p->gstrip) cudaFree(p->gstrip);
-  if (p->gquad) cudaFree(p->gquad);
-  if (p->grow) cudaFree(p->grow);
-  if (p->gline) cudaFree(p->gline);
-  if (p->gslotk) cudaFree(p->gslotk);
-  if (p->krow) cudaFree(p->krow);
-  cudaFree(p->dev);
+  cudaFree(p->block);
   delete p;
   return CCO_OK;
 }
@@ -773,6 +783,8 @@ __global__ void k_make_lanes(EvalLane* lanes, EvalItem* it1, EvalItem* it2, int 
   }
 }
 
+size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
+
 // Device buffers of one batched evaluation: densities, partials and the plan.
 // One problem and one arithmetic, so every lane takes the same form: it1 and
 // it2 hold the items of that form's two passes.
@@ -783,7 +795,8 @@ struct EvalWS {
   double2* rho = nullptr;
   double2* rhow = nullptr;
   double2* part = nullptr;
-  double2* roots = nullptr;   // after the partials
+  double2* roots = nullptr;
+  unsigned char* block = nullptr;   // the allocation that holds them (null: the caller's memory)
   EvalPlan plan{};
   int prec = PREC_FP64;   // arithmetic of every lane of this workspace
 
@@ -806,15 +819,38 @@ struct EvalWS {
     z.roots = z.grid ? eval_roots_words(h) : 0;
     return z;
   }
-  cudaError_t alloc(const cco_problem* p, int B, cudaStream_t st) {
+  // Byte offsets of the buffers in one block of memory.
+  struct Carve {
+    size_t it1, it2, rho, rhow, part, roots, total;
+  };
+  static Carve carve(const cco_problem* p, int B, int prec) {
     const Sizes z = sizes(p, B, prec);
-    cudaError_t e = pool_alloc(&lanes, sizeof(EvalLane) * B, st);
-    if (e == cudaSuccess) e = pool_alloc(&it1, sizeof(EvalItem) * (size_t)B * z.nt1, st);
-    if (e == cudaSuccess) e = pool_alloc(&it2, sizeof(EvalItem) * (size_t)B * z.nt2, st);
-    if (e == cudaSuccess) e = pool_alloc(&rho, sizeof(double2) * (size_t)B * p->M, st);
-    if (e == cudaSuccess) e = pool_alloc(&rhow, sizeof(double2) * (size_t)B * z.rhow, st);
-    if (e == cudaSuccess) e = pool_alloc(&part, sizeof(double2) * (size_t)B * (z.part + z.roots), st);
-    if (e == cudaSuccess) roots = part + (size_t)B * z.part;
+    Carve c;
+    c.it1 = round256(sizeof(EvalLane) * B);
+    c.it2 = c.it1 + round256(sizeof(EvalItem) * (size_t)B * z.nt1);
+    c.rho = c.it2 + round256(sizeof(EvalItem) * (size_t)B * z.nt2);
+    c.rhow = c.rho + round256(sizeof(double2) * (size_t)B * p->M);
+    c.part = c.rhow + round256(sizeof(double2) * (size_t)B * z.rhow);
+    c.roots = c.part + round256(sizeof(double2) * (size_t)B * z.part);
+    c.total = c.roots + round256(sizeof(double2) * (size_t)B * z.roots);
+    return c;
+  }
+  void place(unsigned char* base, const Carve& c) {
+    lanes = reinterpret_cast<EvalLane*>(base);
+    it1 = reinterpret_cast<EvalItem*>(base + c.it1);
+    it2 = reinterpret_cast<EvalItem*>(base + c.it2);
+    rho = reinterpret_cast<double2*>(base + c.rho);
+    rhow = reinterpret_cast<double2*>(base + c.rhow);
+    part = reinterpret_cast<double2*>(base + c.part);
+    roots = reinterpret_cast<double2*>(base + c.roots);
+  }
+  // one stream-ordered allocation per evaluation (six and their frees took a
+  // third of a small call's host time), `extra` bytes of the caller's in front
+  cudaError_t alloc(const cco_problem* p, int B, cudaStream_t st, size_t extra = 0) {
+    const Carve c = carve(p, B, prec);
+    const size_t front = round256(extra);
+    const cudaError_t e = pool_alloc(&block, front + c.total, st);
+    if (e == cudaSuccess) place(block + front, c);
     return e;
   }
   cudaError_t build(const cco_problem* p, int B, const double* s, size_t s_stride, double* f,
@@ -860,15 +896,33 @@ struct EvalWS {
     return cudaGetLastError();
   }
   void release(cudaStream_t st) {
-    cudaFreeAsync(lanes, st);
-    cudaFreeAsync(it1, st);
-    cudaFreeAsync(it2, st);
-    cudaFreeAsync(rho, st);
-    cudaFreeAsync(rhow, st);
-    cudaFreeAsync(part, st);
-    lanes = nullptr;
+    if (block) cudaFreeAsync(block, st);
+    block = nullptr;
   }
 };
+
+}  // namespace
+
+namespace {
+
+// One batched evaluation; `after` gets the run-order densities on the stream.
+template <class After>
+int evaluate_batch(cco_problem* p, void* stream, int batch, const double* s, double* phi,
+                   double* grad, After after) {
+  DeviceGuard guard(p->device);
+  cudaStream_t st = (cudaStream_t)stream;
+  EvalWS ws;
+  CCO_CUDA(ws.alloc(p, batch, st, phi ? 0 : sizeof(double) * batch));
+  const size_t nd = (size_t)p->N * p->d;
+  cudaError_t e = ws.build(p, batch, s, nd, phi ? phi : reinterpret_cast<double*>(ws.block), 1, grad,
+                           nd, st);
+  if (e == cudaSuccess) e = eval_launch(ws.plan, st);
+  if (e == cudaSuccess) e = after(ws.rho, st);
+  ws.release(st);
+  CCO_CUDA(e);
+  CCO_CUDA(cudaGetLastError());
+  return CCO_OK;
+}
 
 }  // namespace
 
@@ -878,18 +932,33 @@ extern "C" int cco_energy_grad(cco_problem* p, void* stream, int batch, const do
   if (batch < 0) return fail(CCO_ERR_ARG, "batch must be >= 0");
   if (batch == 0) return CCO_OK;
   if (!s || !phi) return fail(CCO_ERR_ARG, "null s or phi");
-  DeviceGuard guard(p->device);
-  cudaStream_t st = (cudaStream_t)stream;
-  EvalWS ws;
-  CCO_CUDA(ws.alloc(p, batch, st));
-  const size_t nd = (size_t)p->N * p->d;
-  CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, grad, nd, st));
-  CCO_CUDA(eval_launch(ws.plan, st));
-  if (rho_re || rho_im)
-    CCO_CUDA(rho_scatter(ws.rho, p->run2ref, p->M, batch, p->M, rho_re, rho_im, st));
-  ws.release(st);
-  CCO_CUDA(cudaGetLastError());
-  return CCO_OK;
+  return evaluate_batch(p, stream, batch, s, phi, grad, [&](const double2* rho, cudaStream_t st) {
+    if (!rho_re && !rho_im) return cudaSuccess;
+    return rho_scatter(rho, p->host.run2ref, p->M, batch, p->M, rho_re, rho_im, st);
+  });
+}
+
+extern "C" int cco_energy_grad_rows(cco_problem* p, void* stream, int batch, const double* s,
+                                    double* phi, double* grad, double* rho_re, double* rho_im) {
+  if (!p) return fail(CCO_ERR_ARG, "null problem");
+  if (batch < 0) return fail(CCO_ERR_ARG, "batch must be >= 0");
+  if (batch == 0) return CCO_OK;
+  if (!s || !phi) return fail(CCO_ERR_ARG, "null s or phi");
+  return evaluate_batch(p, stream, batch, s, phi, grad, [&](const double2* rho, cudaStream_t st) {
+    if (!rho_re && !rho_im) return cudaSuccess;
+    return rho_rows(rho, p->row_of, p->total, p->M, p->N, batch, rho_re, rho_im, st);
+  });
+}
+
+extern "C" int cco_structure_sums(cco_problem* p, void* stream, int batch, const double* s,
+                                  double* tot, double* tot2) {
+  if (!p) return fail(CCO_ERR_ARG, "null problem");
+  if (batch < 0) return fail(CCO_ERR_ARG, "batch must be >= 0");
+  if (batch == 0) return CCO_OK;
+  if (!s || !tot || !tot2) return fail(CCO_ERR_ARG, "null argument");
+  return evaluate_batch(p, stream, batch, s, nullptr, nullptr, [&](const double2* rho, cudaStream_t st) {
+    return structure_sums(rho, p->host.run2ref, p->M, p->N, batch, tot, tot2, st);
+  });
 }
 
 extern "C" int cco_energy_grad_fp32(cco_problem* p, void* stream, int batch, const double* s,
@@ -921,15 +990,13 @@ extern "C" int cco_hessian(cco_problem* p, void* stream, int batch, const double
   DeviceGuard guard(p->device);
   cudaStream_t st = (cudaStream_t)stream;
   EvalWS ws;
-  double* phi = nullptr;
-  CCO_CUDA(ws.alloc(p, batch, st));
-  CCO_CUDA(pool_alloc(&phi, sizeof(double) * batch, st));
+  CCO_CUDA(ws.alloc(p, batch, st, sizeof(double) * batch));
+  double* phi = reinterpret_cast<double*>(ws.block);
   const size_t nd = (size_t)p->N * p->d;
   CCO_CUDA(ws.build(p, batch, s, nd, phi, 1, nullptr, 0, st));
   CCO_CUDA(eval_launch(ws.plan, st));   // the density the diagonal blocks need
   CCO_CUDA(hessian_launch(p, st, batch, s, ws.rho, hess));
   ws.release(st);
-  cudaFreeAsync(phi, st);
   CCO_CUDA(cudaGetLastError());
   return CCO_OK;
 }
@@ -963,8 +1030,6 @@ int noalloc_scratch(int device, unsigned char** out) {
   return CCO_OK;
 }
 
-size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
-
 }  // namespace
 
 extern "C" int cco_energy_grad_noalloc(cco_problem* p, void* stream, int batch, const double* s,
@@ -996,39 +1061,17 @@ extern "C" int cco_energy_grad_noalloc(cco_problem* p, void* stream, int batch, 
   if (rc != CCO_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nd = (size_t)p->N * p->d;
-  struct Carve {
-    size_t lanes, it1, it2, rho, rhow, part, roots, total;
-  };
-  auto carve = [&](int b) {
-    const EvalWS::Sizes z = EvalWS::sizes(p, b, PREC_FP64);
-    Carve c;
-    c.lanes = 0;
-    c.it1 = round256(sizeof(EvalLane) * b);
-    c.it2 = c.it1 + round256(sizeof(EvalItem) * (size_t)b * z.nt1);
-    c.rho = c.it2 + round256(sizeof(EvalItem) * (size_t)b * z.nt2);
-    c.rhow = c.rho + round256(sizeof(double2) * (size_t)b * M);
-    c.part = c.rhow + round256(sizeof(double2) * (size_t)b * z.rhow);
-    c.roots = c.part + sizeof(double2) * (size_t)b * z.part;
-    c.total = c.roots + round256(sizeof(double2) * (size_t)b * z.roots);
-    return c;
-  };
   int part_b = batch;
-  while (part_b > 1 && carve(part_b).total > CCO_NOALLOC_SCRATCH_BYTES)
+  while (part_b > 1 && EvalWS::carve(p, part_b, PREC_FP64).total > CCO_NOALLOC_SCRATCH_BYTES)
     part_b = (part_b + 1) / 2;
-  const Carve c = carve(part_b);
+  const EvalWS::Carve c = EvalWS::carve(p, part_b, PREC_FP64);
   if (c.total > CCO_NOALLOC_SCRATCH_BYTES)
     return fail(CCO_ERR_ARG, "one configuration needs %zu bytes of fixed scratch, the limit is %zu",
                 c.total, (size_t)CCO_NOALLOC_SCRATCH_BYTES);
   for (int lo = 0; lo < batch; lo += part_b) {
     const int b = std::min(part_b, batch - lo);
     EvalWS ws;  // carved from the fixed scratch; never released
-    ws.lanes = reinterpret_cast<EvalLane*>(base + c.lanes);
-    ws.it1 = reinterpret_cast<EvalItem*>(base + c.it1);
-    ws.it2 = reinterpret_cast<EvalItem*>(base + c.it2);
-    ws.rho = reinterpret_cast<double2*>(base + c.rho);
-    ws.rhow = reinterpret_cast<double2*>(base + c.rhow);
-    ws.part = reinterpret_cast<double2*>(base + c.part);
-    ws.roots = reinterpret_cast<double2*>(base + c.roots);
+    ws.place(base, c);
     CCO_CUDA(ws.build(p, b, s + (size_t)lo * nd, nd, phi + lo, 1,
                       grad ? grad + (size_t)lo * nd : nullptr, nd, st));
     CCO_CUDA(eval_launch(ws.plan, st));

@@ -280,6 +280,42 @@ __global__ void k_rho_scatter(const double2* __restrict__ rho, const int* __rest
   }
 }
 
+__global__ void k_rho_rows(const double2* __restrict__ rho, const int* __restrict__ row_of,
+                           int total, int M, double n, double* re, double* im) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+  if (c >= total) return;
+  const int k = row_of[c];
+  const double2 v = k >= 0 ? rho[(size_t)b * M + k] : make_double2(n, 0.0);
+  if (re) re[(size_t)b * total + c] = v.x;
+  if (im) im[(size_t)b * total + c] = v.y;
+}
+
+// One thread per row walks the batch, eight densities in flight, so the sums
+// are a sequential scan of the configurations. One pass over the densities
+// where separate array operations took three launches per configuration.
+__global__ void k_structure_sums(const double2* __restrict__ rho, const int* __restrict__ run2ref,
+                                 int M, double n, int batch, double* tot, double* tot2) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= M) return;
+  const int o = run2ref[k];
+  double t = tot[o], t2 = tot2[o];
+  for (int b0 = 0; b0 < batch; b0 += 8) {
+    double2 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (b0 + u < batch) v[u] = rho[(size_t)(b0 + u) * M + k];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (b0 + u < batch) {
+        const double sk = __dadd_rn(__dmul_rn(v[u].x, v[u].x), __dmul_rn(v[u].y, v[u].y)) / n;
+        t = __dadd_rn(t, sk);
+        t2 = __dadd_rn(t2, __dmul_rn(sk, sk));
+      }
+  }
+  tot[o] = t;
+  tot2[o] = t2;
+}
+
 }  // namespace
 
 int pass1_slices(int nseg, int nj) {
@@ -465,6 +501,24 @@ cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream, const EvalSid
     e = launch_pass_all(plan, true, stream, side);
     if (e != cudaSuccess) return e;
   }
+  return cudaGetLastError();
+}
+
+cudaError_t rho_rows(const double2* rho_run, const int* row_of, int total, int M, int N, int batch,
+                     double* re, double* im, cudaStream_t stream) {
+  for (int lo = 0; lo < batch; lo += 65535) {
+    const int b = std::min(batch - lo, 65535);
+    k_rho_rows<<<dim3((total + 127) / 128, b), 128, 0, stream>>>(
+        rho_run + (size_t)lo * M, row_of, total, M, (double)N, re ? re + (size_t)lo * total : nullptr,
+        im ? im + (size_t)lo * total : nullptr);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t structure_sums(const double2* rho_run, const int* run2ref, int M, int N, int batch,
+                           double* tot, double* tot2, cudaStream_t stream) {
+  k_structure_sums<<<(M + 127) / 128, 128, 0, stream>>>(rho_run, run2ref, M, (double)N, batch, tot,
+                                                        tot2);
   return cudaGetLastError();
 }
 

@@ -20,19 +20,12 @@ struct cco_problem {
   int device = 0;
   int d = 0, N = 0, M = 0;
   cco::ProbDev host{};         // pointers are device pointers
+  unsigned char* block = nullptr;   // the device memory all of these lie in
   cco::ProbDev* dev = nullptr; // device copy
-  cco::SegHdr* seg1 = nullptr;
-  cco::SegHdr* seg2 = nullptr;
-  double* w_run = nullptr;
-  int* run2ref = nullptr;
-  cco::GridRun* grun = nullptr;
-  cco::GridBlock* gblk = nullptr;
-  cco::GridStrip* gstrip = nullptr;
-  cco::GridQuad* gquad = nullptr;
-  cco::GridRow* grow = nullptr;
-  cco::GridLine* gline = nullptr;
-  int2* gslotk = nullptr;
   double4* krow = nullptr;     // run-order rows (n_0, n_1, n_2, w) for the Hessian kernels
+  int total = 0;               // columns of the padded row layout, and each one's
+  int* row_of = nullptr;       // run-order row (-1: zero row)
+  std::vector<int> run2ref;    // host copy
   size_t smem1 = 0, smem2 = 0, smemG = 0, smemH = 0;
   int dense_blocks = 0;        // cco_problem_pass1_form
 };

@@ -338,6 +338,15 @@ constexpr long long kPass2TargetCtas = 148 * 3;
 int pass2_split(long long tiles_at_split1);
 cudaError_t eval_configure();   // opt-in to large dynamic shared memory
 
+// The run-order densities in a padded layout: column c holds row row_of[c], or
+// (N, 0) where that is -1.
+cudaError_t rho_rows(const double2* rho_run, const int* row_of, int total, int M, int N, int batch,
+                     double* re, double* im, cudaStream_t stream);
+// tot[k] += |rho_k|^2 / N and tot2[k] += its square over the batch, in batch
+// order, k in the caller's row order.
+cudaError_t structure_sums(const double2* rho_run, const int* run2ref, int M, int N, int batch,
+                           double* tot, double* tot2, cudaStream_t stream);
+
 // Copy the run-order density of lane i out in the caller's row order.
 cudaError_t rho_scatter(const double2* rho_run, const int* run2ref, int M,
                         int batch, size_t lane_stride, double* re, double* im,

@@ -1147,9 +1147,8 @@ extern "C" int cco_md_segment(cco_problem* p, void* stream, int batch, const dou
   DeviceGuard guard(p->device);
   cudaStream_t st = (cudaStream_t)stream;
   // run position of each constrained wave's density
-  std::vector<int> r2r(p->M), pos(p->M), cpos(nc);
-  CCO_CUDA(cudaMemcpy(r2r.data(), p->run2ref, sizeof(int) * p->M, cudaMemcpyDeviceToHost));
-  for (int k = 0; k < p->M; ++k) pos[r2r[k]] = k;
+  std::vector<int> pos(p->M), cpos(nc);
+  for (int k = 0; k < p->M; ++k) pos[p->run2ref[k]] = k;
   for (int c = 0; c < nc; ++c) {
     const int row = wv->constrained_rows[c];
     if (row < 0 || row >= p->M) return fail(CCO_ERR_ARG, "constrained wave %d: row %d outside the problem", c, row);

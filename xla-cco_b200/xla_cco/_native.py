@@ -191,9 +191,16 @@ SIGNATURES = {
         [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, _vp, ctypes.c_double,
          ctypes.POINTER(_vp)],
     ),  # fmt: skip
+    "cco_problem_create_rows": (
+        ctypes.c_int,
+        [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, _vp, ctypes.c_double,
+         ctypes.c_int, _vp, ctypes.POINTER(_vp)],
+    ),  # fmt: skip
     "cco_problem_destroy": (ctypes.c_int, [_vp]),
     "cco_problem_info": (ctypes.c_int, [_vp, _c_int_p, _c_int_p, _c_int_p, _c_int_p, _c_int_p, _c_int_p]),
     "cco_energy_grad": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp]),
+    "cco_energy_grad_rows": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp]),
+    "cco_structure_sums": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp]),
     "cco_energy_grad_noalloc": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp]),
     "cco_energy_grad_fp32": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp]),
     "cco_hessian": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp]),

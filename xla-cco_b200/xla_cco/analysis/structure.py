@@ -106,12 +106,17 @@ def _sk_moments(s: Any, n_vec: np.ndarray) -> Tuple[np.ndarray, np.ndarray]:
     chunk = max(1, min(b, _SCRATCH_BYTES // (16 * m * (tiles + 3))))
     tot = torch.zeros(m, dtype=torch.float64, device=st.device)
     tot2 = torch.zeros_like(tot)
-    for lo in range(0, b, chunk):
-        _, _, re, im = en.evaluate(st[lo:lo + chunk], want_grad=False, want_rho=True)
-        sk = (re * re + im * im) / n
-        for row in sk:   # configuration order, as a sequential scan
-            tot = tot + row
-            tot2 = tot2 + row * row
+    # configuration order, as a sequential scan; one device call per chunk
+    st = st.contiguous()
+    dev = st.device.index if st.device.index is not None else torch.cuda.current_device()
+    h = en.problem_handle(dev, n)
+    with torch.cuda.device(dev):
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        for lo in range(0, b, chunk):
+            hi = min(b, lo + chunk)
+            code = _native.load().cco_structure_sums(h, stream, hi - lo, st[lo:hi].data_ptr(),
+                                                     tot.data_ptr(), tot2.data_ptr())  # fmt: skip
+            _native.check(code, "cco_structure_sums")
     return (tot / b).cpu().numpy(), (tot2 / b).cpu().numpy()
 
 

@@ -90,7 +90,7 @@ class _Problems:
         self._handles: Dict[Tuple[int, int], int] = {}
 
     def get(self, device: int, n_particles: int, n_rows: np.ndarray, w_rows: np.ndarray,
-            volume: float) -> int:  # fmt: skip
+            volume: float, rows: np.ndarray, total: int) -> int:  # fmt: skip
         key = (device, n_particles)
         with self._lock:
             h = self._handles.get(key)
@@ -99,10 +99,13 @@ class _Problems:
             lib = _native.load()
             n32 = np.ascontiguousarray(n_rows, dtype=np.int32)
             w64 = np.ascontiguousarray(w_rows, dtype=np.float64)
+            # the densities' padded layout: zero rows included, the caller's order
+            r32 = np.ascontiguousarray(rows, dtype=np.int32)
             out = _native._vp()
-            code = lib.cco_problem_create(
+            code = lib.cco_problem_create_rows(
                 device, int(n32.shape[1]), int(n_particles), int(n32.shape[0]),
-                n32.ctypes.data, w64.ctypes.data, float(volume), _native.ctypes.byref(out),
+                n32.ctypes.data, w64.ctypes.data, float(volume), int(total), r32.ctypes.data,
+                _native.ctypes.byref(out),
             )  # fmt: skip
             _native.check(code, "cco_problem_create")
             self._handles[key] = int(out.value)
@@ -172,7 +175,7 @@ class StealthyEnergy(AbstractEnergy):
         if self._rows.size == 0:
             raise ValueError("empty k-set: no k-vectors in the shell")
         return self._problems.get(device, n_particles, self._n_int, self._w_dev,
-                                  float(self.volume))  # fmt: skip
+                                  float(self.volume), self._rows, self.n_vectors.shape[0])  # fmt: skip
 
     def evaluate(self, s: Any, want_grad: bool = True, want_rho: bool = False):
         """Batched evaluation: ``s`` is (B, N, d) float64 (NumPy or CUDA tensor).
@@ -193,32 +196,24 @@ class StealthyEnergy(AbstractEnergy):
         b, n, d = st.shape
         dev = st.device.index if st.device.index is not None else torch.cuda.current_device()
         h = self.problem_handle(dev, n)
-        m_dev = int(self._rows.size)
         with torch.cuda.device(dev):
             phi = torch.empty(b, dtype=torch.float64, device=st.device)
             grad = torch.empty_like(st) if want_grad else None
-            re_d = torch.empty((b, m_dev), dtype=torch.float64, device=st.device) if want_rho else None
-            im_d = torch.empty((b, m_dev), dtype=torch.float64, device=st.device) if want_rho else None
+            re = im = None
+            if want_rho:   # every row, padding rows included, written by the device
+                mp = self.n_vectors.shape[0]
+                re = torch.empty((b, mp), dtype=torch.float64, device=st.device)
+                im = torch.empty((b, mp), dtype=torch.float64, device=st.device)
             stream = torch.cuda.current_stream(dev).cuda_stream
-            code = _native.load().cco_energy_grad(
+            code = _native.load().cco_energy_grad_rows(
                 h, stream, b, st.data_ptr(), phi.data_ptr(),
                 grad.data_ptr() if grad is not None else None,
-                re_d.data_ptr() if re_d is not None else None,
-                im_d.data_ptr() if im_d is not None else None,
+                re.data_ptr() if re is not None else None,
+                im.data_ptr() if im is not None else None,
             )  # fmt: skip
-            _native.check(code, "cco_energy_grad")
+            _native.check(code, "cco_energy_grad_rows")
             if self._zero_weight != 0.0:
                 phi = phi + self._zero_weight * float(n) * float(n) / float(self.volume)
-            re = im = None
-            if want_rho:
-                mp = self.n_vectors.shape[0]
-                re = torch.zeros((b, mp), dtype=torch.float64, device=st.device)
-                im = torch.zeros((b, mp), dtype=torch.float64, device=st.device)
-                rows = torch.as_tensor(self._rows, device=st.device)
-                re[:, rows] = re_d
-                im[:, rows] = im_d
-                if self._zero_rows.size:
-                    re[:, torch.as_tensor(self._zero_rows, device=st.device)] = float(n)
         if host:
             to = lambda t: None if t is None else t.cpu().numpy()  # noqa: E731
             return to(phi), to(grad), to(re), to(im)
