@@ -125,6 +125,21 @@ int cco_structure_sums(cco_problem* p, void* stream, int batch, const double* s,
                        double* tot, double* tot2);
 
 /*
+ * Host halves of the isotropic structure factor (no device; host pointers;
+ * src/xla_cco/analysis/structure.py:113-201).
+ * cco_isotropic_rows: the multiples i n, i = 1, 2, ..., of each direction (dir
+ * [n_dir][d], its vector k_dir, |k|^2 q_dir) with |i k|^2 <= limit, in order, at
+ * most `cap`: rows n_vec [count][d], their |i k|^2.
+ * cco_bin_sums: per bin floor(k / width) of `nb`, sums [nb][5] += 1, k, S, k^2,
+ * S^2 in row order.
+ */
+int cco_isotropic_rows(int d, int n_dir, const int64_t* dir, const double* k_dir,
+                       const double* q_dir, double limit, int64_t cap, double* n_vec,
+                       double* sq, int64_t* count);
+int cco_bin_sums(int64_t m, const double* k, const double* s, const double* s2,
+                 double width, int64_t nb, double* sums);
+
+/*
  * Closed-form Hessian d2 Phi / ds_ja ds_lb of `batch` configurations
  *   <- StealthyEnergy.hessian             src/xla_cco/energy.py:272-299
  * (the Jacobian of the ROS2 gradient flow, src/xla_cco/minimize/flow.py:367-398).

@@ -200,6 +200,12 @@ SIGNATURES = {
     "cco_problem_info": (ctypes.c_int, [_vp, _c_int_p, _c_int_p, _c_int_p, _c_int_p, _c_int_p, _c_int_p]),
     "cco_energy_grad": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp]),
     "cco_energy_grad_rows": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp]),
+    "cco_isotropic_rows": (
+        ctypes.c_int,
+        [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, ctypes.c_double, ctypes.c_int64, _vp, _vp,
+         ctypes.POINTER(ctypes.c_int64)],
+    ),  # fmt: skip
+    "cco_bin_sums": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, _vp, ctypes.c_double, ctypes.c_int64, _vp]),
     "cco_structure_sums": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp]),
     "cco_energy_grad_noalloc": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp]),
     "cco_energy_grad_fp32": (ctypes.c_int, [_vp, _vp, ctypes.c_int, _vp, _vp, _vp]),

@@ -15,6 +15,7 @@ from typing import Any, Tuple
 
 import numpy as np
 
+from xla_cco import _native
 from xla_cco._types import require_float64
 from xla_cco.box import Box
 from xla_cco.energy import _density_energy, collective_density
@@ -76,24 +77,24 @@ def _isotropic_kset(basis: np.ndarray, k_dir_max: float, k_max: float):
     if n_dir.shape[0] == 0:
         raise ValueError("no reciprocal-lattice vector below k_dir_max")
     limit = k_max * k_max
-    rows, sq = [], []
-    for nv, kv, q in zip(n_dir, k_dir, q_dir):
-        i = np.arange(1, int(math.sqrt(limit / q)) + 3, dtype=np.float64)
-        m2 = np.zeros(i.size)
-        for c in range(kv.size):
-            comp = i * kv[c]
-            m2 = m2 + comp * comp
-        keep = m2 <= limit
-        rows.append(i[keep, None] * nv[None, :].astype(np.float64))
-        sq.append(m2[keep])
-    return np.concatenate(rows), np.concatenate(sq)
+    d = k_dir.shape[1]
+    # every multiple of every direction, one native pass in direction order
+    cap = int((np.sqrt(limit / q_dir).astype(np.int64) + 2).sum())
+    n_vec, sq = np.empty((cap, d)), np.empty(cap)
+    dirs = np.ascontiguousarray(n_dir, dtype=np.int64)
+    kd = np.ascontiguousarray(k_dir, dtype=np.float64)
+    qd = np.ascontiguousarray(q_dir, dtype=np.float64)
+    got = _native.ctypes.c_int64(0)
+    code = _native.load().cco_isotropic_rows(
+        d, dirs.shape[0], dirs.ctypes.data, kd.ctypes.data, qd.ctypes.data, limit, cap,
+        n_vec.ctypes.data, sq.ctypes.data, _native.ctypes.byref(got))  # fmt: skip
+    _native.check(code, "cco_isotropic_rows")
+    return n_vec[:got.value], sq[:got.value]
 
 
 def _sk_moments(s: Any, n_vec: np.ndarray) -> Tuple[np.ndarray, np.ndarray]:
     """Config means of S and S^2 per k (M,), summed over configs in order."""
     import torch
-
-    from xla_cco import _native
 
     _native.require_gpu()
     b, n = int(s.shape[0]), int(s.shape[1])
@@ -124,19 +125,17 @@ def _bin_moments(k_mod: np.ndarray, s_mean: np.ndarray, s2_mean: np.ndarray, n_c
                  bin_width: float) -> Tuple[np.ndarray, ...]:  # fmt: skip
     """C++ binning: per bin, sums over k and configurations; empty bins dropped."""
     assert k_mod.shape == s_mean.shape == s2_mean.shape, "shape mismatch"
-    idx = np.floor(k_mod / bin_width).astype(np.int64)
-    nb = int(idx.max()) + 1
-    cnt = np.bincount(idx, minlength=nb) * float(n_cfg)
-    nz = cnt != 0
-    cnt = cnt[nz]
-
-    def total(v: np.ndarray) -> np.ndarray:
-        return np.bincount(idx, weights=v, minlength=nb)[nz] * n_cfg
-
-    mean_k = total(k_mod) / cnt
-    mean_s = total(s_mean) / cnt
-    var_k = (total(k_mod * k_mod) / cnt - mean_k**2) / cnt
+    k, sm, s2 = (np.ascontiguousarray(x, dtype=np.float64) for x in (k_mod, s_mean, s2_mean))
+    sums = np.zeros((int(np.floor(k.max() / bin_width)) + 1, 5))   # count, k, S, k^2, S^2
+    code = _native.load().cco_bin_sums(k.size, k.ctypes.data, sm.ctypes.data, s2.ctypes.data,
+                                       float(bin_width), sums.shape[0], sums.ctypes.data)  # fmt: skip
+    _native.check(code, "cco_bin_sums")
+    sums = sums[sums[:, 0] != 0] * float(n_cfg)
+    cnt, total = sums[:, 0], sums.T
+    mean_k = total[1] / cnt
+    mean_s = total[2] / cnt
+    var_k = (total[3] / cnt - mean_k**2) / cnt
     err_k = np.sqrt(np.where(var_k > 0.0, var_k, 0.0))
     with np.errstate(invalid="ignore"):
-        err_s = np.sqrt((total(s2_mean) / cnt - mean_s**2) / cnt)
+        err_s = np.sqrt((total[4] / cnt - mean_s**2) / cnt)
     return mean_k, mean_s, err_k, err_s
