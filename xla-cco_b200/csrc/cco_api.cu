@@ -568,6 +568,10 @@ int cco_problem_create_rows(int device, int d, int n_particles, int m, const int
   P.d = d;
   P.N = n_particles;
   P.M = m;
+  for (int a = 0; a < 3; ++a) P.rmax[a] = R[a];
+  P.compact = compact_smem(P) > kPersistMaxSmem                              ? 0
+              : compact_smem(P) + compact_phase_smem(P) > kPersistMaxSmem ? 1
+                                                                          : 2;
   {
     const int Rv[3] = {R[0], R[1], R[2]};
     P.t1 = make_layout(Rv, d, (int)(kPass1TableBudget / (kPass1Stride * sizeof(double2))));
@@ -703,6 +707,7 @@ int cco_problem_create_rows(int device, int d, int n_particles, int m, const int
     P.gline = static_cast<GridLine*>(at(o_gline));
     P.gslotk = static_cast<int2*>(at(o_gslotk));
     pr->krow = static_cast<double4*>(at(o_krow));
+    P.krow = pr->krow;
     pr->row_of = static_cast<int*>(at(o_row));
     pr->dev = static_cast<ProbDev*>(at(o_dev));
     memcpy(blob.bytes.data() + o_dev, &P, sizeof(ProbDev));

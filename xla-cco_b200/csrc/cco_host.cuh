@@ -331,7 +331,12 @@ constexpr double kPersistMaxFlops = 2.5e5;          // N M F_pair(d) per evaluat
 constexpr size_t kPersistMaxSmem = 200 * 1024;      // dynamic shared memory of the launch
 bool persist_eligible(const cco_problem* p);
 size_t persist_smem(const cco_problem* p);
-// One launch per dimension present (bit d-1 of `dims`) over a.B lanes;
+// Dynamic shared memory of the compact form (the whole lane in shared memory);
+// problems whose lanes fit kPersistMaxSmem take it.
+size_t compact_smem(const ProbDev& p);
+size_t compact_phase_smem(const ProbDev& p);   // on top, if the phases are kept
+// One launch per dimension present (bit d-1 of `dims`; bit 2 + d: of the compact
+// form) over a.B lanes;
 // *d_overrun is set to 1 if a lane reached max_ticks while still RUNNING.
 cudaError_t persist_descent(const DescentArgs& a, const EvalPlan& plan, size_t smem, int dims,
                             int64_t max_ticks, int* d_overrun, cudaStream_t st);

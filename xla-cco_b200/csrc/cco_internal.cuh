@@ -117,6 +117,9 @@ struct ProbDev {
   const GridRow* grow;
   const GridLine* gline;     // line grids: per strip; and per slot its rows n = +c, -c (-1: none)
   const int2* gslotk;
+  int rmax[3];               // largest |n| per axis
+  int compact;               // descent lanes run k_persist_compact (2: and keep their phases)
+  const double4* krow;       // run-order rows (n_0, n_1, n_2, w)
   double vol;                // V
   double gpref;              // 2 (2 pi) / V
   const SegHdr* seg1;

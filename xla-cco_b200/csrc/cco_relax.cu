@@ -605,7 +605,7 @@ struct PersistRun {
         small.push_back(T.refs[i]);
         sprobs.push_back(p);
         smem = std::max(smem, persist_smem(p));
-        dims |= 1 << (p->d - 1);
+        dims |= 1 << (p->d - 1 + (p->host.compact ? 3 : 0));
       } else {
         large.refs.push_back(T.refs[i]);
         large.probs.push_back(p);
