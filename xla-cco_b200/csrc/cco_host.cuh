@@ -280,7 +280,7 @@ struct EvalSet {
 
 // ------------------------------------------------------------ tick schedule
 // A tick evaluates every RUNNING lane once and runs its minimizer update.
-// Ticks are captured into CUDA graphs of `graph_ticks` ticks, with the lanes
+// Ticks are launched as CUDA graphs of up to `graph_ticks` ticks, with the lanes
 // split into `branches` independent graph branches so that one branch's
 // FP64-bound evaluation overlaps another branch's HBM-bound update.
 struct Schedule {
@@ -341,8 +341,9 @@ size_t compact_phase_smem(const ProbDev& p);   // on top, if the phases are kept
 cudaError_t persist_descent(const DescentArgs& a, const EvalPlan& plan, size_t smem, int dims,
                             int64_t max_ticks, int* d_overrun, cudaStream_t st);
 
-// One schedule of a lane table captured as an executable graph of
-// sch.graph_ticks ticks.
+// One schedule of a lane table as an executable graph: a loop on the device
+// over a body of `body` ticks, run until sch.graph_ticks ticks are done or no
+// lane of the table is RUNNING.
 struct TickPlan {
   Method method = Method::Lbfgs;
   Schedule sch;
@@ -354,11 +355,16 @@ struct TickPlan {
   FlArgs fl[kMaxBranches];
   MdArgs md[kMaxBranches];
   cudaGraphExec_t exec = nullptr;
+  cudaGraph_t graph = nullptr;   // owns the loop's condition: outlives the launches
+  TickLoop* loop = nullptr;
+  int body = 1, bodies = 1;      // ticks of the body, bodies of one launch
   int build(const LaneTable& T, const Schedule& sch, cudaStream_t st);
   cudaError_t tick(cudaStream_t s, int b, const EvalSide* side = nullptr) const;
   cudaError_t update(cudaStream_t s, int b) const;
   int launches_per_tick() const;
+  int loop_gates() const { return bodies > 1; }   // condition kernels per body
   void release(cudaStream_t st);
+  void retire(cudaStream_t st, std::vector<cudaGraph_t>* graphs);   // launches in flight
 };
 
 struct RunStats {

@@ -997,9 +997,25 @@ __global__ void k_count_running(const LaneRef* lanes, int B, int* out) {
   if (threadIdx.x == 0) *out = (int)c;
 }
 
-__global__ void k_gather_status(const LaneRef* lanes, int B, int64_t* out) {
+__global__ void k_gather_status(const LaneRef* lanes, int B, int64_t* out, const int64_t* extra) {
+  if (extra && blockIdx.x == 0 && threadIdx.x == 0) out[B] = *extra;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B; i += gridDim.x * blockDim.x)
     out[i] = *rec_status(lanes[i].rec);
+}
+
+__global__ void k_tick_gate(const LaneRef* lanes, int B, TickLoop* loop, int first, int bodies,
+                            cudaGraphConditionalHandle h) {
+  int run = 0;
+  for (int i = threadIdx.x; i < B; i += blockDim.x)
+    run |= *rec_status(lanes[i].rec) == CCO_STATUS_RUNNING;
+  run = __syncthreads_or(run);
+  if (threadIdx.x == 0) {
+    const int left = first ? bodies : loop->left - 1;
+    const bool go = run && left > 0;
+    loop->left = left;
+    loop->done += go;
+    cudaGraphSetConditional(h, go ? 1u : 0u);
+  }
 }
 
 __global__ void k_cancel_lbfgs(double* rec) {
@@ -1059,9 +1075,15 @@ cudaError_t count_running(const LaneRef* lanes, int B, int* out, cudaStream_t st
   k_count_running<<<1, 256, 0, st>>>(lanes, B, out);
   return cudaGetLastError();
 }
-cudaError_t gather_status(const LaneRef* lanes, int B, int64_t* out, cudaStream_t st) {
+cudaError_t gather_status(const LaneRef* lanes, int B, int64_t* out, cudaStream_t st,
+                          const int64_t* extra) {
   int blocks = (B + 255) / 256;
-  k_gather_status<<<blocks < 1 ? 1 : blocks, 256, 0, st>>>(lanes, B, out);
+  k_gather_status<<<blocks < 1 ? 1 : blocks, 256, 0, st>>>(lanes, B, out, extra);
+  return cudaGetLastError();
+}
+cudaError_t tick_gate(const LaneRef* lanes, int B, TickLoop* loop, bool first, int bodies,
+                      cudaGraphConditionalHandle h, cudaStream_t st) {
+  k_tick_gate<<<1, 256, 0, st>>>(lanes, B, loop, first, bodies, h);
   return cudaGetLastError();
 }
 

@@ -219,7 +219,20 @@ cudaError_t lbfgs_finalize(const LbArgs& a, double* s_out, double* e_out, double
 // Count lanes whose status is RUNNING.
 cudaError_t count_running(const LaneRef* lanes, int B, int* out, cudaStream_t st);
 // Copy every lane's status into out[B].
-cudaError_t gather_status(const LaneRef* lanes, int B, int64_t* out, cudaStream_t st);
+// The statuses of the lanes, then (if given) *extra, into out.
+cudaError_t gather_status(const LaneRef* lanes, int B, int64_t* out, cudaStream_t st,
+                          const int64_t* extra = nullptr);
+
+// Progress of a tick loop (device memory of its plan).
+struct TickLoop {
+  int64_t done;   // bodies run since the plan was built
+  int left;       // bodies left in this launch
+  int pad_;
+};
+// Sets the loop's condition: a lane is RUNNING and the launch has bodies left
+// (first: it has `bodies`; else one fewer than before).
+cudaError_t tick_gate(const LaneRef* lanes, int B, TickLoop* loop, bool first, int bodies,
+                      cudaGraphConditionalHandle h, cudaStream_t st);
 // Ends an L-BFGS lane with CCO_STATUS_CANCELLED if it is still RUNNING.
 cudaError_t cancel_lbfgs_lane(double* rec, cudaStream_t st);
 

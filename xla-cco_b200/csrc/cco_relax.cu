@@ -87,6 +87,30 @@ void schedule_clear() {
 }
 
 // ------------------------------------------------------------ tick plans
+namespace {
+
+// Ticks of a loop body. Each body costs about 9 us more (a condition kernel,
+// the loop's own turn, the join of the branches: ticks of 7 empty kernels took
+// 5.9 us in a flat graph, 9.2 / 7.9 / 7.2 us in bodies of 2 / 4 / 8), a run ends
+// up to a body late, and every captured kernel costs host time to instantiate,
+// upload and destroy. So a body holds about 0.6 ms of ticks, estimated from the
+// evaluation's work at 15 TFLOP/s and 2 us per kernel. Bodies of 1 / 2 / 4 / 8 / 16
+// ticks: 11.1 / 11.5 / 12.3 / 14.4 / 18.5 ms for 48 uneven lanes of 20 evaluations
+// (18.7 as one flat graph; the rule takes 1), 8.3 / 8.1 / 8.1 / 8.3 / 8.6 ms for
+// 256 lanes of d=2 N=1000 and 32 evaluations (9.3; the rule takes 4).
+int body_ticks(const std::vector<const cco_problem*>& probs, int launches, int graph_ticks) {
+  double flops = 0.0;
+  for (const cco_problem* p : probs)
+    flops += (double)p->N * p->M * (p->d == 1 ? 7.0 : p->d == 2 ? 21.0 : 35.0);
+  const double us = flops / 15e6 + 2.0 * launches;
+  const int gt = std::max(1, graph_ticks);
+  for (int t = std::max(1, (int)(600.0 / us)); t < gt; ++t)
+    if (gt % t == 0) return t;
+  return gt;
+}
+
+}  // namespace
+
 int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
   release(st);
   this->sch = sch;
@@ -126,8 +150,12 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
       lb[b] = a;
     }
   }
-  // capture graph_ticks ticks of every branch; branches fork from and join
-  // back into the first capture stream
+  body = body_ticks(T.probs, launches_per_tick(), sch.graph_ticks);
+  bodies = std::max(1, sch.graph_ticks) / body;
+  CCO_CUDA(pool_alloc(&loop, sizeof(TickLoop), st));
+  CCO_CUDA(cudaMemsetAsync(loop, 0, sizeof(TickLoop), st));
+  // the condition, then the loop around a body of `body` ticks of every
+  // branch; branches fork from and join back into the first capture stream
   cudaStream_t cap[kMaxBranches] = {};
   cudaEvent_t fork = nullptr, join[kMaxBranches] = {};
   EvalSide side[kMaxBranches] = {};   // per-dimension side streams of each branch
@@ -166,12 +194,37 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventRecord(ready, st);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(cap[0], ready, 0);
-  cudaGraph_t graph = nullptr;
-  if (e == cudaSuccess) e = cudaStreamBeginCapture(cap[0], cudaStreamCaptureModeThreadLocal);
+  cudaGraphConditionalHandle cond{};
+  cudaGraph_t inner = nullptr, cg = nullptr;
+  if (e == cudaSuccess) e = cudaGraphCreate(&graph, 0);
+  if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&cond, graph, 0, 0);
+  if (e == cudaSuccess)
+    e = cudaStreamBeginCaptureToGraph(cap[0], graph, nullptr, nullptr, 0,
+                                      cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    e = tick_gate(T.d_refs, B, loop, true, bodies, cond, cap[0]);
+    cudaError_t e2 = cudaStreamEndCapture(cap[0], &cg);
+    if (e == cudaSuccess) e = e2;
+  }
+  if (e == cudaSuccess) {
+    cudaGraphNode_t gate, node;
+    size_t n = 1;
+    e = cudaGraphGetNodes(graph, &gate, &n);
+    cudaGraphNodeParams np{};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = cond;
+    np.conditional.type = bodies > 1 ? cudaGraphCondTypeWhile : cudaGraphCondTypeIf;
+    np.conditional.size = 1;
+    if (e == cudaSuccess) e = cudaGraphAddNode(&node, graph, &gate, 1, &np);
+    if (e == cudaSuccess) inner = np.conditional.phGraph_out[0];
+  }
+  if (e == cudaSuccess)
+    e = cudaStreamBeginCaptureToGraph(cap[0], inner, nullptr, nullptr, 0,
+                                      cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     e = cudaEventRecord(fork, cap[0]);
     for (int b = 1; b < nbr && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(cap[b], fork, 0);
-    for (int t = 0; t < sch.graph_ticks && e == cudaSuccess; ++t)
+    for (int t = 0; t < body && e == cudaSuccess; ++t)
       for (int b = 0; b < nbr && e == cudaSuccess; ++b) {
         const EvalSide* sd = side[b].fork ? &side[b] : nullptr;
         if (!overlap) {
@@ -191,12 +244,13 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
       e = cudaEventRecord(join[b], cap[b]);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(cap[0], join[b], 0);
     }
-    cudaError_t e2 = cudaStreamEndCapture(cap[0], &graph);
+    if (bodies > 1 && e == cudaSuccess)
+      e = tick_gate(T.d_refs, B, loop, false, bodies, cond, cap[0]);
+    cudaError_t e2 = cudaStreamEndCapture(cap[0], &cg);
     if (e == cudaSuccess) e = e2;
   }
   if (e == cudaSuccess)
     e = cudaGraphInstantiate(&exec, graph, overlap ? cudaGraphInstantiateFlagUseNodePriority : 0);
-  if (graph) cudaGraphDestroy(graph);
   for (int b = 0; b < nbr; ++b) {
     if (cap[b]) cudaStreamDestroy(cap[b]);
     if (join[b]) cudaEventDestroy(join[b]);
@@ -241,8 +295,18 @@ int TickPlan::launches_per_tick() const {
 }
 
 void TickPlan::release(cudaStream_t st) {
-  if (exec) cudaGraphExecDestroy(exec);
+  std::vector<cudaGraph_t> g;
+  retire(st, &g);
+  for (cudaGraph_t x : g) cudaGraphDestroy(x);
+}
+
+void TickPlan::retire(cudaStream_t st, std::vector<cudaGraph_t>* graphs) {
+  if (exec) cudaGraphExecDestroy(exec);   // launches in flight run to their end
+  if (graph) graphs->push_back(graph);
+  if (loop) cudaFreeAsync(loop, st);
   exec = nullptr;
+  graph = nullptr;
+  loop = nullptr;
   for (int b = 0; b < kMaxBranches; ++b) ev[b].release(st);
 }
 
@@ -310,6 +374,7 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
   const size_t nc = cand.size();
   std::vector<cudaEvent_t> t0(2 * nc, nullptr), t1(2 * nc, nullptr);
   std::vector<int> ran(2 * nc, 0);
+  std::vector<cudaGraph_t> graphs;
   int rc = CCO_OK;
   cudaError_t e = cudaSuccess;
   for (size_t c = 0; c < 2 * nc && e == cudaSuccess; ++c) {
@@ -321,16 +386,22 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
     TickPlan P;
     P.method = C.shape.method;
     rc = P.build(C, cand[c], st);
-    if (rc != CCO_OK) break;
+    if (rc != CCO_OK) {
+      P.retire(st, &graphs);
+      break;
+    }
     e = cudaEventRecord(t0[v], st);
     if (e == cudaSuccess) e = cudaGraphLaunch(P.exec, st);
     if (e == cudaSuccess) e = cudaEventRecord(t1[v], st);
     ran[v] = e == cudaSuccess;
     *ticks += cand[c].graph_ticks;
-    *launches += (int64_t)cand[c].graph_ticks * P.launches_per_tick();
-    P.release(st);
+    *launches += (int64_t)cand[c].graph_ticks * P.launches_per_tick() + 1 +
+                 P.bodies * P.loop_gates();
+    P.retire(st, &graphs);
   }
-  if (rc == CCO_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (rc == CCO_OK && e == cudaSuccess) e = es;
+  for (cudaGraph_t g : graphs) cudaGraphDestroy(g);
   std::vector<float> sum(nc, 0.f);
   std::vector<int> cnt(nc, 0);
   for (size_t v = 0; v < 2 * nc && e == cudaSuccess && rc == CCO_OK; ++v) {
@@ -363,7 +434,7 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
   // (their kernels exit at once for finished lanes)
   const double tick_ms = ms[best] < 1e29f ? ms[best] : 0.2;
   const int gt = (int)std::lround(8.0 / std::max(tick_ms, 1e-3));
-  s.graph_ticks = std::max(4, std::min(32, gt));
+  s.graph_ticks = std::max(4, std::min(32, gt & ~3));   // whole bodies of four ticks
   *out = s;
   return CCO_OK;
 }
@@ -381,13 +452,17 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
   const int inflight = std::max(1, std::min(kMaxInflight, env_int("CCO_INFLIGHT", kInflight)));
   const int kSlots = inflight + 1;
   int64_t* d_status = nullptr;
-  int64_t* h_status = pinned_status((size_t)kSlots * B);
+  const int W = B + 1;   // a snapshot: the statuses, then the bodies the plan has run
+  int64_t* h_status = pinned_status((size_t)kSlots * W);
   if (!h_status) return fail(CCO_ERR_OOM, "pinned status buffer");
-  CCO_CUDA(pool_alloc(&d_status, sizeof(int64_t) * kSlots * B, st));
+  CCO_CUDA(pool_alloc(&d_status, sizeof(int64_t) * kSlots * W, st));
   cudaEvent_t ev[kMaxInflight + 1];
   int ver[kMaxInflight + 1] = {}, rows[kMaxInflight + 1] = {};
   for (int i = 0; i < kSlots; ++i) CCO_CUDA(cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming));
-  int64_t ticks = 0, launches = 0;
+  int64_t ticks = 0, launches = 0;   // ticks: the bound; what ran is counted as it lands
+  int64_t ticks_run = 0, seen = 0, per_body[kMaxInflight + 1] = {};
+  int body_of[kMaxInflight + 1] = {}, seen_version = 0;
+  std::vector<cudaGraph_t> graphs;   // of plans with launches in flight
   int rc = CCO_OK;
   cudaError_t e = cudaSuccess;
   bool done = false;
@@ -437,7 +512,9 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     } else if (!schedule_cached(C.probs, C.shape.method, &s) && tune) {
       defer_tune = C.shape.method == Method::Lbfgs && ticks < kTuneAfterTicks;
       if (!defer_tune) {
+        const int64_t before = ticks;
         r = tune_schedule(C, st, max_ticks, &ticks, &launches, &s);
+        ticks_run += ticks - before;
         if (r != CCO_OK) return r;
         schedule_store(C.probs, C.shape.method, s);
       }
@@ -457,7 +534,12 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     const int slot = checked % kSlots;
     CCO_CUDA(cudaEventSynchronize(ev[slot]));
     ++checked;
-    const int64_t* h = h_status + (size_t)slot * B;
+    const int64_t* h = h_status + (size_t)slot * W;
+    if (ver[slot] != seen_version) seen = 0;
+    seen_version = ver[slot];
+    ticks_run += (h[rows[slot]] - seen) * body_of[slot];
+    launches += (h[rows[slot]] - seen) * per_body[slot];
+    seen = h[rows[slot]];
     int running = 0;
     for (int i = 0; i < rows[slot]; ++i) running += h[i] == CCO_STATUS_RUNNING;
     if (running == 0) {
@@ -480,7 +562,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     // (older version, old row order) only feed the all-finished test.
     C.refs.swap(refs);
     C.probs.swap(probs);
-    P.release(st);
+    P.retire(st, &graphs);
     return start();
   };
 
@@ -489,20 +571,22 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     e = cudaGraphLaunch(P.exec, st);
     if (e != cudaSuccess) break;
     ticks += chosen.graph_ticks;
-    launches += (int64_t)chosen.graph_ticks * P.launches_per_tick() + 1;
+    launches += 2;   // the first condition kernel and the snapshot
     const int slot = launched % kSlots;
     const int n = (int)C.refs.size();
-    e = gather_status(C.d_refs, n, d_status + (size_t)slot * B, st);
+    e = gather_status(C.d_refs, n, d_status + (size_t)slot * W, st, &P.loop->done);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(h_status + (size_t)slot * B, d_status + (size_t)slot * B,
-                          sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st);
+      e = cudaMemcpyAsync(h_status + (size_t)slot * W, d_status + (size_t)slot * W,
+                          sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[slot], st);
     ver[slot] = version;
     rows[slot] = n;
+    body_of[slot] = P.body;
+    per_body[slot] = (int64_t)P.body * P.launches_per_tick() + P.loop_gates();
     ++launched;
     if (e == cudaSuccess && launched - checked > inflight) rc = land();
     if (rc == CCO_OK && e == cudaSuccess && !done && defer_tune && ticks >= kTuneAfterTicks) {
-      P.release(st);   // the deferred tuning, on the same table
+      P.retire(st, &graphs);   // the deferred tuning, on the same table
       rc = start();
     }
   }
@@ -512,13 +596,14 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     if (e != cudaSuccess) rc = cuda_fail(e, "relax ticks");
     else if (!done) rc = fail(CCO_ERR_ROUNDS, "relax did not finish within the round bound (%lld ticks)", (long long)max_ticks);
   }
-  P.release(st);
+  P.retire(st, &graphs);
   C.release(st);
   for (int i = 0; i < kSlots; ++i) cudaEventDestroy(ev[i]);
   cudaFreeAsync(d_status, st);
   cudaStreamSynchronize(st);
+  for (cudaGraph_t g : graphs) cudaGraphDestroy(g);
   if (stats) {
-    stats->ticks = ticks;
+    stats->ticks = ticks_run;
     stats->launches = launches;
     stats->schedule = first;
     stats->compactions = version - 1;
