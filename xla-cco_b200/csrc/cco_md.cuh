@@ -3,6 +3,8 @@
 // See cco_md.cu.
 #pragma once
 
+#include <vector>
+
 #include "cco_opt.cuh"
 
 namespace cco {
@@ -96,6 +98,11 @@ struct MdArgs {
   const double* wave_n = nullptr;        // [w][d] reciprocal-basis coefficients
   const double* wave_k = nullptr;        // [w][d] Cartesian wavevectors
   const int* cpos = nullptr;             // [nc] run position of constrained wave c
+  // unconstrained waves on axis tables (k_md_waves_tab): per wave its table
+  // offset on each axis (~o: conjugate) and its index, in an order that keeps
+  // equal leading components together; largest |n| per axis, particles a tile
+  const int4* wave_t = nullptr;          // [w - nc], null: k_md_waves
+  int wave_r[3] = {0, 0, 0}, wave_tp = 0, wave_d = 0;
   int n_rec = 0, trace_every = 0, trace_cap = 0;
   const int64_t* rec_steps = nullptr;    // [n_rec] ascending
   MdSegIO io{};
@@ -106,6 +113,9 @@ struct MdArgs {
 cudaError_t md_init(const MdArgs& a, const double* r0, const double* v0, const double* mats,
                     const uint32_t* keys, const double* acc0, cudaStream_t st);
 cudaError_t md_update(const MdArgs& a, cudaStream_t st);
+// Fills a's wave_r and wave_tp from the rows of wave_n (host, [w][d]) and
+// returns the descriptors for wave_t; empty if the rows take k_md_waves.
+std::vector<int4> md_wave_tables(MdArgs* a, int d, const double* wave_n);
 cudaError_t md_finalize(const MdArgs& a, double* r_out, double* v_out, double* f_out,
                         double* phi_out, double* ke_out, double* drift_out, int64_t* resets_out,
                         double* acc_out, uint32_t* keys_out, int64_t* status_out,

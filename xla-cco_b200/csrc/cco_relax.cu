@@ -1284,6 +1284,7 @@ extern "C" int cco_md_segment(cco_problem* p, void* stream, int batch, const dou
   a.lanes = T.d_refs;
   double *d_mats = nullptr, *d_wn = nullptr, *d_wk = nullptr;
   int* d_cpos = nullptr;
+  int4* d_wt = nullptr;
   int64_t* d_rec = nullptr;
   cudaError_t e = upload(&d_mats, mats, st);
   if (e == cudaSuccess) e = upload(&d_wn, std::vector<double>(wv->n_vectors, wv->n_vectors + (size_t)w * d), st);
@@ -1291,6 +1292,9 @@ extern "C" int cco_md_segment(cco_problem* p, void* stream, int batch, const dou
   if (e == cudaSuccess) e = upload(&d_cpos, cpos, st);
   if (e == cudaSuccess && rec)
     e = upload(&d_rec, std::vector<int64_t>(cfg->record_steps, cfg->record_steps + cfg->n_record_steps), st);
+  const std::vector<int4> wt = md_wave_tables(&a, d, wv->n_vectors);
+  if (e == cudaSuccess && !wt.empty()) e = upload(&d_wt, wt, st);
+  a.wave_t = d_wt;
   a.wave_n = d_wn;
   a.wave_k = d_wk;
   a.cpos = d_cpos;
@@ -1305,7 +1309,7 @@ extern "C" int cco_md_segment(cco_problem* p, void* stream, int batch, const dou
   }
   if (ticks) *ticks = rs.ticks;
   T.release(st);
-  for (void* q : {(void*)d_mats, (void*)d_wn, (void*)d_wk, (void*)d_cpos, (void*)d_rec, (void*)records})
+  for (void* q : {(void*)d_mats, (void*)d_wn, (void*)d_wk, (void*)d_cpos, (void*)d_wt, (void*)d_rec, (void*)records})
     if (q) cudaFreeAsync(q, st);
   e = cudaStreamSynchronize(st);
   if (rc == CCO_OK && e != cudaSuccess) rc = cuda_fail(e, "md segment");
