@@ -91,14 +91,16 @@ __device__ __forceinline__ double min_image_r2(const double* si, const double* s
   return best;
 }
 
-// r2 of the zero shift on a diagonal basis.
-template <int D>
+// r2 of the zero shift on a diagonal basis. SMALL: |t| < 2^51, where the nearest
+// integer is two additions instead of a quarter-rate rounding instruction.
+template <int D, bool SMALL = false>
 __device__ __forceinline__ double diag_r2(const double* si, const double* sj, const double* Bd) {
   double r2 = 0.0;
 #pragma unroll
   for (int c = 0; c < D; ++c) {
     const double t = __dadd_rn(sj[c], -si[c]);
-    const double v = __dmul_rn(__dadd_rn(t, -rint(t)), Bd[c]);
+    const double k = SMALL ? __dadd_rn(__dadd_rn(t, 0x1.8p52), -0x1.8p52) : rint(t);
+    const double v = __dmul_rn(__dadd_rn(t, -k), Bd[c]);
     r2 = __dadd_rn(r2, __dmul_rn(v, v));
   }
   return r2;
@@ -109,7 +111,8 @@ __device__ __forceinline__ double diag_r2(const double* si, const double* sj, co
 // last bin): the largest k with t[k] <= r2.
 __device__ __forceinline__ int bin_of(double r2, const double* t, const PairGeom& g) {
   if (g.inv_w > 0.f) {
-    int k = (int)((sqrtf((float)r2) - g.e0) * g.inv_w);
+    const float f = (float)r2;
+    int k = (int)((f * rsqrtf(f) - g.e0) * g.inv_w);   // a zero r2 gives NaN, bin 0
     k = min(max(k, 0), g.n_bins - 1);
     while (t[k] > r2) --k;
     while (k + 1 < g.n_bins && t[k + 1] <= r2) ++k;
@@ -234,6 +237,386 @@ __global__ void __launch_bounds__(kPairTile) k_nearest(const double* __restrict_
   if (i < g.n) out[(size_t)blockIdx.y * g.n + i] = sqrt(best);
 }
 
+// ------------------------------------------------------------ cell grids
+// Diagonal bases, configurations that fit shared memory: every CTA sorts its
+// configuration into a grid of cells and a row looks only at the cells a
+// partner within range (or nearer than what it has) can be in. A pair that is
+// skipped lies more than K cells apart on some axis; with |s| <= 2^16 its
+// distance as computed exceeds K / G L by no less than kCellMargin, so the
+// counts and the smallest distances stay those of all pairs. A configuration
+// with larger or non-finite coordinates, or most of its particles in a few
+// cells, takes one cell, all pairs.
+// 256 configurations of d=2 N=1000, range 0.2 L, 200 bins: histogram 235 -> 85 us
+// (a ninth of the pairs; 200 us while every tested pair took FP64 and the queue,
+// 133 with the FP32 screen before the queue; 93 / 82 us with 256 / 1024 threads,
+// cells of a half / a third / a quarter of the range 103 / 93 / 92), nearest
+// neighbours 254 -> 37 us, about half of it the sort. Instruction issue bounds
+// both. The all-pairs kernels below stay for sheared bases, ranges that reach
+// most of the box, fewer than 64 particles and configurations past shared memory.
+constexpr int kCellThreads = 512;
+constexpr double kCellReach = 65536.0;     // largest |s| of a cell grid
+constexpr double kCellMargin = 1e-7;       // relative: |s| rounding 2^-37, G <= 2048
+constexpr int kMaxCells = 8192, kMaxAxisCells = 2048;
+constexpr size_t kCellSmem = 200 * 1024;
+constexpr double kHistReach = 3.0;     // cells per histogram range, at least
+constexpr double kHistFill = 4.0, kNearFill = 2.0;   // particles per cell, at least / about
+constexpr double kHistMost = 0.6, kNearMost = 0.5;   // stencil / box
+constexpr int kCellMin = 64, kCellCtas = 148 * 3, kCellSplit = 96;
+constexpr int kCellCrowd = 64;
+
+struct CellGrid {
+  int G[3], K[3], cells;   // cells per axis, stencil reach, all cells
+  float lim;               // histogram: FP32 r2 no pair in range exceeds
+  float eps;               // and bins around an edge that FP32 cannot tell (0: queue every pair)
+};
+
+template <int D>
+__device__ __forceinline__ int cell_of(const double* s, const int* G, int* c) {
+  int id = 0;
+#pragma unroll
+  for (int a = 0; a < D; ++a) {
+    const double u = s[a] - floor(s[a]);
+    c[a] = min(max((int)(u * G[a]), 0), G[a] - 1);
+    id = id * G[a] + c[a];
+  }
+  return id;
+}
+
+// Sorts the configuration by cell: positions to ps, rows to idx (optional),
+// end[c] = one past the last particle of cell c. The order inside a cell is any,
+// so CTAs that share a configuration split it at cells (cell_range). A
+// configuration outside the reach, or with a crowded cell, keeps its order in
+// one cell (G = 1, K = 0). Returns the grid in use. All threads of the CTA.
+template <int D>
+__device__ CellGrid cell_sort(const double* __restrict__ s, int n, CellGrid g, double* ps, int* end,
+                              int* idx) {
+  __shared__ int wsum[kCellThreads / 32];
+  const int tid = threadIdx.x;
+  int cc[3];
+  auto load = [&](int j, double* x) {
+    bool in = true;
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      x[a] = s[(size_t)j * D + a];
+      in = in && fabs(x[a]) <= kCellReach;
+    }
+    return in ? cell_of<D>(x, g.G, cc) : -1;
+  };
+  for (int c = tid; c < g.cells; c += kCellThreads) end[c] = 0;
+  __syncthreads();
+  int bad = 0;
+  const int crowd = kCellCrowd + 4 * n / g.cells;
+  for (int j = tid; j < n; j += kCellThreads) {
+    double x[D];
+    const int c = load(j, x);
+    bad |= c < 0;
+    if (c >= 0) bad |= atomicAdd(end + c, 1) >= crowd;
+  }
+  if (__syncthreads_or(bad)) {
+    for (int q = tid; q < n * D; q += kCellThreads) ps[q] = s[q];
+    if (idx)
+      for (int j = tid; j < n; j += kCellThreads) idx[j] = j;
+    if (tid == 0) end[0] = n;
+    __syncthreads();
+    for (int a = 0; a < 3; ++a) {
+      g.G[a] = 1;
+      g.K[a] = 0;
+    }
+    g.cells = 1;
+    return g;
+  }
+  // exclusive prefix sums: a run of cells per thread
+  const int per = (g.cells + kCellThreads - 1) / kCellThreads;
+  const int c0 = min(tid * per, g.cells), c1 = min(c0 + per, g.cells);
+  int sum = 0;
+  for (int c = c0; c < c1; ++c) sum += end[c];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((tid & 31) >= o) incl += v;
+  }
+  if ((tid & 31) == 31) wsum[tid >> 5] = incl;
+  __syncthreads();
+  int at = incl - sum;
+  for (int w = 0; w < tid >> 5; ++w) at += wsum[w];
+  for (int c = c0; c < c1; ++c) {
+    const int v = end[c];
+    end[c] = at;
+    at += v;
+  }
+  __syncthreads();
+  for (int j = tid; j < n; j += kCellThreads) {
+    double x[D];
+    const int to = atomicAdd(end + load(j, x), 1);   // leaves end[c] at the cell's end
+#pragma unroll
+    for (int a = 0; a < D; ++a) ps[to * D + a] = x[a];
+    if (idx) idx[to] = j;
+  }
+  __syncthreads();
+  return g;
+}
+
+// The particles of this CTA (of gridDim.x): an even split, moved back to the
+// start of a cell.
+__device__ __forceinline__ int cell_range(const CellGrid& g, const int* end, int n, int part) {
+  const int p = (int)((long long)n * part / gridDim.x);
+  if (g.cells == 1 || p == 0 || p == n) return p;
+  int lo = 0, hi = g.cells - 1;   // the first cell that ends past p
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (end[mid] > p) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo > 0 ? end[lo - 1] : 0;
+}
+
+// Particles of columns [c - lo, c + hi] (wrapped) of the cell row `row`:
+// [a, a + n1) and [b, b + n2).
+struct CellSpan {
+  int a, n1, b, n2;
+};
+__device__ __forceinline__ CellSpan cell_span(const int* end, int row, int G, int c, int lo, int hi) {
+  const int base = row * G;
+  auto begin = [&](int k) { return base + k > 0 ? end[base + k - 1] : 0; };
+  CellSpan r;
+  const int f = c - lo, l = c + hi;
+  r.a = begin(max(f, 0));
+  r.n1 = end[base + min(l, G - 1)] - r.a;
+  r.b = 0;
+  r.n2 = 0;
+  if (f < 0) {
+    r.b = begin(f + G);
+    r.n2 = end[base + G - 1] - r.b;
+  } else if (l >= G) {
+    r.b = begin(0);
+    r.n2 = end[base + l - G] - r.b;
+  }
+  return r;
+}
+
+__device__ __forceinline__ int wrap(int x, int G) { return x < 0 ? x + G : x >= G ? x - G : x; }
+
+// The histogram over half the stencil: the rest of the row's own cell, the
+// cells after it, the cell rows after its own. Lanes are neighbours in the sorted
+// order, so their partners are mostly the same. A pair is screened by the FP32
+// distance of wrapped coordinates (the image is known from the cells; lim
+// allows for their rounding, 1e-6 L). On even edges one that lies more than eps
+// bins from every edge is counted at once; the others that pass queue up per
+// warp, 32 at a time are measured in FP64 and binned.
+template <int D>
+__global__ void __launch_bounds__(kCellThreads)
+    k_pair_hist_cells(const double* __restrict__ s, PairGeom g, CellGrid grid,
+                      const double* __restrict__ thresholds, unsigned long long* counts) {
+  // positions, thresholds (if they fit), FP32 wrapped positions, cell ends, bins
+  extern __shared__ double sm[];
+  __shared__ unsigned int queues[kCellThreads / 32][64];
+  const bool local = g.n_bins <= kSmemBins, tl = g.n_bins < kSmemEdges;
+  double* ps = sm;
+  double* ts = ps + (size_t)g.n * D;
+  const double* t = tl ? ts : thresholds;
+  float* pf = reinterpret_cast<float*>(ts + (tl ? g.n_bins + 1 : 0));
+  int* end = reinterpret_cast<int*>(pf + (size_t)(g.n + 1) / 2 * 2 * D);
+  unsigned int* bins = reinterpret_cast<unsigned int*>(end + grid.cells);
+  if (tl)
+    for (int b = threadIdx.x; b <= g.n_bins; b += kCellThreads) ts[b] = thresholds[b];
+  if (local)
+    for (int b = threadIdx.x; b < g.n_bins; b += kCellThreads) bins[b] = 0u;
+  const CellGrid cg = cell_sort<D>(s + (size_t)blockIdx.y * g.n * D, g.n, grid, ps, end, nullptr);
+  const double t_lo = t[0], t_hi = t[g.n_bins];
+  double Bd[D];
+  float L[D];
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    Bd[c] = g.B[c * D + c];
+    L[c] = (float)fabs(Bd[c]);
+  }
+  const float lim = cg.cells > 1 ? cg.lim : INFINITY;   // one cell: every pair is measured
+  for (int q = threadIdx.x; q < g.n * D; q += kCellThreads)
+    pf[q] = cg.cells > 1 ? (float)((ps[q] - floor(ps[q])) * fabs(g.B[(q % D) * (D + 1)])) : 0.f;
+  __syncthreads();
+  // the bin less 1/2 is r inv_w + shift; within `half` of its nearest integer the bin is sure
+  const bool direct = cg.cells > 1 && cg.eps > 0.f;
+  const float shift = -g.e0 * g.inv_w - 0.5f, half = 0.5f - cg.eps;
+  unsigned int* queue = queues[threadIdx.x >> 5];
+  const int wl = threadIdx.x & 31;
+  const unsigned below = (1u << wl) - 1u;
+  int have = 0;
+  auto count = [&](unsigned int ij) {
+    const double *si = ps + (ij >> 16) * D, *sj = ps + (ij & 0xffffu) * D;
+    const double r2 = cg.cells > 1 ? diag_r2<D, true>(si, sj, Bd) : diag_r2<D>(si, sj, Bd);
+    if (!(r2 >= t_lo && r2 < t_hi)) return;   // out of range or NaN
+    const int b = bin_of(r2, t, g);
+    if (local) atomicAdd(bins + b, 1u);
+    else atomicAdd(counts + b, 1ull);
+  };
+  const int rows = D == 1 ? 1 : D == 2 ? cg.K[0] + 1 : cg.K[1] + 1 + cg.K[0] * (2 * cg.K[1] + 1);
+  const int i1 = cell_range(cg, end, g.n, blockIdx.x + 1);
+  for (int i0 = cell_range(cg, end, g.n, blockIdx.x) + (threadIdx.x & ~31); i0 < i1; i0 += kCellThreads) {
+    const int i = i0 + wl;
+    const bool live = i < i1;
+    double si[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) si[c] = ps[(live ? i : 0) * D + c];
+    int cc[3] = {0, 0, 0};
+    if (cg.cells > 1) cell_of<D>(si, cg.G, cc);
+    for (int q = 0; q < rows; ++q) {
+      float x[D];   // this row's image of the particle
+#pragma unroll
+      for (int c = 0; c < D; ++c) x[c] = pf[(live ? i : 0) * D + c];
+      int row = 0;
+      if (D == 2) {
+        row = wrap(cc[0] + q, cg.G[0]);
+        if (cc[0] + q >= cg.G[0]) x[0] -= L[0];
+      }
+      if (D == 3) {
+        const int w = 2 * cg.K[1] + 1, q1 = q - (cg.K[1] + 1);
+        const int r0 = cc[0] + (q1 < 0 ? 0 : q1 / w + 1), r1 = cc[1] + (q1 < 0 ? q : q1 % w - cg.K[1]);
+        row = wrap(r0, cg.G[0]) * cg.G[1] + wrap(r1, cg.G[1]);
+        if (r0 >= cg.G[0]) x[0] -= L[0];
+        if (r1 >= cg.G[1]) x[1] -= L[1];
+        if (r1 < 0) x[1] += L[1];
+      }
+      const int lo = q == 0 ? 0 : cg.K[D - 1];
+      CellSpan sp = cell_span(end, row, cg.G[D - 1], cc[D - 1], lo, cg.K[D - 1]);
+      if (q == 0) {   // the rest of its own cell first
+        sp.n1 -= i + 1 - sp.a;
+        sp.a = i + 1;
+      }
+      const int len = live ? sp.n1 + sp.n2 : 0, gap = sp.b - sp.a - sp.n1;
+      const float x2 = cc[D - 1] < lo ? x[D - 1] + L[D - 1] : x[D - 1] - L[D - 1];   // of the second span
+      const int most = __reduce_max_sync(0xffffffffu, len);
+      auto at = [&](int k) { return k < len ? sp.a + k + (k >= sp.n1 ? gap : 0) : 0; };
+      auto screen = [&](int k, int j) {
+        float r2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+          const float v = pf[j * D + c] - (c == D - 1 && k >= sp.n1 ? x2 : x[c]);
+          r2 = fmaf(v, v, r2);
+        }
+        return r2;
+      };
+      auto push = [&](bool in, int j) {
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) queue[have + __popc(m & below)] = (unsigned)i << 16 | (unsigned)j;
+        have += __popc(m);
+        if (have >= 32) {
+          __syncwarp();
+          count(queue[wl]);
+          have -= 32;
+          const unsigned rest = queue[32 + wl];
+          __syncwarp();
+          if (wl < have) queue[wl] = rest;
+        }
+      };
+      if (direct) {
+#pragma unroll 4
+        for (int k = 0; k < most; ++k) {
+          const int j = at(k);
+          const float r2 = fmaxf(screen(k, j), 1e-30f);
+          const float u = fmaf(r2 * rsqrtf(r2), g.inv_w, shift);   // bin - 1/2
+          const float n = u + 0x1.8p23f;                           // its nearest integer
+          const int b = __float_as_int(n) - 0x4b400000;
+          const bool edge = fabsf(u - (n - 0x1.8p23f)) >= half;
+          const bool in = k < len && r2 <= lim;
+          if (in && !edge && (unsigned)b < (unsigned)g.n_bins) atomicAdd(bins + b, 1u);
+          if (__any_sync(0xffffffffu, in && edge)) push(in && edge, j);
+        }
+      } else {
+#pragma unroll 4
+        for (int k = 0; k < most; ++k) {
+          const int j = at(k);
+          push(k < len && screen(k, j) <= lim, j);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  if (wl < have) count(queue[wl]);
+  if (!local) return;
+  __syncthreads();
+  for (int b = threadIdx.x; b < g.n_bins; b += kCellThreads)
+    if (bins[b]) atomicAdd(counts + b, (unsigned long long)bins[b]);
+}
+
+// Nearest neighbours: the 3^D cells around a particle, then 5^D if the best
+// could be beaten from outside, then everything.
+template <int D>
+__global__ void __launch_bounds__(kCellThreads)
+    k_nearest_cells(const double* __restrict__ s, PairGeom g, CellGrid grid, double* __restrict__ out) {
+  extern __shared__ double sm[];   // positions, cell ends, rows
+  double* ps = sm;
+  int* end = reinterpret_cast<int*>(ps + (size_t)g.n * D);
+  int* idx = end + grid.cells;
+  const CellGrid cg = cell_sort<D>(s + (size_t)blockIdx.y * g.n * D, g.n, grid, ps, end, idx);
+  double Bd[D], side = INFINITY;
+  int gmin = 1 << 30;
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    Bd[c] = g.B[c * D + c];
+    side = fmin(side, fabs(Bd[c]) / cg.G[c] * (1.0 - kCellMargin));
+    gmin = min(gmin, cg.G[c]);
+  }
+  const int i1 = cell_range(cg, end, g.n, blockIdx.x + 1);
+  for (int i = cell_range(cg, end, g.n, blockIdx.x) + threadIdx.x; i < i1; i += kCellThreads) {
+    double si[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) si[c] = ps[i * D + c];
+    double best = min_image_r2<D>(si, si, g, true);   // its own nearest image
+    int cc[3] = {0, 0, 0};
+    if (cg.cells > 1) cell_of<D>(si, cg.G, cc);
+    auto visit = [&](int j) {
+      const double r2 = diag_r2<D, true>(si, ps + j * D, Bd);
+      if (j != i) best = fmin(best, r2);
+    };
+    bool done = false;
+    for (int K = 1; K <= 2 && !done && gmin >= 2 * K + 1; ++K) {
+      const int w = 2 * K + 1, rows = D == 1 ? 1 : D == 2 ? w : w * w;
+      for (int q = 0; q < rows; ++q) {
+        int row = 0;
+        if (D == 2) row = wrap(cc[0] + q - K, cg.G[0]);
+        if (D == 3) row = wrap(cc[0] + q / w - K, cg.G[0]) * cg.G[1] + wrap(cc[1] + q % w - K, cg.G[1]);
+        const CellSpan sp = cell_span(end, row, cg.G[D - 1], cc[D - 1], K, K);
+        for (int k = 0; k < sp.n1; ++k) visit(sp.a + k);
+        for (int k = 0; k < sp.n2; ++k) visit(sp.b + k);
+      }
+      const double reach = K * side;
+      done = best <= reach * reach * (1.0 - kCellMargin);
+    }
+    if (!done)
+      for (int j = 0; j < g.n; ++j) {
+        const double r2 = diag_r2<D>(si, ps + j * D, Bd);
+        if (j != i) best = fmin(best, r2);
+      }
+    out[(size_t)blockIdx.y * g.n + idx[i]] = sqrt(best);
+  }
+}
+
+// Cell grid with cells of about `side`; reach > 0: K covers it, else K = 1. False
+// if the stencil covers too much of the box or the configuration is too large
+// or too small.
+bool cell_grid(const PairGeom& g, int d, double side, double reach, double most, CellGrid* c) {
+  *c = CellGrid{{1, 1, 1}, {0, 0, 0}, 1, 0.f, 0.f};
+  double part = 1.0, longest = 0.0;
+  if (!(side > 0.0) || g.n > 0xffff) return false;
+  for (int a = 0; a < d; ++a) {
+    const double L = std::fabs(g.B[a * d + a]);
+    const double n = std::floor(L / side);
+    if (!(n >= 3.0 && L > 1e-12 && L < 1e12)) return false;
+    longest = std::max(longest, L);
+    c->G[a] = (int)std::min<double>(n, kMaxAxisCells);
+    const double k = reach > 0.0 ? std::ceil(reach * c->G[a] / (L * (1.0 - kCellMargin))) : 1.0;
+    if (!(2.0 * k + 1.0 <= c->G[a])) return false;
+    c->K[a] = (int)k;
+    part *= (2.0 * k + 1.0) / c->G[a];
+    if ((double)c->cells * c->G[a] > kMaxCells) return false;
+    c->cells *= c->G[a];
+  }
+  const double r = reach + 1e-6 * longest;
+  c->lim = (float)(r * r * (1.0 + 1e-6));
+  return part <= most;
+}
+
 // The smallest double t >= 0 with sqrt(t) >= e (e >= 0), or > e with `past`.
 double r2_threshold(double e, bool past) {
   auto in = [&](double t) { return past ? std::sqrt(t) > e : std::sqrt(t) >= e; };
@@ -255,6 +638,22 @@ void launch_hist(bool diag, dim3 grid, size_t smem, cudaStream_t st, const doubl
                  const PairGeom& g, const double* t, unsigned long long* c, int tiles) {
   if (diag) k_pair_hist<D, true><<<grid, kPairTile, smem, st>>>(s, g, t, c, tiles);
   else k_pair_hist<D, false><<<grid, kPairTile, smem, st>>>(s, g, t, c, tiles);
+}
+template <int D>
+cudaError_t launch_hist_cells(dim3 grid, size_t smem, cudaStream_t st, const double* s, const PairGeom& g,
+                              const CellGrid& c, const double* t, unsigned long long* out) {
+  const cudaError_t e = cudaFuncSetAttribute(k_pair_hist_cells<D>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+  if (e == cudaSuccess) k_pair_hist_cells<D><<<grid, kCellThreads, smem, st>>>(s, g, c, t, out);
+  return e;
+}
+template <int D>
+cudaError_t launch_nearest_cells(dim3 grid, size_t smem, cudaStream_t st, const double* s,
+                                 const PairGeom& g, const CellGrid& c, double* out) {
+  const cudaError_t e = cudaFuncSetAttribute(k_nearest_cells<D>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+  if (e == cudaSuccess) k_nearest_cells<D><<<grid, kCellThreads, smem, st>>>(s, g, c, out);
+  return e;
 }
 template <int D>
 void launch_nearest(bool diag, dim3 grid, cudaStream_t st, const double* s, const PairGeom& g,
@@ -316,16 +715,42 @@ int cco_pair_histogram(int device, void* stream, int batch, int n, int d, const 
   double* d_t = nullptr;
   CCO_CUDA(upload(&d_t, ht, st));
   CCO_CUDA(cudaMemsetAsync(counts, 0, sizeof(int64_t) * g.n_bins, st));
+  const bool diag = is_diagonal(g, d);
+  auto* c = reinterpret_cast<unsigned long long*>(counts);
+  const size_t bin_smem = (g.n_bins < kSmemEdges ? sizeof(double) * n_edges : 0) +
+                          (g.n_bins <= kSmemBins ? sizeof(unsigned int) * g.n_bins : 0);
+  double vol = 1.0;
+  for (int a = 0; a < d; ++a) vol *= std::fabs(g.B[a * d + a]);
+  const double side = std::max(edges[g.n_bins] / kHistReach * (1.0 + 4.0 * kCellMargin),
+                               std::pow(kHistFill * vol / n, 1.0 / d));
+  // edges against the even ones, and the longest axis, for the FP32 bins
+  double dev = 0.0, longest = 0.0;
+  for (int k = 0; k < n_edges; ++k) dev = std::max(dev, std::fabs(edges[k] - (edges[0] + k * width)));
+  for (int a = 0; a < d; ++a) longest = std::max(longest, std::fabs(g.B[a * d + a]));
+  const double eps = 1.01 * (1e-6 * longest + 1e-6 * edges[g.n_bins] + dev) / width;
+  CellGrid cg;
+  const size_t pos_smem = sizeof(double) * n * d + sizeof(float) * ((n + 1) / 2 * 2) * d;
+  const size_t cell_smem = pos_smem + bin_smem + sizeof(int) * kMaxCells;
+  if (diag && n >= kCellMin && cell_smem <= kCellSmem &&
+      cell_grid(g, d, side, edges[g.n_bins], kHistMost, &cg)) {
+    const int chunks = (n + kCellSplit - 1) / kCellSplit;
+    const dim3 grid(std::max(1, std::min(chunks, (kCellCtas + batch - 1) / batch)), batch);
+    const size_t smem = pos_smem + bin_smem + sizeof(int) * cg.cells;
+    if (even && g.n_bins <= kSmemBins && eps < 0.1) cg.eps = (float)eps;
+    CCO_CUDA(d == 1   ? launch_hist_cells<1>(grid, smem, st, s, g, cg, d_t, c)
+             : d == 2 ? launch_hist_cells<2>(grid, smem, st, s, g, cg, d_t, c)
+                      : launch_hist_cells<3>(grid, smem, st, s, g, cg, d_t, c));
+    CCO_CUDA(cudaGetLastError());
+    CCO_CUDA(cudaFreeAsync(d_t, st));
+    return CCO_OK;
+  }
   const int tiles = (n + kPairTile - 1) / kPairTile;
   const long long units = (long long)tiles * (tiles + 1) / 2;
   // a CTA's range: enough CTAs to fill the GPU a few times, few flushes of the bins
   long long ctas = std::min<long long>(units, (kPairCtas + batch - 1) / batch);
   ctas = std::max(ctas, (units + kMaxUnits - 1) / kMaxUnits);
   const dim3 grid((unsigned)ctas, batch);
-  const size_t smem = (g.n_bins < kSmemEdges ? sizeof(double) * n_edges : 0) +
-                      (g.n_bins <= kSmemBins ? sizeof(unsigned int) * g.n_bins : 0);
-  auto* c = reinterpret_cast<unsigned long long*>(counts);
-  const bool diag = is_diagonal(g, d);
+  const size_t smem = bin_smem;
   if (d == 1) launch_hist<1>(diag, grid, smem, st, s, g, d_t, c, tiles);
   else if (d == 2) launch_hist<2>(diag, grid, smem, st, s, g, d_t, c, tiles);
   else launch_hist<3>(diag, grid, smem, st, s, g, d_t, c, tiles);
@@ -342,8 +767,23 @@ int cco_nearest_neighbor(int device, void* stream, int batch, int n, int d, cons
   if (!out) return fail(CCO_ERR_ARG, "null output");
   DeviceGuard guard(device);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const dim3 grid((n + kPairTile - 1) / kPairTile, batch);
   const bool diag = is_diagonal(g, d);
+  double vol = 1.0;
+  for (int a = 0; a < d; ++a) vol *= std::fabs(g.B[a * d + a]);
+  CellGrid cg;
+  const size_t cell_smem = (sizeof(double) * d + sizeof(int)) * n + sizeof(int) * kMaxCells;
+  if (diag && n >= kCellMin && cell_smem <= kCellSmem &&
+      cell_grid(g, d, std::pow(kNearFill * vol / n, 1.0 / d), 0.0, kNearMost, &cg)) {
+    const int chunks = (n + kCellSplit - 1) / kCellSplit;
+    const dim3 grid(std::max(1, std::min(chunks, (kCellCtas + batch - 1) / batch)), batch);
+    const size_t smem = (sizeof(double) * d + sizeof(int)) * n + sizeof(int) * cg.cells;
+    CCO_CUDA(d == 1   ? launch_nearest_cells<1>(grid, smem, st, s, g, cg, out)
+             : d == 2 ? launch_nearest_cells<2>(grid, smem, st, s, g, cg, out)
+                      : launch_nearest_cells<3>(grid, smem, st, s, g, cg, out));
+    CCO_CUDA(cudaGetLastError());
+    return CCO_OK;
+  }
+  const dim3 grid((n + kPairTile - 1) / kPairTile, batch);
   if (d == 1) launch_nearest<1>(diag, grid, st, s, g, out);
   else if (d == 2) launch_nearest<2>(diag, grid, st, s, g, out);
   else launch_nearest<3>(diag, grid, st, s, g, out);
