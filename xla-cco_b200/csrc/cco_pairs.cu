@@ -260,7 +260,11 @@ constexpr int kMaxCells = 8192, kMaxAxisCells = 2048;
 constexpr size_t kCellSmem = 200 * 1024;
 constexpr double kHistReach = 3.0;     // cells per histogram range, at least
 constexpr double kHistFill = 4.0, kNearFill = 2.0;   // particles per cell, at least / about
-constexpr double kHistMost = 0.6, kNearMost = 0.5;   // stencil / box
+// The histogram takes cells as long as their stencil fits the box once; in 1-D, where
+// the range's pairs cost what all pairs do, up to 0.6 of it (call times, range
+// 0.25 / 0.3 / 0.4 L, cells against all pairs: 256 configurations of d=2 N=1000 205 /
+// 265 / 374 against 320 / 339 / 399 us, 64 of d=1 190 / 213 / 200 against 150 / 153 / 166).
+constexpr double kHistMost = 1.0, kHistMost1 = 0.6, kNearMost = 0.5;   // stencil / box
 constexpr int kCellMin = 64, kCellCtas = 148 * 3, kCellSplit = 96;
 constexpr int kCellCrowd = 64;
 
@@ -732,7 +736,7 @@ int cco_pair_histogram(int device, void* stream, int batch, int n, int d, const 
   const size_t pos_smem = sizeof(double) * n * d + sizeof(float) * ((n + 1) / 2 * 2) * d;
   const size_t cell_smem = pos_smem + bin_smem + sizeof(int) * kMaxCells;
   if (diag && n >= kCellMin && cell_smem <= kCellSmem &&
-      cell_grid(g, d, side, edges[g.n_bins], kHistMost, &cg)) {
+      cell_grid(g, d, side, edges[g.n_bins], d == 1 ? kHistMost1 : kHistMost, &cg)) {
     const int chunks = (n + kCellSplit - 1) / kCellSplit;
     const dim3 grid(std::max(1, std::min(chunks, (kCellCtas + batch - 1) / batch)), batch);
     const size_t smem = pos_smem + bin_smem + sizeof(int) * cg.cells;
