@@ -871,6 +871,7 @@ struct EvalWS {
     plan.items1 = plan.itemsG = it1;
     plan.items2 = plan.itemsH = it2;
     plan.n_lanes = B;
+    plan.chain = true;
     plan.n_items1 = z.grid ? 0 : B * z.nt1;
     plan.n_items2 = z.grid2 ? 0 : B * z.nt2;
     const int nG = z.grid ? B * z.nt1 : 0, nH = z.grid2 ? B * z.nt2 : 0;

@@ -57,6 +57,7 @@ __device__ __forceinline__ bool grid_lane_runs(const EvalPlan& plan, const EvalL
 
 // Grid form: the phases the tables start from.
 __global__ void __launch_bounds__(kRootChunk) k_grid_roots(EvalPlan plan) {
+  chain_wait();
   const EvalLane& ln = plan.lanes[blockIdx.y];
   if (!grid_lane_runs(plan, ln)) return;
   const ProbDev& P = plan.probs[ln.prob];
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid1(EvalPlan plan
   constexpr int NT = CLS == 2 ? 3 : LINES ? 1 : 2;
   const EvalItem* items = plan.itemsG + plan.q_offG[D - 1][CLS];
   const int n = plan.q_offG[D - 1][CLS + 1] - plan.q_offG[D - 1][CLS];
+  chain_wait<false>();
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     const EvalItem it = items[i];
     const EvalLane ln = plan.lanes[it.lane];
@@ -92,7 +94,7 @@ int grid_ctas(int items) { return std::min(items, kGridCtas * kGridSms); }
 template <int D, int CLS>
 void launch_grid1_class(const EvalPlan& plan, cudaStream_t s) {
   const int n = plan.q_offG[D - 1][CLS + 1] - plan.q_offG[D - 1][CLS];
-  if (n > 0) k_grid1<D, CLS><<<grid_ctas(n), kGridThreads, plan.smemG, s>>>(plan);
+  if (n > 0) launch_chained(plan.chain, k_grid1<D, CLS>, grid_ctas(n), kGridThreads, plan.smemG, s, plan);
 }
 template <int D>
 void launch_grid1(const EvalPlan& plan, cudaStream_t s) {
@@ -111,6 +113,7 @@ template <int D, bool F32>
 __global__ void __launch_bounds__(kPass1Threads, 4) k_pass1(EvalPlan plan) {
   extern __shared__ double2 smem[];
   __shared__ ProbDev sp;
+  chain_wait();
   const EvalItem it = plan.items1[plan.d_off1[D - 1] + blockIdx.x];
   const EvalLane ln = plan.lanes[it.lane];
   if (!lane_active(ln.status)) return;
@@ -137,6 +140,7 @@ __device__ __forceinline__ double* grid_energies(const ProbDev& P, const EvalLan
 // this block reads).
 __global__ void __launch_bounds__(kReduceChunk) k_reduce(EvalPlan plan) {
   __shared__ double red[32];
+  chain_wait();
   const EvalLane ln = plan.lanes[blockIdx.y];
   if (!lane_active(ln.status)) return;
   const ProbDev& P = plan.probs[ln.prob];
@@ -212,6 +216,7 @@ __device__ __forceinline__ void lane_energy(const EvalPlan& plan, const EvalLane
 // the first warp of each lane's first pass-2 tile sums it instead (one launch
 // fewer per evaluation, the same sum).
 __global__ void k_energy(EvalPlan plan) {
+  chain_wait();
   const EvalLane ln = plan.lanes[blockIdx.x];
   if (!lane_active(ln.status)) return;
   lane_energy(plan, ln);
@@ -224,6 +229,7 @@ __global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid2(EvalPlan plan
   __shared__ GridStage stage;
   const EvalItem* items = plan.itemsH + plan.h_off[D - 1][ROOTS];
   const int n = plan.h_off[D - 1][ROOTS + 1] - plan.h_off[D - 1][ROOTS];
+  chain_wait<false>();
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     const EvalItem it = items[i];
     const EvalLane ln = plan.lanes[it.lane];
@@ -237,6 +243,7 @@ template <int D, bool F32>
 __global__ void __launch_bounds__(kPass2Threads, 4) k_pass2(EvalPlan plan) {
   extern __shared__ double2 smem[];
   __shared__ ProbDev sp;
+  chain_wait();
   const EvalItem it = plan.items2[plan.d_off2[D - 1] + blockIdx.x];
   const EvalLane ln = plan.lanes[it.lane];
   if (!lane_active(ln.status)) return;
@@ -396,17 +403,18 @@ cudaError_t configure_grid() {
 template <int D, bool ROOTS>
 void launch_grid2(const EvalPlan& plan, cudaStream_t s) {
   const int n = plan.h_off[D - 1][ROOTS + 1] - plan.h_off[D - 1][ROOTS];
-  if (n > 0) k_grid2<D, ROOTS><<<grid_ctas(n), kGridThreads, plan.smemH, s>>>(plan);
+  if (n > 0) launch_chained(plan.chain, k_grid2<D, ROOTS>, grid_ctas(n), kGridThreads, plan.smemH, s, plan);
 }
 
 template <int D, bool F32>
 void launch_d(const EvalPlan& plan, bool pass2, cudaStream_t stream) {
   if (!pass2) {
     const int n = plan.d_off1[D] - plan.d_off1[D - 1];
-    if (n > 0) k_pass1<D, F32><<<n, kPass1Threads, plan.smem1, stream>>>(plan);
+    if (n > 0) launch_chained(plan.chain, k_pass1<D, F32>, n, kPass1Threads, plan.smem1, stream, plan);
   } else {
     const int n = plan.d_off2[D] - plan.d_off2[D - 1];
-    if (n > 0) k_pass2<D, F32><<<n, kPass2Threads, F32 ? plan.smem2_f32 : plan.smem2, stream>>>(plan);
+    if (n > 0)
+      launch_chained(plan.chain, k_pass2<D, F32>, n, kPass2Threads, F32 ? plan.smem2_f32 : plan.smem2, stream, plan);
   }
 }
 
@@ -490,12 +498,12 @@ cudaError_t launch_pass_all(const EvalPlan& plan, bool pass2, cudaStream_t strea
 
 cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream, const EvalSide* side) {
   if (plan.n_grid > 0)
-    k_grid_roots<<<dim3(plan.root_chunks, plan.n_lanes), kRootChunk, 0, stream>>>(plan);
+    launch_chained(plan.chain, k_grid_roots, dim3(plan.root_chunks, plan.n_lanes), kRootChunk, 0, stream, plan);
   cudaError_t e = launch_pass_all(plan, false, stream, side);
   if (e != cudaSuccess) return e;
   if (plan.n_lanes > 0) {
-    k_reduce<<<dim3(plan.red_chunks, plan.n_lanes), kReduceChunk, 0, stream>>>(plan);
-    if (!plan.want_grad) k_energy<<<plan.n_lanes, 32, 0, stream>>>(plan);
+    launch_chained(plan.chain, k_reduce, dim3(plan.red_chunks, plan.n_lanes), kReduceChunk, 0, stream, plan);
+    if (!plan.want_grad) launch_chained(plan.chain, k_energy, plan.n_lanes, 32, 0, stream, plan);
   }
   if (plan.want_grad) {
     e = launch_pass_all(plan, true, stream, side);

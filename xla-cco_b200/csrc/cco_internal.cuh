@@ -217,9 +217,45 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 }
 
 // ---------------------------------------------------------------- launches
+// Chained launches. The kernels of an evaluation or a tick follow one another on a
+// stream, each needing all of its predecessor. launch_chained lets a kernel be
+// set up, and its CTAs come in, while the predecessor's last ones still run; every
+// CTA of it calls chain_wait first (a grid whose CTAs left without it would let
+// its own successor run beside the predecessor), which returns when the
+// predecessor has finished and its writes are visible. EARLY: the successor's
+// CTAs may come in from then on; the grid kernels, which fill the GPU, leave
+// that to their end (let in early they cost the two passes 2%). Used where a call
+// is one evaluation (256 lanes of d=2 N=1000 166 -> 160 us, one of N=20000 288 -> 281,
+// one of d=1 N=7777 with its synchronisation 82 -> 77, a Hessian 129 -> 123) and by
+// the tick graphs of a lone lane (d=2 N=1000 to the ground state 41.7 -> 39.0 ms);
+// graphs of more lanes lose more to the edges than they gain (64 MD lanes, 40
+// steps: 5.17 -> 5.38 ms; 25 of d=3 N=1492: 6.1 -> 6.4 ms).
+template <bool EARLY = true>
+__device__ __forceinline__ void chain_wait() {
+  cudaGridDependencySynchronize();
+  if (EARLY) cudaTriggerProgrammaticLaunchCompletion();
+}
+
+template <class... P, class... A>
+void launch_chained(bool chain, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                    const A&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = chain ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);   // the error is read by cudaGetLastError
+}
+
 // Three launches per evaluation: partial densities, reduction + energy,
 // gradient. Items index (lane, tile); lanes whose status is not RUNNING exit.
 struct EvalPlan {
+  bool chain = false;       // launch_chained: the kernels as a chain
   const ProbDev* probs;     // device
   const EvalLane* lanes;    // device
   const EvalItem* items1;   // device, grouped by d: d = D items at [d_off1[D-1], d_off1[D])

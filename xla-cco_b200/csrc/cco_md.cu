@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(kMdThreads) k_md_update(MdArgs a, double c, do
   __shared__ MdState S;
   __shared__ double red[kMdThreads / 32][4], tot[4], rcm[3];
   __shared__ int pick;
+  chain_wait();
   const int lane = blockIdx.x;
   const LaneRef R = a.lanes[lane];
   const MdView w = md_view(R.rec, R.ld, a.w);
@@ -420,6 +421,7 @@ __global__ void __launch_bounds__(kMdThreads) k_md_update(MdArgs a, double c, do
 // running sums, and the snapshot and trace rows. Waves are independent, so
 // spreading a lane's waves over blocks changes no result.
 __global__ void __launch_bounds__(kUpdThreads) k_md_observe(MdArgs a) {
+  chain_wait();
   const LaneRef R = a.lanes[blockIdx.x];
   const MdView w = md_view(R.rec, R.ld, a.w);
   const MdState* S = w.st;
@@ -815,10 +817,10 @@ cudaError_t md_update(const MdArgs& a, cudaStream_t st) {
       k_md_waves<<<grid, kUpdThreads, 0, st>>>(a);
     }
   }
-  k_md_update<<<a.B, kMdThreads, 0, st>>>(a, c, noise_var);
+  launch_chained(a.chain, k_md_update, a.B, kMdThreads, 0, st, a, c, noise_var);
   if (a.w > 0) {
     const dim3 grid(a.B, (a.w + kUpdThreads - 1) / kUpdThreads);
-    k_md_observe<<<grid, kUpdThreads, 0, st>>>(a);
+    launch_chained(a.chain, k_md_observe, grid, kUpdThreads, 0, st, a);
   }
   return cudaGetLastError();
 }

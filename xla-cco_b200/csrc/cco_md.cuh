@@ -86,6 +86,7 @@ struct MdSegIO {
 };
 
 struct MdArgs {
+  bool chain = false;   // launch_chained
   int B;
   const LaneRef* lanes;
   double dt, gamma, temperature, andersen_p, drift_tol;

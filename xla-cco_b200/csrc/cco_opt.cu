@@ -59,6 +59,7 @@ __global__ void k_descent_init(DescentArgs a, const double* __restrict__ s0) {
 namespace {
 
 __global__ void __launch_bounds__(kUpdThreads) k_descent_update(DescentArgs a) {
+  chain_wait();
   descent_update_lane(a, blockIdx.x);
 }
 
@@ -417,6 +418,7 @@ __global__ void k_lbfgs_init(LbArgs A, const double* __restrict__ s0) {
 // places the next probe or ends the iteration.
 __global__ void __launch_bounds__(kUpdThreads, 2) k_lbfgs_probe(LbArgs A) {
   __shared__ LbShared sh;
+  chain_wait();
   const int lane = blockIdx.x;
   const LaneRef R = A.lanes[lane];
   const LbView v = lane_view(A, R);
@@ -566,6 +568,7 @@ __global__ void __launch_bounds__(kUpdThreads, 2) k_lbfgs_probe(LbArgs A) {
 // y_p.y_n. One warp per (pair, chunk) with four double2 words per lane in
 // flight; a lane of one chunk writes the dots, a wide lane its partials.
 __global__ void __launch_bounds__(kUpdThreads) k_lbfgs_passA(LbArgs A) {
+  chain_wait();
   const int lane = blockIdx.y;
   const LaneRef R = A.lanes[lane];
   const int chunk = blockIdx.x % A.nchA, pblk = blockIdx.x / A.nchA;
@@ -699,6 +702,7 @@ __global__ void __launch_bounds__(kUpdThreads) k_lbfgs_scalar(LbArgs A) {
   __shared__ int sl[kScalarMaxPairs];
   __shared__ double red[32];
   __shared__ double gam_s;
+  chain_wait();
   const int lane = blockIdx.x;
   const LaneRef R = A.lanes[lane];
   const LbView v = lane_view(A, R);
@@ -854,6 +858,7 @@ __global__ void __launch_bounds__(kUpdThreads) k_lbfgs_scalar(LbArgs A) {
 __global__ void __launch_bounds__(kUpdThreads) k_lbfgs_passB(LbArgs A) {
   __shared__ double cyv[kPassBMaxPairs], csv[kPassBMaxPairs];
   __shared__ double red[32];
+  chain_wait();
   const int lane = blockIdx.y;
   const LaneRef R = A.lanes[lane];
   if ((int)blockIdx.x >= lb_nblk(R.ld)) return;   // this lane has fewer element blocks
@@ -1033,7 +1038,7 @@ cudaError_t descent_init(const DescentArgs& a, const double* s0, cudaStream_t st
   return cudaGetLastError();
 }
 cudaError_t descent_update(const DescentArgs& a, cudaStream_t st) {
-  k_descent_update<<<a.B, kUpdThreads, 0, st>>>(a);
+  launch_chained(a.chain, k_descent_update, a.B, kUpdThreads, 0, st, a);
   return cudaGetLastError();
 }
 cudaError_t descent_finalize(const DescentArgs& a, double* s_out, double* e_out, double* gn_out,
@@ -1056,12 +1061,12 @@ cudaError_t lbfgs_init(const LbArgs& a, const double* s0, cudaStream_t st) {
 // One tick of the minimizer: the probe kernel for every lane, then the three
 // direction stages, which exit at once for lanes that are mid line search.
 cudaError_t lbfgs_update(const LbArgs& a, cudaStream_t st) {
-  k_lbfgs_probe<<<a.B, kUpdThreads, 0, st>>>(a);
+  launch_chained(a.chain, k_lbfgs_probe, a.B, kUpdThreads, 0, st, a);
   const dim3 ga((a.m + kUpdThreads / 32 - 1) / (kUpdThreads / 32) * a.nchA, a.B);
-  k_lbfgs_passA<<<ga, kUpdThreads, 0, st>>>(a);
-  k_lbfgs_scalar<<<a.B, kUpdThreads, a.smem_tri, st>>>(a);
+  launch_chained(a.chain, k_lbfgs_passA, ga, kUpdThreads, 0, st, a);
+  launch_chained(a.chain, k_lbfgs_scalar, a.B, kUpdThreads, a.smem_tri, st, a);
   const dim3 gb(a.nblkB, a.B);
-  k_lbfgs_passB<<<gb, kUpdThreads, 0, st>>>(a);
+  launch_chained(a.chain, k_lbfgs_passB, gb, kUpdThreads, 0, st, a);
   return cudaGetLastError();
 }
 cudaError_t lbfgs_finalize(const LbArgs& a, double* s_out, double* e_out, double* gn_out,

@@ -80,6 +80,7 @@ __host__ __device__ __forceinline__ size_t ds_record_doubles(int ld, size_t scra
 }
 
 struct DescentArgs {
+  bool chain = false;   // launch_chained
   int B;
   const LaneRef* lanes;
   double step_init, step_min, shrink, grow, rel_tol, energy_tol;
@@ -187,6 +188,7 @@ __host__ __device__ __forceinline__ size_t lb_record_doubles(int m, int tri_len,
 }
 
 struct LbArgs {
+  bool chain = false;   // launch_chained
   int B, m, n_pass, tri_len;
   const LaneRef* lanes;
   double rescales[CCO_MAX_RESCALES];

@@ -121,6 +121,8 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
     const int lo = bounds[b], hi = bounds[b + 1];
     const bool may_fp32 = T.shape.method == Method::Lbfgs && T.lb.prec0 == PREC_FP32;
     CCO_CUDA(ev[b].build(T.shape, T.refs, T.probs, lo, hi, st, may_fp32));
+    const bool chain = B == 1;   // launch_chained
+    ev[b].plan.chain = chain;
     int nblk = 1, nch = 1;
     for (int i = lo; i < hi; ++i) {
       nblk = std::max(nblk, lb_nblk(T.refs[i].ld));
@@ -133,16 +135,19 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
       fl[b] = a;
     } else if (T.shape.method == Method::Md) {
       MdArgs a = T.md;
+      a.chain = chain;
       a.B = hi - lo;
       a.lanes = T.d_refs + lo;
       md[b] = a;
     } else if (T.shape.method == Method::Descent) {
       DescentArgs a = T.ds;
+      a.chain = chain;
       a.B = hi - lo;
       a.lanes = T.d_refs + lo;
       ds[b] = a;
     } else {
       LbArgs a = T.lb;
+      a.chain = chain;
       a.B = hi - lo;
       a.lanes = T.d_refs + lo;
       a.nblkB = nblk;
