@@ -247,7 +247,7 @@ typedef struct {
   int64_t ticks;        /* out: device ticks (one energy evaluation per running lane each) */
   int64_t launches;     /* out: kernel launches issued by the call */
   int32_t branches;     /* out: graph branches of the tick schedule used */
-  int32_t graph_ticks;  /* out: ticks per captured graph of that schedule */
+  int32_t graph_ticks;  /* out: most ticks of one launch of that schedule */
   int32_t overlap;      /* out: 1 if that schedule ran the branches half a tick apart with
                            the update kernels at high stream priority */
   int32_t reserved;     /* zero */
@@ -481,9 +481,9 @@ int cco_md_segment(cco_problem* p, void* stream, int batch, const double* basis,
  * N M bucketed by powers of two, largest d) and cached for the process;
  * results never depend on the schedule. This forgets every cached schedule.
  * The environment variables CCO_BRANCHES, CCO_GRAPH_TICKS and CCO_OVERLAP
- * (0 or 1) force a schedule, CCO_AUTOTUNE=0 keeps the default (2 branches,
- * 16 ticks, no overlap). CCO_INFLIGHT (1..16, default 3) sets how many
- * graphs the driver keeps queued ahead of its completion checks.
+ * (0 or 1) force a schedule, CCO_AUTOTUNE=0 keeps the default (one branch, two
+ * from 64 lanes, 16 ticks, no overlap). CCO_INFLIGHT (1..16, default 3) sets how
+ * many graphs the driver keeps queued ahead of its completion checks.
  */
 int cco_schedule_reset(void);
 
@@ -507,7 +507,7 @@ typedef struct {
   int64_t max_lanes;        /* lanes on the device at once (0: 4096) */
   int64_t hbm_budget_bytes; /* admission budget for lane records (0: 150 GB), clamped to 90%
                                of the device memory free at creation */
-  int32_t graph_ticks;      /* ticks per launched graph (0: 8) */
+  int32_t graph_ticks;      /* most ticks of one launch (0: 8) */
   int32_t branches;         /* graph branches (0: 2 when >= 64 lanes run, else 1) */
 } cco_server_config;
 

@@ -36,6 +36,7 @@
 //     w(Im rho cos - Re rho sin) and two accumulations; prefix axes are
 //     weighted once per segment.
 #include <algorithm>
+#include <vector>
 #include <cstdio>
 #include <cstdlib>
 
@@ -435,11 +436,11 @@ cudaError_t eval_configure() {
 
 namespace {
 
-// The pass kernels of dimension D on stream s (per-segment and grid forms).
-// FP64 lanes run the F32 = false kernels whatever the plan; a plan that may
-// hold FP32 lanes (dyn_prec) launches the F32 = true kernels as well.
+// The pass kernels of dimension D (per-segment and grid forms). FP64 lanes run
+// the F32 = false kernels whatever the plan; a plan that may hold FP32 lanes
+// (dyn_prec) launches the F32 = true kernels as well.
 template <int D>
-void launch_dim_d(const EvalPlan& plan, bool pass2, cudaStream_t s) {
+void launch_dim(const EvalPlan& plan, bool pass2, cudaStream_t s) {
   launch_d<D, false>(plan, pass2, s);
   if (plan.dyn_prec) launch_d<D, true>(plan, pass2, s);
   if (pass2) {
@@ -450,63 +451,54 @@ void launch_dim_d(const EvalPlan& plan, bool pass2, cudaStream_t s) {
   }
 }
 void launch_dim(const EvalPlan& plan, bool pass2, int D, cudaStream_t s) {
-  if (D == 1) launch_dim_d<1>(plan, pass2, s);
-  else if (D == 2) launch_dim_d<2>(plan, pass2, s);
-  else launch_dim_d<3>(plan, pass2, s);
+  if (D == 1) launch_dim<1>(plan, pass2, s);
+  else if (D == 2) launch_dim<2>(plan, pass2, s);
+  else launch_dim<3>(plan, pass2, s);
 }
 
-// One pass over every dimension present: in order on `stream`, or, with side
-// streams and more than one dimension, the first dimension on `stream` and the
-// others on side streams forked from it and joined back before returning.
-cudaError_t launch_pass_all(const EvalPlan& plan, bool pass2, cudaStream_t stream,
-                            const EvalSide* side) {
-  bool has[4] = {false, false, false, false};
-  int nd = 0;
-  for (int D = 1; D <= 3; ++D) {
-    has[D] = eval_has_dim(plan, D);
-    nd += has[D];
-  }
-  if (!side || nd < 2) {
-    for (int D = 1; D <= 3; ++D)
-      if (has[D]) launch_dim(plan, pass2, D, stream);
-    return cudaGetLastError();
-  }
-  cudaError_t e = cudaEventRecord(side->fork, stream);
-  cudaStream_t sd[4] = {stream, stream, stream, stream};
-  int used = 0;
-  bool first = true;
+// The nodes that the next operation captured on a stream depends on.
+cudaError_t capture_front(cudaStream_t s, std::vector<cudaGraphNode_t>* front) {
+  cudaStreamCaptureStatus status;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t n = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &n);
+  if (e == cudaSuccess) front->assign(deps, deps + n);
+  return e;
+}
+
+// One pass over every dimension present: in order on `stream`, or, while a tick
+// graph is captured (fork), every dimension's kernels as a chain of nodes of
+// their own, from what came before and joined before what follows.
+cudaError_t launch_pass_all(const EvalPlan& plan, bool pass2, cudaStream_t stream, bool fork) {
+  std::vector<cudaGraphNode_t> base, at, ends;
+  cudaError_t e = fork ? capture_front(stream, &base) : cudaSuccess;
   for (int D = 1; D <= 3 && e == cudaSuccess; ++D) {
-    if (!has[D]) continue;
-    if (first) {
-      first = false;
-      continue;
-    }
-    sd[D] = side->aux[used++];
-    e = cudaStreamWaitEvent(sd[D], side->fork, 0);
+    if (fork)
+      e = cudaStreamUpdateCaptureDependencies(stream, base.data(), base.size(),
+                                              cudaStreamSetCaptureDependencies);
+    if (e == cudaSuccess) launch_dim(plan, pass2, D, stream);
+    if (fork && e == cudaSuccess) e = capture_front(stream, &at);
+    if (fork && at != base) ends.insert(ends.end(), at.begin(), at.end());
   }
-  if (e != cudaSuccess) return e;
-  for (int D = 1; D <= 3; ++D)
-    if (has[D]) launch_dim(plan, pass2, D, sd[D]);
-  for (int u = 0; u < used && e == cudaSuccess; ++u) {
-    e = cudaEventRecord(side->join[u], side->aux[u]);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, side->join[u], 0);
-  }
+  if (e == cudaSuccess && !ends.empty())
+    e = cudaStreamUpdateCaptureDependencies(stream, ends.data(), ends.size(),
+                                            cudaStreamSetCaptureDependencies);
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace
 
-cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream, const EvalSide* side) {
+cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream, bool fork) {
   if (plan.n_grid > 0)
     launch_chained(plan.chain, k_grid_roots, dim3(plan.root_chunks, plan.n_lanes), kRootChunk, 0, stream, plan);
-  cudaError_t e = launch_pass_all(plan, false, stream, side);
+  cudaError_t e = launch_pass_all(plan, false, stream, fork);
   if (e != cudaSuccess) return e;
   if (plan.n_lanes > 0) {
     launch_chained(plan.chain, k_reduce, dim3(plan.red_chunks, plan.n_lanes), kReduceChunk, 0, stream, plan);
     if (!plan.want_grad) launch_chained(plan.chain, k_energy, plan.n_lanes, 32, 0, stream, plan);
   }
   if (plan.want_grad) {
-    e = launch_pass_all(plan, true, stream, side);
+    e = launch_pass_all(plan, true, stream, fork);
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();

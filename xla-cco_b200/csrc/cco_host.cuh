@@ -293,6 +293,11 @@ struct Schedule {
   int overlap = 0;
 };
 constexpr int kMaxBranches = 8;
+// Before a shape class is tuned: one branch below 64 lanes, where a second one costs
+// more to set up and join than it overlaps (32 evaluations of d=2 N=1000: 2 / 4 /
+// 16 lanes 2.68 / 2.76 / 2.91 ms in one branch, 3.13 / 3.21 / 3.39 in two; 256 lanes
+// 8.30 and 8.13).
+inline int default_branches(size_t lanes) { return lanes >= 64 ? 2 : 1; }
 constexpr int kInflight = 3;    // graphs in flight before the host checks completion
 constexpr int kMaxInflight = 16;   // CCO_INFLIGHT bound (and the round bounds' slack)
 
@@ -358,8 +363,9 @@ struct TickPlan {
   cudaGraph_t graph = nullptr;   // owns the loop's condition: outlives the launches
   TickLoop* loop = nullptr;
   int body = 1, bodies = 1;      // ticks of the body, bodies of one launch
+  bool forks[kMaxBranches] = {}; // dimensions of a pass as parallel nodes
   int build(const LaneTable& T, const Schedule& sch, cudaStream_t st);
-  cudaError_t tick(cudaStream_t s, int b, const EvalSide* side = nullptr) const;
+  cudaError_t tick(cudaStream_t s, int b) const;
   cudaError_t update(cudaStream_t s, int b) const;
   int launches_per_tick() const;
   int loop_gates() const { return bodies > 1; }   // condition kernels per body

@@ -252,8 +252,8 @@ void launch_chained(bool chain, void (*kernel)(P...), dim3 grid, int threads, si
   cudaLaunchKernelEx(&cfg, kernel, P(args)...);   // the error is read by cudaGetLastError
 }
 
-// Three launches per evaluation: partial densities, reduction + energy,
-// gradient. Items index (lane, tile); lanes whose status is not RUNNING exit.
+// Launches of an evaluation: (phase roots,) partial densities, reduction +
+// energy, gradient. Items index (lane, tile); lanes whose status is not RUNNING exit.
 struct EvalPlan {
   bool chain = false;       // launch_chained: the kernels as a chain
   const ProbDev* probs;     // device
@@ -322,17 +322,9 @@ __host__ __device__ __forceinline__ size_t eval_scratch_words(const ProbDev& p) 
   return (size_t)p.M + eval_rhow_words(p) + eval_part_words(p) + eval_roots_words(p);
 }
 
-// Side streams of one launching stream: when a plan holds lanes of several
-// dimensions, each dimension's pass kernels run on their own stream (forked
-// from and joined back into the launching stream with these events), so the
-// small per-dimension grids of a mixed plan overlap instead of running back
-// to back. The kernels and their results are the same either way.
-struct EvalSide {
-  cudaStream_t aux[2];
-  cudaEvent_t fork, join[2];
-};
-cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream,
-                        const EvalSide* side = nullptr);
+// fork: `stream` is being captured into a tick graph; the dimensions of a pass
+// become parallel nodes.
+cudaError_t eval_launch(const EvalPlan& plan, cudaStream_t stream, bool fork = false);
 // Kernels one eval_launch of a plan issues: per dimension the per-segment and
 // grid pass kernels that have items, plus the reduction (and the energy kernel
 // when there is no pass 2).
@@ -347,18 +339,6 @@ inline int eval_kernels(const EvalPlan& p) {
       n += per * (p.d_off2[D] > p.d_off2[D - 1]) + (p.h_off[D - 1][1] > p.h_off[D - 1][0]) +
            (p.h_off[D - 1][2] > p.h_off[D - 1][1]);
   }
-  return n;
-}
-
-// Whether a plan launches pass kernels of dimension D.
-inline bool eval_has_dim(const EvalPlan& p, int D) {
-  return p.d_off1[D] > p.d_off1[D - 1] || p.q_offG[D - 1][kGridClasses] > p.q_offG[D - 1][0] ||
-         p.d_off2[D] > p.d_off2[D - 1] || p.h_off[D - 1][2] > p.h_off[D - 1][0];
-}
-// Dimensions whose pass kernels a plan launches (side streams pay off from 2).
-inline int eval_dims(const EvalPlan& p) {
-  int n = 0;
-  for (int D = 1; D <= 3; ++D) n += eval_has_dim(p, D);
   return n;
 }
 size_t eval_smem1(const ProbDev& p);

@@ -4,11 +4,12 @@
 // A tick of the graph driver (cco_relax.cu) is five to eight dependent kernel
 // launches; for a problem of a few thousand (k, particle) pairs - the
 // reference README's d=3 N=100 chi=0.05 relax has 1300 - their launch
-// latency is the whole cost of an iteration. Here a CTA of 128 threads (the
-// evaluation bodies' size) owns one lane and loops: pass 1 over the lane's
-// particle tiles (per-segment form), the tile-order reduction to rho,
-// w rho and Phi, pass 2 over its tiles, and the descent update, with block
-// barriers between the stages and no host round trip. Lanes never wait on
+// latency is the whole cost of an iteration. Here a CTA owns one lane and loops
+// with block barriers between the stages and no host round trip. Lanes that fit
+// shared memory altogether run k_persist_compact (512 threads, below); the others
+// k_persist_descent (128 threads, the evaluation bodies' size): pass 1 over the
+// lane's particle tiles (per-segment form), the tile-order reduction to rho,
+// w rho and Phi, pass 2 over its tiles, and the descent update. Lanes never wait on
 // one another, so there is no inter-CTA synchronization; the loop ends when
 // the lane's status leaves RUNNING or after the same tick bound as the graph
 // driver (then the launch reports an overrun, the host CCO_ERR_ROUNDS).

@@ -6,8 +6,8 @@
 // Reference: relax (src/xla_cco/minimize/__init__.py:102-151) runs host
 // rounds of jitted chunks over the RUNNING lanes, padded to a power of two,
 // with a host sync per round. Here every lane is a device state machine
-// (cco_opt.cu); the host only launches captured graphs of ticks and checks,
-// a few graphs behind, whether any lane is still RUNNING.
+// (cco_opt.cu); the host only launches graphs that loop over ticks until every
+// lane has finished, and looks a few launches behind which lanes have.
 #include <cmath>
 #include <cstdlib>
 #include <map>
@@ -89,6 +89,25 @@ void schedule_clear() {
 // ------------------------------------------------------------ tick plans
 namespace {
 
+double eval_flops(const cco_problem* p) {
+  return (double)p->N * p->M * (p->d == 1 ? 7.0 : p->d == 2 ? 21.0 : 35.0);
+}
+
+// Whether the dimensions of a branch's passes run as parallel nodes. A fork and
+// its join cost a tick tens of us on the device, so they pay only for ticks of
+// much work (20 evaluations, forked against in order: 48 lanes of N <= 8000,
+// 3.5 GFLOP a tick, 10.9 against 11.3 ms; 16 of them, 1.2 GFLOP, 6.6 against
+// 6.2 ms; 48 of N <= 2000 6.7 against 5.1 ms, 8 of them 7.5 against 4.1 ms).
+bool eval_forks(const std::vector<const cco_problem*>& probs, int lo, int hi) {
+  double flops = 0.0;
+  int dims = 0;
+  for (int i = lo; i < hi; ++i) {
+    flops += eval_flops(probs[i]);
+    dims |= 1 << probs[i]->d;
+  }
+  return (dims & (dims - 1)) != 0 && flops >= 1.5e9;
+}
+
 // Ticks of a loop body. Each body costs about 9 us more (a condition kernel,
 // the loop's own turn, the join of the branches: ticks of 7 empty kernels took
 // 5.9 us in a flat graph, 9.2 / 7.9 / 7.2 us in bodies of 2 / 4 / 8), a run ends
@@ -100,8 +119,7 @@ namespace {
 // 256 lanes of d=2 N=1000 and 32 evaluations (9.3; the rule takes 4).
 int body_ticks(const std::vector<const cco_problem*>& probs, int launches, int graph_ticks) {
   double flops = 0.0;
-  for (const cco_problem* p : probs)
-    flops += (double)p->N * p->M * (p->d == 1 ? 7.0 : p->d == 2 ? 21.0 : 35.0);
+  for (const cco_problem* p : probs) flops += eval_flops(p);
   const double us = flops / 15e6 + 2.0 * launches;
   const int gt = std::max(1, graph_ticks);
   for (int t = std::max(1, (int)(600.0 / us)); t < gt; ++t)
@@ -123,6 +141,7 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
     CCO_CUDA(ev[b].build(T.shape, T.refs, T.probs, lo, hi, st, may_fp32));
     const bool chain = B == 1;   // launch_chained
     ev[b].plan.chain = chain;
+    forks[b] = eval_forks(T.probs, lo, hi);
     int nblk = 1, nch = 1;
     for (int i = lo; i < hi; ++i) {
       nblk = std::max(nblk, lb_nblk(T.refs[i].ld));
@@ -163,18 +182,9 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
   // branch; branches fork from and join back into the first capture stream
   cudaStream_t cap[kMaxBranches] = {};
   cudaEvent_t fork = nullptr, join[kMaxBranches] = {};
-  EvalSide side[kMaxBranches] = {};   // per-dimension side streams of each branch
   cudaError_t e = cudaSuccess;
   for (int b = 0; b < nbr && e == cudaSuccess; ++b)
     e = cudaStreamCreateWithFlags(&cap[b], cudaStreamNonBlocking);
-  for (int b = 0; b < nbr && e == cudaSuccess; ++b) {
-    if (eval_dims(ev[b].plan) < 2) continue;   // one dimension: no side streams
-    for (int u = 0; u < 2 && e == cudaSuccess; ++u) {
-      e = cudaStreamCreateWithFlags(&side[b].aux[u], cudaStreamNonBlocking);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&side[b].join[u], cudaEventDisableTiming);
-    }
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&side[b].fork, cudaEventDisableTiming);
-  }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
   for (int b = 0; b < nbr && e == cudaSuccess; ++b)
     e = cudaEventCreateWithFlags(&join[b], cudaEventDisableTiming);
@@ -231,13 +241,12 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
     for (int b = 1; b < nbr && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(cap[b], fork, 0);
     for (int t = 0; t < body && e == cudaSuccess; ++t)
       for (int b = 0; b < nbr && e == cudaSuccess; ++b) {
-        const EvalSide* sd = side[b].fork ? &side[b] : nullptr;
         if (!overlap) {
-          e = tick(cap[b], b, sd);
+          e = tick(cap[b], b);
           continue;
         }
         if (t == 0 && b > 0) e = cudaStreamWaitEvent(cap[b], phase, 0);
-        if (e == cudaSuccess) e = eval_launch(ev[b].plan, cap[b], sd);
+        if (e == cudaSuccess) e = eval_launch(ev[b].plan, cap[b], forks[b]);
         if (e == cudaSuccess && t == 0 && b == 0) e = cudaEventRecord(phase, cap[0]);
         if (e == cudaSuccess) e = cudaEventRecord(ev_done[b], cap[b]);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(up[b], ev_done[b], 0);
@@ -262,11 +271,6 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
     if (up[b]) cudaStreamDestroy(up[b]);
     if (ev_done[b]) cudaEventDestroy(ev_done[b]);
     if (up_done[b]) cudaEventDestroy(up_done[b]);
-    for (int u = 0; u < 2; ++u) {
-      if (side[b].aux[u]) cudaStreamDestroy(side[b].aux[u]);
-      if (side[b].join[u]) cudaEventDestroy(side[b].join[u]);
-    }
-    if (side[b].fork) cudaEventDestroy(side[b].fork);
   }
   if (fork) cudaEventDestroy(fork);
   if (phase) cudaEventDestroy(phase);
@@ -275,8 +279,9 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
   return CCO_OK;
 }
 
-cudaError_t TickPlan::tick(cudaStream_t s, int b, const EvalSide* side) const {
-  cudaError_t e = eval_launch(ev[b].plan, s, side);
+// Captures one tick of branch b.
+cudaError_t TickPlan::tick(cudaStream_t s, int b) const {
+  cudaError_t e = eval_launch(ev[b].plan, s, forks[b]);
   if (e != cudaSuccess) return e;
   return update(s, b);
 }
@@ -510,6 +515,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     C.md.lanes = C.d_refs;
     C.md.B = (int)C.refs.size();
     Schedule s;
+    s.branches = default_branches(C.refs.size());
     if (force_br > 0 || force_gt > 0 || force_ov >= 0) {
       if (force_br > 0) s.branches = force_br;
       if (force_gt > 0) s.graph_ticks = force_gt;

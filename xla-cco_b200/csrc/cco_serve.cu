@@ -388,7 +388,7 @@ class Driver {
     table_.lb.lanes = table_.d_refs;
     Schedule sch;
     sch.graph_ticks = S_->graph_ticks;
-    sch.branches = S_->branches > 0 ? S_->branches : (live_.size() >= 64 ? 2 : 1);
+    sch.branches = S_->branches > 0 ? S_->branches : default_branches(live_.size());
     plan_.reset(new TickPlan());
     plan_->method = Method::Lbfgs;
     rc = plan_->build(table_, sch, st_);
