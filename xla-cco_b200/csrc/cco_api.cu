@@ -804,33 +804,38 @@ struct EvalWS {
   unsigned char* block = nullptr;   // the allocation that holds them (null: the caller's memory)
   EvalPlan plan{};
   int prec = PREC_FP64;   // arithmetic of every lane of this workspace
+  int cap = 0, split = 1;   // lanes that fit, pass-2 threads per particle: of the carve
 
-  // Element counts of a batch of B (b_*: of the whole batch).
+  // Element counts of one lane.
   struct Sizes {
     bool grid, grid2;   // the grid form in pass 1, in pass 2
-    int split, nt1, nt2;
-    size_t rhow, part, roots;   // double2 words per lane
+    int nt1, nt2;
+    size_t rhow, part, roots;   // double2 words
   };
-  static Sizes sizes(const cco_problem* p, int B, int prec) {
+  static Sizes sizes(const cco_problem* p, int prec, int split) {
     Sizes z;
     const ProbDev& h = p->host;
     z.grid = h.grid && prec == PREC_FP64;
-    z.split = pass2_split((long long)B * h.ntile2);
     z.nt1 = z.grid ? h.gntile * h.ngblk : h.ntile1;
     z.grid2 = z.grid && h.grid == 1;
-    z.nt2 = z.grid2 ? (h.N + kGridTile2 - 1) / kGridTile2 : pass2_tiles(h, z.split);
+    z.nt2 = z.grid2 ? (h.N + kGridTile2 - 1) / kGridTile2 : pass2_tiles(h, split);
     z.rhow = z.grid ? (size_t)h.grhow : (size_t)h.M;
     z.part = z.grid ? 2 * (size_t)h.gntile * h.gslots : (size_t)h.ntile1 * h.M;
     z.roots = z.grid ? eval_roots_words(h) : 0;
     return z;
   }
-  // Byte offsets of the buffers in one block of memory.
+  // Byte offsets of the buffers of up to B lanes in one block of memory. The
+  // pass-2 split is part of it: fewer lanes would choose a larger one, and with
+  // it more items than the block has room for.
   struct Carve {
+    int lanes, split;
     size_t it1, it2, rho, rhow, part, roots, total;
   };
   static Carve carve(const cco_problem* p, int B, int prec) {
-    const Sizes z = sizes(p, B, prec);
     Carve c;
+    c.lanes = B;
+    c.split = pass2_split((long long)B * p->host.ntile2);
+    const Sizes z = sizes(p, prec, c.split);
     c.it1 = round256(sizeof(EvalLane) * B);
     c.it2 = c.it1 + round256(sizeof(EvalItem) * (size_t)B * z.nt1);
     c.rho = c.it2 + round256(sizeof(EvalItem) * (size_t)B * z.nt2);
@@ -841,6 +846,8 @@ struct EvalWS {
     return c;
   }
   void place(unsigned char* base, const Carve& c) {
+    cap = c.lanes;
+    split = c.split;
     lanes = reinterpret_cast<EvalLane*>(base);
     it1 = reinterpret_cast<EvalItem*>(base + c.it1);
     it2 = reinterpret_cast<EvalItem*>(base + c.it2);
@@ -860,7 +867,8 @@ struct EvalWS {
   }
   cudaError_t build(const cco_problem* p, int B, const double* s, size_t s_stride, double* f,
                     size_t f_stride, double* g, size_t g_stride, cudaStream_t st) {
-    const Sizes z = sizes(p, B, prec);
+    if (B > cap) return cudaErrorInvalidValue;
+    const Sizes z = sizes(p, prec, split);
     const int total = B * std::max(z.nt1, z.nt2) + B;
     const int blocks = std::min(1024, (total + 255) / 256);
     k_make_lanes<<<blocks, 256, 0, st>>>(lanes, it1, it2, B, z.nt1, z.nt2, total, s, s_stride, f,
@@ -893,9 +901,9 @@ struct EvalWS {
     plan.dyn_prec = prec == PREC_FP32 ? 1 : 0;
     plan.max_d = p->d;
     plan.smem1 = p->smem1;
-    plan.smem2 = eval_smem2(p->host, z.split);
-    plan.smem2_f32 = eval_smem2(p->host, z.split, true);
-    plan.split2 = z.split;
+    plan.smem2 = eval_smem2(p->host, split);
+    plan.smem2_f32 = eval_smem2(p->host, split, true);
+    plan.split2 = split;
     plan.chunks1 = 1;
     plan.red_chunks = reduce_chunks(z.grid ? p->host.gslots : p->M);
     plan.want_grad = g != nullptr;
