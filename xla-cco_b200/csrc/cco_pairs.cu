@@ -256,6 +256,7 @@ __global__ void __launch_bounds__(kPairTile) k_nearest(const double* __restrict_
 constexpr int kCellThreads = 512;
 constexpr double kCellReach = 65536.0;     // largest |s| of a cell grid
 constexpr double kCellMargin = 1e-7;       // relative: |s| rounding 2^-37, G <= 2048
+constexpr double kCellLeast = 1e-7;        // shortest FP32 distance / longest axis
 constexpr int kMaxCells = 8192, kMaxAxisCells = 2048;
 constexpr size_t kCellSmem = 200 * 1024;
 constexpr double kHistReach = 3.0;     // cells per histogram range, at least
@@ -271,6 +272,8 @@ constexpr int kCellCrowd = 64;
 struct CellGrid {
   int G[3], K[3], cells;   // cells per axis, stencil reach, all cells
   float lim;               // histogram: FP32 r2 no pair in range exceeds
+  float least;             // FP32 r2 below which a pair counts as that far apart: of the
+                           // box's own size, so that every allowance scales with it
   float eps;               // and bins around an edge that FP32 cannot tell (0: queue every pair)
 };
 
@@ -517,7 +520,7 @@ __global__ void __launch_bounds__(kCellThreads)
 #pragma unroll 4
         for (int k = 0; k < most; ++k) {
           const int j = at(k);
-          const float r2 = fmaxf(screen(k, j), 1e-30f);
+          const float r2 = fmaxf(screen(k, j), cg.least);
           const float u = fmaf(r2 * rsqrtf(r2), g.inv_w, shift);   // bin - 1/2
           const float n = u + 0x1.8p23f;                           // its nearest integer
           const int b = __float_as_int(n) - 0x4b400000;
@@ -600,7 +603,7 @@ __global__ void __launch_bounds__(kCellThreads)
 // if the stencil covers too much of the box or the configuration is too large
 // or too small.
 bool cell_grid(const PairGeom& g, int d, double side, double reach, double most, CellGrid* c) {
-  *c = CellGrid{{1, 1, 1}, {0, 0, 0}, 1, 0.f, 0.f};
+  *c = CellGrid{{1, 1, 1}, {0, 0, 0}, 1, 0.f, 0.f, 0.f};
   double part = 1.0, longest = 0.0;
   if (!(side > 0.0) || g.n > 0xffff) return false;
   for (int a = 0; a < d; ++a) {
@@ -618,6 +621,7 @@ bool cell_grid(const PairGeom& g, int d, double side, double reach, double most,
   }
   const double r = reach + 1e-6 * longest;
   c->lim = (float)(r * r * (1.0 + 1e-6));
+  c->least = (float)(kCellLeast * longest * kCellLeast * longest);
   return part <= most;
 }
 
@@ -727,11 +731,12 @@ int cco_pair_histogram(int device, void* stream, int batch, int n, int d, const 
   for (int a = 0; a < d; ++a) vol *= std::fabs(g.B[a * d + a]);
   const double side = std::max(edges[g.n_bins] / kHistReach * (1.0 + 4.0 * kCellMargin),
                                std::pow(kHistFill * vol / n, 1.0 / d));
-  // edges against the even ones, and the longest axis, for the FP32 bins
+  // FP32 bins: what rounding and the shortest distance can move a pair by, and the
+  // edges against the even ones
   double dev = 0.0, longest = 0.0;
   for (int k = 0; k < n_edges; ++k) dev = std::max(dev, std::fabs(edges[k] - (edges[0] + k * width)));
   for (int a = 0; a < d; ++a) longest = std::max(longest, std::fabs(g.B[a * d + a]));
-  const double eps = 1.01 * (1e-6 * longest + 1e-6 * edges[g.n_bins] + dev) / width;
+  const double eps = 1.01 * ((1e-6 + kCellLeast) * longest + 1e-6 * edges[g.n_bins] + dev) / width;
   CellGrid cg;
   const size_t pos_smem = sizeof(double) * n * d + sizeof(float) * ((n + 1) / 2 * 2) * d;
   const size_t cell_smem = pos_smem + bin_smem + sizeof(int) * kMaxCells;
