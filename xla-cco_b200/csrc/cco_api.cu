@@ -658,9 +658,7 @@ int cco_problem_create_rows(int device, int d, int n_particles, int m, const int
                 P.t1.nrows, P.t2.nrows);
 
   DeviceGuard guard(device);
-  static std::once_flag once;
-  static cudaError_t cfg_err = cudaSuccess;
-  std::call_once(once, [] { cfg_err = eval_configure(); });
+  const cudaError_t cfg_err = eval_configure();
   if (cfg_err != cudaSuccess) return cuda_fail(cfg_err, "eval_configure");
 
   auto* pr = new cco_problem();

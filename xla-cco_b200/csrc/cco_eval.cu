@@ -422,16 +422,19 @@ void launch_d(const EvalPlan& plan, bool pass2, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t eval_configure() {
-  cudaError_t e = configure_grid<1>();
-  if (e == cudaSuccess) e = configure_grid<2>();
-  if (e == cudaSuccess) e = configure_grid<3>();
-  if (e == cudaSuccess) e = configure_d<1, false>();
-  if (e == cudaSuccess) e = configure_d<2, false>();
-  if (e == cudaSuccess) e = configure_d<3, false>();
-  if (e == cudaSuccess) e = configure_d<1, true>();
-  if (e == cudaSuccess) e = configure_d<2, true>();
-  if (e == cudaSuccess) e = configure_d<3, true>();
-  return e;
+  static OncePerDevice once;
+  return once.run([] {
+    cudaError_t e = configure_grid<1>();
+    if (e == cudaSuccess) e = configure_grid<2>();
+    if (e == cudaSuccess) e = configure_grid<3>();
+    if (e == cudaSuccess) e = configure_d<1, false>();
+    if (e == cudaSuccess) e = configure_d<2, false>();
+    if (e == cudaSuccess) e = configure_d<3, false>();
+    if (e == cudaSuccess) e = configure_d<1, true>();
+    if (e == cudaSuccess) e = configure_d<2, true>();
+    if (e == cudaSuccess) e = configure_d<3, true>();
+    return e;
+  });
 }
 
 namespace {

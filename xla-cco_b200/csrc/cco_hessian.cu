@@ -274,8 +274,11 @@ cudaError_t launch_hessian(const cco_problem* p, cudaStream_t st, int batch, con
   const int T = (N + kHessTile - 1) / kHessTile;
   const size_t nd = (size_t)N * D;
   const double pref = 2.0 * (2.0 * M_PI) * (2.0 * M_PI) / p->host.vol;
-  static const cudaError_t opt = cudaFuncSetAttribute(
-      k_hess_tiles<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hess_smem<D>());
+  static OncePerDevice once;
+  const cudaError_t opt = once.run([] {
+    return cudaFuncSetAttribute(k_hess_tiles<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)hess_smem<D>());
+  });
   if (opt != cudaSuccess) return opt;
   // lanes, then k rows, at a time: phases within kPhaseBytes
   const size_t per_k = (size_t)N * sizeof(double2);

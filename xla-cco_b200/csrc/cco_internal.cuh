@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "cco.h"
 
 namespace cco {
@@ -252,6 +254,27 @@ void launch_chained(bool chain, void (*kernel)(P...), dim3 grid, int threads, si
   cudaLaunchKernelEx(&cfg, kernel, P(args)...);   // the error is read by cudaGetLastError
 }
 
+// Kernel attributes belong to a device: `set` (host code that opts kernels in to
+// large dynamic shared memory) runs once on each device it is asked for on.
+class OncePerDevice {
+  std::mutex mu_;
+  uint64_t done_ = 0;
+
+ public:
+  template <class F>
+  cudaError_t run(F set) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;   // others: every time
+    std::lock_guard<std::mutex> lk(mu_);
+    if (done_ & bit) return cudaSuccess;
+    e = set();
+    if (e == cudaSuccess) done_ |= bit;
+    return e;
+  }
+};
+
 // Launches of an evaluation: (phase roots,) partial densities, reduction +
 // energy, gradient. Items index (lane, tile); lanes whose status is not RUNNING exit.
 struct EvalPlan {
@@ -355,7 +378,7 @@ int pass2_tiles(const ProbDev& p, int split);
 // It changes how work is spread, never the arithmetic.
 constexpr long long kPass2TargetCtas = 148 * 3;
 int pass2_split(long long tiles_at_split1);
-cudaError_t eval_configure();   // opt-in to large dynamic shared memory
+cudaError_t eval_configure();   // the current device: opt-in to large dynamic shared memory
 
 // The run-order densities in a padded layout: column c holds row row_of[c], or
 // (N, 0) where that is -1.

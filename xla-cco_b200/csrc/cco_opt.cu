@@ -1050,9 +1050,12 @@ cudaError_t descent_finalize(const DescentArgs& a, double* s_out, double* e_out,
 }
 
 size_t lbfgs_update_smem(int m) { return 2 * ((size_t)m * (m + 1) / 2) * sizeof(double); }
-cudaError_t lbfgs_configure(size_t smem) {
-  return cudaFuncSetAttribute(k_lbfgs_scalar, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem);
+cudaError_t lbfgs_configure() {
+  static OncePerDevice once;
+  return once.run([] {
+    return cudaFuncSetAttribute(k_lbfgs_scalar, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kScalarSmem);
+  });
 }
 cudaError_t lbfgs_init(const LbArgs& a, const double* s0, cudaStream_t st) {
   k_lbfgs_init<<<a.B, kUpdThreads, 0, st>>>(a, s0);

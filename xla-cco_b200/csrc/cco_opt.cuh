@@ -211,7 +211,8 @@ cudaError_t descent_finalize(const DescentArgs& a, double* s_out, double* e_out,
                              int64_t* st_out, int64_t* lat_out, cudaStream_t st);
 
 size_t lbfgs_update_smem(int m);
-cudaError_t lbfgs_configure(size_t smem);
+constexpr size_t kScalarSmem = 200 * 1024;   // the scalar kernel's triangles, at most
+cudaError_t lbfgs_configure();   // the current device: opt-in to kScalarSmem
 cudaError_t lbfgs_init(const LbArgs& a, const double* s0, cudaStream_t st);
 cudaError_t lbfgs_update(const LbArgs& a, cudaStream_t st);
 cudaError_t lbfgs_finalize(const LbArgs& a, double* s_out, double* e_out, double* gn_out,

@@ -397,7 +397,8 @@ size_t persist_smem(const cco_problem* p) {
 
 cudaError_t persist_descent(const DescentArgs& a, const EvalPlan& plan, size_t smem, int dims,
                             int64_t max_ticks, int* d_overrun, cudaStream_t st) {
-  static const cudaError_t configured = [] {
+  static OncePerDevice once;
+  const cudaError_t configured = once.run([] {
     cudaError_t e = cudaSuccess;
     for (const void* k : {(const void*)k_persist_descent<1>, (const void*)k_persist_descent<2>,
                           (const void*)k_persist_descent<3>, (const void*)k_persist_compact<1>,
@@ -405,7 +406,7 @@ cudaError_t persist_descent(const DescentArgs& a, const EvalPlan& plan, size_t s
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistMaxSmem);
     return e;
-  }();
+  });
   if (configured != cudaSuccess) return configured;
   if (dims & 8) k_persist_compact<1><<<a.B, kCompactThreads, smem, st>>>(a, plan, max_ticks, d_overrun);
   if (dims & 16) k_persist_compact<2><<<a.B, kCompactThreads, smem, st>>>(a, plan, max_ticks, d_overrun);

@@ -822,9 +822,6 @@ int relax_descent_set(cco_problem* const* probs, int B, cudaStream_t st, const d
   return rc;
 }
 
-std::mutex g_cfg_mu;
-size_t g_scalar_smem_configured = 0;
-
 int relax_lbfgs_set(cco_problem* const* probs, int B, cudaStream_t st, const double* s0,
                     const cco_lbfgs_settings* cfg, cco_relax_out* out) {
   if (!cfg || !s0) return fail(CCO_ERR_ARG, "null argument");
@@ -914,16 +911,10 @@ int lbfgs_args(const cco_lbfgs_settings* cfg, LbArgs* A, RecordShape* shape) {
   A->prec0 = cfg->precision == 1 ? PREC_FP32 : PREC_FP64;
   A->keep_s0 = cfg->precision == 1 ? 1 : 0;
   const size_t tri_bytes = lbfgs_update_smem(m);
-  const bool in_smem = tri_bytes <= 200 * 1024;
+  const bool in_smem = tri_bytes <= kScalarSmem;
   A->smem_tri = in_smem ? tri_bytes : 0;
   A->tri_len = in_smem ? 0 : m * (m + 1);
-  if (in_smem) {
-    std::lock_guard<std::mutex> lk(g_cfg_mu);
-    if (g_scalar_smem_configured < 200 * 1024) {
-      CCO_CUDA(lbfgs_configure(200 * 1024));
-      g_scalar_smem_configured = 200 * 1024;
-    }
-  }
+  if (in_smem) CCO_CUDA(lbfgs_configure());
   shape->method = Method::Lbfgs;
   shape->m = m;
   shape->tri_len = A->tri_len;
