@@ -371,11 +371,18 @@ int64_t* pinned_status(size_t count) {
   return buf;
 }
 
+constexpr int kMaxTrials = 2 * 6;   // visits of the candidates
+
 // Online tuning: graphs of each candidate on the live lanes C, timed with
 // events, then the fastest per tick. Every candidate advances every lane by
 // the same ticks, so results do not depend on which schedule wins.
-int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_t* ticks,
-                  int64_t* launches, Schedule* out) {
+// Only whole trials count: a loop that ended early has no time per tick (one
+// whose lanes were done before it spends a few us on none). The first that did
+// ends the tuning, since the lanes are done; then *out is set only if two
+// candidates were timed (*tuned). *ticks counts the ticks launched, *ran and
+// *launches what ran; done: kMaxTrials pinned words.
+int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_t* done,
+                  int64_t* ticks, int64_t* ran, int64_t* launches, Schedule* out, bool* tuned) {
   // Two rounds, the second in reverse order, each candidate timed once per
   // round: the lanes' work drifts while they advance (histories fill, rescale
   // passes restart them), and the mean of a forward and a backward visit
@@ -383,15 +390,18 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
   const std::vector<Schedule> cand = candidates((int)C.refs.size());
   const size_t nc = cand.size();
   std::vector<cudaEvent_t> t0(2 * nc, nullptr), t1(2 * nc, nullptr);
-  std::vector<int> ran(2 * nc, 0);
+  std::vector<int64_t> bodies(2 * nc, 0), body(2 * nc, 0), per_body(2 * nc, 0);
   std::vector<cudaGraph_t> graphs;
+  *tuned = false;
   int rc = CCO_OK;
   cudaError_t e = cudaSuccess;
   for (size_t c = 0; c < 2 * nc && e == cudaSuccess; ++c) {
     e = cudaEventCreate(&t0[c]);
     if (e == cudaSuccess) e = cudaEventCreate(&t1[c]);
   }
-  for (size_t v = 0; v < 2 * nc && rc == CCO_OK && e == cudaSuccess && *ticks < max_ticks; ++v) {
+  size_t launched = 0;
+  bool early = false;
+  for (size_t v = 0; v < 2 * nc && e == cudaSuccess && !early && *ticks < max_ticks; ++v) {
     const size_t c = v < nc ? v : 2 * nc - 1 - v;
     TickPlan P;
     P.method = C.shape.method;
@@ -402,20 +412,32 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
     }
     e = cudaEventRecord(t0[v], st);
     if (e == cudaSuccess) e = cudaGraphLaunch(P.exec, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(done + v, &P.loop->done, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaEventRecord(t1[v], st);
-    ran[v] = e == cudaSuccess;
-    *ticks += cand[c].graph_ticks;
-    *launches += (int64_t)cand[c].graph_ticks * P.launches_per_tick() + 1 +
-                 P.bodies * P.loop_gates();
+    body[v] = P.body;
+    per_body[v] = (int64_t)P.body * P.launches_per_tick() + P.loop_gates();
+    bodies[v] = P.bodies;
     P.retire(st, &graphs);
+    if (e != cudaSuccess) break;
+    launched = v + 1;
+    *ticks += cand[c].graph_ticks;
+    // the trial before, while this one runs
+    if (v > 0) e = cudaEventSynchronize(t1[v - 1]);
+    if (e != cudaSuccess) break;
+    early = v > 0 && done[v - 1] < bodies[v - 1];
   }
   const cudaError_t es = cudaStreamSynchronize(st);
   if (rc == CCO_OK && e == cudaSuccess) e = es;
   for (cudaGraph_t g : graphs) cudaGraphDestroy(g);
+  for (size_t v = 0; v < launched && e == cudaSuccess; ++v) {
+    *ran += done[v] * body[v];
+    *launches += 1 + done[v] * per_body[v];
+  }
   std::vector<float> sum(nc, 0.f);
   std::vector<int> cnt(nc, 0);
-  for (size_t v = 0; v < 2 * nc && e == cudaSuccess && rc == CCO_OK; ++v) {
-    if (!ran[v]) continue;
+  for (size_t v = 0; v < launched && e == cudaSuccess && rc == CCO_OK; ++v) {
+    if (done[v] < bodies[v]) continue;
     const size_t c = v < nc ? v : 2 * nc - 1 - v;
     float x = 0.f;
     if (cudaEventElapsedTime(&x, t0[v], t1[v]) == cudaSuccess) {
@@ -426,10 +448,11 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
     }
   }
   std::vector<float> ms(nc, 1e30f);
-  int best = 0;
+  int best = 0, timed = 0;
   for (size_t c = 0; c < nc; ++c) {
     if (cnt[c] > 0) ms[c] = sum[c] / cnt[c];
     if (ms[c] < ms[best]) best = (int)c;
+    timed += cnt[c] > 0;
   }
   for (size_t c = 0; c < 2 * nc; ++c) {
     if (t0[c]) cudaEventDestroy(t0[c]);
@@ -437,15 +460,16 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
   }
   if (rc != CCO_OK) return rc;
   if (e != cudaSuccess) return cuda_fail(e, "schedule tuning");
+  if (timed < (int)std::min<size_t>(nc, 2)) return CCO_OK;
   Schedule s = cand[best];
   // graphs of about 8 ms of device work: with three in flight the device has
   // ~20 ms queued, so a host thread descheduled on a busy host does not leave
   // it idle; the graphs that run past the last lane's completion cost little
   // (their kernels exit at once for finished lanes)
-  const double tick_ms = ms[best] < 1e29f ? ms[best] : 0.2;
-  const int gt = (int)std::lround(8.0 / std::max(tick_ms, 1e-3));
+  const int gt = (int)std::lround(8.0 / std::max((double)ms[best], 1e-3));
   s.graph_ticks = std::max(4, std::min(32, gt & ~3));   // whole bodies of four ticks
   *out = s;
+  *tuned = true;
   return CCO_OK;
 }
 
@@ -463,7 +487,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
   const int kSlots = inflight + 1;
   int64_t* d_status = nullptr;
   const int W = B + 1;   // a snapshot: the statuses, then the bodies the plan has run
-  int64_t* h_status = pinned_status((size_t)kSlots * W);
+  int64_t* h_status = pinned_status((size_t)kSlots * W + kMaxTrials);
   if (!h_status) return fail(CCO_ERR_OOM, "pinned status buffer");
   CCO_CUDA(pool_alloc(&d_status, sizeof(int64_t) * kSlots * W, st));
   cudaEvent_t ev[kMaxInflight + 1];
@@ -495,10 +519,12 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
   TickPlan P;
   P.method = T.shape.method;
   int version = 0;
-  // An L-BFGS table is tuned only once its lanes' histories have filled: in
-  // the first ticks the HBM-bound update is short, so schedules that overlap
-  // it with the FP64-bound evaluation of another branch cannot show their
-  // gain. Until then it runs the default schedule.
+  // A table is tuned only once it has run for a while, on the default schedule
+  // until then. Short runs (a 40-step segment, a flow to a first stop) end inside
+  // the trials, which tell nothing then and cost a graph each (about 1 ms); and
+  // in an L-BFGS table's first ticks, before its lanes' histories have filled, the
+  // HBM-bound update is short, so schedules that overlap it with the FP64-bound
+  // evaluation of another branch cannot show their gain.
   constexpr int64_t kTuneAfterTicks = 128;
   bool defer_tune = false;
 
@@ -516,18 +542,19 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     C.md.B = (int)C.refs.size();
     Schedule s;
     s.branches = default_branches(C.refs.size());
+    defer_tune = false;
     if (force_br > 0 || force_gt > 0 || force_ov >= 0) {
       if (force_br > 0) s.branches = force_br;
       if (force_gt > 0) s.graph_ticks = force_gt;
       if (force_ov >= 0) s.overlap = force_ov;
     } else if (!schedule_cached(C.probs, C.shape.method, &s) && tune) {
-      defer_tune = C.shape.method == Method::Lbfgs && ticks < kTuneAfterTicks;
+      defer_tune = ticks_run < kTuneAfterTicks;
       if (!defer_tune) {
-        const int64_t before = ticks;
-        r = tune_schedule(C, st, max_ticks, &ticks, &launches, &s);
-        ticks_run += ticks - before;
+        bool tuned = false;
+        r = tune_schedule(C, st, max_ticks, h_status + (size_t)kSlots * W, &ticks, &ticks_run,
+                          &launches, &s, &tuned);
         if (r != CCO_OK) return r;
-        schedule_store(C.probs, C.shape.method, s);
+        if (tuned) schedule_store(C.probs, C.shape.method, s);
       }
     }
     chosen = s;
@@ -596,7 +623,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     per_body[slot] = (int64_t)P.body * P.launches_per_tick() + P.loop_gates();
     ++launched;
     if (e == cudaSuccess && launched - checked > inflight) rc = land();
-    if (rc == CCO_OK && e == cudaSuccess && !done && defer_tune && ticks >= kTuneAfterTicks) {
+    if (rc == CCO_OK && e == cudaSuccess && !done && defer_tune && ticks_run >= kTuneAfterTicks) {
       P.retire(st, &graphs);   // the deferred tuning, on the same table
       rc = start();
     }
