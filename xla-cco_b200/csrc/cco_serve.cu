@@ -83,8 +83,10 @@ struct Flight {
   cudaEvent_t ev = nullptr;
   std::vector<Request*> lanes;
   Pinned h_status;
-  int64_t* d_status = nullptr;
+  int64_t* d_status = nullptr;   // the lanes' statuses, then the bodies the plan has run
   size_t d_cap = 0;
+  int64_t plan = 0;              // which plan, and the ticks of its body
+  int body = 1;
 };
 
 // One batch of retiring lanes: finalize outputs on their way to the host.
@@ -228,6 +230,8 @@ class Driver {
   std::vector<Request*> live_;       // lanes of the current table
   LaneTable table_;
   std::unique_ptr<TickPlan> plan_;
+  int64_t plan_id_ = 0;                   // plans built
+  int64_t seen_plan_ = 0, seen_ = 0;      // of the last landed launch: its plan, bodies that had run
   std::vector<OldPlan> old_;
   bool dirty_ = false;
   size_t used_ = 0;      // bytes of the resident records
@@ -390,6 +394,7 @@ class Driver {
     sch.graph_ticks = S_->graph_ticks;
     sch.branches = S_->branches > 0 ? S_->branches : default_branches(live_.size());
     plan_.reset(new TickPlan());
+    ++plan_id_;
     plan_->method = Method::Lbfgs;
     rc = plan_->build(table_, sch, st_);
     std::lock_guard<std::mutex> lk(S_->mu);
@@ -413,23 +418,24 @@ class Driver {
   int launch() {
     Flight& f = fl_[(fl_head_ + fl_count_) % kServeSlots];
     const size_t n = live_.size();
-    if (f.d_cap < n) {
+    if (f.d_cap < n + 1) {
       if (f.d_status) CCO_CUDA(cudaFreeAsync(f.d_status, st_));
       f.d_status = nullptr;
-      f.d_cap = std::max<size_t>(n, 256);
+      f.d_cap = std::max<size_t>(n + 1, 256);
       CCO_CUDA(pool_alloc(&f.d_status, sizeof(int64_t) * f.d_cap, st_));
     }
-    CCO_CUDA(f.h_status.reserve(sizeof(int64_t) * n));
+    CCO_CUDA(f.h_status.reserve(sizeof(int64_t) * (n + 1)));
     CCO_CUDA(cudaGraphLaunch(plan_->exec, st_));
-    CCO_CUDA(gather_status(table_.d_refs, (int)n, f.d_status, st_));
-    CCO_CUDA(cudaMemcpyAsync(f.h_status.ptr, f.d_status, sizeof(int64_t) * n,
+    CCO_CUDA(gather_status(table_.d_refs, (int)n, f.d_status, st_, &plan_->loop->done));
+    CCO_CUDA(cudaMemcpyAsync(f.h_status.ptr, f.d_status, sizeof(int64_t) * (n + 1),
                              cudaMemcpyDeviceToHost, st_));
     CCO_CUDA(cudaEventRecord(f.ev, st_));
     f.lanes = live_;
+    f.plan = plan_id_;
+    f.body = plan_->body;
     ++fl_count_;
     std::lock_guard<std::mutex> lk(S_->mu);
     S_->graphs += 1;
-    S_->ticks += plan_->sch.graph_ticks;
     return CCO_OK;
   }
 
@@ -438,6 +444,13 @@ class Driver {
     Flight& f = fl_[fl_head_];
     CCO_CUDA(cudaEventSynchronize(f.ev));
     const int64_t* h = static_cast<const int64_t*>(f.h_status.ptr);
+    if (f.plan != seen_plan_) seen_ = 0;   // launches land in order
+    seen_plan_ = f.plan;
+    {
+      std::lock_guard<std::mutex> lk(S_->mu);
+      S_->ticks += (h[f.lanes.size()] - seen_) * f.body;
+    }
+    seen_ = h[f.lanes.size()];
     std::vector<Request*> done;
     for (size_t i = 0; i < f.lanes.size(); ++i) {
       Request* r = f.lanes[i];
