@@ -214,7 +214,17 @@ void grid_layout(std::vector<GridRun> runs, int d, int max_cols, int max_strips,
     }
     const int range = hi - lo + 1, nw = (range + max_cols - 1) / max_cols;
     const int width = ((range + nw - 1) / nw + 7) / 8 * 8;
-    for (int w = lo; w <= hi; w += width) {
+    std::vector<int> wins;   // first columns of the windows
+    if (nw <= 64) {
+      for (int w = lo; w <= hi; w += width) wins.push_back(w);
+    } else {   // those with columns of a run: far-apart runs leave most of them empty
+      for (int r = 8 * s0; r < std::min(nr, 8 * s1); ++r)
+        for (int w = (fold_lo(runs[r]) - lo) / width; w <= (fold_hi(runs[r]) - lo) / width; ++w)
+          wins.push_back(lo + w * width);
+      std::sort(wins.begin(), wins.end());
+      wins.erase(std::unique(wins.begin(), wins.end()), wins.end());
+    }
+    for (const int w : wins) {
       GridBlock b{};
       b.strip0 = (int)out->strips.size();
       b.lo = w;
@@ -387,11 +397,13 @@ void grid_sizes(ProbDev* P, const GridPlan& gp) {
   const size_t own = (size_t)P->M + P->grhow + 2 * (size_t)P->gntile * P->gslots + eval_roots_words(*P);
   if (sizeof(double2) * own > CCO_NOALLOC_SCRATCH_BYTES - 65536 &&
       sizeof(double2) * seg <= CCO_NOALLOC_SCRATCH_BYTES)
-    P->grid = 0;
+    P->grid = P->groots = 0;
 }
 
 void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
-  if (runs.empty()) return;
+  // every strip of 8 runs takes a quad (32 slots) or more: sets of short runs are
+  // refused before a layout is made (90 000 runs of about one row: 11 layouts took 290 ms)
+  if (runs.empty() || 32ll * (long long)((runs.size() + 7) / 8) > 2ll * P->M) return;
   // the layout that costs least per particle: products and table entries (both
   // passes), among block shapes whose tables fit
   int step = 1;
@@ -634,6 +646,7 @@ int cco_problem_create_rows(int device, int d, int n_particles, int m, const int
       for (int a = 0; a < d; ++a) rows[(size_t)k * d + a] = n_vectors[(size_t)order[k] * d + a];
     plan_lines(rows, &P, &gp);
   }
+  if (!P.grid) gp = GridPlan{};   // nothing to upload of a refused layout
   // longest segments first: pass-1 warps share trip counts, pass 2 pairs
   // segments of similar length
   auto by_len = [](const SegHdr& x, const SegHdr& y) { return x.len > y.len; };
