@@ -88,13 +88,13 @@ int cco_problem_destroy(cco_problem* p);
 /* Sizes of the device k-set layout (runs split into pass-1/pass-2 segments). */
 int cco_problem_info(const cco_problem* p, int* d, int* n_particles, int* m,
                      int* n_seg1, int* n_seg2, int* table_rows);
-/* Density class of a k-set: *gemm_blocks > 0, the number of (24-run x last-axis
- * window) blocks, for d >= 2 when the blocks hold at least half (d = 3: all) as
- * many rows as cells; 0 for sparser k-sets and for d = 1. FP64 lanes of the
- * dense ones always run the tensor-core grid form of both passes; sparser and
- * 1-D sets do when their padded grid has at most two slots per row.
- * CCO_PASS1_GEMM=0 when the problem is created turns the grid form off (and
- * this number to 0). No reference counterpart. */
+/* Density class of a k-set whose FP64 lanes run the tensor-core grid form of
+ * both passes (a set does when its padded grid has at most two slots per row):
+ * *gemm_blocks > 0, the number of (24-run x last-axis window) blocks, for d >= 2
+ * when the blocks hold at least half (d = 3: all) as many rows as cells. 0 for
+ * sparser k-sets and for d = 1, whatever form they run, and for every set that
+ * does not run the grid form. CCO_PASS1_GEMM=0 when the problem is created turns
+ * the grid form off. No reference counterpart. */
 int cco_problem_pass1_form(const cco_problem* p, int* gemm_blocks);
 
 /*

@@ -145,7 +145,8 @@ void sort_by_fold(std::vector<GridRun>& runs) {
   });
 }
 
-// What cco_problem_pass1_form reports: the (24-run x 16 cq-column) blocks of a
+// The density class of cco_problem_pass1_form, which is also part of the scratch
+// cco_energy_grad_noalloc has always asked for: the (24-run x 16 cq-column) blocks of a
 // k-set of d >= 2 whose blocks hold at least half (d = 3: all) as many rows as
 // cells, cells counted per 6 runs; 0 for sparser ones and in 1-D.
 int folded_blocks(std::vector<GridRun> runs, int d, int m) {
@@ -760,7 +761,7 @@ int cco_problem_info(const cco_problem* p, int* d, int* n_particles, int* m, int
 
 int cco_problem_pass1_form(const cco_problem* p, int* gemm_blocks) {
   if (!p || !gemm_blocks) return fail(CCO_ERR_ARG, "null argument");
-  *gemm_blocks = p->dense_blocks;
+  *gemm_blocks = p->host.grid == 1 ? p->dense_blocks : 0;
   return CCO_OK;
 }
 
