@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import abc
 import threading
+from collections import OrderedDict
 from typing import Any, Dict, List, Optional, Tuple
 
 import numpy as np
@@ -304,25 +305,38 @@ def collective_density(s: Any, n_vectors: Any, chunk_size: Optional[int] = None)
     return re[0], im[0]
 
 
-# unit-weight energies of the k-sets density calls have named, by content:
-# newest last, at most _DENSITY_KEEP of them
-_DENSITY_KEEP = 64
-_DENSITY_CACHE: List[StealthyEnergy] = []
+# Unit-weight energies of the k-sets density calls have named, by content, most
+# recently used last: as many as hold _DENSITY_ROWS rows (about 150 bytes of device
+# memory each) and at most _DENSITY_SETS.
+_DENSITY_ROWS = 8 << 20
+_DENSITY_SETS = 4096
+_DENSITY_CACHE: "OrderedDict[tuple, List[StealthyEnergy]]" = OrderedDict()
 _DENSITY_LOCK = threading.Lock()
 
 
 def _density_energy(nv: np.ndarray) -> StealthyEnergy:
-    # compared element by element: hashing the bytes of a 97 000-row set took 1.6 ms
+    # found by a sample of the entries, then compared element by element: hashing
+    # all bytes of a 97 000-row set took 1.6 ms
+    flat = nv.reshape(-1)
+    key = (nv.shape, flat[:: flat.size // 64 + 1].tobytes())
     with _DENSITY_LOCK:
-        for i in range(len(_DENSITY_CACHE) - 1, -1, -1):
-            en = _DENSITY_CACHE[i]
-            if en.n_vectors.shape == nv.shape and np.array_equal(en.n_vectors, nv):
-                _DENSITY_CACHE.append(_DENSITY_CACHE.pop(i))
+        for en in _DENSITY_CACHE.get(key, ()):
+            if np.array_equal(en.n_vectors, nv):
+                _DENSITY_CACHE.move_to_end(key)
                 return en
     en = StealthyEnergy(nv.copy(), np.ones(nv.shape[0]), np.float64(1.0))
+    old = []   # destroyed after the lock is free
     with _DENSITY_LOCK:
-        _DENSITY_CACHE.append(en)
-        del _DENSITY_CACHE[:-_DENSITY_KEEP]
+        _DENSITY_CACHE.setdefault(key, []).append(en)
+        _DENSITY_CACHE.move_to_end(key)
+        sets = sum(len(x) for x in _DENSITY_CACHE.values())
+        rows = sum(e.n_vectors.shape[0] for x in _DENSITY_CACHE.values() for e in x)
+        while len(_DENSITY_CACHE) > 1 and (sets > _DENSITY_SETS or rows > _DENSITY_ROWS):
+            _, x = _DENSITY_CACHE.popitem(last=False)
+            old.append(x)
+            sets -= len(x)
+            rows -= sum(e.n_vectors.shape[0] for e in x)
+    del old
     return en
 
 
