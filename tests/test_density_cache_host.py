@@ -1,5 +1,6 @@
 """Energies kept for density calls (no device): programs that cycle through many
-k-sets find them again, and what is kept is bounded."""
+k-sets find them again, what is kept is bounded, and one that a captured stream has
+used is never destroyed under the graph."""
 
 from __future__ import annotations
 
@@ -53,3 +54,27 @@ def test_what_is_kept_is_bounded(monkeypatch):
     energy._density_energy(_sets(401)[-1])
     gc.collect()
     assert sum(r() is not None for r in refs) <= 64
+
+
+def test_a_set_used_under_capture_outlives_its_place_in_the_cache(monkeypatch):
+    import torch
+
+    class OnDevice(np.ndarray):   # an input that says it is a CUDA tensor
+        is_cuda = True
+
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    monkeypatch.setattr(energy, "require_float64", lambda *a: None)
+    seen = []
+
+    def evaluate(self, s, want_grad=True, want_rho=False):
+        seen.append(weakref.ref(self))
+        return None, None, np.zeros((1, 7)), np.zeros((1, 7))
+
+    monkeypatch.setattr(energy.StealthyEnergy, "evaluate", evaluate)
+    nv = _sets(1)[0]
+    energy.collective_density(np.zeros((5, 2)).view(OnDevice), nv)
+    monkeypatch.setattr(energy, "_DENSITY_SETS", 8, raising=False)
+    for other in _sets(200)[1:]:
+        energy._density_energy(other)
+    gc.collect()
+    assert seen[0]() is not None

@@ -301,6 +301,9 @@ def collective_density(s: Any, n_vectors: Any, chunk_size: Optional[int] = None)
     assert chunk_size is None or chunk_size >= 1, "chunk_size must be >= 1"
     nv = np.asarray(n_vectors)
     en = _density_energy(nv)
+    if getattr(s, "is_cuda", False) and _torch().cuda.is_current_stream_capturing():
+        with _DENSITY_LOCK:
+            _DENSITY_CAPTURED[id(en)] = en
     _, _, re, im = en.evaluate(s[None], want_grad=False, want_rho=True)
     return re[0], im[0]
 
@@ -311,6 +314,9 @@ def collective_density(s: Any, n_vectors: Any, chunk_size: Optional[int] = None)
 _DENSITY_ROWS = 8 << 20
 _DENSITY_SETS = 4096
 _DENSITY_CACHE: "OrderedDict[tuple, List[StealthyEnergy]]" = OrderedDict()
+# Those a captured stream has used: a graph holds their device memory by address, and
+# nobody but this module holds them, so they stay.
+_DENSITY_CAPTURED: Dict[int, StealthyEnergy] = {}
 _DENSITY_LOCK = threading.Lock()
 
 
