@@ -121,14 +121,13 @@ template <int D, bool ROOTS>
 __device__ __forceinline__ void grid_seeds(const ProbDev& P, const EvalLane& ln, const GridUnit& A,
                                            const GridUnit& C, int j, double2& za, double2& a0,
                                            double2& zc, double2& c0) {
-  a0 = c0 = make_double2(1.0, 0.0);
   if constexpr (ROOTS) {
     const double2* ra = ln.roots + (size_t)P.groff[A.v] * P.N + j;
     const double2* rc = ln.roots + (size_t)P.groff[C.v] * P.N + j;
     za = ra[0];
     zc = rc[0];
-    if (A.q != 0) a0 = ra[(size_t)abs(A.q) * P.N];
-    if (C.q != 0) c0 = rc[(size_t)abs(C.q) * P.N];
+    a0 = A.q != 0 ? ra[(size_t)abs(A.q) * P.N] : zeroth_power(za);
+    c0 = C.q != 0 ? rc[(size_t)abs(C.q) * P.N] : zeroth_power(zc);
     if (A.q < 0) a0.y = -a0.y;
     if (C.q < 0) c0.y = -c0.y;
   } else {
@@ -137,6 +136,8 @@ __device__ __forceinline__ void grid_seeds(const ProbDev& P, const EvalLane& ln,
     const int ka = A.v == 0 ? P.gstep : 1, kc = C.v == 0 ? P.gstep : 1;
     sincos_2pi_ms((double)ka, sa, &za.y, &za.x);
     sincos_2pi_ms((double)kc, sc, &zc.y, &zc.x);
+    a0 = zeroth_power(za);
+    c0 = zeroth_power(zc);
     if (A.q != 0 || C.q != 0) {   // warp-uniform
       sincos_2pi_ms((double)(16 * A.q * ka), sa, &a0.y, &a0.x);
       sincos_2pi_ms((double)(16 * C.q * kc), sc, &c0.y, &c0.x);
@@ -210,8 +211,9 @@ __device__ __forceinline__ void grid_line_tables(const ProbDev& P, const GridBlo
       nS[a] = (double)(L.n[a] * L.step);
       nQ[a] = (double)(L.n[a] * L.step * L.q0);
     }
-    double2 z, y, c0 = make_double2(1.0, 0.0), r0 = c0;
+    double2 z, y, r0 = make_double2(1.0, 0.0);
     sincos_2pi_dot<D>(n1, sj, &z.y, &z.x);
+    double2 c0 = zeroth_power(z);
     sincos_2pi_dot<D>(nS, sj, &y.y, &y.x);
     if (L.q0 != 0) sincos_2pi_dot<D>(nQ, sj, &r0.y, &r0.x);
     if (!live) r0 = make_double2(0.0, 0.0);

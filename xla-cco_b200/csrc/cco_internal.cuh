@@ -195,6 +195,12 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
+// z^0 of a phase z as a table entry: 1, but NaN for a NaN z, so that a particle
+// with a non-finite coordinate makes every row NaN (n . s is, also where n_a = 0).
+__device__ __forceinline__ double2 zeroth_power(double2 z) {
+  return make_double2(fma(0.0, z.x, 1.0), 0.0);
+}
+
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }

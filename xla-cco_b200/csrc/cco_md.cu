@@ -570,8 +570,9 @@ __global__ void __cluster_dims__(kWaveRanks, 1, 1) __launch_bounds__(kWaveThread
       const int e0 = 8 * u, e1 = min(e0 + 8, a.wave_r[c] + 1);
       double2* col = tab + (size_t)base[c] * ld + j;
       const double x = w.ps[(size_t)(j0 + j) * D + c];
-      double2 z, p = make_double2(1.0, 0.0);
+      double2 z, p;
       sincos_2pi_ms(1.0, x, &z.y, &z.x);
+      p = zeroth_power(z);
       if (e0 > 0) sincos_2pi_ms((double)e0, x, &p.y, &p.x);
       for (int e = e0; e < e1; ++e) {
         col[(size_t)e * ld] = p;

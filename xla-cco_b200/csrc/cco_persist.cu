@@ -216,8 +216,9 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
         }
       const double x = ps[j * D + c];
       const int e0 = 8 * u, e1 = min(e0 + 8, P.rmax[c] + 1);
-      double2 z, p = make_double2(1.0, 0.0);
+      double2 z, p;
       sincos_2pi_ms(1.0, x, &z.y, &z.x);
+      p = zeroth_power(z);
       if (e0 > 0) sincos_2pi_ms((double)e0, x, &p.y, &p.x);
       for (int e = e0; e < e1; ++e) {
         tab[(size_t)(base[c] + e) * N + j] = p;
