@@ -363,6 +363,7 @@ struct TickPlan {
   cudaGraph_t graph = nullptr;   // owns the loop's condition: outlives the launches
   TickLoop* loop = nullptr;
   int body = 1, bodies = 1;      // ticks of the body, bodies of one launch
+  double launch_us = 0.0;        // a whole launch, about
   bool forks[kMaxBranches] = {}; // dimensions of a pass as parallel nodes
   int build(const LaneTable& T, const Schedule& sch, cudaStream_t st);
   cudaError_t tick(cudaStream_t s, int b) const;

@@ -117,10 +117,12 @@ bool eval_forks(const std::vector<const cco_problem*>& probs, int lo, int hi) {
 // ticks: 11.1 / 11.5 / 12.3 / 14.4 / 18.5 ms for 48 uneven lanes of 20 evaluations
 // (18.7 as one flat graph; the rule takes 1), 8.3 / 8.1 / 8.1 / 8.3 / 8.6 ms for
 // 256 lanes of d=2 N=1000 and 32 evaluations (9.3; the rule takes 4).
-int body_ticks(const std::vector<const cco_problem*>& probs, int launches, int graph_ticks) {
+double tick_us(const std::vector<const cco_problem*>& probs, int launches) {
   double flops = 0.0;
   for (const cco_problem* p : probs) flops += eval_flops(p);
-  const double us = flops / 15e6 + 2.0 * launches;
+  return flops / 15e6 + 2.0 * launches;
+}
+int body_ticks(double us, int graph_ticks) {
   const int gt = std::max(1, graph_ticks);
   for (int t = std::max(1, (int)(600.0 / us)); t < gt; ++t)
     if (gt % t == 0) return t;
@@ -174,7 +176,9 @@ int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
       lb[b] = a;
     }
   }
-  body = body_ticks(T.probs, launches_per_tick(), sch.graph_ticks);
+  const double us = tick_us(T.probs, launches_per_tick());
+  body = body_ticks(us, sch.graph_ticks);
+  launch_us = us * sch.graph_ticks;
   bodies = std::max(1, sch.graph_ticks) / body;
   CCO_CUDA(pool_alloc(&loop, sizeof(TickLoop), st));
   CCO_CUDA(cudaMemsetAsync(loop, 0, sizeof(TickLoop), st));
@@ -480,7 +484,12 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
 // whenever at most half of it still runs, so finished lanes stop costing
 // launch slots (the reference's per-round compaction of active lanes,
 // minimize/__init__.py:75-99, without moving any lane's state). Each
-// compaction looks up or re-tunes the schedule for the smaller table.
+// compaction looks up or re-tunes the schedule for the smaller table. Where a
+// launch takes less than a new plan does, the next snapshot has to show it too:
+// lanes that end at about the same tick straddle a launch, and the plan would serve
+// the last of them for a tick or two (200 lanes of d=2 N=60 that end after 16 and
+// 17 ticks: 3.3 ms, 2.2 without it). Longer launches do not wait for one (256 lanes
+// of d=2 N=1000 to the ground state 202.3 ms, 204.6 with the wait).
 int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* stats) {
   const int B = (int)T.refs.size();
   const int inflight = std::max(1, std::min(kMaxInflight, env_int("CCO_INFLIGHT", kInflight)));
@@ -519,6 +528,8 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
   TickPlan P;
   P.method = T.shape.method;
   int version = 0;
+  int low = 0;   // snapshots in a row with at most half of the current table running
+  constexpr double kPlanUs = 1000.0;   // host time of a new plan
   // A table is tuned only once it has run for a while, on the default schedule
   // until then. Short runs (a 40-step segment, a flow to a first stop) end inside
   // the trials, which tell nothing then and cost a graph each (about 1 ms); and
@@ -563,6 +574,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
       first_set = true;
     }
     ++version;
+    low = 0;
     return P.build(C, chosen, st);
   };
   rc = start();
@@ -585,7 +597,9 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
       return CCO_OK;
     }
     const int n = (int)C.refs.size();
-    if (!compact || ver[slot] != version || n < 2 || 2 * running > n) return CCO_OK;
+    if (ver[slot] != version) return CCO_OK;
+    low = 2 * running > n ? 0 : low + 1;
+    if (!compact || n < 2 || low < (P.launch_us < kPlanUs ? 2 : 1)) return CCO_OK;
     // compaction: keep the lanes this snapshot of the current table shows running
     std::vector<LaneRef> refs;
     std::vector<const cco_problem*> probs;
