@@ -39,7 +39,7 @@ def _system(n, d, chi, b):
     return box, make_stealthy_energy(box, ks), s0
 
 
-@pytest.mark.parametrize("evals", [2, 40, 240, 300])
+@pytest.mark.parametrize("evals", [2, 40, 240, 270, 300, 310])
 def test_short_runs_neither_choose_nor_leave_a_schedule(evals):
     """Runs that end at once, inside the first trials of an immediate tuning, and
     shortly before and after the tick from which a table is tuned."""
@@ -95,3 +95,4 @@ def test_md_segments_count_the_ticks_that_ran(monkeypatch):
     simulate(en, waves, box.basis, st, state, 40)
     assert seen[0] >= 1 and seen[0] < 1 + BODY
     assert 41 <= seen[1] < 41 + BODY
+

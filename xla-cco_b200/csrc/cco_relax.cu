@@ -47,6 +47,10 @@ namespace {
 using ShapeKey = std::tuple<int, int, int, int>;
 std::mutex g_sched_mu;
 std::map<ShapeKey, Schedule> g_sched;
+// Ticks from which a table of the class is tuned: kTuneAfterTicks, and twice what the
+// last one had behind it whose lanes ended inside the trials.
+std::map<ShapeKey, int64_t> g_tune_after;
+constexpr int64_t kTuneAfterTicks = 128;
 
 ShapeKey shape_key(const std::vector<const cco_problem*>& probs, Method method) {
   double work = 0.0;
@@ -84,7 +88,23 @@ void schedule_store(const std::vector<const cco_problem*>& probs, Method method,
 void schedule_clear() {
   std::lock_guard<std::mutex> lk(g_sched_mu);
   g_sched.clear();
+  g_tune_after.clear();
 }
+
+namespace {
+
+int64_t tune_after(const std::vector<const cco_problem*>& probs, Method method) {
+  std::lock_guard<std::mutex> lk(g_sched_mu);
+  auto it = g_tune_after.find(shape_key(probs, method));
+  return it == g_tune_after.end() ? kTuneAfterTicks : it->second;
+}
+
+void set_tune_after(const std::vector<const cco_problem*>& probs, Method method, int64_t ticks) {
+  std::lock_guard<std::mutex> lk(g_sched_mu);
+  g_tune_after[shape_key(probs, method)] = ticks;
+}
+
+}  // namespace
 
 // ------------------------------------------------------------ tick plans
 namespace {
@@ -380,12 +400,12 @@ constexpr int kMaxTrials = 2 * 6;   // visits of the candidates
 // Online tuning: graphs of each candidate on the live lanes C, timed with
 // events, then the fastest per tick. Every candidate advances every lane by
 // the same ticks, so results do not depend on which schedule wins.
-// Only whole trials count: a loop that ended early has no time per tick (one
-// whose lanes were done before it spends a few us on none). The first that did
-// ends the tuning, since the lanes are done; then *out is set only if two
-// candidates were timed (*tuned). *ticks counts the ticks launched, *ran and
-// *launches what ran; done: kMaxTrials pinned words.
-int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_t* done,
+// Only whole trials count: a loop that ended early, or whose last ticks had no
+// RUNNING lane left, has no time per tick (one whose lanes were done before it
+// spends a few us on none). The first such trial ends the tuning; then *out is set
+// only if two candidates had both their visits (*tuned). *ticks counts the ticks launched, *ran
+// and *launches what ran; seen: kMaxTrials pairs of pinned words.
+int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_t* seen,
                   int64_t* ticks, int64_t* ran, int64_t* launches, Schedule* out, bool* tuned) {
   // Two rounds, the second in reverse order, each candidate timed once per
   // round: the lanes' work drifts while they advance (histories fill, rescale
@@ -393,7 +413,7 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
   // cancels a drift that is linear in time.
   const std::vector<Schedule> cand = candidates((int)C.refs.size());
   const size_t nc = cand.size();
-  std::vector<cudaEvent_t> t0(2 * nc, nullptr), t1(2 * nc, nullptr);
+  std::vector<cudaEvent_t> t0(2 * nc, nullptr), t1(2 * nc, nullptr), landed(2 * nc, nullptr);
   std::vector<int64_t> bodies(2 * nc, 0), body(2 * nc, 0), per_body(2 * nc, 0);
   std::vector<cudaGraph_t> graphs;
   *tuned = false;
@@ -402,7 +422,13 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
   for (size_t c = 0; c < 2 * nc && e == cudaSuccess; ++c) {
     e = cudaEventCreate(&t0[c]);
     if (e == cudaSuccess) e = cudaEventCreate(&t1[c]);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&landed[c], cudaEventDisableTiming);
   }
+  // per trial: the bodies it ran, then the lanes still RUNNING
+  int64_t* d_seen = nullptr;
+  if (e == cudaSuccess) e = pool_alloc(&d_seen, sizeof(int64_t) * 4 * nc, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_seen, 0, sizeof(int64_t) * 4 * nc, st);
+  auto whole = [&](size_t v) { return seen[2 * v] >= bodies[v] && seen[2 * v + 1] > 0; };
   size_t launched = 0;
   bool early = false;
   for (size_t v = 0; v < 2 * nc && e == cudaSuccess && !early && *ticks < max_ticks; ++v) {
@@ -416,9 +442,15 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
     }
     e = cudaEventRecord(t0[v], st);
     if (e == cudaSuccess) e = cudaGraphLaunch(P.exec, st);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(done + v, &P.loop->done, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaEventRecord(t1[v], st);
+    int64_t* ds = d_seen + 2 * v;
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(ds, &P.loop->done, sizeof(int64_t), cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess)
+      e = count_running(C.d_refs, (int)C.refs.size(), reinterpret_cast<int*>(ds + 1), st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(seen + 2 * v, ds, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaEventRecord(landed[v], st);
     body[v] = P.body;
     per_body[v] = (int64_t)P.body * P.launches_per_tick() + P.loop_gates();
     bodies[v] = P.bodies;
@@ -427,21 +459,21 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
     launched = v + 1;
     *ticks += cand[c].graph_ticks;
     // the trial before, while this one runs
-    if (v > 0) e = cudaEventSynchronize(t1[v - 1]);
+    if (v > 0) e = cudaEventSynchronize(landed[v - 1]);
     if (e != cudaSuccess) break;
-    early = v > 0 && done[v - 1] < bodies[v - 1];
+    early = v > 0 && !whole(v - 1);
   }
   const cudaError_t es = cudaStreamSynchronize(st);
   if (rc == CCO_OK && e == cudaSuccess) e = es;
   for (cudaGraph_t g : graphs) cudaGraphDestroy(g);
   for (size_t v = 0; v < launched && e == cudaSuccess; ++v) {
-    *ran += done[v] * body[v];
-    *launches += 1 + done[v] * per_body[v];
+    *ran += seen[2 * v] * body[v];
+    *launches += 2 + seen[2 * v] * per_body[v];
   }
   std::vector<float> sum(nc, 0.f);
   std::vector<int> cnt(nc, 0);
   for (size_t v = 0; v < launched && e == cudaSuccess && rc == CCO_OK; ++v) {
-    if (done[v] < bodies[v]) continue;
+    if (!whole(v)) continue;
     const size_t c = v < nc ? v : 2 * nc - 1 - v;
     float x = 0.f;
     if (cudaEventElapsedTime(&x, t0[v], t1[v]) == cudaSuccess) {
@@ -454,14 +486,16 @@ int tune_schedule(const LaneTable& C, cudaStream_t st, int64_t max_ticks, int64_
   std::vector<float> ms(nc, 1e30f);
   int best = 0, timed = 0;
   for (size_t c = 0; c < nc; ++c) {
-    if (cnt[c] > 0) ms[c] = sum[c] / cnt[c];
+    if (cnt[c] == 2) ms[c] = sum[c] / 2;   // one visit alone keeps the drift
     if (ms[c] < ms[best]) best = (int)c;
-    timed += cnt[c] > 0;
+    timed += cnt[c] == 2;
   }
   for (size_t c = 0; c < 2 * nc; ++c) {
     if (t0[c]) cudaEventDestroy(t0[c]);
     if (t1[c]) cudaEventDestroy(t1[c]);
+    if (landed[c]) cudaEventDestroy(landed[c]);
   }
+  if (d_seen) cudaFreeAsync(d_seen, st);
   if (rc != CCO_OK) return rc;
   if (e != cudaSuccess) return cuda_fail(e, "schedule tuning");
   if (timed < (int)std::min<size_t>(nc, 2)) return CCO_OK;
@@ -496,7 +530,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
   const int kSlots = inflight + 1;
   int64_t* d_status = nullptr;
   const int W = B + 1;   // a snapshot: the statuses, then the bodies the plan has run
-  int64_t* h_status = pinned_status((size_t)kSlots * W + kMaxTrials);
+  int64_t* h_status = pinned_status((size_t)kSlots * W + 2 * kMaxTrials);
   if (!h_status) return fail(CCO_ERR_OOM, "pinned status buffer");
   CCO_CUDA(pool_alloc(&d_status, sizeof(int64_t) * kSlots * W, st));
   cudaEvent_t ev[kMaxInflight + 1];
@@ -536,8 +570,8 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
   // in an L-BFGS table's first ticks, before its lanes' histories have filled, the
   // HBM-bound update is short, so schedules that overlap it with the FP64-bound
   // evaluation of another branch cannot show their gain.
-  constexpr int64_t kTuneAfterTicks = 128;
   bool defer_tune = false;
+  int64_t tune_from = 0;
 
   // (re)start on table C: schedule, graph
   auto start = [&]() -> int {
@@ -559,13 +593,16 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
       if (force_gt > 0) s.graph_ticks = force_gt;
       if (force_ov >= 0) s.overlap = force_ov;
     } else if (!schedule_cached(C.probs, C.shape.method, &s) && tune) {
-      defer_tune = ticks_run < kTuneAfterTicks;
+      tune_from = tune_after(C.probs, C.shape.method);
+      defer_tune = ticks < tune_from;
       if (!defer_tune) {
         bool tuned = false;
+        const int64_t before = ticks;
         r = tune_schedule(C, st, max_ticks, h_status + (size_t)kSlots * W, &ticks, &ticks_run,
                           &launches, &s, &tuned);
         if (r != CCO_OK) return r;
         if (tuned) schedule_store(C.probs, C.shape.method, s);
+        else set_tune_after(C.probs, C.shape.method, 2 * before);
       }
     }
     chosen = s;
@@ -637,7 +674,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     per_body[slot] = (int64_t)P.body * P.launches_per_tick() + P.loop_gates();
     ++launched;
     if (e == cudaSuccess && launched - checked > inflight) rc = land();
-    if (rc == CCO_OK && e == cudaSuccess && !done && defer_tune && ticks_run >= kTuneAfterTicks) {
+    if (rc == CCO_OK && e == cudaSuccess && !done && defer_tune && ticks >= tune_from) {
       P.retire(st, &graphs);   // the deferred tuning, on the same table
       rc = start();
     }
