@@ -261,13 +261,15 @@ constexpr double kCellMargin = 1e-7;       // relative: |s| rounding 2^-37, G <=
 constexpr double kCellLeast = 1e-7;        // shortest FP32 distance / longest axis
 constexpr int kMaxCells = 8192, kMaxAxisCells = 2048;
 constexpr size_t kCellSmem = 200 * 1024;
-constexpr double kHistReach = 3.0;     // cells per histogram range, at least
+// cells per histogram range, at least: in 1-D a row's cells are one span, so that
+// finer ones cost nothing (one configuration of N=6000, range 0.4 L: 12 / 24 / 48
+// cells 263 / 147 / 96 us; 256 of N=1000, 0.2 L: 140 / 136 / 109)
+constexpr double kHistReach = 3.0, kHistReach1 = 48.0;
 constexpr double kHistFill = 4.0, kNearFill = 2.0;   // particles per cell, at least / about
-// The histogram takes cells as long as their stencil fits the box once; in 1-D, where
-// the range's pairs cost what all pairs do, up to 0.6 of it (call times, range
-// 0.25 / 0.3 / 0.4 L, cells against all pairs: 256 configurations of d=2 N=1000 205 /
-// 265 / 374 against 320 / 339 / 399 us, 64 of d=1 190 / 213 / 200 against 150 / 153 / 166).
-constexpr double kHistMost = 1.0, kHistMost1 = 0.6, kNearMost = 0.5;   // stencil / box
+// Stencil / box. In 1-D the range's pairs then cost what all pairs do (four
+// configurations of N=9000, range 0.4 L: all pairs 537 us, cells 1150).
+constexpr double kHistMost = 1.0, kHistMost1 = 0.6, kNearMost = 0.5;
+constexpr int kHistCells1 = 512;       // 1-D cells, at most
 constexpr int kCellMin = 64, kCellCtas = 148 * 3, kCellSplit = 96;
 constexpr int kCellCrowd = 64;
 
@@ -277,6 +279,7 @@ struct CellGrid {
   float least;             // FP32 r2 below which a pair counts as that far apart: of the
                            // box's own size, so that every allowance scales with it
   float eps;               // and bins around an edge that FP32 cannot tell (0: queue every pair)
+  float part;              // stencil / box
 };
 
 template <int D>
@@ -413,7 +416,7 @@ __device__ __forceinline__ int wrap(int x, int G) { return x < 0 ? x + G : x >= 
 // allows for their rounding, 1e-6 L). On even edges one that lies more than eps
 // bins from every edge is counted at once; the others that pass queue up per
 // warp, 32 at a time are measured in FP64 and binned.
-template <int D>
+template <int D, bool SLICED>
 __global__ void __launch_bounds__(kCellThreads)
     k_pair_hist_cells(const double* __restrict__ s, PairGeom g, CellGrid grid,
                       const double* __restrict__ thresholds, unsigned long long* counts) {
@@ -460,8 +463,20 @@ __global__ void __launch_bounds__(kCellThreads)
     else atomicAdd(counts + b, 1ull);
   };
   const int rows = D == 1 ? 1 : D == 2 ? cg.K[0] + 1 : cg.K[1] + 1 + cg.K[0] * (2 * cg.K[1] + 1);
-  const int i1 = cell_range(cg, end, g.n, blockIdx.x + 1);
-  for (int i0 = cell_range(cg, end, g.n, blockIdx.x) + (threadIdx.x & ~31); i0 < i1; i0 += kCellThreads) {
+  const int ib = cell_range(cg, end, g.n, blockIdx.x), i1 = cell_range(cg, end, g.n, blockIdx.x + 1);
+  // the CTA's particles, a warp each 32. SLICED (a CTA has few of them): several warps
+  // share 32 particles and take a slice of every span each
+  const int groups = SLICED ? (i1 - ib + 31) >> 5 : 0;
+  const int slices = SLICED ? max(1, kCellThreads / 32 / max(groups, 1)) : 1;
+  for (int u = threadIdx.x & ~31;; u += kCellThreads) {   // the warp's first thread
+    int i0 = ib + u, sl = 0;
+    if (SLICED) {
+      if (u >= 32 * groups * slices) break;
+      sl = u / max(32 * groups, 1);
+      i0 -= 32 * groups * sl;
+    } else if (i0 >= i1) {
+      break;
+    }
     const int i = i0 + wl;
     const bool live = i < i1;
     double si[D];
@@ -494,7 +509,11 @@ __global__ void __launch_bounds__(kCellThreads)
       }
       const int len = live ? sp.n1 + sp.n2 : 0, gap = sp.b - sp.a - sp.n1;
       const float x2 = cc[D - 1] < lo ? x[D - 1] + L[D - 1] : x[D - 1] - L[D - 1];   // of the second span
-      const int most = __reduce_max_sync(0xffffffffu, len);
+      int k0 = 0, most = __reduce_max_sync(0xffffffffu, len);
+      if (SLICED) {
+        k0 = most * sl / slices;
+        most = most * (sl + 1) / slices;
+      }
       auto at = [&](int k) { return k < len ? sp.a + k + (k >= sp.n1 ? gap : 0) : 0; };
       auto screen = [&](int k, int j) {
         float r2 = 0.f;
@@ -520,7 +539,7 @@ __global__ void __launch_bounds__(kCellThreads)
       };
       if (direct) {
 #pragma unroll 4
-        for (int k = 0; k < most; ++k) {
+        for (int k = k0; k < most; ++k) {
           const int j = at(k);
           const float r2 = fmaxf(screen(k, j), cg.least);
           const float u = fmaf(r2 * rsqrtf(r2), g.inv_w, shift);   // bin - 1/2
@@ -533,7 +552,7 @@ __global__ void __launch_bounds__(kCellThreads)
         }
       } else {
 #pragma unroll 4
-        for (int k = 0; k < most; ++k) {
+        for (int k = k0; k < most; ++k) {
           const int j = at(k);
           push(k < len && screen(k, j) <= lim, j);
         }
@@ -605,7 +624,7 @@ __global__ void __launch_bounds__(kCellThreads)
 // if the stencil covers too much of the box or the configuration is too large
 // or too small.
 bool cell_grid(const PairGeom& g, int d, double side, double reach, double most, CellGrid* c) {
-  *c = CellGrid{{1, 1, 1}, {0, 0, 0}, 1, 0.f, 0.f, 0.f};
+  *c = CellGrid{{1, 1, 1}, {0, 0, 0}, 1, 0.f, 0.f, 0.f, 1.f};
   double part = 1.0, longest = 0.0;
   if (!(side > 0.0) || g.n > 0xffff) return false;
   for (int a = 0; a < d; ++a) {
@@ -624,7 +643,42 @@ bool cell_grid(const PairGeom& g, int d, double side, double reach, double most,
   const double r = reach + 1e-6 * longest;
   c->lim = (float)(r * r * (1.0 + 1e-6));
   c->least = (float)(kCellLeast * longest * kCellLeast * longest);
+  c->part = (float)part;
   return part <= most;
+}
+
+// CTAs per configuration of a histogram on cells: 96 particles each, fewer (32 at
+// least) while that leaves SMs without one, more when the batch alone fills the GPU
+// (one / 16 configurations of d=2 N=1000, range 0.28 L: 96 particles 24.9 / 31.4 us,
+// 32 particles 20.6 / 37.7).
+int hist_chunks(int n, int batch) {
+  const int few = (n + kCellSplit - 1) / kCellSplit, most = (n + 31) / 32;
+  const int chunks = std::min(most, std::max(few, 148 / batch));
+  return std::max(1, std::min(chunks, (kCellCtas + batch - 1) / batch));
+}
+
+// Whether a histogram takes cells: an estimate of both forms' time in us, fitted to
+// ranges of 5 to 45% of the box, 64 to 9000 particles and 1 to 256 configurations.
+// All pairs: a cost per pair of the tiles and per pair in range. Cells: the CTAs'
+// sorts, then the stencil's pairs at the rate of the CTAs that have cells of their
+// own, at most the GPU's. One configuration of d=2 N=6000, range 0.05 / 0.2 / 0.28 /
+// 0.4 L: all pairs 37 / 42 / 46 / 56 us, cells 23 / 45 / 67 / 173; 256 of N=1000: 200 /
+// 234 / 264 / 332 against 38 / 93 / 149 / 312; 64 of d=3 N=500, 0.05 / 0.2: 32 / 34
+// against 32 / 60.
+bool cells_pay(int n, int batch, int d, const CellGrid& c, double range, double vol, size_t smem) {
+  const double pairs = 0.5 * n * n * batch;
+  const double ball = d == 1 ? 2.0 * range : d == 2 ? M_PI * range * range : 4.0 / 3.0 * M_PI * range * range * range;
+  const double in = std::min(1.0, ball / vol);
+  const double tiles = (n + kPairTile - 1) / kPairTile;
+  const double tested = 0.5 * tiles * (tiles + 1) * kPairTile * kPairTile * batch;
+  const double all = std::max(24.0 + 16.0 * in,
+                              8.0 + tested * (d == 1 ? 1.15e-6 : d == 2 ? 1.3e-6 : 1.6e-6) + pairs * in * 2.1e-6);
+  const int ctas = hist_chunks(n, batch);
+  const double fit = std::max<double>(1.0, std::min<double>(4.0, std::floor(227.0 * 1024 / (smem + 6 * 1024))));
+  const double per_sm = std::min(fit, ctas * (double)batch / 148);
+  const double busy = (double)std::min(ctas, c.cells) * batch;
+  const double rate = std::min(4e5, (d == 1 ? 1300.0 : d == 2 ? 2000.0 : 800.0) * busy);
+  return 0.9 * (10.0 + per_sm * (4.0 + 2e-3 * n) + pairs * c.part / rate) < all;
 }
 
 // The smallest double t >= 0 with sqrt(t) >= e (e >= 0), or > e with `past`.
@@ -652,9 +706,13 @@ void launch_hist(bool diag, dim3 grid, size_t smem, cudaStream_t st, const doubl
 template <int D>
 cudaError_t launch_hist_cells(dim3 grid, size_t smem, cudaStream_t st, const double* s, const PairGeom& g,
                               const CellGrid& c, const double* t, unsigned long long* out) {
-  const cudaError_t e = cudaFuncSetAttribute(k_pair_hist_cells<D>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
-  if (e == cudaSuccess) k_pair_hist_cells<D><<<grid, kCellThreads, smem, st>>>(s, g, c, t, out);
+  // two warps or more for every 32 particles, and SMs with warps to spare (256
+  // configurations of d=2 N=300, three CTAs an SM: 97 us sliced, 91 not)
+  const bool sliced = (size_t)g.n <= (size_t)grid.x * (kCellThreads / 2) && grid.x * grid.y <= 2 * 148;
+  const auto kernel = sliced ? k_pair_hist_cells<D, true> : k_pair_hist_cells<D, false>;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+  if (e == cudaSuccess) kernel<<<grid, kCellThreads, smem, st>>>(s, g, c, t, out);
   return e;
 }
 template <int D>
@@ -731,8 +789,9 @@ int cco_pair_histogram(int device, void* stream, int batch, int n, int d, const 
                           (g.n_bins <= kSmemBins ? sizeof(unsigned int) * g.n_bins : 0);
   double vol = 1.0;
   for (int a = 0; a < d; ++a) vol *= std::fabs(g.B[a * d + a]);
-  const double side = std::max(edges[g.n_bins] / kHistReach * (1.0 + 4.0 * kCellMargin),
-                               std::pow(kHistFill * vol / n, 1.0 / d));
+  double side = std::max(edges[g.n_bins] / (d == 1 ? kHistReach1 : kHistReach) * (1.0 + 4.0 * kCellMargin),
+                         std::pow(kHistFill * vol / n, 1.0 / d));
+  if (d == 1) side = std::max(side, vol / kHistCells1);
   // FP32 bins: what rounding and the shortest distance can move a pair by, and the
   // edges against the even ones
   double dev = 0.0, longest = 0.0;
@@ -743,9 +802,9 @@ int cco_pair_histogram(int device, void* stream, int batch, int n, int d, const 
   const size_t pos_smem = sizeof(double) * n * d + sizeof(float) * ((n + 1) / 2 * 2) * d;
   const size_t cell_smem = pos_smem + bin_smem + sizeof(int) * kMaxCells;
   if (diag && n >= kCellMin && cell_smem <= kCellSmem &&
-      cell_grid(g, d, side, edges[g.n_bins], d == 1 ? kHistMost1 : kHistMost, &cg)) {
-    const int chunks = (n + kCellSplit - 1) / kCellSplit;
-    const dim3 grid(std::max(1, std::min(chunks, (kCellCtas + batch - 1) / batch)), batch);
+      cell_grid(g, d, side, edges[g.n_bins], d == 1 ? kHistMost1 : kHistMost, &cg) &&
+      cells_pay(n, batch, d, cg, edges[g.n_bins], vol, pos_smem + bin_smem + sizeof(int) * cg.cells)) {
+    const dim3 grid(hist_chunks(n, batch), batch);
     const size_t smem = pos_smem + bin_smem + sizeof(int) * cg.cells;
     if (even && g.n_bins <= kSmemBins && eps < 0.1) cg.eps = (float)eps;
     CCO_CUDA(d == 1   ? launch_hist_cells<1>(grid, smem, st, s, g, cg, d_t, c)
