@@ -724,16 +724,24 @@ cudaError_t launch_hist_cells(dim3 grid, size_t smem, cudaStream_t st, const dou
   // configurations of d=2 N=300, three CTAs an SM: 97 us sliced, 91 not)
   const bool sliced = (size_t)g.n <= (size_t)grid.x * (kCellThreads / 2) && grid.x * grid.y <= 2 * 148;
   const auto kernel = sliced ? k_pair_hist_cells<D, true> : k_pair_hist_cells<D, false>;
-  const cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+  static OncePerDevice once;
+  const cudaError_t e = once.run([] {
+    const cudaError_t a = cudaFuncSetAttribute(k_pair_hist_cells<D, true>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+    return a != cudaSuccess ? a
+                            : cudaFuncSetAttribute(k_pair_hist_cells<D, false>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+  });
   if (e == cudaSuccess) kernel<<<grid, kCellThreads, smem, st>>>(s, g, c, t, out);
   return e;
 }
 template <int D>
 cudaError_t launch_nearest_cells(dim3 grid, size_t smem, cudaStream_t st, const double* s,
                                  const PairGeom& g, const CellGrid& c, double* out) {
-  const cudaError_t e = cudaFuncSetAttribute(k_nearest_cells<D>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+  static OncePerDevice once;   // on every call it is 0.7 of 18 us
+  const cudaError_t e = once.run([] {
+    return cudaFuncSetAttribute(k_nearest_cells<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
+  });
   if (e == cudaSuccess) k_nearest_cells<D><<<grid, kCellThreads, smem, st>>>(s, g, c, out);
   return e;
 }
