@@ -29,11 +29,13 @@ int main() {
       check("hessian", d, cco::hessian_launch(&p, nullptr, 1, nullptr, nullptr, nullptr));
     }
     cco::DescentArgs a{};
-    a.B = 1;
-    for (int d = 1; d <= 3; ++d)
-      for (int bit : {d - 1, d + 2})
-        check("descent", d,
-              cco::persist_descent(a, cco::EvalPlan{}, cco::kPersistMaxSmem, 1 << bit, 1, nullptr, nullptr));
+    for (int lanes : {1, 1000}) {
+      a.B = lanes;
+      for (int d = 1; d <= 3; ++d)
+        for (int bit : {d - 1, d + 2})
+          check("descent", d,
+                cco::persist_descent(a, cco::EvalPlan{}, cco::kPersistMaxSmem, 1 << bit, 1, nullptr, nullptr));
+    }
   }
   std::printf("%d bad\n", bad);
   return bad != 0;

@@ -117,7 +117,10 @@ __global__ void __launch_bounds__(kPersistThreads) k_persist_descent(DescentArgs
 // table builds, two particle tiles one after the other, trips through global
 // memory and ~25 barriers; this form takes 3.6 us, a chain of latencies (sincospi,
 // shuffles, barriers) that neither the 1300 pairs nor memory bound.
+// (With more lanes than SMs fewer threads take a lane, see launch_compact; sums are
+// then formed as the 512 form them.)
 constexpr int kCompactThreads = 512;
+constexpr int kPersistSms = 148;   // SMs of a B200
 
 // Every thread's copy of the descent state of a lane.
 struct CompactState {
@@ -126,15 +129,14 @@ struct CompactState {
   bool nonzero;
 };
 
-template <int D>
-__global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs a, EvalPlan plan,
-                                                                     int64_t max_ticks,
-                                                                     int* overrun) {
+template <int D, int T>
+__global__ void __launch_bounds__(T) k_persist_compact(DescentArgs a, EvalPlan plan, int64_t max_ticks,
+                                                       int* overrun) {
   extern __shared__ double2 smem[];
   __shared__ ProbDev P;
   __shared__ double red[kCompactThreads / 32], f_s;
   const int lane = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, wl = tid & 31;
-  constexpr int NWARP = kCompactThreads / 32;
+  constexpr int NWARP = T / 32, VWARP = kCompactThreads / 32;
   const EvalLane ln = plan.lanes[lane];
   if (tid == 0) P = plan.probs[ln.prob];
   __syncthreads();
@@ -160,7 +162,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
   const bool keep = P.compact == 2;
   const int pst = N | 1;
   double2* ph = reinterpret_cast<double2*>(ek + ((M + 4 * nd + 1) & ~1));
-  for (int k = tid; k < M; k += kCompactThreads) {
+  for (int k = tid; k < M; k += T) {
     const double4 r = P.krow[k];
     const double nv[3] = {r.x, r.y, r.z};
     int o[3] = {0, 0, 0};
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
     row[k] = r;
     ro[k] = make_int4(o[0], o[1], o[2], 0);
   }
-  for (int e = tid; e < nd; e += kCompactThreads) {
+  for (int e = tid; e < nd; e += T) {
     s[e] = v.s[e];
     g[e] = v.g[e];
     ps[e] = v.ps[e];
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
       break;
     }
     // tables
-    for (int w = tid; w < nunit * N; w += kCompactThreads) {
+    for (int w = tid; w < nunit * N; w += T) {
       const int j = w % N;
       int u = w / N, c = 0;
 #pragma unroll
@@ -261,40 +263,43 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
         }
     }
     __syncthreads();
-    // gradient, |g|^2, energy
-    double ss = 0.0;
+    // gradient, |g|^2, energy: as kCompactThreads threads do it, whatever T (the
+    // warps take the 16 warps' parts one after the other)
     int nz = 0;
     const int per = kCompactThreads / tpp, q = tid & (tpp - 1);
-    for (int j0 = 0; j0 < N; j0 += per) {
-      const int j = j0 + tid / tpp;
-      double G[D];
+    for (int vw = warp; vw < VWARP; vw += NWARP) {
+      double ss = 0.0;
+      for (int j0 = 0; j0 < N; j0 += per) {
+        const int j = j0 + (32 * vw + wl) / tpp;
+        double G[D];
 #pragma unroll
-      for (int c = 0; c < D; ++c) G[c] = 0.0;
-      if (j < N)
-        for (int k = q; k < M; k += tpp) {
-          const double4 r = row[k];
-          const double2 z = keep ? ph[(size_t)k * pst + j] : phase(ro[k], j), w = rw[k];
-          const double h = w.y * z.x - w.x * z.y;
-          const double nv[3] = {r.x, r.y, r.z};
+        for (int c = 0; c < D; ++c) G[c] = 0.0;
+        if (j < N)
+          for (int k = q; k < M; k += tpp) {
+            const double4 r = row[k];
+            const double2 z = keep ? ph[(size_t)k * pst + j] : phase(ro[k], j), w = rw[k];
+            const double h = w.y * z.x - w.x * z.y;
+            const double nv[3] = {r.x, r.y, r.z};
 #pragma unroll
-          for (int c = 0; c < D; ++c) G[c] += nv[c] * h;
-        }
-      for (int o = tpp >> 1; o > 0; o >>= 1)
+            for (int c = 0; c < D; ++c) G[c] += nv[c] * h;
+          }
+        for (int o = tpp >> 1; o > 0; o >>= 1)
 #pragma unroll
-        for (int c = 0; c < D; ++c) G[c] += __shfl_xor_sync(0xffffffffu, G[c], o);
-      if (j < N && q == 0) {
+          for (int c = 0; c < D; ++c) G[c] += __shfl_xor_sync(0xffffffffu, G[c], o);
+        if (j < N && q == 0) {
 #pragma unroll
-        for (int c = 0; c < D; ++c) {
-          const double x = P.gpref * G[c];
-          pg[j * D + c] = x;
-          ss += x * x;
-          nz |= x != 0.0;
+          for (int c = 0; c < D; ++c) {
+            const double x = P.gpref * G[c];
+            pg[j * D + c] = x;
+            ss += x * x;
+            nz |= x != 0.0;
+          }
         }
       }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (wl == 0) red[warp] = ss;
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (wl == 0) red[vw] = ss;
+    }
     if (warp == NWARP - 1) {
       double e = 0.0;
       for (int k = wl; k < M; k += 32) e += ek[k];
@@ -304,9 +309,9 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
     }
     nz = __syncthreads_or(nz);
     // the descent rule (descent.py:121-175), every thread on the same numbers
-    ss = 0.0;
+    double ss = 0.0;
 #pragma unroll
-    for (int w = 0; w < NWARP; ++w) ss += red[w];
+    for (int w = 0; w < VWARP; ++w) ss += red[w];
     const double f2 = f_s;
     bool take = true;
     if (!init) {
@@ -329,7 +334,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
     }
     status = descent_status(S.f, S.nonzero, S.step, S.it, a);
     const bool rec = a.traj_count && S.it % a.rec_every == 0 && S.rec < a.rec_cap;
-    for (int e = tid; e < nd; e += kCompactThreads) {
+    for (int e = tid; e < nd; e += T) {
       if (take) {
         s[e] = S.it == 0 ? s[e] : ps[e];
         g[e] = pg[e];
@@ -352,7 +357,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_persist_compact(DescentArgs
     __syncthreads();
   }
   __syncthreads();
-  for (int e = tid; e < nd; e += kCompactThreads) {
+  for (int e = tid; e < nd; e += T) {
     v.s[e] = s[e];
     v.g[e] = g[e];
     v.ps[e] = ps[e];
@@ -396,22 +401,63 @@ size_t persist_smem(const cco_problem* p) {
   return std::max(p->smem1, eval_smem2(p->host, 1));
 }
 
+namespace {
+
+template <int D, int T>
+void launch_compact(const DescentArgs& a, const EvalPlan& plan, size_t smem, int64_t max_ticks,
+                    int* d_overrun, cudaStream_t st) {
+  k_persist_compact<D, T><<<a.B, T, smem, st>>>(a, plan, max_ticks, d_overrun);
+}
+
+// Rounds of CTAs that a.B lanes take with T threads each, times what an iteration
+// costs next to 512 threads.
+template <int D, int T>
+double compact_cost(const DescentArgs& a, size_t smem) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist_compact<D, T>, T, smem) !=
+          cudaSuccess || per_sm < 1)
+    return 1e300;
+  const int rounds = (a.B + kPersistSms * per_sm - 1) / (kPersistSms * per_sm);
+  return rounds * (T == 512 ? 1.0 : T == 256 ? 1.25 : 1.9);
+}
+
+// A lane gives the same bits with any number of threads. 512 are the fastest for one
+// lane per SM (relaxations of 100 evaluations with 512 / 256 / 128 threads, 5 lanes: d=3
+// N=100 278 / 351 / 462 us, d=1 N=60 301 / 326 / 467); more lanes run in fewer rounds
+// with smaller CTAs where shared memory lets several share an SM (1500 lanes: 2255 /
+// 1924 / 1552 and 2006 / 1171 / 1268 us; the general form 3342 and 1456).
+template <int D>
+void launch_compact(const DescentArgs& a, const EvalPlan& plan, size_t smem, int64_t max_ticks,
+                    int* d_overrun, cudaStream_t st) {
+  const double c512 = a.B <= kPersistSms ? 0.0 : compact_cost<D, 512>(a, smem);
+  const double c256 = c512 == 0.0 ? 1.0 : compact_cost<D, 256>(a, smem);
+  const double c128 = c512 == 0.0 ? 1.0 : compact_cost<D, 128>(a, smem);
+  if (c512 <= c256 && c512 <= c128) launch_compact<D, 512>(a, plan, smem, max_ticks, d_overrun, st);
+  else if (c256 <= c128) launch_compact<D, 256>(a, plan, smem, max_ticks, d_overrun, st);
+  else launch_compact<D, 128>(a, plan, smem, max_ticks, d_overrun, st);
+}
+
+}  // namespace
+
 cudaError_t persist_descent(const DescentArgs& a, const EvalPlan& plan, size_t smem, int dims,
                             int64_t max_ticks, int* d_overrun, cudaStream_t st) {
   static OncePerDevice once;
   const cudaError_t configured = once.run([] {
     cudaError_t e = cudaSuccess;
     for (const void* k : {(const void*)k_persist_descent<1>, (const void*)k_persist_descent<2>,
-                          (const void*)k_persist_descent<3>, (const void*)k_persist_compact<1>,
-                          (const void*)k_persist_compact<2>, (const void*)k_persist_compact<3>})
+                          (const void*)k_persist_descent<3>, (const void*)k_persist_compact<1, 512>,
+                          (const void*)k_persist_compact<2, 512>, (const void*)k_persist_compact<3, 512>,
+                          (const void*)k_persist_compact<1, 256>, (const void*)k_persist_compact<2, 256>,
+                          (const void*)k_persist_compact<3, 256>, (const void*)k_persist_compact<1, 128>,
+                          (const void*)k_persist_compact<2, 128>, (const void*)k_persist_compact<3, 128>})
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistMaxSmem);
     return e;
   });
   if (configured != cudaSuccess) return configured;
-  if (dims & 8) k_persist_compact<1><<<a.B, kCompactThreads, smem, st>>>(a, plan, max_ticks, d_overrun);
-  if (dims & 16) k_persist_compact<2><<<a.B, kCompactThreads, smem, st>>>(a, plan, max_ticks, d_overrun);
-  if (dims & 32) k_persist_compact<3><<<a.B, kCompactThreads, smem, st>>>(a, plan, max_ticks, d_overrun);
+  if (dims & 8) launch_compact<1>(a, plan, smem, max_ticks, d_overrun, st);
+  if (dims & 16) launch_compact<2>(a, plan, smem, max_ticks, d_overrun, st);
+  if (dims & 32) launch_compact<3>(a, plan, smem, max_ticks, d_overrun, st);
   if (dims & 1) k_persist_descent<1><<<a.B, kPersistThreads, smem, st>>>(a, plan, max_ticks, d_overrun);
   if (dims & 2) k_persist_descent<2><<<a.B, kPersistThreads, smem, st>>>(a, plan, max_ticks, d_overrun);
   if (dims & 4) k_persist_descent<3><<<a.B, kPersistThreads, smem, st>>>(a, plan, max_ticks, d_overrun);
