@@ -238,10 +238,16 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // the tick graphs of a lone lane (d=2 N=1000 to the ground state 41.7 -> 39.0 ms);
 // graphs of more lanes lose more to the edges than they gain (64 MD lanes, 40
 // steps: 5.17 -> 5.38 ms; 25 of d=3 N=1492: 6.1 -> 6.4 ms).
+//
+// A kernel of more than kChainCtas CTAs (one per SM) does not let them in early either:
+// they would pile up on the SMs that it leaves first, and a successor of few CTAs per SM
+// run as long as its fullest SM (gradient of 256 lanes of d=1 N=36, 2003 rows, after
+// their reduction 383 -> 320 us; one lane of d=1 N=7777 after its roots 50.9 -> 47.1).
+constexpr unsigned kChainCtas = 148;
 template <bool EARLY = true>
 __device__ __forceinline__ void chain_wait() {
   cudaGridDependencySynchronize();
-  if (EARLY) cudaTriggerProgrammaticLaunchCompletion();
+  if (EARLY && gridDim.x * gridDim.y <= kChainCtas) cudaTriggerProgrammaticLaunchCompletion();
 }
 
 template <class... P, class... A>
