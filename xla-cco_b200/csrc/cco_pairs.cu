@@ -27,10 +27,11 @@
 // 64-bit result once, so the counts are exact and independent of the launch
 // order. On 256 configurations of d=2 N=1000 (200 bins) histogram and nearest
 // neighbours went from 1423 and 1712 us to 235 and 254 us; bound: instruction
-// issue (FP64: 6 operations per axis and pair). The column loops are unrolled for
-// one image only: with 27 images four times over, nearest neighbours of 8 sheared
-// configurations of d=3 N=900 take 584 us instead of 505. Screening pairs by FP32 distances
-// of fixed-point differences first ran 272 and 242 us (conversions) and was not kept.
+// issue (FP64: 6 operations per axis and pair). The column loops are not unrolled
+// over 27 images: four times over, nearest neighbours of 8 sheared configurations of
+// d=3 N=900 take 584 us instead of 505 (9 images: 164 unrolled, 208 not). Screening
+// pairs by FP32 distances of fixed-point differences first ran 272 and 242 us
+// (conversions) and was not kept.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(kPairTile) k_pair_hist(const double* __restric
     for (int c = 0; c < D; ++c) si[c] = i < g.n ? sc[(size_t)i * D + c] : 0.0;
     // the row's first column: past the diagonal, past the end for a dead row
     const int first = i >= g.n ? nj : tj == ti ? (int)threadIdx.x + 1 : 0;
-#pragma unroll (DIAG ? 4 : 1)
+#pragma unroll (DIAG || D < 3 ? 4 : 1)
     for (int jj = 0; jj < nj; ++jj) {
       const double r2 = DIAG ? diag_r2<D>(si, col + jj * D, Bd)
                              : min_image_r2<D>(si, col + jj * D, g, false);
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(kPairTile) k_nearest(const double* __restrict_
     for (int u = threadIdx.x; u < nj * D; u += blockDim.x) col[u] = sc[(size_t)j0 * D + u];
     __syncthreads();
     const int self = i - j0;
-#pragma unroll (DIAG ? 4 : 1)
+#pragma unroll (DIAG || D < 3 ? 4 : 1)
     for (int jj = 0; jj < nj; ++jj) {
       const double r2 = DIAG ? diag_r2<D>(si, col + jj * D, Bd)
                              : min_image_r2<D>(si, col + jj * D, g, false);
