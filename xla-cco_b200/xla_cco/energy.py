@@ -324,10 +324,10 @@ def _density_energy(nv: np.ndarray) -> StealthyEnergy:
     # found by a sample of the entries, then compared element by element: hashing
     # all bytes of a 97 000-row set took 1.6 ms
     flat = nv.reshape(-1)
-    key = (nv.shape, flat[:: flat.size // 64 + 1].tobytes())
+    key = (nv.shape, flat[:: flat.size // 16 + 1].tobytes())
     with _DENSITY_LOCK:
         for en in _DENSITY_CACHE.get(key, ()):
-            if np.array_equal(en.n_vectors, nv):
+            if (en.n_vectors == nv).all():
                 _DENSITY_CACHE.move_to_end(key)
                 return en
     en = StealthyEnergy(nv.copy(), np.ones(nv.shape[0]), np.float64(1.0))
