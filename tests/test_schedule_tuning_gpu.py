@@ -17,7 +17,7 @@ from xla_cco.minimize.descent import DescentSettings
 
 pytestmark = pytest.mark.gpu
 
-DEFAULT = (2, 16)   # branches and ticks of a launch from 64 lanes on
+DEFAULT = (1, 16)   # branches and ticks of a launch of so small a tick
 BODY = 16           # a run ends at most one loop body late
 
 
@@ -96,3 +96,33 @@ def test_md_segments_count_the_ticks_that_ran(monkeypatch):
     assert seen[0] >= 1 and seen[0] < 1 + BODY
     assert 41 <= seen[1] < 41 + BODY
 
+
+def test_md_of_many_steps_is_tuned_before_its_first_step(monkeypatch):
+    """A segment that lasts as long as the trials counts its own ticks and no others,
+    in the call that tunes and in the next."""
+    n, d, b = 60, 2, 64
+    box, en, _ = _system(n, d, 0.3, b)
+    seen = []
+    lib = _native.load()
+
+    class Recorder:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def cco_md_segment(self, *args):
+            code = lib.cco_md_segment(*args)
+            seen.append(args[-1]._obj.value)
+            return code
+
+    rng = np.random.default_rng(5)
+    k = k_outer_from_ka(ka_from_chi(0.3, 0.05, d), 0.05, d)
+    waves = make_waves(box.basis, k, 1.1 * k)
+    keys = np.stack([make_key(i) for i in range(b)])
+    st = MDSettings(dt=0.01, scheme="baoab", gamma=1.0, chunk_steps=400, drift_tol=np.inf)
+    r0 = rng.uniform(size=(b, n, d)) * box.basis[0, 0]
+    state = init_state(en, waves, box.basis, r0, rng.normal(size=(b, n, d)), np.full(b, 0.5), keys, st)
+    monkeypatch.setattr(_native, "load", lambda: Recorder())
+    one = simulate(en, waves, box.basis, st, state, 400).state
+    two = simulate(en, waves, box.basis, st, state, 400).state
+    assert all(401 <= x < 401 + 2 * BODY for x in seen), seen
+    assert np.array_equal(one.r, two.r) and np.array_equal(one.v, two.v)

@@ -298,6 +298,11 @@ constexpr int kMaxBranches = 8;
 // 16 lanes 2.68 / 2.76 / 2.91 ms in one branch, 3.13 / 3.21 / 3.39 in two; 256 lanes
 // 8.30 and 8.13).
 inline int default_branches(size_t lanes) { return lanes >= 64 ? 2 : 1; }
+// Other minimizers than L-BFGS have no long update to overlap: two branches only for
+// ticks of much work (200 MD steps in one / two branches: 64 lanes of d=2 N=60 6.5 /
+// 7.1 ms, 200 of d=3 N=300 15.5 / 15.1, 400 of d=2 N=500 22.4 / 20.7; 40 steps 2.6 / 2.9,
+// 4.3 / 4.6, 5.7 / 5.6).
+int default_branches(size_t lanes, Method method, const std::vector<const cco_problem*>& probs);
 constexpr int kInflight = 3;    // graphs in flight before the host checks completion
 constexpr int kMaxInflight = 16;   // CCO_INFLIGHT bound (and the round bounds' slack)
 
@@ -323,6 +328,7 @@ struct LaneTable {
   LbArgs lb{};
   FlArgs fl{};
   MdArgs md{};
+  int64_t steps = 0;   // ticks the lanes run, where that is known (MD)
   int upload_refs(cudaStream_t st);
   void release(cudaStream_t st);
 };

@@ -151,6 +151,12 @@ int body_ticks(double us, int graph_ticks) {
 
 }  // namespace
 
+int default_branches(size_t lanes, Method method, const std::vector<const cco_problem*>& probs) {
+  double flops = 0.0;
+  for (const cco_problem* p : probs) flops += eval_flops(p);
+  return method == Method::Lbfgs || flops >= 1.2e9 ? default_branches(lanes) : 1;
+}
+
 int TickPlan::build(const LaneTable& T, const Schedule& sch, cudaStream_t st) {
   release(st);
   this->sch = sch;
@@ -569,7 +575,8 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
   // the trials, which tell nothing then and cost a graph each (about 1 ms); and
   // in an L-BFGS table's first ticks, before its lanes' histories have filled, the
   // HBM-bound update is short, so schedules that overlap it with the FP64-bound
-  // evaluation of another branch cannot show their gain.
+  // evaluation of another branch cannot show their gain. A run known to last as long
+  // as the trials is tuned at once.
   bool defer_tune = false;
   int64_t tune_from = 0;
 
@@ -586,7 +593,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
     C.md.lanes = C.d_refs;
     C.md.B = (int)C.refs.size();
     Schedule s;
-    s.branches = default_branches(C.refs.size());
+    s.branches = default_branches(C.refs.size(), C.shape.method, C.probs);
     defer_tune = false;
     if (force_br > 0 || force_gt > 0 || force_ov >= 0) {
       if (force_br > 0) s.branches = force_br;
@@ -594,7 +601,9 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
       if (force_ov >= 0) s.overlap = force_ov;
     } else if (!schedule_cached(C.probs, C.shape.method, &s) && tune) {
       tune_from = tune_after(C.probs, C.shape.method);
-      defer_tune = ticks < tune_from;
+      const int64_t trials = 2 * 16 * (int64_t)candidates((int)C.refs.size()).size();
+      const bool lasts = tune_from == kTuneAfterTicks && T.steps - ticks >= trials;
+      defer_tune = ticks < tune_from && !lasts;
       if (!defer_tune) {
         bool tuned = false;
         const int64_t before = ticks;
@@ -602,7 +611,7 @@ int run_lane_table(LaneTable& T, cudaStream_t st, int64_t max_ticks, RunStats* s
                           &launches, &s, &tuned);
         if (r != CCO_OK) return r;
         if (tuned) schedule_store(C.probs, C.shape.method, s);
-        else set_tune_after(C.probs, C.shape.method, 2 * before);
+        else set_tune_after(C.probs, C.shape.method, 2 * std::max(before, kTuneAfterTicks));
       }
     }
     chosen = s;
@@ -1223,6 +1232,7 @@ extern "C" int cco_md_run(cco_problem* const* problems, void* stream, int batch,
   a.andersen_p = cfg->andersen_p;
   a.drift_tol = cfg->drift_tol;
   a.n_steps = cfg->n_steps;
+  T.steps = cfg->n_steps;
   a.scheme = cfg->scheme;
   a.andersen = cfg->scheme == MD_VERLET ? cfg->andersen : ANDERSEN_OFF;
   double* records = nullptr;
@@ -1330,6 +1340,7 @@ extern "C" int cco_md_segment(cco_problem* p, void* stream, int batch, const dou
   a.andersen_p = cfg->andersen_p;
   a.drift_tol = 0.0;
   a.n_steps = cfg->n_steps;
+  T.steps = cfg->n_steps;
   a.scheme = cfg->scheme;
   a.andersen = cfg->scheme == MD_VERLET ? cfg->andersen : ANDERSEN_OFF;
   a.w = w;
