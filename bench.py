@@ -37,7 +37,9 @@ METRIC = "relaxations/s to Phi<1e-20 (batched L-BFGS, plain FP64)"
 UNIT = "relaxations/s"
 N_PART, DIM, CHI, PHI_PACK, BATCH, SEED = 1000, 2, 0.40, 0.05, 256, 0
 TOL = 1e-20
-F_PAIR = {1: 7, 2: 21, 3: 35}  # algorithmic FP64 flops per (k, particle) pair and evaluation
+# algorithmic FP64 flops per (k, particle) pair and evaluation: 2 FMAs for the density,
+# 4 for the gradient (the grid form's products without its padded cells and tables)
+F_PAIR = {1: 12, 2: 12, 3: 12}
 
 
 def workload():
@@ -873,8 +875,9 @@ def run_md(args) -> None:
     w = int(waves.n_vectors.shape[0])
     cpu_s = None if args.no_cpu_baseline else _md_host_sample(ks, basis, waves, r0[0], v0[0], 20)
     # device-side algorithmic flops per lane-step: force (F_PAIR N M) + fresh waves every 10 steps
+    # (the product of two table entries, added up: 4 FMAs)
     flops = lanes * n_steps * (F_PAIR[DIM] * N_PART * ks.n.shape[0] +
-                               0.1 * 40.0 * N_PART * (w - waves.n_constrained))  # fmt: skip
+                               0.1 * 8.0 * N_PART * (w - waves.n_constrained))  # fmt: skip
     peak = fp64_peak_tflops()
     line = {
         "metric": "MD lane-steps/s (simulate: BAOAB + tracked-wave observables)", "value": value,
@@ -890,7 +893,7 @@ def run_md(args) -> None:
         "roofline": {"kernel": "whole MD segment (evaluations + step + observables)", "bound": "fp64",
                      "achieved": flops / (ms / 1e3) / 1e12, "peak": peak, "unit": "TFLOP/s",
                      "frac": flops / (ms / 1e3) / 1e12 / peak if peak else None,
-                     "algorithmic": "F_PAIR N M per force + 40 flops per (fresh wave, particle) every 10 steps"},
+                     "algorithmic": "F_PAIR N M per force + 8 flops per (fresh wave, particle) every 10 steps"},
         "e2e": {"value": lanes * n_steps / e2e_s, "unit": "lane-steps/s",
                 "h2d_bytes_per_step": buf_bytes, "d2h_bytes_per_step": buf_bytes,
                 "note": "simulate() with a NumPy state: one upload and one download of the state"},

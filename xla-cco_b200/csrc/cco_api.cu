@@ -284,11 +284,8 @@ std::vector<GridRun> split_runs_1d(const std::vector<GridRun>& runs, int C) {
   return out;
 }
 
-// Whether and how FP64 lanes of a problem run the grid form. The form costs 12
-// FMAs per grid cell and particle (4 density, 8 gradient) plus the tables,
-// where the recurrences need 14 or more instructions per k-set row: it is taken
-// when the slots (cells with their padding) are at most twice the rows.
 void grid_sizes(ProbDev* P, const GridPlan& gp);
+
 // A line grid: `rows` holds the k-set in run order (M x d). Rows are multiples
 // i v of primitive vectors v; a line's multiples are cut into strips of 8 rows
 // i = q step + c, |c| < 4 nq, step = 8 nq - 1, with the nq (at most 4) that
@@ -401,6 +398,10 @@ void grid_sizes(ProbDev* P, const GridPlan& gp) {
     P->grid = P->groots = 0;
 }
 
+// Whether and how FP64 lanes of a problem run the grid form. The form costs 12
+// FMAs per grid cell and particle (4 density, 8 gradient) plus the tables,
+// where the recurrences need 14 or more instructions per k-set row: it is taken
+// when the slots (cells with their padding) are at most twice the rows.
 void plan_grid(const std::vector<GridRun>& runs, ProbDev* P, GridPlan* gp) {
   // every strip of 8 runs takes a quad (32 slots) or more: sets of short runs are
   // refused before a layout is made (90 000 runs of about one row: 11 layouts took 290 ms)

@@ -501,7 +501,6 @@ __global__ void __launch_bounds__(kUpdThreads) k_md_waves(MdArgs a) {
   }
 }
 
-// Segment runs: each lane's record from the batched state.
 // The same sums when the components of the waves are small: z_a^0 .. z_a^R of a
 // tile of particles in shared memory (anchors every 8 powers from the exactly
 // reduced argument, products between), then a thread per two waves over the
@@ -626,6 +625,7 @@ __global__ void __cluster_dims__(kWaveRanks, 1, 1) __launch_bounds__(kWaveThread
   cl.sync();   // no CTA leaves while its sums are read
 }
 
+// Segment runs: each lane's record from the batched state.
 __global__ void k_md_seg_init(MdArgs a, const double* __restrict__ mats) {
   const LaneRef R = a.lanes[blockIdx.x];
   const MdView w = md_view(R.rec, R.ld, a.w);

@@ -221,7 +221,6 @@ cudaError_t lbfgs_finalize(const LbArgs& a, double* s_out, double* e_out, double
 
 // Count lanes whose status is RUNNING.
 cudaError_t count_running(const LaneRef* lanes, int B, int* out, cudaStream_t st);
-// Copy every lane's status into out[B].
 // The statuses of the lanes, then (if given) *extra, into out.
 cudaError_t gather_status(const LaneRef* lanes, int B, int64_t* out, cudaStream_t st,
                           const int64_t* extra = nullptr);

@@ -267,7 +267,9 @@ __global__ void __launch_bounds__(T) k_persist_compact(DescentArgs a, EvalPlan p
     // warps take the 16 warps' parts one after the other)
     int nz = 0;
     const int per = kCompactThreads / tpp, q = tid & (tpp - 1);
-    for (int vw = warp; vw < VWARP; vw += NWARP) {
+#pragma unroll 1
+    for (int i = 0; i < VWARP / NWARP; ++i) {
+      const int vw = warp + i * NWARP;
       double ss = 0.0;
       for (int j0 = 0; j0 < N; j0 += per) {
         const int j = j0 + (32 * vw + wl) / tpp;
