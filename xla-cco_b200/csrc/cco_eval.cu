@@ -58,7 +58,7 @@ __device__ __forceinline__ bool grid_lane_runs(const EvalPlan& plan, const EvalL
 
 // Grid form: the phases the tables start from.
 __global__ void __launch_bounds__(kRootChunk) k_grid_roots(EvalPlan plan) {
-  chain_wait();
+  chain_wait<CHAIN_FEW>();
   const EvalLane& ln = plan.lanes[blockIdx.y];
   if (!grid_lane_runs(plan, ln)) return;
   const ProbDev& P = plan.probs[ln.prob];
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid1(EvalPlan plan
   constexpr int NT = CLS == 2 ? 3 : LINES ? 1 : 2;
   const EvalItem* items = plan.itemsG + plan.q_offG[D - 1][CLS];
   const int n = plan.q_offG[D - 1][CLS + 1] - plan.q_offG[D - 1][CLS];
-  chain_wait<false>();
+  chain_wait<CHAIN_LATE>();
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     const EvalItem it = items[i];
     const EvalLane ln = plan.lanes[it.lane];
@@ -141,7 +141,7 @@ __device__ __forceinline__ double* grid_energies(const ProbDev& P, const EvalLan
 // this block reads).
 __global__ void __launch_bounds__(kReduceChunk) k_reduce(EvalPlan plan) {
   __shared__ double red[32];
-  chain_wait();
+  chain_wait<CHAIN_FEW>();
   const EvalLane ln = plan.lanes[blockIdx.y];
   if (!lane_active(ln.status)) return;
   const ProbDev& P = plan.probs[ln.prob];
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kGridThreads, kGridCtas) k_grid2(EvalPlan plan
   __shared__ GridStage stage;
   const EvalItem* items = plan.itemsH + plan.h_off[D - 1][ROOTS];
   const int n = plan.h_off[D - 1][ROOTS + 1] - plan.h_off[D - 1][ROOTS];
-  chain_wait<false>();
+  chain_wait<CHAIN_LATE>();
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     const EvalItem it = items[i];
     const EvalLane ln = plan.lanes[it.lane];

@@ -230,24 +230,27 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // set up, and its CTAs come in, while the predecessor's last ones still run; every
 // CTA of it calls chain_wait first (a grid whose CTAs left without it would let
 // its own successor run beside the predecessor), which returns when the
-// predecessor has finished and its writes are visible. EARLY: the successor's
+// predecessor has finished and its writes are visible. CHAIN_EARLY: the successor's
 // CTAs may come in from then on; the grid kernels, which fill the GPU, leave
-// that to their end (let in early they cost the two passes 2%). Used where a call
+// that to their end (CHAIN_LATE; let in early they cost the two passes 2%). Used where a call
 // is one evaluation (256 lanes of d=2 N=1000 166 -> 160 us, one of N=20000 288 -> 281,
 // one of d=1 N=7777 with its synchronisation 82 -> 77, a Hessian 129 -> 123) and by
 // the tick graphs of a lone lane (d=2 N=1000 to the ground state 41.7 -> 39.0 ms);
 // graphs of more lanes lose more to the edges than they gain (64 MD lanes, 40
 // steps: 5.17 -> 5.38 ms; 25 of d=3 N=1492: 6.1 -> 6.4 ms).
 //
-// A kernel of more than kChainCtas CTAs (one per SM) does not let them in early either:
-// they would pile up on the SMs that it leaves first, and a successor of few CTAs per SM
-// run as long as its fullest SM (gradient of 256 lanes of d=1 N=36, 2003 rows, after
-// their reduction 383 -> 320 us; one lane of d=1 N=7777 after its roots 50.9 -> 47.1).
+// The reduction and the phase roots do so only up to kChainCtas CTAs (one per SM): of
+// more, the successor's CTAs would pile up on the SMs that are left first, and a pass of
+// few CTAs per SM runs as long as its fullest SM (gradient of 256 lanes of d=1 N=36, 2003
+// rows, after their reduction 383 -> 320 us; one lane of d=1 N=7777 after its roots 50.9
+// -> 47.1). The minimizers' kernels always do: looking at their grids cost a tick 1.5 us.
 constexpr unsigned kChainCtas = 148;
-template <bool EARLY = true>
+enum ChainLet { CHAIN_LATE, CHAIN_EARLY, CHAIN_FEW };
+template <ChainLet LET = CHAIN_EARLY>
 __device__ __forceinline__ void chain_wait() {
   cudaGridDependencySynchronize();
-  if (EARLY && gridDim.x * gridDim.y <= kChainCtas) cudaTriggerProgrammaticLaunchCompletion();
+  if (LET == CHAIN_EARLY || (LET == CHAIN_FEW && gridDim.x * gridDim.y <= kChainCtas))
+    cudaTriggerProgrammaticLaunchCompletion();
 }
 
 template <class... P, class... A>
