@@ -478,11 +478,13 @@ int cco_md_segment(cco_problem* p, void* stream, int batch, const double* basis,
 /*
  * Tick schedules (graph branches, ticks per graph) are tuned online on the
  * first relaxation of each shape class (minimizer, lane count and total
- * N M bucketed by powers of two, largest d) and cached for the process;
+ * N M bucketed by powers of two, largest d) that runs on past 128 ticks, or
+ * on an MD segment that lasts as long as the trials, and cached for the process;
  * results never depend on the schedule. This forgets every cached schedule.
  * The environment variables CCO_BRANCHES, CCO_GRAPH_TICKS and CCO_OVERLAP
  * (0 or 1) force a schedule, CCO_AUTOTUNE=0 keeps the default (one branch, two
- * from 64 lanes, 16 ticks, no overlap). CCO_INFLIGHT (1..16, default 3) sets how
+ * from 64 lanes, where other minimizers than L-BFGS take two only for ticks of
+ * much work; 16 ticks, no overlap). CCO_INFLIGHT (1..16, default 3) sets how
  * many graphs the driver keeps queued ahead of its completion checks.
  */
 int cco_schedule_reset(void);

@@ -338,7 +338,7 @@ struct LaneTable {
 // their whole descent in one persistent launch (cco_persist.cu) instead of
 // graph ticks. The choice depends on the problem alone, so a lane gives the
 // same bits alone and in any batch.
-constexpr double kPersistMaxFlops = 2.5e5;          // N M F_pair(d) per evaluation
+constexpr double kPersistMaxFlops = 2.5e5;          // N M times 7 / 21 / 35 (d = 1, 2, 3) per evaluation
 constexpr size_t kPersistMaxSmem = 200 * 1024;      // dynamic shared memory of the launch
 bool persist_eligible(const cco_problem* p);
 size_t persist_smem(const cco_problem* p);
